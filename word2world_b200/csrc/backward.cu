@@ -21,10 +21,11 @@
 #include "kernels.h"
 #include "tile_walk.cuh"
 
+#include <type_traits>
+
 namespace w2w {
 namespace {
 
-constexpr int kValues = 10;
 // Heavy tiles: each warp's walk is cut into kSplitWays segments, one CTA per
 // segment.  The CTA of a segment first replays the state recurrences of the
 // entries behind it (alpha and the transmittance / suffix updates only: no
@@ -61,131 +62,150 @@ __device__ __forceinline__ void segment_of(int walk, int k, int& lo, int& hi) {
   lo = max(0, min(lo, hi));
 }
 
-// Where each of the ten per-entry sums goes: after the transposed reduction
-// below, lane L (L even) holds the warp's sum of value (L >> 1); lanes 0..18
-// each add one of them to its gradient array.
-struct Target {
-  float* base;
-  int mult, off;
-  bool active;
-  bool second = false;  // flush_pair: the lane's value belongs to the second entry
+// ---------------------------------------------------------------------------
+// Per-pixel pass.  One warp per 8x4 pixel block (of two in a CTA; warps never
+// wait for one another), walking its block's part of the tile's list back to
+// front, the entries its block mask names packed into groups of 32:
+//
+//   1. lane j gathers entry j's record (the next group's loads are in flight
+//      while this one is evaluated) and puts it in shared memory;
+//   2. every lane evaluates the group's entries in order for its pixel -- the
+//      transmittance chain -- and writes two numbers per pair: u, from which
+//      every geometric gradient of the pair follows, and w, the pair's colour
+//      weight;
+//   3. the 32 x 32 table of (u, w) is read across: lane j sums entry j over the
+//      block's 32 pixels (the moments of u over the pixel offsets, and w times
+//      each upstream plane), turns the sums into the entry's gradients and adds
+//      each with one atomic.
+//
+// What bounds it: instruction issue, and for scenes that leave SMs idle the
+// busiest warp's chain.  Summing across the warp in step 3 costs about 12
+// instructions per entry; a shuffle tree per entry (ten values through 21
+// shuffles per pair of entries, with their products computed per pixel) cost
+// about 60, and groups of 32 mask-selected entries replace list chunks of 32
+// of which a quarter were evaluated.  Two-warp CTAs give a block's slot back
+// when it ends; an eight-warp CTA held its registers until the slowest of its
+// blocks had ended.
+// ---------------------------------------------------------------------------
+constexpr int kBwdWarps = 2;               // blocks (warps) per CTA
+constexpr int kBwdParts = 8 / kBwdWarps;   // CTAs per tile (and segment)
+constexpr int kGroup = 32;                 // entries per group, one per lane
+
+// A warp's shared memory.  The rows of `uw` are one pair longer than the
+// group, so that reading down a column touches every bank once.
+struct __align__(16) BwdWarp {
+  float4 rec[kGroup * kRecVec];  // the group's records; the third float4's w is the entry's list position
+  float4 up[32];                 // per pixel: upstream dL/dcolour and dL/ddepth
+  float2 uw[kGroup][33];
+  uint32_t slot[kGroup];         // list positions of the group being packed
 };
 
-// The gradient array and component of value idx (0..kValues-1).
-__device__ __forceinline__ Target value_target(const BackwardArgs& a, int mode, int idx, bool active) {
-  Target t{nullptr, 0, 0, active && idx >= 0 && idx < kValues};
-  if (idx < 0) return t;
-  if (idx < 3) t = Target{a.dL_dcolors, 3, idx, t.active};
-  else if (idx == 3) t = Target{a.acc_depth, 1, 0, t.active};
-  else if (idx < 6) t = Target{a.dL_dmean2D, 3, idx - 4, t.active};
-  else if (idx < 9) t = Target{a.acc_cov, 4, mode == 0 ? (idx == 8 ? 3 : idx - 6) : idx - 6, t.active};
-  else if (idx == 9) t = Target{a.dL_dopacity, 1, 0, t.active};
-  return t;
-}
+// Positions [lo, top) of a block's part of a tile's list, highest first, in
+// groups of up to 32.  words: the block's mask row, or null (each entry is
+// tested against the block here).
+struct BlockWalk {
+  const uint32_t* words;
+  const float* record;
+  const uint32_t* list;   // the tile's first list entry
+  uint32_t num_records;
+  int bx, by, lo, top, wi, wb;
+  uint32_t bits, cache;
 
-__device__ __forceinline__ Target lane_target(const BackwardArgs& a, int mode) {
-  const int lane = threadIdx.x & 31, idx = (lane >> 1) & 15;
-  return value_target(a, mode, idx, (lane & 1) == 0);
-}
-
-// flush_pair's lane roles: lane bit 4 picks the entry; within it the 16 lanes
-// of bits 0-3 hold values 5 * b3 + {0, 1, 2, 3, 4} at (b2, b1, b0) = (000,
-// 001, 010, 100, 101), and the other three hold the tree's zero padding.
-__device__ __forceinline__ Target lane_target_pair(const BackwardArgs& a, int mode) {
-  const int lane = threadIdx.x & 31;
-  const int b0 = lane & 1, b1 = (lane >> 1) & 1, b2 = (lane >> 2) & 1, b3 = (lane >> 3) & 1;
-  const int sub = b2 ? (b1 ? -1 : 3 + b0) : (b1 && b0 ? -1 : 2 * b1 + b0);
-  Target t = value_target(a, mode, sub < 0 ? -1 : 5 * b3 + sub, true);
-  t.second = (lane & 16) != 0;
-  return t;
-}
-
-// Sum ten values over the warp with 16 shuffles (each step exchanges the half
-// of the partial sums a lane does not keep) and add each total with one
-// atomic, issued by ten lanes at once.
-__device__ __forceinline__ void flush(const float (&c)[kValues], bool any_contrib, uint32_t id, const Target& t) {
-  if (!__any_sync(0xffffffffu, any_contrib)) return;
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  float v[16];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) v[k] = k < kValues ? c[k] : 0.0f;
-  float w8[8], w4[4], w2[2];
-  bool b = lane & 16;
-#pragma unroll
-  for (int k = 0; k < 8; ++k) w8[k] = (b ? v[k + 8] : v[k]) + __shfl_xor_sync(full, b ? v[k] : v[k + 8], 16);
-  b = lane & 8;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) w4[k] = (b ? w8[k + 4] : w8[k]) + __shfl_xor_sync(full, b ? w8[k] : w8[k + 4], 8);
-  b = lane & 4;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) w2[k] = (b ? w4[k + 2] : w4[k]) + __shfl_xor_sync(full, b ? w4[k] : w4[k + 2], 4);
-  b = lane & 2;
-  float w1 = (b ? w2[1] : w2[0]) + __shfl_xor_sync(full, b ? w2[0] : w2[1], 2);
-  w1 += __shfl_xor_sync(full, w1, 1);
-  if (t.active) atomicAdd(t.base + size_t(t.mult) * id + t.off, w1);
-}
-
-// Two entries' sums at once: their 20 values halve over five exchange steps
-// (10, 5, 3, 2 and 1 shuffles, the odd counts padded with a zero) instead of
-// 16 shuffles per entry; 20 lanes then add one total each (lane_target_pair).
-// An entry no lane contributes to is left out: the other goes alone (flush).
-__device__ __forceinline__ void flush_pair(const float (&c0)[kValues], const float (&c1)[kValues], bool any0,
-                                           bool any1, uint32_t id0, uint32_t id1, const Target& t,
-                                           const Target& tp) {
-  const bool has0 = __any_sync(0xffffffffu, any0), has1 = __any_sync(0xffffffffu, any1);
-  if (!has0 || !has1) {
-    if (has0) flush(c0, true, id0, t);
-    if (has1) flush(c1, true, id1, t);
-    return;
+  __device__ __forceinline__ void start(int lo_, int top_) {
+    lo = lo_;
+    top = top_;
+    wi = ((top - 1) >> 5) + 1;  // words [0, wi) are still to come
+    wb = wi;
+    bits = 0;
   }
-  static_assert(kValues == 10, "pair tree layout");
-  const unsigned full = 0xffffffffu;
-  const int lane = threadIdx.x & 31;
-  float w10[10], w5[6], w3[4], w2[2];
-  bool b = lane & 16;
-#pragma unroll
-  for (int k = 0; k < 10; ++k) w10[k] = (b ? c1[k] : c0[k]) + __shfl_xor_sync(full, b ? c0[k] : c1[k], 16);
-  b = lane & 8;
-#pragma unroll
-  for (int k = 0; k < 5; ++k) w5[k] = (b ? w10[k + 5] : w10[k]) + __shfl_xor_sync(full, b ? w10[k] : w10[k + 5], 8);
-  w5[5] = 0.0f;
-  b = lane & 4;
-#pragma unroll
-  for (int k = 0; k < 3; ++k) w3[k] = (b ? w5[k + 3] : w5[k]) + __shfl_xor_sync(full, b ? w5[k] : w5[k + 3], 4);
-  w3[3] = 0.0f;
-  b = lane & 2;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) w2[k] = (b ? w3[k + 2] : w3[k]) + __shfl_xor_sync(full, b ? w3[k] : w3[k + 2], 2);
-  b = lane & 1;
-  const float w1 = (b ? w2[1] : w2[0]) + __shfl_xor_sync(full, b ? w2[0] : w2[1], 1);
-  if (tp.active) atomicAdd(tp.base + size_t(tp.mult) * (tp.second ? id1 : id0) + tp.off, w1);
-}
+  // Word w's bits inside [lo, top).
+  __device__ __forceinline__ uint32_t word(int w) {
+    const int lane = threadIdx.x & 31;
+    uint32_t b;
+    if (words != nullptr) {
+      if (w < wb) {  // 32 words at a time, one per lane
+        wb = max(w - 31, 0);
+        cache = wb + lane <= w ? __ldg(words + wb + lane) : 0u;
+      }
+      b = __shfl_sync(0xffffffffu, cache, w - wb);
+    } else {
+      const int pos = 32 * w + lane;
+      bool reach = false;
+      if (pos >= lo && pos < top) {
+        const uint32_t id = __ldg(list + pos);
+        if (id < num_records) {
+          const float4* r = reinterpret_cast<const float4*>(record) + 4 * size_t(id);
+          const float4 r0 = __ldg(r), r2 = __ldg(r + 2), r3 = __ldg(r + 3);
+          reach = block_test(r0.x, r0.y, r2.w, r3.x, r3.y, r3.z, r3.w, bx, by);
+        }
+      }
+      b = __ballot_sync(0xffffffffu, reach);
+    }
+    const int above = top - 32 * w, below = lo - 32 * w;
+    if (above < 32) b &= (1u << above) - 1u;
+    if (below > 0) b &= 0xffffffffu << below;
+    return b;
+  }
+  // Packs the next group's positions into slot[0, count), highest first.
+  // Warp-collective; the caller has synchronised the warp after its last read of slot.
+  __device__ __forceinline__ int next(uint32_t* slot) {
+    const int lane = threadIdx.x & 31;
+    int count = 0;
+    if (top <= lo) return 0;
+    const int first = lo >> 5;
+    while (true) {
+      if (bits == 0u) {
+        if (wi <= first) break;
+        bits = word(--wi);
+        continue;
+      }
+      const int n = __popc(bits), room = kGroup - count;
+      const int rank = __popc((bits >> lane) >> 1);  // set bits above this lane's
+      const bool mine = (bits >> lane) & 1u;
+      if (mine && rank < room) slot[count + rank] = uint32_t(32 * wi + lane);
+      if (n > room) {
+        bits = __ballot_sync(0xffffffffu, mine && rank >= room);
+        count = kGroup;
+        break;
+      }
+      count += n;
+      bits = 0u;
+      if (count == kGroup) break;
+    }
+    __syncwarp();
+    return count;
+  }
+};
+
+// Entry records of a group in flight: lane j's entry.
+struct GroupLoad {
+  float4 r0, r1, r2;
+  uint32_t id;
+  int count;
+};
 
 // Pixel-loop prologue shared by both modes: this thread's pixel, its
-// upstream gradients and contributor count, the tile's walk length.
+// upstream gradients and contributor count, the warp's walk length.
 struct BwdPixel {
   int tile;
   TilePixel tp;
   bool inside;
-  size_t pix, hw;
+  size_t pix;
   uint2 range;
   int walk;  // list positions [0, walk) may hold contributors of this warp's pixels
-  uint32_t last, warp_last;
+  uint32_t last;
   float dLp0 = 0.f, dLp1 = 0.f, dLp2 = 0.f, dLd = 0.f, dLa = 0.f;
   int W, H;         // this tile's image size
-  size_t pbase;     // its first pixel in the (packed) per-pixel buffers
   const float* bg;
-  __device__ __forceinline__ BwdPixel(const BackwardArgs& a, int tile_, int local_tile, int W_, int H_, size_t pbase_,
-                                      const float* bg_)
-      : tile(tile_), tp(local_tile, (W_ + kTile - 1) / kTile), W(W_), H(H_), pbase(pbase_), bg(bg_) {
+  __device__ __forceinline__ BwdPixel(const BackwardArgs& a, int tile_, int local_tile, int block, int W_, int H_,
+                                      size_t pbase, const float* bg_)
+      : tile(tile_), tp(local_tile, (W_ + kTile - 1) / kTile, block), W(W_), H(H_), bg(bg_) {
     inside = tp.px < W && tp.py < H;
     range = a.ranges[tile];
-    hw = size_t(W) * H;
+    const size_t hw = size_t(W) * H;
     pix = inside ? pbase + size_t(tp.py) * W + tp.px : 0;
     last = inside ? a.n_contrib[pix] : 0u;
-    warp_last = __reduce_max_sync(0xffffffffu, last);
-    walk = int(min(warp_last, range.y - range.x));
+    walk = int(min(__reduce_max_sync(0xffffffffu, last), range.y - range.x));
     if (inside) {
       // colour planes: an image's three planes sit together at 3 * pbase
       const size_t cp = 3 * pbase + (pix - pbase);
@@ -195,99 +215,6 @@ struct BwdPixel {
       dLd = a.dL_ddepth != nullptr ? a.dL_ddepth[pix] : 0.f;  // absent: no loss on depth / alpha
       dLa = a.dL_dalpha != nullptr ? a.dL_dalpha[pix] : 0.f;
     }
-  }
-};
-
-// Reference formulas (backward.cu:552-663), per pixel, for one entry:
-// q0 = (mx, my, conic a, conic b), q1 = (conic c, opacity, depth, r), q2 = (g, b, skip, _).
-// kDA: a loss reaches depth or alpha.  Without one (dL/ddepth and dL/dalpha
-// absent, read as zero) every depth and alpha term adds exactly zero, so
-// RefChain<false> leaves them out (the suffix depth and alpha, their terms of
-// dL/dopacity, the depth contribution): the same results with about 7 % fewer
-// instructions per pair.
-template <bool kDA>
-struct RefChain {
-  float T, T_final, bg_dot;
-  float acc0 = 0.f, acc1 = 0.f, acc2 = 0.f, acc_d = 0.f, acc_a = 0.f;
-  float last_alpha = 0.f, lc0 = 0.f, lc1 = 0.f, lc2 = 0.f, last_depth = 0.f;
-
-  // The state after entry (opacity-weighted alpha `alpha`, colour in q1.w,
-  // q2.x, q2.y, depth q1.z).  T in [~1e-4, 1] (the forward stops before
-  // T < 1e-4) and 1 - alpha in [0.01, 1]: the division is in div_markstein's
-  // range, which equals /.
-  struct Next {
-    float Tn, n0, n1, n2, nd, na, y;  // y: RN(1 / (1 - alpha)), shared by the step's two quotients
-  };
-  __device__ __forceinline__ Next next(float alpha) const {
-    Next x;
-    x.y = rcp_markstein(1.f - alpha);
-    x.Tn = div_markstein_y(T, 1.f - alpha, x.y);
-    x.n0 = last_alpha * lc0 + (1.f - last_alpha) * acc0;
-    x.n1 = last_alpha * lc1 + (1.f - last_alpha) * acc1;
-    x.n2 = last_alpha * lc2 + (1.f - last_alpha) * acc2;
-    if constexpr (kDA) {
-      x.nd = last_alpha * last_depth + (1.f - last_alpha) * acc_d;
-      x.na = last_alpha + (1.f - last_alpha) * acc_a;
-    } else {
-      x.nd = 0.f;
-      x.na = 0.f;
-    }
-    return x;
-  }
-  __device__ __forceinline__ void commit(bool ok, const Next& x, float4 q1, float4 q2, float alpha) {
-    if (ok) {
-      T = x.Tn;
-      acc0 = x.n0; acc1 = x.n1; acc2 = x.n2;
-      lc0 = q1.w; lc1 = q2.x; lc2 = q2.y;
-      if constexpr (kDA) {
-        acc_d = x.nd; acc_a = x.na;
-        last_depth = q1.z;
-      }
-      last_alpha = alpha;
-    }
-  }
-  // State only (the walk of a later segment's prefix, see render_ref_kernel).
-  __device__ __forceinline__ void advance(bool ok, float4 q1, float4 q2, float alpha) {
-    commit(ok, next(alpha), q1, q2, alpha);
-  }
-
-  // ok false: the entry is skipped (state unchanged, contributions zero).
-  __device__ __forceinline__ void step(bool ok, const BwdPixel& p, float4 q0, float4 q1, float4 q2, float dx, float dy,
-                                       float G, float alpha, float ddelx_dx, float ddely_dy, float (&c)[kValues]) {
-    const Next x = next(alpha);
-    const float Tn = x.Tn, n0 = x.n0, n1 = x.n1, n2 = x.n2, nd = x.nd, na = x.na;
-    // a skipped entry's contributions are zeroed through three of their
-    // factors: alpha <= 0.99 and T_final / T finite keep dL_dopa finite, and
-    // the conic (inverse of a covariance with +0.3 on its diagonal) keeps dx,
-    // dy and the products finite, so each contribution is exactly +-0
-    const float dchdc = ok ? alpha * Tn : 0.f;
-    float dL_dopa = 0.0f;
-    dL_dopa += (q1.w - n0) * p.dLp0;
-    dL_dopa += (q2.x - n1) * p.dLp1;
-    dL_dopa += (q2.y - n2) * p.dLp2;
-    if constexpr (kDA) {
-      const float c_d = q1.z;
-      dL_dopa += (c_d - nd) * p.dLd;
-      dL_dopa += (1 - na) * p.dLa;
-    }
-    dL_dopa *= Tn;
-    dL_dopa += div_markstein_y(-T_final, 1.f - alpha, x.y) * bg_dot;
-    const float Gz = ok ? G : 0.f;  // G itself may be infinite where the entry is skipped
-    const float dL_dG = ok ? q1.y * dL_dopa : 0.f;
-    const float gdx = Gz * dx, gdy = Gz * dy;
-    const float dG_ddelx = -gdx * q0.z - gdy * q0.w;
-    const float dG_ddely = -gdy * q1.x - gdx * q0.w;
-    c[0] = dchdc * p.dLp0;
-    c[1] = dchdc * p.dLp1;
-    c[2] = dchdc * p.dLp2;
-    c[3] = kDA ? dchdc * p.dLd : 0.f;
-    c[4] = dL_dG * dG_ddelx * ddelx_dx;
-    c[5] = dL_dG * dG_ddely * ddely_dy;
-    c[6] = -0.5f * gdx * dx * dL_dG;
-    c[7] = -0.5f * gdx * dy * dL_dG;
-    c[8] = -0.5f * gdy * dy * dL_dG;
-    c[9] = Gz * dL_dopa;
-    commit(ok, x, q1, q2, alpha);
   }
 };
 
@@ -303,129 +230,97 @@ __device__ __forceinline__ bool ref_eval(float4 q0, float4 q1, float4 q2, float 
   return power <= 0.0f && power >= q2.z && alpha >= 1.0f / 255.0f;
 }
 
-// Walk list positions [lo, top) back to front, kChunk at a time; body(bits,
-// hi) handles one staged chunk whose entry j is list position hi - 1 - j and
-// whose set bits are the entries that may reach this warp's block.
-// wmask / wbit: the warp's block-mask array and bit (the blend's masks), or null.
-template <typename Body>
-__device__ __forceinline__ void walk_back(const float* records, const uint32_t* point_list, uint32_t num_records,
-                                          const uint8_t* wmask, int wbit, uint32_t base, int lo, int top,
-                                          WarpChunk& wc, const TilePixel& tp, Body&& body) {
-  const int len = top - lo;
-  const int nc = len > 0 ? (len + kChunk - 1) / kChunk : 0;
-  ChunkLoad ld;
-  uint32_t reach = 0;
-  if (nc > 0) {
-    chunk_load(ld, records, point_list, base + top - 1 - tp.lane, tp.lane < len, num_records, wmask, wbit);
-    reach = chunk_store(wc, ld, tp.bx, tp.by);
+// Reference formulas (backward.cu:552-663) for one pixel; records
+// (mx, my, conic a, conic b), (conic c, opacity, depth, r), (g, b, skip, position).
+// The reference keeps the colour, depth and alpha composited behind the current
+// entry per channel and multiplies their differences by the upstream planes;
+// the chain is linear in them, so one number serves: B, the upstream-weighted
+// composite behind the entry.  kDA: a loss reaches depth or alpha.
+template <bool kDA>
+struct RefChain {
+  float T, B = 0.f, tf_bg;  // tf_bg: T_final times (background . upstream colour)
+  __device__ __forceinline__ RefChain(const BackwardArgs& a, const BwdPixel& p) {
+    const float tf = p.inside ? 1.0f - a.out_alpha[p.pix] : 0.0f;
+    T = tf;
+    tf_bg = tf * (p.bg[0] * p.dLp0 + p.bg[1] * p.dLp1 + p.bg[2] * p.dLp2);
   }
-  for (int c = 0; c < nc; ++c) {
-    const int hi = top - c * kChunk;
-    const int hn = hi - kChunk;
-    const bool more = c + 1 < nc;
-    if (more)
-      chunk_load(ld, records, point_list, base + hn - 1 - tp.lane, hn - 1 - tp.lane >= lo, num_records, wmask,
-                 wbit);
-    body(reach, hi);
-    if (more) {
-      __syncwarp();
-      reach = chunk_store(wc, ld, tp.bx, tp.by);
+  static __device__ __forceinline__ const float* records(const BackwardArgs& a) { return a.bwd_record; }
+
+  // Two entries, in order (has1: the second exists); u, w of each.  T in
+  // [~1e-4, 1] (the forward stops before T < 1e-4) and 1 - alpha in [0.01, 1]:
+  // the division is in div_markstein's range, which equals /.  kFull false:
+  // state only (the entries behind a split tile's segment).
+  template <bool kFull>
+  __device__ __forceinline__ void pair(const float4* e0, const float4* e1, bool has1, const BwdPixel& p, float pxf,
+                                       float pyf, float2& o0, float2& o1) {
+    const float4 a0 = e0[0], a1 = e0[1], a2 = e0[2], b0 = e1[0], b1 = e1[1], b2 = e1[2];
+    float dx, dy, G0, al0, G1, al1;
+    const bool ok0 = ref_eval(a0, a1, a2, pxf, pyf, dx, dy, G0, al0) && __float_as_uint(a2.w) < p.last;
+    const bool ok1 = ref_eval(b0, b1, b2, pxf, pyf, dx, dy, G1, al1) && has1 && __float_as_uint(b2.w) < p.last;
+    step<kFull>(ok0, p, a1, a2, G0, al0, o0);
+    step<kFull>(ok1, p, b1, b2, G1, al1, o1);
+  }
+  template <bool kFull>
+  __device__ __forceinline__ void step(bool ok, const BwdPixel& p, float4 q1, float4 q2, float G, float alpha,
+                                       float2& o) {
+    const float y = rcp_markstein(1.f - alpha);
+    const float Tn = div_markstein_y(T, 1.f - alpha, y);
+    float q = q1.w * p.dLp0 + q2.x * p.dLp1 + q2.y * p.dLp2;
+    if constexpr (kDA) q += q1.z * p.dLd + p.dLa;
+    const float d = q - B;
+    // alpha <= 0.99 and T finite keep both factors finite; G itself may be
+    // infinite where the entry is skipped
+    if constexpr (kFull) o = make_float2(ok ? G * (d * Tn - tf_bg * y) : 0.f, ok ? alpha * Tn : 0.f);
+    if (ok) {
+      T = Tn;
+      B += alpha * d;
     }
   }
-}
 
-// CTA b's tile and segment: the first kSplitWays * split CTAs are the
-// segments of the `split` heaviest tiles (segment 0..kSplitWays-1), the rest
-// one whole tile each (segment -1), heaviest first.
-// Pixel-loop prologue for CTA blockIdx.x: its tile's image (the call's, or its
-// batch item's) and segment role.
-__device__ __forceinline__ BwdPixel make_bwd_pixel(const BackwardArgs& a, int tile, const float*& bg) {
-  if (a.items == nullptr) {
-    bg = a.bg;
-    return BwdPixel(a, tile, tile, a.W, a.H, 0, a.bg);
-  }
-  const BatchItem& it = a.items[find_item_tile(a.items, a.num_items, uint32_t(tile))];
-  bg = it.bg;
-  return BwdPixel(a, tile, tile - int(it.tile_base), it.W, it.H, size_t(it.pix_base), it.bg);
-}
-
-template <int kSplitWays>
-__device__ __forceinline__ int cta_tile(const BackwardArgs& a, int& seg) {
-  const int b = int(blockIdx.x);
-  if (b < kSplitWays * a.split) {
-    seg = b % kSplitWays;
-    return int(a.order_bwd[b / kSplitWays]);
-  }
-  seg = -1;
-  return int(a.order_bwd[b - (kSplitWays - 1) * a.split]);
-}
-
-template <int kSplitWays, bool kDA>
-__global__ void __launch_bounds__(kBlendThreads, 2) render_ref_kernel(BackwardArgs a) {
-  __shared__ WarpChunk s_chunk[kBlendThreads / 32];
-  int role;
-  const int gtile = cta_tile<kSplitWays>(a, role);
-  const float* bgp;
-  const BwdPixel p = make_bwd_pixel(a, gtile, bgp);
-  RefChain<kDA> ch;
-  ch.T_final = p.inside ? 1.0f - a.out_alpha[p.pix] : 0.0f;
-  ch.T = ch.T_final;
-  ch.bg_dot = bgp[0] * p.dLp0 + bgp[1] * p.dLp1 + bgp[2] * p.dLp2;
-  const float ddelx_dx = 0.5f * float(p.W), ddely_dy = 0.5f * float(p.H);
-  const float pxf = float(p.tp.px), pyf = float(p.tp.py);
-  const Target tgt = lane_target(a, 0);
-  const Target tgt2 = lane_target_pair(a, 0);
-  WarpChunk& wc = s_chunk[threadIdx.x >> 5];
-  // the blend's block masks, when this binning state has them: warps 0-3 read
-  // the top array, 4-7 the bottom one, bit = block within that half
-  const bool use_masks = a.masks_valid != nullptr && *a.masks_valid != 0u;
-  const uint8_t* wmask = use_masks ? ((threadIdx.x >> 5) < 4 ? a.mask_top : a.mask_bottom) : nullptr;
-  const int wbit = int(threadIdx.x >> 5) & 3;
-  const float4* s = wc.rec;
-  auto full = [&](uint32_t bits, int hi) {
-    while (bits != 0u) {
-      const int j0 = pop_entry(bits);
-      const int j1r = pop_entry(bits);
-      const bool has1 = j1r >= 0;
-      const int j1 = has1 ? j1r : j0;
-      const float4 a0 = s[kRecVec * j0], a1 = s[kRecVec * j0 + 1], a2 = s[kRecVec * j0 + 2];
-      const float4 b0 = s[kRecVec * j1], b1 = s[kRecVec * j1 + 1], b2 = s[kRecVec * j1 + 2];
-      float dx0, dy0, G0, al0, dx1, dy1, G1, al1;
-      const bool ok0 = ref_eval(a0, a1, a2, pxf, pyf, dx0, dy0, G0, al0) && uint32_t(hi - 1 - j0) < p.last;
-      const bool ok1 = ref_eval(b0, b1, b2, pxf, pyf, dx1, dy1, G1, al1) && has1 &&
-                       uint32_t(hi - 1 - j1) < p.last;
-      float c0[kValues], c1[kValues];
-      ch.step(ok0, p, a0, a1, a2, dx0, dy0, G0, al0, ddelx_dx, ddely_dy, c0);
-      ch.step(ok1, p, b0, b1, b2, dx1, dy1, G1, al1, ddelx_dx, ddely_dy, c1);
-      flush_pair(c0, c1, ok0, ok1, wc.id[j0], wc.id[j1], tgt, tgt2);
+  // Lane j's entry over the block's 32 pixels, and its atomics.
+  static __device__ __forceinline__ void reduce(const BackwardArgs& a, const BwdWarp& s, int j, uint32_t id, float bx,
+                                                float by, float hW, float hH) {
+    const float4 q0 = s.rec[kRecVec * j], q1 = s.rec[kRecVec * j + 1];
+    float S = 0.f, Sx = 0.f, Sy = 0.f, Sxx = 0.f, Sxy = 0.f, Syy = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f, cd = 0.f;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float dy = q0.y - (by + float(r));
+      float rs = 0.f, rx = 0.f;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float2 uw = s.uw[j][8 * r + c];
+        const float4 up = s.up[8 * r + c];
+        const float dx = q0.x - (bx + float(c)), t = uw.x * dx;
+        rs += uw.x;
+        rx += t;
+        Sxx += t * dx;
+        c0 += uw.y * up.x;
+        c1 += uw.y * up.y;
+        c2 += uw.y * up.z;
+        if constexpr (kDA) cd += uw.y * up.w;
+      }
+      S += rs;
+      Sx += rx;
+      Sxy += dy * rx;
+      const float t = dy * rs;
+      Sy += t;
+      Syy += t * dy;
     }
-  };
-  auto state_only = [&](uint32_t bits, int hi) {
-    while (bits != 0u) {
-      const int j0 = pop_entry(bits);
-      const int j1r = pop_entry(bits);
-      const bool has1 = j1r >= 0;
-      const int j1 = has1 ? j1r : j0;
-      const float4 a0 = s[kRecVec * j0], a1 = s[kRecVec * j0 + 1], a2 = s[kRecVec * j0 + 2];
-      const float4 b0 = s[kRecVec * j1], b1 = s[kRecVec * j1 + 1], b2 = s[kRecVec * j1 + 2];
-      float dx0, dy0, G0, al0, dx1, dy1, G1, al1;
-      const bool ok0 = ref_eval(a0, a1, a2, pxf, pyf, dx0, dy0, G0, al0) && uint32_t(hi - 1 - j0) < p.last;
-      const bool ok1 = ref_eval(b0, b1, b2, pxf, pyf, dx1, dy1, G1, al1) && has1 &&
-                       uint32_t(hi - 1 - j1) < p.last;
-      ch.advance(ok0, a1, a2, al0);
-      ch.advance(ok1, b1, b2, al1);
-    }
-  };
-  if (role < 0) {
-    walk_back(a.bwd_record, a.point_list, uint32_t(a.P), wmask, wbit, p.range.x, 0, p.walk, wc, p.tp, full);
-  } else {
-    int lo, hi;
-    segment_of<kSplitWays>(p.walk, role, lo, hi);
-    walk_back(a.bwd_record, a.point_list, uint32_t(a.P), wmask, wbit, p.range.x, hi, p.walk, wc, p.tp, state_only);
-    __syncwarp();
-    walk_back(a.bwd_record, a.point_list, uint32_t(a.P), wmask, wbit, p.range.x, lo, hi, wc, p.tp, full);
+    // no pixel of the block took the entry
+    if (S == 0.f && Sxx == 0.f && Syy == 0.f && c0 == 0.f && c1 == 0.f && c2 == 0.f && cd == 0.f) return;
+    const float h = -0.5f * q1.y;
+    atomicAdd(a.dL_dcolors + 3 * size_t(id), c0);
+    atomicAdd(a.dL_dcolors + 3 * size_t(id) + 1, c1);
+    atomicAdd(a.dL_dcolors + 3 * size_t(id) + 2, c2);
+    if constexpr (kDA) atomicAdd(a.acc_depth + id, cd);
+    atomicAdd(a.dL_dmean2D + 3 * size_t(id), -q1.y * hW * (q0.z * Sx + q0.w * Sy));
+    atomicAdd(a.dL_dmean2D + 3 * size_t(id) + 1, -q1.y * hH * (q1.x * Sy + q0.w * Sx));
+    atomicAdd(a.acc_cov + 4 * size_t(id), h * Sxx);
+    atomicAdd(a.acc_cov + 4 * size_t(id) + 1, h * Sxy);
+    atomicAdd(a.acc_cov + 4 * size_t(id) + 3, h * Syy);
+    atomicAdd(a.dL_dopacity + id, S);
   }
-}
+};
 
 // The forward's Gaussian value (blend.cu), split at its division so that a
 // warp's divisions can run branch-free together.
@@ -438,101 +333,26 @@ __device__ __forceinline__ float gauss_num_fwd(float px, float py, float mx, flo
   return s2<BL_NUM>(tX, dx, tY, dy);
 }
 
-// Exact derivative of the forward blend, per pixel, for one entry:
-// q0 = (mx, my, cxx, cxy), q1 = (cyy, det, opacity, depth), q2 = (r, g, b, _).
+// Exact derivative of the forward blend for one pixel; records
+// (mx, my, cxx, cxy), (cyy, det, opacity, depth), (r, g, b, position).  The
+// suffix sums behind the current entry (colour including the background,
+// depth, weight) enter only through their upstream-weighted sum D.
 struct ExactChain {
-  float T;
-  float S0, S1, S2, SD = 0.f, SW = 0.f;  // suffix sums behind the current entry (colour includes the background)
-
-  // State only (the walk of a later segment's prefix).
-  __device__ __forceinline__ void advance(bool ok, float4 q1, float4 q2, float a_) {
-    const float ia = rcp_markstein(1.0f - a_);
-    const float Tn = T * ia;
-    const float aT = a_ * Tn;
-    if (ok) {
-      T = Tn;
-      S0 += q2.x * aT;
-      S1 += q2.y * aT;
-      S2 += q2.z * aT;
-      SD += q1.w * aT;
-      SW += aT;
-    }
+  float T, D;
+  __device__ __forceinline__ ExactChain(const BackwardArgs& a, const BwdPixel& p) {
+    T = p.inside ? a.T_final[p.pix] : 0.0f;
+    D = T * (p.bg[0] * p.dLp0 + p.bg[1] * p.dLp1 + p.bg[2] * p.dLp2);
   }
+  static __device__ __forceinline__ const float* records(const BackwardArgs& a) { return a.record; }
 
-  // ok false: the entry is skipped (state unchanged, contributions zero).
-  __device__ __forceinline__ void step(bool ok, const BwdPixel& p, float4 q0, float4 q1, float4 q2, float pxf,
-                                       float pyf, float g, float og, float a_, float mahal, float hW, float hH,
-                                       float (&c)[kValues]) {
-    const float ia = rcp_markstein(1.0f - a_);  // 1 - alpha in [0.01, 1]
-    const float Tn = T * ia;  // transmittance in front of this entry
-    const float aT = a_ * Tn;
-    float dLda = p.dLp0 * (q2.x * Tn - S0 * ia) + p.dLp1 * (q2.y * Tn - S1 * ia) + p.dLp2 * (q2.z * Tn - S2 * ia);
-    dLda += p.dLd * (q1.w * Tn - SD * ia);
-    dLda += p.dLa * (Tn - SW * ia);
-    // skipped entries' contributions are zeroed through one factor each:
-    // 1 - alpha >= 0.01, g <= 1, det >= 0.09 and the mahalanobis distance
-    // (a quotient by det) keep every other factor finite
-    const float aTz = ok ? aT : 0.f;
-    c[0] = aTz * p.dLp0;
-    c[1] = aTz * p.dLp1;
-    c[2] = aTz * p.dLp2;
-    c[3] = aTz * p.dLd;
-    if (ok) {
-      T = Tn;
-      S0 += q2.x * aT;
-      S1 += q2.y * aT;
-      S2 += q2.z * aT;
-      SD += q1.w * aT;
-      SW += aT;
-    }
-    const bool unclamped = ok && og < 0.99f;
-    c[9] = dLda * (unclamped ? g : 0.f);
-    const bool inner = unclamped && mahal >= 0.0f;
-    const float dLdm = inner ? dLda * q1.z * (-0.5f * g) : 0.f;
-    const float cxx = q0.z, cxy = q0.w, cyy = q1.x, det = q1.y;
-    const float dx = pxf - q0.x, dy = pyf - q0.y;
-    // det >= 0.09 (the forward's +0.3 low-pass on a positive semi-definite
-    // covariance), where rcp_markstein is the correctly rounded 1/det
-    const float idet = rcp_markstein(det);
-    const float num = mahal * det;
-    c[4] = -dLdm * (2.f * cyy * dx - 2.f * cxy * dy) * idet * hW;
-    c[5] = -dLdm * (2.f * cxx * dy - 2.f * cxy * dx) * idet * hH;
-    c[6] = dLdm * (dy * dy * idet - num * cyy * idet * idet);
-    c[7] = dLdm * (-2.f * dx * dy * idet + 2.f * num * cxy * idet * idet);
-    c[8] = dLdm * (dx * dx * idet - num * cxx * idet * idet);
-  }
-};
-
-template <int kSplitWays>
-__global__ void __launch_bounds__(kBlendThreads, 2) render_exact_kernel(BackwardArgs a) {
-  __shared__ WarpChunk s_chunk[kBlendThreads / 32];
-  int role;
-  const int gtile = cta_tile<kSplitWays>(a, role);
-  const float* bgp;
-  const BwdPixel p = make_bwd_pixel(a, gtile, bgp);
-  ExactChain ch;
-  const float Tf = p.inside ? a.T_final[p.pix] : 0.0f;
-  ch.T = Tf;
-  ch.S0 = Tf * bgp[0];
-  ch.S1 = Tf * bgp[1];
-  ch.S2 = Tf * bgp[2];
-  const float hW = 0.5f * float(p.W), hH = 0.5f * float(p.H);
-  const float pxf = float(p.tp.px), pyf = float(p.tp.py);
-  const Target tgt = lane_target(a, 1);
-  const Target tgt2 = lane_target_pair(a, 1);
-  WarpChunk& wc = s_chunk[threadIdx.x >> 5];
-  // the blend's block masks, when this binning state has them: warps 0-3 read
-  // the top array, 4-7 the bottom one, bit = block within that half
-  const bool use_masks = a.masks_valid != nullptr && *a.masks_valid != 0u;
-  const uint8_t* wmask = use_masks ? ((threadIdx.x >> 5) < 4 ? a.mask_top : a.mask_bottom) : nullptr;
-  const int wbit = int(threadIdx.x >> 5) & 3;
-  const float4* s = wc.rec;
-  // the forward's Gaussian values of two entries (same division as the blend)
-  auto eval2 = [&](int j0, int j1, float& m0, float& m1, float& g0, float& g1) {
-    const float4 a0 = s[kRecVec * j0], a1 = s[kRecVec * j0 + 1];
-    const float4 b0 = s[kRecVec * j1], b1 = s[kRecVec * j1 + 1];
+  template <bool kFull>
+  __device__ __forceinline__ void pair(const float4* e0, const float4* e1, bool has1, const BwdPixel& p, float pxf,
+                                       float pyf, float2& o0, float2& o1) {
+    const float4 a0 = e0[0], a1 = e0[1], a2 = e0[2], b0 = e1[0], b1 = e1[1], b2 = e1[2];
+    // the forward's Gaussian values of the two entries (same division as the blend)
     const float n0 = gauss_num_fwd(pxf, pyf, a0.x, a0.y, a0.z, a0.w, a1.x);
     const float n1 = gauss_num_fwd(pxf, pyf, b0.x, b0.y, b0.z, b0.w, b1.x);
+    float m0, m1;
     if (__all_sync(0xffffffffu, div_in_range(n0, a1.y) && div_in_range(n1, b1.y))) {
       m0 = div_markstein(n0, a1.y);
       m1 = div_markstein(n1, b1.y);
@@ -540,53 +360,188 @@ __global__ void __launch_bounds__(kBlendThreads, 2) render_exact_kernel(Backward
       m0 = div(n0, a1.y);
       m1 = div(n1, b1.y);
     }
-    g0 = expf(mul(-0.5f, m0 < 0.0f ? 1000.0f : m0));
-    g1 = expf(mul(-0.5f, m1 < 0.0f ? 1000.0f : m1));
+    const float g0 = expf(mul(-0.5f, m0 < 0.0f ? 1000.0f : m0));
+    const float g1 = expf(mul(-0.5f, m1 < 0.0f ? 1000.0f : m1));
+    const float og0 = mul(a1.z, g0), og1 = mul(b1.z, g1);
+    const float al0 = fminf(0.99f, og0), al1 = fminf(0.99f, og1);
+    const bool ok0 = al0 >= 1.0f / 255.0f && __float_as_uint(a2.w) < p.last;
+    const bool ok1 = al1 >= 1.0f / 255.0f && has1 && __float_as_uint(b2.w) < p.last;
+    step<kFull>(ok0, p, a1, a2, g0, og0, al0, o0);
+    step<kFull>(ok1, p, b1, b2, g1, og1, al1, o1);
+  }
+  // u = dL/dalpha g: nothing passes the 0.99 clamp (a negative mahalanobis
+  // distance, mapped to 1000 by the forward, has g = 0)
+  template <bool kFull>
+  __device__ __forceinline__ void step(bool ok, const BwdPixel& p, float4 q1, float4 q2, float g, float og, float al,
+                                       float2& o) {
+    const float ia = rcp_markstein(1.0f - al);  // 1 - alpha in [0.01, 1]
+    const float Tn = T * ia;                    // transmittance in front of this entry
+    const float aT = al * Tn;
+    const float q = q2.x * p.dLp0 + q2.y * p.dLp1 + q2.z * p.dLp2 + q1.w * p.dLd + p.dLa;
+    if constexpr (kFull) o = make_float2(ok && og < 0.99f ? (q * Tn - D * ia) * g : 0.f, ok ? aT : 0.f);
+    if (ok) {
+      T = Tn;
+      D += q * aT;
+    }
+  }
+
+  // With e = cyy dx - cxy dy and f = cxx dy - cxy dx (offsets from the mean),
+  // d(num / det) = 2 (e, f) / det over the offsets and -(e e, 2 e f, f f) / det^2
+  // over the covariance.
+  static __device__ __forceinline__ void reduce(const BackwardArgs& a, const BwdWarp& s, int j, uint32_t id, float bx,
+                                                float by, float hW, float hH) {
+    const float4 q0 = s.rec[kRecVec * j], q1 = s.rec[kRecVec * j + 1];
+    float S = 0.f, Se = 0.f, Sf = 0.f, See = 0.f, Sef = 0.f, Sff = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f, cd = 0.f;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const float dy = (by + float(r)) - q0.y, ey = -q0.w * dy, fy = q0.z * dy;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float2 uw = s.uw[j][8 * r + c];
+        const float4 up = s.up[8 * r + c];
+        const float dx = (bx + float(c)) - q0.x;
+        const float e = q1.x * dx + ey, f = fy - q0.w * dx;
+        const float te = uw.x * e, tf = uw.x * f;
+        S += uw.x;
+        Se += te;
+        Sf += tf;
+        See += te * e;
+        Sef += te * f;
+        Sff += tf * f;
+        c0 += uw.y * up.x;
+        c1 += uw.y * up.y;
+        c2 += uw.y * up.z;
+        cd += uw.y * up.w;
+      }
+    }
+    if (S == 0.f && See == 0.f && Sff == 0.f && c0 == 0.f && c1 == 0.f && c2 == 0.f && cd == 0.f) return;
+    // det >= 0.09 (the forward's +0.3 low-pass on a positive semi-definite
+    // covariance), where rcp_markstein is the correctly rounded 1/det
+    const float idet = rcp_markstein(q1.y), k1 = q1.z * idet, k2 = k1 * idet;
+    atomicAdd(a.dL_dcolors + 3 * size_t(id), c0);
+    atomicAdd(a.dL_dcolors + 3 * size_t(id) + 1, c1);
+    atomicAdd(a.dL_dcolors + 3 * size_t(id) + 2, c2);
+    atomicAdd(a.acc_depth + id, cd);
+    atomicAdd(a.dL_dmean2D + 3 * size_t(id), k1 * hW * Se);
+    atomicAdd(a.dL_dmean2D + 3 * size_t(id) + 1, k1 * hH * Sf);
+    atomicAdd(a.acc_cov + 4 * size_t(id), 0.5f * k2 * See);
+    atomicAdd(a.acc_cov + 4 * size_t(id) + 1, k2 * Sef);
+    atomicAdd(a.acc_cov + 4 * size_t(id) + 2, 0.5f * k2 * Sff);
+    atomicAdd(a.dL_dopacity + id, S);
+  }
+};
+
+// Pixel-loop prologue for block `block` of tile `tile`: the call's image, or
+// its batch item's.
+__device__ __forceinline__ BwdPixel make_bwd_pixel(const BackwardArgs& a, int tile, int block) {
+  if (a.items == nullptr) return BwdPixel(a, tile, tile, block, a.W, a.H, 0, a.bg);
+  const BatchItem& it = a.items[find_item_tile(a.items, a.num_items, uint32_t(tile))];
+  return BwdPixel(a, tile, tile - int(it.tile_base), block, it.W, it.H, size_t(it.pix_base), it.bg);
+}
+
+// Work item b's tile and segment: the first kSplitWays * split items are the
+// segments of the `split` heaviest tiles (segment 0..kSplitWays-1), the rest
+// one whole tile each (segment -1), heaviest first.
+template <int kSplitWays>
+__device__ __forceinline__ int item_tile(const BackwardArgs& a, int b, int& seg) {
+  if (b < kSplitWays * a.split) {
+    seg = b % kSplitWays;
+    return int(a.order_bwd[b / kSplitWays]);
+  }
+  seg = -1;
+  return int(a.order_bwd[b - (kSplitWays - 1) * a.split]);
+}
+
+template <typename Chain, int kSplitWays>
+__global__ void __launch_bounds__(32 * kBwdWarps) render_bwd_kernel(BackwardArgs a) {
+  __shared__ BwdWarp s_warp[kBwdWarps];
+  int seg;
+  const int tile = item_tile<kSplitWays>(a, int(blockIdx.x) / kBwdParts, seg);
+  const int warp = int(threadIdx.x >> 5), lane = int(threadIdx.x & 31);
+  const int block = (int(blockIdx.x) % kBwdParts) * kBwdWarps + warp;
+  const BwdPixel p = make_bwd_pixel(a, tile, block);
+  if (p.walk <= 0) return;  // warp-uniform
+  BwdWarp& s = s_warp[warp];
+  s.up[lane] = make_float4(p.dLp0, p.dLp1, p.dLp2, p.dLd);
+  Chain ch(a, p);
+  const float pxf = float(p.tp.px), pyf = float(p.tp.py);
+  const float hW = 0.5f * float(p.W), hH = 0.5f * float(p.H);
+  const float4* records = reinterpret_cast<const float4*>(Chain::records(a));
+  const uint32_t* list = a.point_list + p.range.x;
+  BlockWalk walk;
+  // the blend's block masks, when this binning state has them
+  const bool use_masks = a.masks_valid != nullptr && *a.masks_valid != 0u;
+  walk.words = use_masks ? a.masks + mask_row(p.range.x, tile, int(p.range.y - p.range.x), block) : nullptr;
+  walk.record = Chain::records(a);
+  walk.list = list;
+  walk.num_records = uint32_t(a.P);
+  walk.bx = p.tp.bx;
+  walk.by = p.tp.by;
+
+  // Positions of the next group, and lane j's id in it (an id of num_records
+  // or more -- a list left inconsistent by a sort whose bounded wait ran out,
+  // which its error word reports -- is skipped, never read).
+  auto pack = [&](uint32_t& pos, uint32_t& id) {
+    __syncwarp();
+    const int n = walk.next(s.slot);
+    pos = lane < n ? s.slot[lane] : 0u;
+    id = lane < n ? __ldg(list + pos) : ~0u;
+    return n;
   };
-  auto full = [&](uint32_t bits, int hi) {
-    while (bits != 0u) {
-      const int j0 = pop_entry(bits);
-      const int j1r = pop_entry(bits);
-      const bool has1 = j1r >= 0;
-      const int j1 = has1 ? j1r : j0;
-      float m0, m1, g0, g1;
-      eval2(j0, j1, m0, m1, g0, g1);
-      const float4 a0 = s[kRecVec * j0], a1 = s[kRecVec * j0 + 1];
-      const float4 b0 = s[kRecVec * j1], b1 = s[kRecVec * j1 + 1];
-      const float og0 = mul(a1.z, g0), og1 = mul(b1.z, g1);
-      const float al0 = fminf(0.99f, og0), al1 = fminf(0.99f, og1);
-      const bool ok0 = al0 >= 1.0f / 255.0f && uint32_t(hi - 1 - j0) < p.last;
-      const bool ok1 = al1 >= 1.0f / 255.0f && has1 && uint32_t(hi - 1 - j1) < p.last;
-      float c0[kValues], c1[kValues];
-      ch.step(ok0, p, a0, a1, s[kRecVec * j0 + 2], pxf, pyf, g0, og0, al0, m0, hW, hH, c0);
-      ch.step(ok1, p, b0, b1, s[kRecVec * j1 + 2], pxf, pyf, g1, og1, al1, m1, hW, hH, c1);
-      flush_pair(c0, c1, ok0, ok1, wc.id[j0], wc.id[j1], tgt, tgt2);
+  auto gather = [&](GroupLoad& g, uint32_t pos, uint32_t id, int n) {
+    g.id = id;
+    g.count = n;
+    g.r0 = g.r1 = g.r2 = make_float4(0.f, 0.f, 0.f, 0.f);  // opacity 0: contributes nothing
+    if (id < uint32_t(a.P)) {
+      const float4* r = records + 4 * size_t(id);
+      g.r0 = __ldg(r);
+      g.r1 = __ldg(r + 1);
+      g.r2 = __ldg(r + 2);
+    }
+    g.r2.w = __uint_as_float(id < uint32_t(a.P) ? pos : ~0u);  // past every pixel's last contributor
+  };
+  auto run = [&](int lo, int top, auto full) {
+    constexpr bool kFull = decltype(full)::value;
+    walk.start(lo, top);
+    GroupLoad g;
+    uint32_t pos, id;
+    int n = pack(pos, id);
+    gather(g, pos, id, n);
+    n = n > 0 ? pack(pos, id) : 0;
+    while (g.count > 0) {
+      const int count = g.count;
+      const uint32_t cur = g.id;
+      s.rec[kRecVec * lane] = g.r0;
+      s.rec[kRecVec * lane + 1] = g.r1;
+      s.rec[kRecVec * lane + 2] = g.r2;
+      gather(g, pos, id, n);             // the next group's records and
+      n = n > 0 ? pack(pos, id) : 0;     // the ids of the one after it are in flight below
+      __syncwarp();
+      for (int j = 0; j < count; j += 2) {
+        const bool has1 = j + 1 < count;
+        float2 o0, o1;
+        ch.template pair<kFull>(s.rec + kRecVec * j, s.rec + kRecVec * (has1 ? j + 1 : j), has1, p, pxf, pyf, o0, o1);
+        if constexpr (kFull) {
+          s.uw[j][lane] = o0;
+          s.uw[j + 1][lane] = o1;
+        }
+      }
+      __syncwarp();
+      if constexpr (kFull) {
+        if (lane < count && cur < uint32_t(a.P))
+          Chain::reduce(a, s, lane, cur, float(p.tp.bx), float(p.tp.by), hW, hH);
+        __syncwarp();
+      }
     }
   };
-  auto state_only = [&](uint32_t bits, int hi) {
-    while (bits != 0u) {
-      const int j0 = pop_entry(bits);
-      const int j1r = pop_entry(bits);
-      const bool has1 = j1r >= 0;
-      const int j1 = has1 ? j1r : j0;
-      float m0, m1, g0, g1;
-      eval2(j0, j1, m0, m1, g0, g1);
-      const float4 a1 = s[kRecVec * j0 + 1], b1 = s[kRecVec * j1 + 1];
-      const float al0 = fminf(0.99f, mul(a1.z, g0)), al1 = fminf(0.99f, mul(b1.z, g1));
-      const bool ok0 = al0 >= 1.0f / 255.0f && uint32_t(hi - 1 - j0) < p.last;
-      const bool ok1 = al1 >= 1.0f / 255.0f && has1 && uint32_t(hi - 1 - j1) < p.last;
-      ch.advance(ok0, a1, s[kRecVec * j0 + 2], al0);
-      ch.advance(ok1, b1, s[kRecVec * j1 + 2], al1);
-    }
-  };
-  if (role < 0) {
-    walk_back(a.record, a.point_list, uint32_t(a.P), wmask, wbit, p.range.x, 0, p.walk, wc, p.tp, full);
+  if (seg < 0) {
+    run(0, p.walk, std::true_type{});
   } else {
     int lo, hi;
-    segment_of<kSplitWays>(p.walk, role, lo, hi);
-    walk_back(a.record, a.point_list, uint32_t(a.P), wmask, wbit, p.range.x, hi, p.walk, wc, p.tp, state_only);
+    segment_of<kSplitWays>(p.walk, seg, lo, hi);
+    run(hi, p.walk, std::false_type{});
     __syncwarp();
-    walk_back(a.record, a.point_list, uint32_t(a.P), wmask, wbit, p.range.x, lo, hi, wc, p.tp, full);
+    run(lo, hi, std::true_type{});
   }
 }
 
@@ -1455,16 +1410,17 @@ void launch_backward_render(const BackwardArgs& a, cudaStream_t stream) {
   b.split = min(tiles / 4, sms * tune_value(kTuneBwdSplit) / 4);
   const int ways = tune_value(kTuneBwdWays);
   stage_begin(kStBwdRender, stream);
-  const int grid = tiles + (ways - 1) * b.split;
+  const int grid = (tiles + (ways - 1) * b.split) * kBwdParts;
   const bool da = a.dL_ddepth != nullptr || a.dL_dalpha != nullptr;  // a loss reaches depth or alpha
+  auto launch = [&](auto kernel) { kernel<<<grid, 32 * kBwdWarps, 0, stream>>>(b); };
   if (ways == 3) {
-    if (a.grad_mode == 1) render_exact_kernel<3><<<grid, kBlendThreads, 0, stream>>>(b);
-    else if (da) render_ref_kernel<3, true><<<grid, kBlendThreads, 0, stream>>>(b);
-    else render_ref_kernel<3, false><<<grid, kBlendThreads, 0, stream>>>(b);
+    if (a.grad_mode == 1) launch(render_bwd_kernel<ExactChain, 3>);
+    else if (da) launch(render_bwd_kernel<RefChain<true>, 3>);
+    else launch(render_bwd_kernel<RefChain<false>, 3>);
   } else {
-    if (a.grad_mode == 1) render_exact_kernel<2><<<grid, kBlendThreads, 0, stream>>>(b);
-    else if (da) render_ref_kernel<2, true><<<grid, kBlendThreads, 0, stream>>>(b);
-    else render_ref_kernel<2, false><<<grid, kBlendThreads, 0, stream>>>(b);
+    if (a.grad_mode == 1) launch(render_bwd_kernel<ExactChain, 2>);
+    else if (da) launch(render_bwd_kernel<RefChain<true>, 2>);
+    else launch(render_bwd_kernel<RefChain<false>, 2>);
   }
   stage_end(kStBwdRender, stream, 1);
 }

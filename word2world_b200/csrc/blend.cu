@@ -128,19 +128,18 @@ __global__ void __launch_bounds__(32 * kBlendWarps, (blend_min_blocks<kBlendWarp
     }
     if constexpr (kAsync) cp_async_commit();
   };
-  // block masks for the backward: the upper half's CTA (or the whole tile's)
-  // writes the top array, the lower half's the bottom one
-  uint8_t* lo_dst = a.mask_top == nullptr ? nullptr : (part == 0 ? a.mask_top : a.mask_bottom) + range.x;
-  uint8_t* hi_dst = a.mask_top == nullptr || kBlendParts != 1 ? nullptr : a.mask_bottom + range.x;
+  // this CTA's rows of block-mask words for the backward (mask_row)
+  const int row_words = (n + 31) >> 5;
+  uint32_t* rows = a.masks == nullptr ? nullptr : a.masks + mask_row(range.x, tile, n, first_block);
   auto store = [&](int buf, int base) {
     if constexpr (kAsync) cp_async_wait_all();
 #pragma unroll
     for (int r = 0; r < kStagePer; ++r) {
       const int j = r * kBlendCta + int(threadIdx.x);
-      uint8_t* lo = lo_dst ? lo_dst + base : nullptr;
-      uint8_t* hi = hi_dst ? hi_dst + base : nullptr;
-      if constexpr (kAsync) stage_mask(sm, buf, staged[r], j, tp.X0, tp.Y0, first_block, lo, hi);
-      else stage_store(sm, buf, st[r], j, tp.X0, tp.Y0, first_block, lo, hi);
+      uint32_t* dst = rows ? rows + (base >> 5) : nullptr;
+      const int words = row_words - (base >> 5);
+      if constexpr (kAsync) stage_mask(sm, buf, staged[r], j, tp.X0, tp.Y0, first_block, dst, row_words, words);
+      else stage_store(sm, buf, st[r], j, tp.X0, tp.Y0, first_block, dst, row_words, words);
     }
   };
   if (nb > 0) {

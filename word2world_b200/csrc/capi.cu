@@ -499,8 +499,7 @@ int w2w_forward_render(const w2w_settings* s, const void* geom_state, const w2w_
   b.num_records = uint32_t(s->P);
   if (R > 0) {
     const BinLayout BL(R, T);
-    b.mask_top = at<uint8_t>(binning_state, BL.masks);
-    b.mask_bottom = b.mask_top + R;
+    b.masks = at<uint32_t>(binning_state, BL.masks);
     b.masks_valid = &at<BinHeader>(binning_state, BL.header)->masks_valid;
   }
   b.bg = s->background;
@@ -711,8 +710,7 @@ int w2w_forward_render_planned(const w2w_settings* s, const void* geom_state, lo
   b.point_list = valsA;
   b.record = at<float>(geom_state, GL.record);
   b.num_records = uint32_t(s->P);
-  b.mask_top = at<uint8_t>(binning_state, BL.masks);
-  b.mask_bottom = b.mask_top + capacity;
+  b.masks = at<uint32_t>(binning_state, BL.masks);
   b.masks_valid = &bh->masks_valid;
   b.bg = s->background;
   b.out_color = out_color; b.out_depth = out_depth; b.out_alpha = out_alpha;
@@ -792,8 +790,7 @@ static int backward_impl(const w2w_settings* s, const float* means3D, const floa
   a.point_list = R > 0 ? at<uint32_t>(binning_state, BinLayout(R, num_tiles(W, H)).valsA) : nullptr;
   if (R > 0) {
     const BinLayout BL(R, num_tiles(W, H));
-    a.mask_top = at<uint8_t>(binning_state, BL.masks);
-    a.mask_bottom = a.mask_top + R;
+    a.masks = at<uint32_t>(binning_state, BL.masks);
     a.masks_valid = &at<BinHeader>(binning_state, BL.header)->masks_valid;
   }
   a.n_contrib = at<uint32_t>(image_state, IL.n_contrib);
@@ -1401,8 +1398,7 @@ int w2w_batch_forward_render(const w2w_batch_item* items, int n, const void* geo
   b.num_records = uint32_t(E);
   if (R > 0) {
     const BinLayout BL(R, T);
-    b.mask_top = at<uint8_t>(binning_state, BL.masks);
-    b.mask_bottom = b.mask_top + R;
+    b.masks = at<uint32_t>(binning_state, BL.masks);
     b.masks_valid = &at<BinHeader>(binning_state, BL.header)->masks_valid;
   }
   b.bg = nullptr;
@@ -1471,8 +1467,7 @@ static int batch_backward_begin(const w2w_batch_item* items, int n, const void* 
   a.point_list = R > 0 ? at<uint32_t>(binning_state, BinLayout(R, T).valsA) : nullptr;
   if (R > 0) {
     const BinLayout BL(R, T);
-    a.mask_top = at<uint8_t>(binning_state, BL.masks);
-    a.mask_bottom = a.mask_top + R;
+    a.masks = at<uint32_t>(binning_state, BL.masks);
     a.masks_valid = &at<BinHeader>(binning_state, BL.header)->masks_valid;
   }
   a.n_contrib = at<uint32_t>(image_state, IL.n_contrib);

@@ -430,8 +430,8 @@ struct BinLayout {
     const size_t chunks = num_tiles > 0 && num_tiles <= kMaxBinTiles ? (r + kBinChunk - 1) / kBinChunk : 0;
     bin_counts = take(chunks * size_t(num_tiles > 0 ? num_tiles : 0) * 4);
     warp_start = take(chunks ? ((r + kBinShare - 1) / kBinShare + 1) * 4 : 0);
-    // the blend's block masks per list position: the tile's upper blocks, then its lower blocks
-    masks = take(2 * r);
+    // the blend's block masks: 8 words per 32 list positions, and up to one more group per tile (mask_row)
+    masks = take((r / 32 + size_t(num_tiles > 0 ? num_tiles : 0) + 1) * 32);
     total = align256(o);
   }
 };

@@ -1,21 +1,9 @@
 // Shared machinery of the per-tile pixel loops (forward blend, both backward
 // pixel passes).
 //
-// A CTA of 256 threads owns one 16x16 tile; warp w owns the 8x4 pixel block
-// w (columns 8*(w & 1) .. +7, rows 4*(w >> 1) .. +3), lane l its pixel
+// A tile is cut into eight 8x4 pixel blocks, one warp each: warp w owns
+// columns 8*(w & 1) .. +7, rows 4*(w >> 1) .. +3, lane l its pixel
 // (l & 7, l >> 3) inside the block.
-//
-// Independent warps (backward passes): each warp walks the tile's list on its
-// own, down from its pixels' largest contributor count, kChunk entries at a
-// time: lane j gathers entry j's 64-byte record by
-// Gaussian id (the tile's warps gather the same records, so after the first
-// they come from L1), tests whether the Gaussian can reach the warp's block
-// with alpha >= 1/255 (block_test in common.cuh) and stores the record's first
-// 48 bytes to the warp's shared-memory slot; the ballot of the tests is the
-// list of entries the warp evaluates, in list order.  The next chunk's records
-// are gathered while the current one is walked.  Warps never wait for one
-// another: a warp whose block has little to do, or whose pixels have all
-// terminated, finishes early instead of idling at a per-batch barrier.
 #pragma once
 
 #include "common.cuh"
@@ -23,12 +11,6 @@
 namespace w2w {
 
 constexpr int kRecVec = 3;  // float4s of a record staged in shared memory
-constexpr int kChunk = 32;  // list entries staged per warp step (one per lane)
-
-struct WarpChunk {
-  float4 rec[kChunk * kRecVec];
-  uint32_t id[kChunk];
-};
 
 // Pixel of this thread in tile `tile` of a grid `gw` tiles wide.
 struct TilePixel {
@@ -57,76 +39,17 @@ struct TilePixel {
 __global__ void tile_order_kernel(const uint2* ranges, const uint32_t* counts, int num_tiles, uint32_t* order,
                                   uint32_t* zero, uint32_t* counter);
 
-// One entry's record held in registers between its gather and its store.
-struct ChunkLoad {
-  float4 r0, r1, r2, r3;
-  uint32_t id;
-  bool has;
-  bool masked;  // `has` already means "may reach the warp's block" (from the blend's block masks)
-};
-
-// Block masks the forward blend leaves for the backward passes: per list
-// position, 4 bits for the tile's upper four 8x4 blocks (array `top`) and 4
-// for its lower four (`bottom`), bit b set when the entry may reach block b
-// (block_mask).  `valid` points at the binning header's flag; a state the
-// blend did not write (a replayed list) has it clear, and the walk tests
-// every entry itself.
-struct BlockMasks {
-  const uint8_t* top;
-  const uint8_t* bottom;
-  const uint32_t* valid;
-};
-
-// Gather entry `pos` of the point list (when `has`).  Records are four float4s;
-// r2.w and r3 hold the culling parameters (hy; beta, gamma, eps, vr).  An id
-// of num_records or more (a list left inconsistent by a sort whose bounded
-// wait ran out, which its error word reports) is skipped, never read.  With
-// `mask` (the warp's mask array, or null) only entries whose bit `bit` is set
-// are gathered.
-__device__ __forceinline__ void chunk_load(ChunkLoad& st, const float* record, const uint32_t* point_list, size_t pos,
-                                           bool has, uint32_t num_records, const uint8_t* mask = nullptr,
-                                           int bit = 0) {
-  st.has = false;
-  st.masked = mask != nullptr;
-  if (has && mask != nullptr) has = (mask[pos] >> bit) & 1u;
-  if (has) {
-    st.id = point_list[pos];
-    st.has = st.id < num_records;
-  }
-  if (st.has) {
-    const float4* rec = reinterpret_cast<const float4*>(record);
-    const float4* r = rec + 4 * size_t(st.id);
-    st.r0 = __ldg(r);
-    st.r1 = __ldg(r + 1);
-    st.r2 = __ldg(r + 2);
-    st.r3 = __ldg(r + 3);
-  }
-}
-
-// Store lane j's gathered entry in slot j and return the ballot of "may reach
-// the block at (bx, by)".  Warp-collective; the caller has synchronised the
-// warp after its last read of the previous chunk.
-__device__ __forceinline__ uint32_t chunk_store(WarpChunk& c, const ChunkLoad& st, int bx, int by) {
-  const int lane = threadIdx.x & 31;
-  bool reach = false;
-  if (st.has) {
-    float4* s = &c.rec[kRecVec * lane];
-    s[0] = st.r0;
-    s[1] = st.r1;
-    s[2] = st.r2;
-    c.id[lane] = st.id;
-    reach = st.masked || block_test(st.r0.x, st.r0.y, st.r2.w, st.r3.x, st.r3.y, st.r3.z, st.r3.w, bx, by);
-  }
-  __syncwarp();
-  return __ballot_sync(0xffffffffu, reach);
-}
-
-// Next set bit of `bits` (cleared), or -1.
-__device__ __forceinline__ int pop_entry(uint32_t& bits) {
-  if (bits == 0u) return -1;
-  const int j = __ffs(bits) - 1;
-  bits &= bits - 1u;
-  return j;
+// Block masks the forward blend leaves for the backward passes: for every
+// tile and 8x4 block one bit per list position, set when the entry may reach
+// the block (block_mask), packed into words of 32 positions counted from the
+// tile's first one.  A tile of n entries has 8 rows (one per block) of
+// ceil(n / 32) words; its rows start at word mask_row(...), which keeps the
+// tiles' regions apart without a prefix over them: a tile's list starts at
+// position x, and floor(x / 32) + tile grows by at least ceil(n / 32) from one
+// tile to the next.  A state the blend did not write (a replayed list) has the
+// binning header's flag clear, and the backward tests every entry itself.
+__host__ __device__ __forceinline__ size_t mask_row(uint32_t first, int tile, int n, int block) {
+  return 8 * (size_t(first >> 5) + size_t(tile)) + size_t(block) * size_t((n + 31) >> 5);
 }
 
 // ---------------------------------------------------------------------------
@@ -175,22 +98,20 @@ __device__ __forceinline__ int build_list(TileWalkShared<kW, kVec>& sm, int buf,
 
 // Block bits of one entry for the CTA's kW blocks (the tile's blocks
 // first_block .. first_block + kW - 1), published as the CTA's ballot words of
-// slot j; the masks also go to global memory for the backward passes
-// (BlockMasks): bits 0-3 to lo_dst[j], bits 4-7 (eight-warp CTAs) to
-// hi_dst[j], where the callers offset the arrays to the batch's first list
-// position.  Every thread of a warp must call this for the same chunk (the
-// ballots are full-warp).
+// slot j; the words also go to global memory for the backward passes
+// (mask_row): block b's word to rows[b * row_words + chunk], where the caller
+// offsets `rows` (or null) to the CTA's first block and the batch's first word
+// and gives how many of the batch's words the row holds.  Every thread of a
+// warp must call this for the same chunk (the ballots are full-warp).
 template <int kW, int kVec>
 __device__ __forceinline__ void publish_mask(TileWalkShared<kW, kVec>& sm, int buf, bool has, float mx, float my,
                                              float hy, float4 c, int j, int X0, int Y0, int first_block,
-                                             uint8_t* lo_dst, uint8_t* hi_dst) {
+                                             uint32_t* rows, int row_words, int words) {
   const int lane = j & 31, chunk = j >> 5;
   uint32_t mask = 0;
   if (has) {
     // the CTA's blocks are kW / 2 rows of two, starting at row group first_block / 2
     mask = block_mask<kW / 2>(mx, my, hy, c.x, c.y, c.z, c.w, X0, Y0 + kBlockH * (first_block / 2));
-    if (lo_dst != nullptr) lo_dst[j] = uint8_t(mask & 15u);
-    if (hi_dst != nullptr) hi_dst[j] = uint8_t(mask >> 4);
   }
   uint32_t mine = 0;
 #pragma unroll
@@ -198,7 +119,10 @@ __device__ __forceinline__ void publish_mask(TileWalkShared<kW, kVec>& sm, int b
     const uint32_t w = __ballot_sync(0xffffffffu, (mask >> b) & 1u);
     if (lane == b) mine = w;
   }
-  if (lane < kW) sm.bal[buf][lane][chunk] = mine;
+  if (lane < kW) {
+    sm.bal[buf][lane][chunk] = mine;
+    if (rows != nullptr && chunk < words) rows[size_t(lane) * row_words + chunk] = mine;
+  }
 }
 
 // One entry's record held in registers between its gather and its store.
@@ -209,7 +133,9 @@ struct Staged {
 
 // Gather entry `pos` of the point list (when `has`) into registers.  Records
 // are four float4s; r2.w and r3 hold the culling parameters (hy; beta, gamma,
-// eps, vr).  Ids of num_records or more are skipped (see chunk_load).
+// eps, vr).  An id of num_records or more (a list left inconsistent by a sort
+// whose bounded wait ran out, which its error word reports) is skipped, never
+// read.
 __device__ __forceinline__ void stage_load(Staged& st, const float* record, const uint32_t* point_list, size_t pos,
                                            bool has, uint32_t num_records) {
   st.has = false;
@@ -231,14 +157,14 @@ __device__ __forceinline__ void stage_load(Staged& st, const float* record, cons
 // publish its block masks (publish_mask).
 template <int kW>
 __device__ __forceinline__ void stage_store(TileWalkShared<kW, kRecVec>& sm, int buf, const Staged& st, int j, int X0,
-                                            int Y0, int first_block, uint8_t* lo_dst, uint8_t* hi_dst) {
+                                            int Y0, int first_block, uint32_t* rows, int row_words, int words) {
   if (st.has) {
     float4* s = &sm.rec[buf][kRecVec * j];
     s[0] = st.r0;
     s[1] = st.r1;
     s[2] = st.r2;
   }
-  publish_mask(sm, buf, st.has, st.r0.x, st.r0.y, st.r2.w, st.r3, j, X0, Y0, first_block, lo_dst, hi_dst);
+  publish_mask(sm, buf, st.has, st.r0.x, st.r0.y, st.r2.w, st.r3, j, X0, Y0, first_block, rows, row_words, words);
 }
 
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
@@ -267,7 +193,7 @@ __device__ __forceinline__ bool stage_copy(float4* dst, const float* record, con
 // by this thread, whose copies have landed).
 template <int kW>
 __device__ __forceinline__ void stage_mask(TileWalkShared<kW, kStageVec>& sm, int buf, bool has, int j, int X0,
-                                           int Y0, int first_block, uint8_t* lo_dst, uint8_t* hi_dst) {
+                                           int Y0, int first_block, uint32_t* rows, int row_words, int words) {
   float2 m = make_float2(0.f, 0.f);
   float hy = 0.f;
   float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -277,7 +203,7 @@ __device__ __forceinline__ void stage_mask(TileWalkShared<kW, kStageVec>& sm, in
     hy = s[2].w;
     c = s[3];
   }
-  publish_mask(sm, buf, has, m.x, m.y, hy, c, j, X0, Y0, first_block, lo_dst, hi_dst);
+  publish_mask(sm, buf, has, m.x, m.y, hy, c, j, X0, Y0, first_block, rows, row_words, words);
 }
 
 }  // namespace w2w
