@@ -63,9 +63,9 @@ __device__ __forceinline__ void segment_of(int walk, int k, int& lo, int& hi) {
 }
 
 // ---------------------------------------------------------------------------
-// Per-pixel pass.  One warp per 8x4 pixel block (of two in a CTA; warps never
-// wait for one another), walking its block's part of the tile's list back to
-// front, the entries its block mask names packed into groups of 32:
+// Per-pixel pass.  One warp, and one CTA, per 8x4 pixel block, walking its
+// block's part of the tile's list back to front, the entries its block mask
+// names packed into groups of 32:
 //
 //   1. lane j gathers entry j's record (the next group's loads are in flight
 //      while this one is evaluated) and puts it in shared memory;
@@ -83,13 +83,20 @@ __device__ __forceinline__ void segment_of(int walk, int k, int& lo, int& hi) {
 // instructions per entry; a shuffle tree per entry (ten values through 21
 // shuffles per pair of entries, with their products computed per pixel) cost
 // about 60, and groups of 32 mask-selected entries replace list chunks of 32
-// of which a quarter were evaluated.  Two-warp CTAs give a block's slot back
-// when it ends; an eight-warp CTA held its registers until the slowest of its
-// blocks had ended.
+// of which a quarter were evaluated.  Four entries are evaluated together: their
+// exponentials and reciprocals overlap, and only the chain of T and B runs
+// through them (two together: 128.8 us per view against 119.3, 500k Gaussians,
+// 512x512).  One-warp CTAs give a block's slot back when it ends; an eight-warp
+// CTA held its registers until the slowest of its blocks had ended (two warps:
+// 125.5 us, four: 139.6 with two entries together).  Sixteen CTAs per SM (128
+// registers): 283 us at 1M / 1024x1024 and 336 us for a 12-view batch, against
+// 299 and 359 at 150 registers; the busiest warps' chain, which a full SM slows,
+// makes 500k / 512x512 124 us against 119.
 // ---------------------------------------------------------------------------
-constexpr int kBwdWarps = 2;               // blocks (warps) per CTA
+constexpr int kBwdWarps = 1;               // blocks (warps) per CTA
 constexpr int kBwdParts = 8 / kBwdWarps;   // CTAs per tile (and segment)
 constexpr int kGroup = 32;                 // entries per group, one per lane
+constexpr int kIlp = 4;                    // entries evaluated together
 
 // A warp's shared memory.  The rows of `uw` are one pair longer than the
 // group, so that reading down a column touches every bank once.
@@ -219,15 +226,13 @@ struct BwdPixel {
 };
 
 // The reference's pair test and Gaussian value: power from the conic, skipped
-// when positive or (certainly) below alpha 1/255, alpha = min(0.99, o G).
-__device__ __forceinline__ bool ref_eval(float4 q0, float4 q1, float4 q2, float pxf, float pyf, float& dx, float& dy,
-                                         float& G, float& alpha) {
-  dx = q0.x - pxf;
-  dy = q0.y - pyf;
+// when positive or below alpha 1/255, alpha = min(0.99, o G).
+__device__ __forceinline__ bool ref_eval(float4 q0, float4 q1, float pxf, float pyf, float& G, float& alpha) {
+  const float dx = q0.x - pxf, dy = q0.y - pyf;
   const float power = -0.5f * (q0.z * dx * dx + q1.x * dy * dy) - q0.w * dx * dy;
   G = expf(power);
   alpha = fminf(0.99f, q1.y * G);
-  return power <= 0.0f && power >= q2.z && alpha >= 1.0f / 255.0f;
+  return power <= 0.0f && alpha >= 1.0f / 255.0f;
 }
 
 // Reference formulas (backward.cu:552-663) for one pixel; records
@@ -246,34 +251,35 @@ struct RefChain {
   }
   static __device__ __forceinline__ const float* records(const BackwardArgs& a) { return a.bwd_record; }
 
-  // Two entries, in order (has1: the second exists); u, w of each.  T in
-  // [~1e-4, 1] (the forward stops before T < 1e-4) and 1 - alpha in [0.01, 1]:
-  // the division is in div_markstein's range, which equals /.  kFull false:
-  // state only (the entries behind a split tile's segment).
+  // kIlp entries, in order, at e (past the group's end: records that contribute
+  // nothing); o: u, w of each.  The evaluations are independent and overlap;
+  // only T and B run through the entries.  kFull false: state only (the entries
+  // behind a split tile's segment).
   template <bool kFull>
-  __device__ __forceinline__ void pair(const float4* e0, const float4* e1, bool has1, const BwdPixel& p, float pxf,
-                                       float pyf, float2& o0, float2& o1) {
-    const float4 a0 = e0[0], a1 = e0[1], a2 = e0[2], b0 = e1[0], b1 = e1[1], b2 = e1[2];
-    float dx, dy, G0, al0, G1, al1;
-    const bool ok0 = ref_eval(a0, a1, a2, pxf, pyf, dx, dy, G0, al0) && __float_as_uint(a2.w) < p.last;
-    const bool ok1 = ref_eval(b0, b1, b2, pxf, pyf, dx, dy, G1, al1) && has1 && __float_as_uint(b2.w) < p.last;
-    step<kFull>(ok0, p, a1, a2, G0, al0, o0);
-    step<kFull>(ok1, p, b1, b2, G1, al1, o1);
-  }
-  template <bool kFull>
-  __device__ __forceinline__ void step(bool ok, const BwdPixel& p, float4 q1, float4 q2, float G, float alpha,
-                                       float2& o) {
-    const float y = rcp_markstein(1.f - alpha);
-    const float Tn = div_markstein_y(T, 1.f - alpha, y);
-    float q = q1.w * p.dLp0 + q2.x * p.dLp1 + q2.y * p.dLp2;
-    if constexpr (kDA) q += q1.z * p.dLd + p.dLa;
-    const float d = q - B;
-    // alpha <= 0.99 and T finite keep both factors finite; G itself may be
-    // infinite where the entry is skipped
-    if constexpr (kFull) o = make_float2(ok ? G * (d * Tn - tf_bg * y) : 0.f, ok ? alpha * Tn : 0.f);
-    if (ok) {
-      T = Tn;
-      B += alpha * d;
+  __device__ __forceinline__ void step(const float4* e, const BwdPixel& p, float pxf, float pyf, float2 (&o)[kIlp]) {
+    float G[kIlp], al[kIlp], y[kIlp], q[kIlp];
+    bool ok[kIlp];
+#pragma unroll
+    for (int k = 0; k < kIlp; ++k) {
+      const float4 q0 = e[kRecVec * k], q1 = e[kRecVec * k + 1], q2 = e[kRecVec * k + 2];
+      ok[k] = ref_eval(q0, q1, pxf, pyf, G[k], al[k]) && __float_as_uint(q2.w) < p.last;
+      y[k] = rcp_markstein(1.f - al[k]);
+      q[k] = q1.w * p.dLp0 + q2.x * p.dLp1 + q2.y * p.dLp2;
+      if constexpr (kDA) q[k] += q1.z * p.dLd + p.dLa;
+    }
+#pragma unroll
+    for (int k = 0; k < kIlp; ++k) {
+      // T / (1 - alpha), T in [~1e-4, 1] (the forward stops before T < 1e-4)
+      // and 1 - alpha in [0.01, 1]: the quotient from the correctly rounded
+      // reciprocal and one remainder correction
+      const float t = T * y[k], Tn = fma(fma(-(1.f - al[k]), t, T), y[k], t);
+      const float d = q[k] - B;
+      // alpha <= 0.99 and T finite keep both factors finite; G itself may be
+      // infinite where the entry is skipped
+      if constexpr (kFull)
+        o[k] = make_float2(ok[k] ? G[k] * (d * Tn - tf_bg * y[k]) : 0.f, ok[k] ? al[k] * Tn : 0.f);
+      T = ok[k] ? Tn : T;
+      B = ok[k] ? B + al[k] * d : B;
     }
   }
 
@@ -345,43 +351,47 @@ struct ExactChain {
   }
   static __device__ __forceinline__ const float* records(const BackwardArgs& a) { return a.record; }
 
+  // As RefChain::step.  u = dL/dalpha g: nothing passes the 0.99 clamp (a
+  // negative mahalanobis distance, mapped to 1000 by the forward, has g = 0).
   template <bool kFull>
-  __device__ __forceinline__ void pair(const float4* e0, const float4* e1, bool has1, const BwdPixel& p, float pxf,
-                                       float pyf, float2& o0, float2& o1) {
-    const float4 a0 = e0[0], a1 = e0[1], a2 = e0[2], b0 = e1[0], b1 = e1[1], b2 = e1[2];
-    // the forward's Gaussian values of the two entries (same division as the blend)
-    const float n0 = gauss_num_fwd(pxf, pyf, a0.x, a0.y, a0.z, a0.w, a1.x);
-    const float n1 = gauss_num_fwd(pxf, pyf, b0.x, b0.y, b0.z, b0.w, b1.x);
-    float m0, m1;
-    if (__all_sync(0xffffffffu, div_in_range(n0, a1.y) && div_in_range(n1, b1.y))) {
-      m0 = div_markstein(n0, a1.y);
-      m1 = div_markstein(n1, b1.y);
-    } else {
-      m0 = div(n0, a1.y);
-      m1 = div(n1, b1.y);
+  __device__ __forceinline__ void step(const float4* e, const BwdPixel& p, float pxf, float pyf, float2 (&o)[kIlp]) {
+    float num[kIlp], det[kIlp], opac[kIlp], q[kIlp];
+    bool ok[kIlp], in_range = true;
+#pragma unroll
+    for (int k = 0; k < kIlp; ++k) {
+      const float4 q0 = e[kRecVec * k], q1 = e[kRecVec * k + 1], q2 = e[kRecVec * k + 2];
+      num[k] = gauss_num_fwd(pxf, pyf, q0.x, q0.y, q0.z, q0.w, q1.x);
+      det[k] = q1.y;
+      opac[k] = q1.z;
+      in_range = in_range && div_in_range(num[k], q1.y);
+      q[k] = q2.x * p.dLp0 + q2.y * p.dLp1 + q2.z * p.dLp2 + q1.w * p.dLd + p.dLa;
+      ok[k] = __float_as_uint(q2.w) < p.last;
     }
-    const float g0 = expf(mul(-0.5f, m0 < 0.0f ? 1000.0f : m0));
-    const float g1 = expf(mul(-0.5f, m1 < 0.0f ? 1000.0f : m1));
-    const float og0 = mul(a1.z, g0), og1 = mul(b1.z, g1);
-    const float al0 = fminf(0.99f, og0), al1 = fminf(0.99f, og1);
-    const bool ok0 = al0 >= 1.0f / 255.0f && __float_as_uint(a2.w) < p.last;
-    const bool ok1 = al1 >= 1.0f / 255.0f && has1 && __float_as_uint(b2.w) < p.last;
-    step<kFull>(ok0, p, a1, a2, g0, og0, al0, o0);
-    step<kFull>(ok1, p, b1, b2, g1, og1, al1, o1);
-  }
-  // u = dL/dalpha g: nothing passes the 0.99 clamp (a negative mahalanobis
-  // distance, mapped to 1000 by the forward, has g = 0)
-  template <bool kFull>
-  __device__ __forceinline__ void step(bool ok, const BwdPixel& p, float4 q1, float4 q2, float g, float og, float al,
-                                       float2& o) {
-    const float ia = rcp_markstein(1.0f - al);  // 1 - alpha in [0.01, 1]
-    const float Tn = T * ia;                    // transmittance in front of this entry
-    const float aT = al * Tn;
-    const float q = q2.x * p.dLp0 + q2.y * p.dLp1 + q2.z * p.dLp2 + q1.w * p.dLd + p.dLa;
-    if constexpr (kFull) o = make_float2(ok && og < 0.99f ? (q * Tn - D * ia) * g : 0.f, ok ? aT : 0.f);
-    if (ok) {
-      T = Tn;
-      D += q * aT;
+    // the forward's Gaussian values (same division as the blend)
+    float m[kIlp], g[kIlp], og[kIlp], ia[kIlp];
+    if (__all_sync(0xffffffffu, in_range)) {
+#pragma unroll
+      for (int k = 0; k < kIlp; ++k) m[k] = div_markstein(num[k], det[k]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < kIlp; ++k) m[k] = div(num[k], det[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < kIlp; ++k) {
+      g[k] = expf(mul(-0.5f, m[k] < 0.0f ? 1000.0f : m[k]));
+      og[k] = mul(opac[k], g[k]);
+      ok[k] = ok[k] && og[k] >= 1.0f / 255.0f;
+      ia[k] = rcp_markstein(1.0f - fminf(0.99f, og[k]));  // 1 - alpha in [0.01, 1]
+    }
+#pragma unroll
+    for (int k = 0; k < kIlp; ++k) {
+      const float al = fminf(0.99f, og[k]);
+      const float Tn = T * ia[k];  // transmittance in front of this entry
+      const float aT = al * Tn;
+      if constexpr (kFull)
+        o[k] = make_float2(ok[k] && og[k] < 0.99f ? (q[k] * Tn - D * ia[k]) * g[k] : 0.f, ok[k] ? aT : 0.f);
+      T = ok[k] ? Tn : T;
+      D = ok[k] ? D + q[k] * aT : D;
     }
   }
 
@@ -453,7 +463,7 @@ __device__ __forceinline__ int item_tile(const BackwardArgs& a, int b, int& seg)
 }
 
 template <typename Chain, int kSplitWays>
-__global__ void __launch_bounds__(32 * kBwdWarps) render_bwd_kernel(BackwardArgs a) {
+__global__ void __launch_bounds__(32 * kBwdWarps, 16 / kBwdWarps) render_bwd_kernel(BackwardArgs a) {
   __shared__ BwdWarp s_warp[kBwdWarps];
   int seg;
   const int tile = item_tile<kSplitWays>(a, int(blockIdx.x) / kBwdParts, seg);
@@ -517,13 +527,12 @@ __global__ void __launch_bounds__(32 * kBwdWarps) render_bwd_kernel(BackwardArgs
       gather(g, pos, id, n);             // the next group's records and
       n = n > 0 ? pack(pos, id) : 0;     // the ids of the one after it are in flight below
       __syncwarp();
-      for (int j = 0; j < count; j += 2) {
-        const bool has1 = j + 1 < count;
-        float2 o0, o1;
-        ch.template pair<kFull>(s.rec + kRecVec * j, s.rec + kRecVec * (has1 ? j + 1 : j), has1, p, pxf, pyf, o0, o1);
+      for (int j = 0; j < count; j += kIlp) {
+        float2 o[kIlp];
+        ch.template step<kFull>(s.rec + kRecVec * j, p, pxf, pyf, o);
         if constexpr (kFull) {
-          s.uw[j][lane] = o0;
-          s.uw[j + 1][lane] = o1;
+#pragma unroll
+          for (int k = 0; k < kIlp; ++k) s.uw[j + k][lane] = o[k];
         }
       }
       __syncwarp();
