@@ -142,8 +142,8 @@ struct BlockWalk {
         const uint32_t id = __ldg(list + pos);
         if (id < num_records) {
           const float4* r = reinterpret_cast<const float4*>(record) + 4 * size_t(id);
-          const float4 r0 = __ldg(r), r2 = __ldg(r + 2), r3 = __ldg(r + 3);
-          reach = block_test(r0.x, r0.y, r2.w, r3.x, r3.y, r3.z, r3.w, bx, by);
+          const float4 r0 = __ldg(r), r1 = __ldg(r + 1);  // the blend's record
+          reach = block_test(r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, bx, by);
         }
       }
       b = __ballot_sync(0xffffffffu, reach);
@@ -235,7 +235,7 @@ __device__ __forceinline__ bool ref_eval(float4 q0, float4 q1, float pxf, float 
   return power <= 0.0f && alpha >= 1.0f / 255.0f;
 }
 
-// Reference formulas (backward.cu:552-663) for one pixel; records
+// Reference formulas (backward.cu:552-663) for one pixel; slots
 // (mx, my, conic a, conic b), (conic c, opacity, depth, r), (g, b, skip, position).
 // The reference keeps the colour, depth and alpha composited behind the current
 // entry per channel and multiplies their differences by the upstream planes;
@@ -249,7 +249,13 @@ struct RefChain {
     T = tf;
     tf_bg = tf * (p.bg[0] * p.dLp0 + p.bg[1] * p.dLp1 + p.bg[2] * p.dLp2);
   }
-  static __device__ __forceinline__ const float* records(const BackwardArgs& a) { return a.bwd_record; }
+  // Gaussian id's record as its slot's three float4s
+  static __device__ __forceinline__ void gather(const BackwardArgs& a, uint32_t id, float4& r0, float4& r1, float4& r2) {
+    const float4* r = reinterpret_cast<const float4*>(a.bwd_record) + 4 * size_t(id);
+    r0 = __ldg(r);
+    r1 = __ldg(r + 1);
+    r2 = __ldg(r + 2);
+  }
 
   // kIlp entries, in order, at e (past the group's end: records that contribute
   // nothing); o: u, w of each.  The evaluations are independent and overlap;
@@ -339,7 +345,7 @@ __device__ __forceinline__ float gauss_num_fwd(float px, float py, float mx, flo
   return s2<BL_NUM>(tX, dx, tY, dy);
 }
 
-// Exact derivative of the forward blend for one pixel; records
+// Exact derivative of the forward blend for one pixel; slots
 // (mx, my, cxx, cxy), (cyy, det, opacity, depth), (r, g, b, position).  The
 // suffix sums behind the current entry (colour including the background,
 // depth, weight) enter only through their upstream-weighted sum D.
@@ -349,7 +355,13 @@ struct ExactChain {
     T = p.inside ? a.T_final[p.pix] : 0.0f;
     D = T * (p.bg[0] * p.dLp0 + p.bg[1] * p.dLp1 + p.bg[2] * p.dLp2);
   }
-  static __device__ __forceinline__ const float* records(const BackwardArgs& a) { return a.record; }
+  static __device__ __forceinline__ void gather(const BackwardArgs& a, uint32_t id, float4& r0, float4& r1, float4& r2) {
+    const float4* r = reinterpret_cast<const float4*>(a.record) + 4 * size_t(id);
+    const float4 m = __ldg(r), o = __ldg(r + 1), c = __ldg(r + 2), dc = __ldg(r + 3);
+    r0 = make_float4(m.x, m.y, c.x, c.y);
+    r1 = make_float4(c.z, c.w, o.w, dc.x);
+    r2 = make_float4(dc.y, dc.z, dc.w, 0.f);
+  }
 
   // As RefChain::step.  u = dL/dalpha g: nothing passes the 0.99 clamp (a
   // negative mahalanobis distance, mapped to 1000 by the forward, has g = 0).
@@ -476,13 +488,12 @@ __global__ void __launch_bounds__(32 * kBwdWarps, 16 / kBwdWarps) render_bwd_ker
   Chain ch(a, p);
   const float pxf = float(p.tp.px), pyf = float(p.tp.py);
   const float hW = 0.5f * float(p.W), hH = 0.5f * float(p.H);
-  const float4* records = reinterpret_cast<const float4*>(Chain::records(a));
   const uint32_t* list = a.point_list + p.range.x;
   BlockWalk walk;
   // the blend's block masks, when this binning state has them
   const bool use_masks = a.masks_valid != nullptr && *a.masks_valid != 0u;
   walk.words = use_masks ? a.masks + mask_row(p.range.x, tile, int(p.range.y - p.range.x), block) : nullptr;
-  walk.record = Chain::records(a);
+  walk.record = a.record;
   walk.list = list;
   walk.num_records = uint32_t(a.P);
   walk.bx = p.tp.bx;
@@ -502,12 +513,7 @@ __global__ void __launch_bounds__(32 * kBwdWarps, 16 / kBwdWarps) render_bwd_ker
     g.id = id;
     g.count = n;
     g.r0 = g.r1 = g.r2 = make_float4(0.f, 0.f, 0.f, 0.f);  // opacity 0: contributes nothing
-    if (id < uint32_t(a.P)) {
-      const float4* r = records + 4 * size_t(id);
-      g.r0 = __ldg(r);
-      g.r1 = __ldg(r + 1);
-      g.r2 = __ldg(r + 2);
-    }
+    if (id < uint32_t(a.P)) Chain::gather(a, id, g.r0, g.r1, g.r2);
     g.r2.w = __uint_as_float(id < uint32_t(a.P) ? pos : ~0u);  // past every pixel's last contributor
   };
   auto run = [&](int lo, int top, auto full) {

@@ -1,12 +1,12 @@
 // Per-tile front-to-back alpha blending (reference pixelGaussiansFull.cu:3-98,
 // pixelGaussiansDev.cuh:5-96, gaussEval.h:7-29).
 //
-// One CTA per 16x16 tile, one thread per pixel, one warp per 8x4 pixel block
-// (tile_walk.cuh).  Each warp walks only the list entries that can reach its
-// block with alpha >= 1/255, kBlendIlp at a time: all their Gaussian values are
-// evaluated before the sequential transmittance/colour updates, so the
-// evaluations overlap.  The CTA stops as soon as every pixel of the tile has
-// terminated (the reference keeps loading every batch of the tile).
+// One warp per 8x4 pixel block (tile_walk.cuh), one thread per pixel.  Each
+// warp walks the tile's list on its own, tests every entry against its block,
+// evaluates the ones that can reach it with alpha >= 1/255, 32 at a time (all
+// their alphas at the block's pixels before the sequential transmittance and
+// colour updates), and stops when its pixels have all terminated (the
+// reference keeps loading every batch of the tile).
 //
 // Per pixel the arithmetic is the reference's, in its operation order: the
 // Gaussian is evaluated from the 2-D covariance and its determinant
@@ -25,8 +25,7 @@
 namespace w2w {
 namespace {
 
-constexpr int kBlendIlp = 4;  // list entries evaluated together per warp (the list is read 4 bytes at a time)
-static_assert(kBlendIlp == 4, "packed list read");
+constexpr int kBlendIlp = 4;  // list entries the queue-fed blend evaluates together per warp
 
 // The reference's Gaussian value (gaussEval.h:7-29) in two halves: the
 // mahalanobis numerator, then exp(-0.5 * num / det) with negative distances
@@ -48,50 +47,164 @@ struct BlendPixel {
   uint32_t last = 0;
   bool done;
 
-  // Entry with alpha `al` (record words q1, q2), 1-based list position `pos`.
+  // Eight entries of the list in order: alphas `v` (0 where an entry is skipped
+  // or the pixel has terminated), depths and colours dc[k]; `at` becomes e + k of
+  // the last one blended.  Only the transmittance runs through them: it never
+  // grows, so the entry that would take it below 1e-4 and all after it are the
+  // ones whose product lies below, and their weight is 0.
+  __device__ __forceinline__ void step(const float (&v)[8], const float4* dc, int e, int& at) {
+    float t = T;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float nT = mul(t, sub(1.0f, v[k]));
+      const bool alive = nT >= 0.0001f;
+      const float aT = alive ? mul(v[k], t) : 0.0f;
+      const float4 q = dc[k];
+      C0 = fma(q.y, aT, C0);
+      C1 = fma(q.z, aT, C1);
+      C2 = fma(q.w, aT, C2);
+      Wt = add(Wt, aT);
+      D = s1<fp::BL_DEPTH>(q.x, aT, D);
+      T = alive ? nT : T;
+      at = aT > 0.0f ? e + k : at;
+      t = nT;
+    }
+    done = done || t < 0.0001f;
+  }
+
+  // Entry with alpha `al` and depth and colour `dc`, 1-based list position `pos`.
   // Branch-free: the updates are selected, so a warp's lanes never diverge.
   // An entry that does not accumulate adds exactly zero: its weight aT is
   // selected to 0, colours and depth are finite, and C, Wt and D are never
   // -0 (non-negative colours and weights, positive depths), so x + c * 0 = x.
-  __device__ __forceinline__ void step(float al, float4 q1, float4 q2, uint32_t pos) {
+  __device__ __forceinline__ void step(float al, float4 dc, uint32_t pos) {
     const bool blend = !done && al >= 1.0f / 255.0f;
     const float nT = mul(T, sub(1.0f, al));
     const bool term = blend && nT < 0.0001f;
     const bool acc = blend && !term;
     const float aT = acc ? mul(al, T) : 0.0f;
-    C0 = fma(q2.x, aT, C0);
-    C1 = fma(q2.y, aT, C1);
-    C2 = fma(q2.z, aT, C2);
+    C0 = fma(dc.y, aT, C0);
+    C1 = fma(dc.z, aT, C1);
+    C2 = fma(dc.w, aT, C2);
     Wt = add(Wt, aT);
-    D = s1<fp::BL_DEPTH>(q1.w, aT, D);
+    D = s1<fp::BL_DEPTH>(dc.x, aT, D);
     T = acc ? nT : T;
     last = acc ? pos : last;
     done = done || term;
   }
 };
 
-// Warps per CTA, kBlendWarps: 8 (one CTA per tile) or 4 (two CTAs per tile,
-// upper and lower eight rows; see tile_walk.cuh), chosen at run time (the
-// tuning knob "blend_warps"); kAsync: the next batch is copied into shared
-// memory with cp.async instead of gathered into registers (the knob
-// "blend_stage"), which leaves the 4-warp CTA few enough registers for five
-// CTAs per SM instead of four.  Results are identical in every combination.
-template <int kBlendWarps, bool kAsync>
-constexpr int blend_min_blocks() {
-  return kAsync && kBlendWarps == 4 ? 5 : 16 / kBlendWarps;
+// kBlendIlp Gaussian values' alphas at one pixel: entry k's position and
+// opacity (mx, my, opacity) and its covariance (cxx, cxy, cyy, det).
+// Warp-collective: the branch-free division when every lane's operands allow it.
+__device__ __forceinline__ void blend_alphas(const float4 (&m)[kBlendIlp], const float4 (&cov)[kBlendIlp], float pxf,
+                                             float pyf, float (&al)[kBlendIlp]) {
+  float num[kBlendIlp], d[kBlendIlp];
+  bool in_range = true;
+#pragma unroll
+  for (int k = 0; k < kBlendIlp; ++k) {
+    num[k] = gauss_num(pxf, pyf, m[k].x, m[k].y, cov[k].x, cov[k].y, cov[k].z);
+    in_range = in_range && div_in_range(num[k], cov[k].w);
+  }
+  if (__all_sync(0xffffffffu, in_range)) {
+#pragma unroll
+    for (int k = 0; k < kBlendIlp; ++k) d[k] = div_markstein(num[k], cov[k].w);
+  } else {
+#pragma unroll
+    for (int k = 0; k < kBlendIlp; ++k) d[k] = div(num[k], cov[k].w);
+  }
+#pragma unroll
+  for (int k = 0; k < kBlendIlp; ++k) al[k] = fminf(0.99f, mul(m[k].z, gauss_from_m(d[k])));
 }
 
-template <int kBlendWarps, bool kAsync>
-__global__ void __launch_bounds__(32 * kBlendWarps, (blend_min_blocks<kBlendWarps, kAsync>()))
-    blend_kernel(BlendArgs a) {
-  constexpr int kBlendParts = 8 / kBlendWarps;  // CTAs per tile
-  constexpr int kBlendCta = 32 * kBlendWarps;
-  constexpr int kStagePer = kBatch / kBlendCta;  // entries each thread stages per batch
-  constexpr int kVec = kAsync ? kStageVec : kRecVec;  // float4s per staged record
-  static_assert(kBatch % kBlendCta == 0, "whole entries per thread");
-  __shared__ TileWalkShared<kBlendWarps, kVec> sm;
-  const int part = int(blockIdx.x) % kBlendParts;
-  const int tile = int(a.order[blockIdx.x / kBlendParts]);
+constexpr int kBlendWarps = 1;      // blocks (warps) per CTA
+constexpr int kBlendResident = 16;  // warps per SM the registers are sized for
+constexpr int kTestChunks = 4;      // 32-entry chunks tested together
+constexpr int kRing = 256;          // waiting entries: a group of 32, up to 31 after it and 128 newly tested
+constexpr int kAlphaStride = 36;    // floats per pixel row of the alpha table: rows start on 16 bytes, 8 rows cover the banks
+
+// A warp's shared memory.
+struct __align__(16) BlendWarp {
+  float alpha[33 * kAlphaStride];  // [pixel of the block][entry of the group], and a row of zeros
+  float4 dc[32];                   // the group's depths and colours
+  uint2 ring[kRing];               // entries that can reach the block: (id, 1-based list position)
+};
+
+// A lane's entry of the group to evaluate next: its record.
+struct BlendEntry {
+  float4 m, c, dc;  // (mx, my, opacity, _), (cxx, cxy, cyy, det), (depth, r, g, b)
+};
+
+// Alphas of a group's entries at the block's 32 pixels, into the alpha table (0
+// where an entry is skipped): up to 32 / kLanes entries, a lane per entry and
+// 4 / kLanes pixel rows.  The entry stays in the lane's registers, so its
+// reciprocal determinant and the per-row and per-column products are computed
+// once; a row's pixels go through each stage together, so their divisions and
+// exponentials overlap.
+//
+// Per value the arithmetic is gauss_num's and gauss_from_m's, with the quotient
+// by the determinant from div_markstein and its sign from the numerator.  Both
+// hold while the determinant and the variances are in [2^-20, 2^20] and the
+// mean is not within 2^-12 of a pixel in both coordinates without being on it:
+// then a numerator is 0 or above 2^-126 in magnitude (each of its two nested
+// sums of products cancels to no less than 2^-47 of its terms), its quotient
+// does not underflow, and one too small for div_markstein's range still gives
+// exp(-quotient / 2) = 1.  Any other entry is evaluated with the IEEE division.
+template <int kLanes>
+__device__ __forceinline__ void group_alphas(BlendWarp& s, const BlendEntry& en, float bx, float by) {
+  constexpr int kEntries = 32 / kLanes, kRows = 4 / kLanes;
+  const int lane = int(threadIdx.x & 31u), e = lane % kEntries, r0 = (lane / kEntries) * kRows;
+  float* out = s.alpha + 8 * r0 * kAlphaStride + e;
+  const float4 m = en.m, c = en.c;
+  const float y = rcp_markstein(c.w);
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) {
+    float num[8], g[8];
+#pragma unroll
+    for (int col = 0; col < 8; ++col)
+      num[col] = gauss_num(bx + float(col), by + float(r0 + r), m.x, m.y, c.x, c.y, c.z);
+#pragma unroll
+    for (int col = 0; col < 8; ++col) g[col] = div_markstein_y(num[col], c.w, y);
+#pragma unroll
+    for (int col = 0; col < 8; ++col) g[col] = expf(mul(-0.5f, g[col]));
+#pragma unroll
+    for (int col = 0; col < 8; ++col) {
+      const float al = fminf(0.99f, mul(m.z, g[col]));
+      out[(8 * r + col) * kAlphaStride] = al >= 1.0f / 255.0f && !(num[col] < 0.0f) ? al : 0.0f;
+    }
+  }
+  const float fx = fabsf(m.x - rintf(m.x)), fy = fabsf(m.y - rintf(m.y));
+  auto in = [](float v) { return v >= 0x1p-20f && v <= 0x1p20f; };
+  if (!(in(c.w) && in(c.x) && in(c.z) && fabsf(m.x) <= 0x1p24f && fabsf(m.y) <= 0x1p24f &&
+        (fmaxf(fx, fy) >= 0x1p-12f || fmaxf(fx, fy) == 0.0f))) {
+#pragma unroll 1
+    for (int p = 0; p < 8 * kRows; ++p) {
+      const float num = gauss_num(bx + float(p & 7), by + float(r0 + (p >> 3)), m.x, m.y, c.x, c.y, c.z);
+      const float al = fminf(0.99f, mul(m.z, gauss_from_m(div(num, c.w))));
+      out[p * kAlphaStride] = al >= 1.0f / 255.0f ? al : 0.0f;
+    }
+  }
+}
+
+// One CTA per kBlendWarps blocks of a tile; its warps never wait for one
+// another.  A warp tests the tile's entries against its block 128 at a time
+// (four per lane; the next 128 entries' culling sectors, and the ids of the 128
+// after them, are in flight meanwhile) and queues the ones that can reach it;
+// the ballots of the tests are the block's mask words for the backward.  It
+// takes them from the queue 32 at a time: every lane evaluates one entry at all
+// 32 pixels (group_alphas), the next group's records are requested, and then
+// every lane runs its pixel through the group's alphas.
+//
+// What bounds it: at 500k Gaussians instruction issue (about 24 instructions
+// per entry and 32 pixels for the alphas, 16 for the pixels' chains, 1.3 per
+// tested entry); at small scenes, and at the end of large ones, the busiest
+// warp's chain.
+__global__ void __launch_bounds__(32 * kBlendWarps, kBlendResident / kBlendWarps) blend_kernel(BlendArgs a) {
+  constexpr int kParts = 8 / kBlendWarps;  // CTAs per tile
+  __shared__ BlendWarp s_warp[kBlendWarps];
+  const int tile = int(a.order[blockIdx.x / kParts]);
+  const int warp = int(threadIdx.x >> 5);
+  const int block = (int(blockIdx.x) % kParts) * kBlendWarps + warp;
   // this tile's image: the call's, or its batch item's
   int W = a.W, H = a.H, ltile = tile;
   size_t pbase = 0;
@@ -104,96 +217,122 @@ __global__ void __launch_bounds__(32 * kBlendWarps, (blend_min_blocks<kBlendWarp
     pbase = size_t(it.pix_base);
     bg = it.bg;
   }
-  const int gw = (W + kTile - 1) / kTile;
-  const int warp = int(threadIdx.x >> 5), first_block = part * kBlendWarps;
-  const TilePixel tp(ltile, gw, first_block + warp);
+  const TilePixel tp(ltile, (W + kTile - 1) / kTile, block);
+  const int lane = tp.lane;
   const bool inside = tp.px < W && tp.py < H;
   const uint2 range = a.ranges[tile];
   const int n = int(range.y - range.x);
-  const float pxf = float(tp.px), pyf = float(tp.py);
+  const uint32_t* ids = a.point_list + range.x;
+  const float4* records = reinterpret_cast<const float4*>(a.record);
+  uint32_t* row = a.masks == nullptr ? nullptr : a.masks + mask_row(range.x, tile, n, block);
+  BlendWarp& s = s_warp[warp];
+  const uint32_t lt = lanemask_lt();
+  s.alpha[32 * kAlphaStride + lane] = 0.0f;
 
   BlendPixel pix;
   pix.done = !inside;
-  const int nb = (n + kBatch - 1) / kBatch;
-  Staged st[kAsync ? 1 : kStagePer];    // register staging: the batch in flight
-  bool staged[kAsync ? kStagePer : 1];  // cp.async staging: slot r * kBlendCta + threadIdx.x holds a record
-  auto load = [&](int buf, int base) {
+  bool done = __all_sync(0xffffffffu, pix.done) != 0;
+  const int chunks = done ? 0 : (n + 31) >> 5;
+  // the culling sectors of the chunks to test next (lane j: entry j of each),
+  // their ids and the ids of the chunks after them.  An id of num_records or
+  // more (a list left inconsistent by a sort whose bounded wait ran out, which
+  // its error word reports) is skipped, never read.
+  uint32_t id[kTestChunks], id_next[kTestChunks];
+  float4 t0[kTestChunks], t1[kTestChunks];
+  auto load_ids = [&](int c) {
 #pragma unroll
-    for (int r = 0; r < kStagePer; ++r) {
-      const int j = r * kBlendCta + int(threadIdx.x), e = base + j;
-      if constexpr (kAsync)
-        staged[r] = stage_copy(&sm.rec[buf][kVec * j], a.record, a.point_list, range.x + e, e < n, a.num_records);
-      else
-        stage_load(st[r], a.record, a.point_list, range.x + e, e < n, a.num_records);
-    }
-    if constexpr (kAsync) cp_async_commit();
-  };
-  // this CTA's rows of block-mask words for the backward (mask_row)
-  const int row_words = (n + 31) >> 5;
-  uint32_t* rows = a.masks == nullptr ? nullptr : a.masks + mask_row(range.x, tile, n, first_block);
-  auto store = [&](int buf, int base) {
-    if constexpr (kAsync) cp_async_wait_all();
-#pragma unroll
-    for (int r = 0; r < kStagePer; ++r) {
-      const int j = r * kBlendCta + int(threadIdx.x);
-      uint32_t* dst = rows ? rows + (base >> 5) : nullptr;
-      const int words = row_words - (base >> 5);
-      if constexpr (kAsync) stage_mask(sm, buf, staged[r], j, tp.X0, tp.Y0, first_block, dst, row_words, words);
-      else stage_store(sm, buf, st[r], j, tp.X0, tp.Y0, first_block, dst, row_words, words);
+    for (int q = 0; q < kTestChunks; ++q) {
+      const int e = 32 * (c + q) + lane;
+      id_next[q] = e < n ? __ldg(ids + e) : ~0u;
     }
   };
-  if (nb > 0) {
-    load(0, 0);
-    store(0, 0);
-  }
-  for (int b = 0; b < nb; ++b) {
-    const int cur = b & 1;
-    // barrier: batch b is staged; every warp has finished batch b-1
-    if (__syncthreads_count(pix.done ? 1 : 0) == kBlendCta) break;
-    const int next_base = (b + 1) * kBatch;
-    if (b + 1 < nb) load(cur ^ 1, next_base);  // in flight while batch b is walked
-    if (!__all_sync(0xffffffffu, pix.done)) {
-      const float4* s = sm.rec[cur];
-      const int cnt = build_list(sm, cur, warp, tp.lane);
-      const uint8_t* lst = sm.list[warp];
-      const uint32_t base = uint32_t(b * kBatch) + 1u;
-      for (int k0 = 0; k0 < cnt; k0 += kBlendIlp) {
-        // kBlendIlp entries in flight: their Gaussian values are independent,
-        // only the transmittance/colour updates are sequential
-        const uint32_t packed = *reinterpret_cast<const uint32_t*>(lst + k0);
-        int j[kBlendIlp];
+  auto load_tests = [&]() {
 #pragma unroll
-        for (int k = 0; k < kBlendIlp; ++k) j[k] = k0 + k < cnt ? int((packed >> (8 * k)) & 255u) : -1;
-        float al[kBlendIlp], num[kBlendIlp], m[kBlendIlp];
-        float4 q1[kBlendIlp], q2[kBlendIlp];
-        bool in_range = true;
-#pragma unroll
-        for (int k = 0; k < kBlendIlp; ++k) {
-          const int jj = j[k] < 0 ? j[0] : j[k];
-          const float4 q0 = s[kVec * jj];
-          q1[k] = s[kVec * jj + 1];
-          q2[k] = s[kVec * jj + 2];
-          num[k] = gauss_num(pxf, pyf, q0.x, q0.y, q0.z, q0.w, q1[k].x);
-          in_range = in_range && div_in_range(num[k], q1[k].y);
-        }
-        // the branch-free division when every lane's operands allow it
-        if (__all_sync(0xffffffffu, in_range)) {
-#pragma unroll
-          for (int k = 0; k < kBlendIlp; ++k) m[k] = div_markstein(num[k], q1[k].y);
-        } else {
-#pragma unroll
-          for (int k = 0; k < kBlendIlp; ++k) m[k] = div(num[k], q1[k].y);
-        }
-#pragma unroll
-        for (int k = 0; k < kBlendIlp; ++k)
-          al[k] = j[k] < 0 ? 0.0f : fminf(0.99f, mul(q1[k].z, gauss_from_m(m[k])));
-#pragma unroll
-        for (int k = 0; k < kBlendIlp; ++k) pix.step(al[k], q1[k], q2[k], base + uint32_t(j[k]));
-        if (__all_sync(0xffffffffu, pix.done)) break;
+    for (int q = 0; q < kTestChunks; ++q) {
+      id[q] = id_next[q];
+      t0[q] = make_float4(0.f, 0.f, -1.f, 0.f);  // hy < 0: reaches nothing
+      t1[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (id[q] < a.num_records) {
+        t0[q] = __ldg(records + 4 * size_t(id[q]));
+        t1[q] = __ldg(records + 4 * size_t(id[q]) + 1);
       }
     }
-    if (b + 1 < nb) store(cur ^ 1, next_base);
+  };
+  int c = 0;                    // next chunk to test
+  uint32_t head = 0, tail = 0;  // queue: [head, tail)
+  uint32_t word = 0;            // lane l: the mask word of chunk 32 * (c / 32) + l
+  // Tests chunks until 32 entries wait or the list ends.
+  auto refill = [&]() {
+    while (tail - head < 32u && c < chunks) {
+#pragma unroll
+      for (int q = 0; q < kTestChunks; ++q) {
+        const bool reach = block_test(t0[q].x, t0[q].y, t0[q].z, t0[q].w, t1[q].x, t1[q].y, t1[q].z, tp.bx, tp.by);
+        const uint32_t bits = __ballot_sync(0xffffffffu, reach);
+        if (lane == ((c + q) & 31)) word = bits;
+        if (reach) s.ring[(tail + __popc(bits & lt)) & (kRing - 1)] = make_uint2(id[q], uint32_t(32 * (c + q) + lane + 1));
+        tail += __popc(bits);
+      }
+      c += kTestChunks;
+      load_tests();
+      load_ids(c + kTestChunks);
+      // a full set of 32 words, or the list's last ones
+      if (row != nullptr && ((c & 31) == 0 || c >= chunks)) {
+        const int w = ((c - 1) & ~31) + lane;
+        if (w < chunks) row[w] = word;
+      }
+    }
+    __syncwarp();
+  };
+  // The lane's entry of the next group: `count` entries from `head`, spread over the lanes as group_alphas wants them.
+  BlendEntry en;
+  auto load_group = [&](int count) {
+    const int e = count > 16 ? lane : count > 8 ? lane & 15 : lane & 7;
+    // past the count: opacity 0, so alpha 0, and operands in group_alphas' range
+    en.m = make_float4(-1024.f, -1024.f, 0.f, 0.f);
+    en.c = make_float4(1.f, 0.f, 1.f, 1.f);
+    en.dc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (e < count) {
+      const float4* r = records + 4 * size_t(s.ring[(head + uint32_t(e)) & (kRing - 1)].x);
+      en.m = __ldg(r);
+      en.m.z = __ldg(reinterpret_cast<const float*>(r) + 7);
+      en.c = __ldg(r + 2);
+      en.dc = __ldg(r + 3);
+    }
+  };
+  int count = 0;
+  if (chunks > 0) {
+    load_ids(0);
+    load_tests();
+    load_ids(kTestChunks);
+    refill();
+    count = int(min(tail - head, 32u));
+    load_group(count);
   }
+  while (count > 0 && !done) {
+    if (count > 16) group_alphas<1>(s, en, float(tp.bx), float(tp.by));
+    else if (count > 8) group_alphas<2>(s, en, float(tp.bx), float(tp.by));
+    else group_alphas<4>(s, en, float(tp.bx), float(tp.by));
+    s.dc[lane] = en.dc;
+    const uint32_t first = head;
+    head += uint32_t(count);
+    refill();  // synchronises the warp
+    const int next = int(min(tail - head, 32u));
+    load_group(next);
+    const float* mine = s.alpha + (pix.done ? 32 : lane) * kAlphaStride;  // a terminated pixel: zeros
+    int at = -1;  // this pixel's last blended entry of the group
+    for (int e = 0; e < count; e += 8) {
+      const float4 a0 = *reinterpret_cast<const float4*>(mine + e), a1 = *reinterpret_cast<const float4*>(mine + e + 4);
+      const float v[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+      pix.step(v, s.dc + e, e, at);
+      if (pix.done) mine = s.alpha + 32 * kAlphaStride;
+    }
+    if (at >= 0) pix.last = s.ring[(first + uint32_t(at)) & (kRing - 1)].y;
+    done = __all_sync(0xffffffffu, pix.done) != 0;
+    __syncwarp();
+    count = next;
+  }
+  // the mask words not yet written (the backward reads none past the last contributor)
+  if (row != nullptr && (c & 31) != 0 && c < chunks && lane < (c & 31)) row[(c & ~31) + lane] = word;
   if (inside) {
     const size_t q = size_t(tp.py) * W + tp.px;
     const size_t p = pbase + q, cp = 3 * pbase + q;
@@ -207,17 +346,9 @@ __global__ void __launch_bounds__(32 * kBlendWarps, (blend_min_blocks<kBlendWarp
     a.out_color[2 * hw + cp] = fma(pix.T, bg[2], pix.C2);
   }
   // largest contributor count in the tile (the backward starts there); the
-  // tile's CTAs combine theirs (tile_max is cleared before the launch)
-  __shared__ uint32_t s_max[kBlendWarps];
+  // tile's warps combine theirs (tile_max is cleared before the launch)
   const uint32_t wm = __reduce_max_sync(0xffffffffu, pix.last);
-  if (tp.lane == 0) s_max[warp] = wm;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t mx = 0;
-    for (int w = 0; w < kBlendWarps; ++w) mx = max(mx, s_max[w]);
-    if (kBlendParts == 1) a.tile_max[tile] = mx;
-    else atomicMax(&a.tile_max[tile], mx);
-  }
+  if (lane == 0 && wm != 0u) atomicMax(&a.tile_max[tile], wm);
 }
 
 // ---------------------------------------------------------------------------
@@ -486,8 +617,8 @@ __global__ void __launch_bounds__(32 * (kW + 1)) blend_queue_kernel(BlendArgs a,
         bool reach = false;
         if ((vw >> lane) & 1u) {
           const int j = 32 * c + lane;
-          const float4 r0 = sr[kQRec * j], r2 = sr[kQRec * j + 2], r3 = sr[kQRec * j + 3];
-          reach = block_test(r0.x, r0.y, r2.w, r3.x, r3.y, r3.z, r3.w, tp.bx, tp.by);
+          const float4 r0 = sr[kQRec * j], r1 = sr[kQRec * j + 1];
+          reach = block_test(r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, tp.bx, tp.by);
         }
         const uint32_t bits = __ballot_sync(0xffffffffu, reach);
         if (reach) s.list[warp][cnt + __popc(bits & lt)] = uint8_t(32 * c + lane);
@@ -501,30 +632,21 @@ __global__ void __launch_bounds__(32 * (kW + 1)) blend_queue_kernel(BlendArgs a,
         int j[kBlendIlp];
 #pragma unroll
         for (int kk = 0; kk < kBlendIlp; ++kk) j[kk] = k0 + kk < cnt ? int((packed >> (8 * kk)) & 255u) : -1;
-        float al[kBlendIlp], num[kBlendIlp], m[kBlendIlp];
-        float4 q1[kBlendIlp], q2[kBlendIlp];
-        bool in_range = true;
+        float al[kBlendIlp];
+        float4 m[kBlendIlp], cov[kBlendIlp];
 #pragma unroll
         for (int kk = 0; kk < kBlendIlp; ++kk) {
           const int jj = j[kk] < 0 ? j[0] : j[kk];
-          const float4 q0 = sr[kQRec * jj];
-          q1[kk] = sr[kQRec * jj + 1];
-          q2[kk] = sr[kQRec * jj + 2];
-          num[kk] = gauss_num(pxf, pyf, q0.x, q0.y, q0.z, q0.w, q1[kk].x);
-          in_range = in_range && div_in_range(num[kk], q1[kk].y);
+          m[kk] = sr[kQRec * jj];
+          m[kk].z = sr[kQRec * jj + 1].w;
+          cov[kk] = sr[kQRec * jj + 2];
         }
-        if (__all_sync(0xffffffffu, in_range)) {
+        blend_alphas(m, cov, pxf, pyf, al);
 #pragma unroll
-          for (int kk = 0; kk < kBlendIlp; ++kk) m[kk] = div_markstein(num[kk], q1[kk].y);
-        } else {
-#pragma unroll
-          for (int kk = 0; kk < kBlendIlp; ++kk) m[kk] = div(num[kk], q1[kk].y);
+        for (int kk = 0; kk < kBlendIlp; ++kk) {
+          const int jj = j[kk] < 0 ? j[0] : j[kk];
+          pix.step(j[kk] < 0 ? 0.0f : al[kk], sr[kQRec * jj + 3], base + uint32_t(j[kk]));
         }
-#pragma unroll
-        for (int kk = 0; kk < kBlendIlp; ++kk)
-          al[kk] = j[kk] < 0 ? 0.0f : fminf(0.99f, mul(q1[kk].z, gauss_from_m(m[kk])));
-#pragma unroll
-        for (int kk = 0; kk < kBlendIlp; ++kk) pix.step(al[kk], q1[kk], q2[kk], base + uint32_t(j[kk]));
         if (__all_sync(0xffffffffu, pix.done)) break;
       }
     }
@@ -643,22 +765,15 @@ void launch_blend(const BlendArgs& a, cudaStream_t stream) {
   const int tiles = a.items ? a.total_tiles : ((a.W + kTile - 1) / kTile) * ((a.H + kTile - 1) / kTile);
   if (tiles <= 0) return;
   const int warps = tune_value(kTuneBlendWarps);
-  const bool async = tune_value(kTuneBlendStage) == 1;
   const bool queue = tune_value(kTuneBlendQueue) == 1 && a.queue != nullptr;
   stage_begin(kStOther, stream);
-  // with two CTAs per tile (or the queue) the tile's maxima combine with
-  // atomics: clear first; the queue counter starts at zero
-  tile_order_kernel<<<1, 1024, 0, stream>>>(a.ranges, nullptr, tiles, a.order,
-                                            (warps == 4 || queue) ? a.tile_max : nullptr, queue ? a.queue : nullptr);
+  // a tile's warps combine their contributor counts in its maximum: clear
+  // first; the queue counter starts at zero
+  tile_order_kernel<<<1, 1024, 0, stream>>>(a.ranges, nullptr, tiles, a.order, a.tile_max, queue ? a.queue : nullptr);
   stage_end(kStOther, stream, 1);
   stage_begin(kStBlend, stream);
   const bool queued = queue && (warps == 4 ? launch_queue<4>(a, tiles, stream) : launch_queue<8>(a, tiles, stream));
-  if (!queued) {
-    if (warps == 4 && async) blend_kernel<4, true><<<tiles * 2, 128, 0, stream>>>(a);
-    else if (warps == 4) blend_kernel<4, false><<<tiles * 2, 128, 0, stream>>>(a);
-    else if (async) blend_kernel<8, true><<<tiles, 256, 0, stream>>>(a);
-    else blend_kernel<8, false><<<tiles, 256, 0, stream>>>(a);
-  }
+  if (!queued) blend_kernel<<<tiles * (8 / kBlendWarps), 32 * kBlendWarps, 0, stream>>>(a);
   stage_end(kStBlend, stream, 1);
   // the backward's order: by the largest contributor count the blend just found
   stage_begin(kStOther, stream);

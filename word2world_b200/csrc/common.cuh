@@ -226,18 +226,18 @@ __device__ __forceinline__ bool block_test(float mx, float my, float hy, float b
 }
 
 // ---------------------------------------------------------------------------
-// Per-Gaussian blend record (forward blend and exact backward), 64 bytes.
-// The first 48 bytes are what the per-pixel loops read from shared memory;
-// the last 20 are the block-culling parameters.
+// Per-Gaussian blend record (forward blend and exact backward), 64 bytes: one
+// 32-byte sector with what a block's culling test reads (and the opacity), one
+// with what only the evaluation of an entry that passed it reads.
 // ---------------------------------------------------------------------------
 struct __align__(16) BlendRecord {
   float mx, my;          // screen position (pixels)
+  float hy, beta, gamma, eps, vr;  // CullParams
+  float opacity;
   float cxx, cxy, cyy;   // 2-D covariance
   float det;             // the blend's own determinant of the covariance
-  float opacity;
   float depth;           // NDC z
   float r, g, b;         // colour (unclamped)
-  float hy, beta, gamma, eps, vr;  // CullParams
 };
 static_assert(sizeof(BlendRecord) == 64, "BlendRecord layout");
 

@@ -418,10 +418,10 @@ preprocess_kernel(PreprocessArgs a) {
       cp = make_cull_params(g.conic[0], g.conic[1], g.conic[2], opacity);
     }
     float4* rp = reinterpret_cast<float4*>(a.record) + 4 * size_t(i);
-    rp[0] = make_float4(rec.mx, rec.my, rec.cxx, rec.cxy);
-    rp[1] = make_float4(rec.cyy, rec.det, rec.opacity, rec.depth);
-    rp[2] = make_float4(rec.r, rec.g, rec.b, cp.hy);
-    rp[3] = make_float4(cp.beta, cp.gamma, cp.eps, cp.vr);
+    rp[0] = make_float4(rec.mx, rec.my, cp.hy, cp.beta);
+    rp[1] = make_float4(cp.gamma, cp.eps, cp.vr, rec.opacity);
+    rp[2] = make_float4(rec.cxx, rec.cxy, rec.cyy, rec.det);
+    rp[3] = make_float4(rec.depth, rec.r, rec.g, rec.b);
     float4* bp = reinterpret_cast<float4*>(a.bwd_record) + 4 * size_t(i);
     if (g.visible) {
       bp[0] = make_float4(g.mx, g.my, g.conic[0], g.conic[1]);
