@@ -253,8 +253,7 @@ __global__ void __launch_bounds__(32 * kBlendWarps, kBlendResident / kBlendWarps
       t0[q] = make_float4(0.f, 0.f, -1.f, 0.f);  // hy < 0: reaches nothing
       t1[q] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (id[q] < a.num_records) {
-        t0[q] = __ldg(records + 4 * size_t(id[q]));
-        t1[q] = __ldg(records + 4 * size_t(id[q]) + 1);
+        ldg32(records + 4 * size_t(id[q]), t0[q], t1[q]);
       }
     }
   };
@@ -293,10 +292,10 @@ __global__ void __launch_bounds__(32 * kBlendWarps, kBlendResident / kBlendWarps
     en.dc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (e < count) {
       const float4* r = records + 4 * size_t(s.ring[(head + uint32_t(e)) & (kRing - 1)].x);
-      en.m = __ldg(r);
-      en.m.z = __ldg(reinterpret_cast<const float*>(r) + 7);
-      en.c = __ldg(r + 2);
-      en.dc = __ldg(r + 3);
+      float4 o;
+      ldg32(r, en.m, o);
+      en.m.z = o.w;
+      ldg32(r + 2, en.c, en.dc);
     }
   };
   int count = 0;
