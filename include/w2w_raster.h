@@ -462,15 +462,15 @@ int w2w_throughput_probe(int kind, long long iters, int blocks, float* out, long
  * (word2world_b200/autotune.py) from timings of the caller's workload.  No
  * counterpart in the reference, whose launch shapes are fixed
  * (pixelGaussiansFull.cu:99-122).  Knobs (w2w_tune_name): 0 "blend_warps"
- * (4: two 4-warp CTAs per tile, 8: one 8-warp CTA; default 4), 1
- * "backward_split" (the per-pixel backward splits its heaviest tiles, up to
- * this many quarters of the SM count, across CTAs; 0..16, default 2), 2
- * "backward_ways" (segments per split tile, 2 or 3; default 2), 3 "binning"
+ * (consumer warps per CTA of the queue-fed blend, 4: half a tile each, 8: a
+ * tile; default 4), 1 "backward_split" (0..16, default 2) and 2
+ * "backward_ways" (2 or 3, default 2) (accepted, without effect: the per-pixel
+ * backward runs one warp per 8x4 block of a tile and splits no walk), 3 "binning"
  * (how a single-view call of at most 4096 tiles builds its sorted list: 0
  * key emission and the radix sort, 1 binning from the depth-ordered
  * Gaussians; default 0; w2w_forward_geometry records the path taken in
  * w2w_geometry_info.reserved, bit 0, and w2w_forward_render follows it), 4
- * "blend_queue" (0: one CTA per tile part, launched heaviest first; 1: a
+ * "blend_queue" (0: one warp per 8x4 block of a tile, launched heaviest first; 1: a
  * persistent blend, one CTA per resident slot, pulling tile parts from a
  * device queue in the same order, each CTA a producer warp that gathers the
  * batches' records with TMA into a three-stage shared-memory ring and
@@ -479,9 +479,8 @@ int w2w_throughput_probe(int kind, long long iters, int blocks, float* out, long
  * 64 registers, 3 at 80, 2 at 128; default 4), 6 "planned_forward" (the torch
  * binding's planned forward for repeated image sizes, 1 on, 0 off; default 1;
  * not tuned, the C ABI's entry points take the plan explicitly), 7
- * "blend_stage" (how the per-tile blend gathers a batch's records while it
- * walks the previous one: 0 into registers, 1 into shared memory with
- * cp.async, which fits five 4-warp CTAs per SM instead of four; default 1).
+ * "blend_stage" (0 or 1, default 1; accepted, without effect: the per-tile
+ * blend has one way of gathering its records).
  * Results do not depend on them beyond the order of float atomic additions.
  * w2w_tune_set returns the previous value, or -1 (and changes nothing) for an
  * unknown knob or value. */

@@ -1,9 +1,8 @@
-"""Launch-shape autotuner: picks the library's tuning knobs (blend CTA shape,
-per-tile or persistent queue-fed blend, the blend's batch staging (registers
-or cp.async), how many heavy tiles the per-pixel backward splits and into how
-many segments, radix or depth-ordered binning, the projection pass's register
-budget) for a workload by timing it, and remembers the choice per shape
-bucket.
+"""Launch-shape autotuner: picks the library's tuning knobs (per-tile or
+persistent queue-fed blend and its consumer warps, radix or depth-ordered
+binning, the projection pass's register budget; backward_split, backward_ways
+and blend_stage are still accepted but select nothing) for a workload by
+timing it, and remembers the choice per shape bucket.
 
 The reference's launch shapes are constants (pixelGaussiansFull.cu:99-122,
 backward.cu:521-665).  Here they are run-time knobs of the C ABI

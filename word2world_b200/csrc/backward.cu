@@ -21,46 +21,8 @@
 #include "kernels.h"
 #include "tile_walk.cuh"
 
-#include <type_traits>
-
 namespace w2w {
 namespace {
-
-// Heavy tiles: each warp's walk is cut into kSplitWays segments, one CTA per
-// segment.  The CTA of a segment first replays the state recurrences of the
-// entries behind it (alpha and the transmittance / suffix updates only: no
-// gradients, no reduction, about kReplayCost of a full entry's work) to reach
-// the state at its segment's end, then walks its segment in full.  All CTAs
-// compute the state with the same code in the same order, so each starts from
-// exactly the state a single walk would have reached; only the order of the
-// atomic additions changes.  Segment lengths (from the back) make the
-// segments' work equal: L_0 = W, L_i = W - kReplayCost * (L_0 + ... + L_{i-1}).
-// kSplitWays (2 or 3) and the number of split tiles are run-time tuning
-// knobs (W2W_TUNE_BWD_WAYS, W2W_TUNE_BWD_SPLIT); only the order of the atomic
-// additions depends on them.
-constexpr float kReplayCost = 0.22f;
-
-// List positions [lo, hi) of segment k (0 = the back-most) of a walk of
-// length `walk`.
-template <int kSplitWays>
-__device__ __forceinline__ void segment_of(int walk, int k, int& lo, int& hi) {
-  float len[kSplitWays], before = 0.f, total = 0.f;
-#pragma unroll
-  for (int i = 0; i < kSplitWays; ++i) {
-    len[i] = 1.0f - kReplayCost * before;
-    before += len[i];
-  }
-  total = before;
-  float b0 = 0.f, b1 = 0.f;
-#pragma unroll
-  for (int i = 0; i < kSplitWays; ++i) {
-    if (i < k) b0 += len[i];
-    if (i <= k) b1 += len[i];
-  }
-  hi = walk - int(float(walk) * (b0 / total));
-  lo = k == kSplitWays - 1 ? 0 : walk - int(float(walk) * (b1 / total));
-  lo = max(0, min(lo, hi));
-}
 
 // ---------------------------------------------------------------------------
 // Per-pixel pass.  One warp, and one CTA, per 8x4 pixel block, walking its
@@ -68,127 +30,136 @@ __device__ __forceinline__ void segment_of(int walk, int k, int& lo, int& hi) {
 // names packed into groups of 32:
 //
 //   1. lane j gathers entry j's record (the next group's loads are in flight
-//      while this one is evaluated) and puts it in shared memory;
-//   2. every lane evaluates the group's entries in order for its pixel -- the
-//      transmittance chain -- and writes two numbers per pair: u, from which
-//      every geometric gradient of the pair follows, and w, the pair's colour
-//      weight;
-//   3. the 32 x 32 table of (u, w) is read across: lane j sums entry j over the
-//      block's 32 pixels (the moments of u over the pixel offsets, and w times
-//      each upstream plane), turns the sums into the entry's gradients and adds
-//      each with one atomic.
+//      while this one is worked on) and evaluates it at the block's 32 pixels:
+//      alpha and Gaussian value of every pair, 0 where the pair is skipped,
+//      into two 32 x 32 tables;
+//   2. every lane runs its pixel through the group's entries in order -- the
+//      transmittance chain, which needs no decisions: a skipped pair's alpha is
+//      0 -- and puts two numbers per pair in their place: u, from which every
+//      geometric gradient of the pair follows, and w, its colour weight;
+//   3. lane j sums entry j over the block's 32 pixels (the moments of u over the
+//      pixel offsets, and w times each upstream plane), turns the sums into the
+//      entry's gradients and adds each with one atomic.
+//
+// A group of up to 16 (8) entries spreads steps 1 and 3 over two (four) lanes
+// per entry.
 //
 // What bounds it: instruction issue, and for scenes that leave SMs idle the
-// busiest warp's chain.  Summing across the warp in step 3 costs about 12
-// instructions per entry; a shuffle tree per entry (ten values through 21
-// shuffles per pair of entries, with their products computed per pixel) cost
-// about 60, and groups of 32 mask-selected entries replace list chunks of 32
-// of which a quarter were evaluated.  Four entries are evaluated together: their
-// exponentials and reciprocals overlap, and only the chain of T and B runs
-// through them (two together: 128.8 us per view against 119.3, 500k Gaussians,
-// 512x512).  One-warp CTAs give a block's slot back when it ends; an eight-warp
-// CTA held its registers until the slowest of its blocks had ended (two warps:
-// 125.5 us, four: 139.6 with two entries together).  Sixteen CTAs per SM (128
-// registers): 283 us at 1M / 1024x1024 and 336 us for a 12-view batch, against
-// 299 and 359 at 150 registers; the busiest warps' chain, which a full SM slows,
-// makes 500k / 512x512 124 us against 119.
+// busiest warp's chain.  About 20 + 18 + 13 instructions per entry in the three
+// steps.  A shuffle tree per entry (ten values through 21 shuffles per pair of
+// entries, with their products computed per pixel) cost about 60 for step 3
+// alone; evaluating the pairs in step 2, four entries at a time, left the
+// busiest warps waiting for each one's exponential and reciprocal (119 us
+// against 96 per view at 500k / 512x512, 30 against 23 at 16k / 256x256).
+// One-warp CTAs give a block's slot back when it ends; an eight-warp CTA held
+// its registers until the slowest of its blocks had ended.  Cutting the
+// heaviest tiles' walks into segments, each replaying the chain behind it, no
+// longer pays: a replay costs steps 1 and 2, three quarters of the work (470
+// us per 4 views at 500k without, 678 with half an SM count of tiles cut).
 // ---------------------------------------------------------------------------
-constexpr int kBwdWarps = 1;               // blocks (warps) per CTA
-constexpr int kBwdParts = 8 / kBwdWarps;   // CTAs per tile (and segment)
-constexpr int kGroup = 32;                 // entries per group, one per lane
-constexpr int kIlp = 4;                    // entries evaluated together
+constexpr int kGroup = 32;        // entries per group
+constexpr int kSteps = 8;         // of them in flight through a pixel's chain
+constexpr int kWindow = 512;      // list positions whose mask bits are expanded together, 16 per lane
+constexpr int kTableStride = 36;  // floats per pixel row: rows start on 16 bytes, 8 rows cover the banks
 
-// A warp's shared memory.  The rows of `uw` are one pair longer than the
-// group, so that reading down a column touches every bank once.
+// A warp's shared memory.
 struct __align__(16) BwdWarp {
-  float4 rec[kGroup * kRecVec];  // the group's records; the third float4's w is the entry's list position
-  float4 up[32];                 // per pixel: upstream dL/dcolour and dL/ddepth
-  float2 uw[kGroup][33];
-  uint32_t slot[kGroup];         // list positions of the group being packed
+  float alpha[32 * kTableStride];  // [pixel of the block][entry of the group]: alpha, then w
+  float value[32 * kTableStride];  // the Gaussian value, then u
+  float4 up[32];                   // per pixel: upstream dL/dcolour and dL/ddepth
+  float4 dc[kGroup];               // per entry: depth and colour
+  uint32_t last[32];               // per pixel: contributor count
+  uint32_t queue[kWindow + kGroup];  // list positions waiting, highest first: under a group, and one window's
 };
 
 // Positions [lo, top) of a block's part of a tile's list, highest first, in
 // groups of up to 32.  words: the block's mask row, or null (each entry is
-// tested against the block here).
+// tested against the block here).  A lane expands 16 positions' bits of a
+// window at the offset a scan over the lanes gives it: about 80 instructions
+// per 512 positions, where taking the words one by one cost 40 per 32 and was
+// the longest walks' largest part (91k of 222k cycles).
 struct BlockWalk {
   const uint32_t* words;
   const float* record;
   const uint32_t* list;   // the tile's first list entry
   uint32_t num_records;
-  int bx, by, lo, top, wi, wb;
-  uint32_t bits, cache;
+  int bx, by, lo, top, window, head, tail;
+  uint32_t ahead;  // the lane's mask word of the next window to expand
 
-  __device__ __forceinline__ void start(int lo_, int top_) {
-    lo = lo_;
-    top = top_;
-    wi = ((top - 1) >> 5) + 1;  // words [0, wi) are still to come
-    wb = wi;
-    bits = 0;
-  }
-  // Word w's bits inside [lo, top).
-  __device__ __forceinline__ uint32_t word(int w) {
+  // Window w's mask word of this lane (two lanes share one).
+  __device__ __forceinline__ uint32_t load(int w) const {
     const int lane = threadIdx.x & 31;
-    uint32_t b;
-    if (words != nullptr) {
-      if (w < wb) {  // 32 words at a time, one per lane
-        wb = max(w - 31, 0);
-        cache = wb + lane <= w ? __ldg(words + wb + lane) : 0u;
-      }
-      b = __shfl_sync(0xffffffffu, cache, w - wb);
-    } else {
-      const int pos = 32 * w + lane;
+    const int i = w * (kWindow / 32) + (lane >> 1);
+    if (words != nullptr) return w >= (lo >> 9) && 32 * i < top ? __ldg(words + i) : 0u;
+    uint32_t mine = 0u;
+    for (int k = 0; k < kWindow / 32 && w >= (lo >> 9); ++k) {
+      const int pos = kWindow * w + 32 * k + lane;
       bool reach = false;
       if (pos >= lo && pos < top) {
         const uint32_t id = __ldg(list + pos);
         if (id < num_records) {
-          const float4* r = reinterpret_cast<const float4*>(record) + 4 * size_t(id);
-          const float4 r0 = __ldg(r), r1 = __ldg(r + 1);  // the blend's record
+          float4 r0, r1;  // the blend's record
+          ldg32(record + 16 * size_t(id), r0, r1);
           reach = block_test(r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, bx, by);
         }
       }
-      b = __ballot_sync(0xffffffffu, reach);
+      const uint32_t b = __ballot_sync(0xffffffffu, reach);
+      if ((lane >> 1) == k) mine = b;
     }
-    const int above = top - 32 * w, below = lo - 32 * w;
-    if (above < 32) b &= (1u << above) - 1u;
-    if (below > 0) b &= 0xffffffffu << below;
-    return b;
+    return mine;
   }
-  // Packs the next group's positions into slot[0, count), highest first.
-  // Warp-collective; the caller has synchronised the warp after its last read of slot.
-  __device__ __forceinline__ int next(uint32_t* slot) {
+  __device__ __forceinline__ void start(int lo_, int top_) {
+    static_assert(kWindow == 512, "window index");
+    lo = lo_;
+    top = top_;
+    head = tail = 0;
+    window = top > lo ? (top - 1) >> 9 : -1;
+    ahead = window >= 0 ? load(window) : 0u;
+  }
+  // Queues positions until a group waits or none are left; returns the next
+  // group's size (its positions: queue[head, head + size)).  Warp-collective;
+  // the caller has synchronised the warp after its last read of the queue.
+  __device__ __forceinline__ int fill(uint32_t* queue) {
     const int lane = threadIdx.x & 31;
-    int count = 0;
-    if (top <= lo) return 0;
-    const int first = lo >> 5;
-    while (true) {
-      if (bits == 0u) {
-        if (wi <= first) break;
-        bits = word(--wi);
-        continue;
+    while (tail - head < kGroup && window >= 0 && window >= (lo >> 9)) {
+      if (head > 0) {  // what waits moves to the front
+        const uint32_t v = head + lane < tail ? queue[head + lane] : 0u;
+        __syncwarp();
+        queue[lane] = v;
+        tail -= head;
+        head = 0;
+        __syncwarp();
       }
-      const int n = __popc(bits), room = kGroup - count;
-      const int rank = __popc((bits >> lane) >> 1);  // set bits above this lane's
-      const bool mine = (bits >> lane) & 1u;
-      if (mine && rank < room) slot[count + rank] = uint32_t(32 * wi + lane);
-      if (n > room) {
-        bits = __ballot_sync(0xffffffffu, mine && rank >= room);
-        count = kGroup;
-        break;
+      const int base = kWindow * window + 16 * lane;
+      uint32_t bits = (lane & 1) ? ahead >> 16 : ahead & 0xffffu;
+      if (top - base < 16) bits &= top > base ? (1u << (top - base)) - 1u : 0u;
+      if (lo - base > 0) bits &= lo - base < 16 ? 0xffffffffu << (lo - base) : 0u;
+      --window;
+      ahead = window >= 0 ? load(window) : 0u;
+      int n = __popc(bits), from = n;  // from: this lane's bits and those of the lanes above
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_down_sync(0xffffffffu, from, d);
+        if (lane + d < 32) from += o;
       }
-      count += n;
-      bits = 0u;
-      if (count == kGroup) break;
+      int at = tail + from - n;
+      while (bits != 0u) {
+        const int b = 31 - __clz(bits);
+        queue[at++] = uint32_t(base + b);
+        bits ^= 1u << b;
+      }
+      tail += __shfl_sync(0xffffffffu, from, 0);
     }
     __syncwarp();
-    return count;
+    return min(tail - head, kGroup);
   }
 };
 
-// Entry records of a group in flight: lane j's entry.
+// A group in flight: the lane's entry.
 struct GroupLoad {
-  float4 r0, r1, r2;
-  uint32_t id;
-  int count;
+  float4 q0, q1, q2;  // Chain::gather's
+  uint32_t id = ~0u, pos = ~0u;
+  int count = 0;
 };
 
 // Pixel-loop prologue shared by both modes: this thread's pixel, its
@@ -226,17 +197,32 @@ struct BwdPixel {
 };
 
 // The reference's pair test and Gaussian value: power from the conic, skipped
-// when positive or below alpha 1/255, alpha = min(0.99, o G).
+// when positive or below alpha 1/255, alpha = min(0.99, o G).  q0 = (mx, my,
+// conic a, conic b), q1 = (conic c, opacity, _, _).  The roundings of the
+// power are written out, so that a pair at a threshold is decided the same
+// whatever the compiler shares between the pixels of a row or a column: one
+// decided differently changes every gradient behind it by 1/255.
 __device__ __forceinline__ bool ref_eval(float4 q0, float4 q1, float pxf, float pyf, float& G, float& alpha) {
-  const float dx = q0.x - pxf, dy = q0.y - pyf;
-  const float power = -0.5f * (q0.z * dx * dx + q1.x * dy * dy) - q0.w * dx * dy;
+  const float dx = sub(q0.x, pxf), dy = sub(q0.y, pyf);
+  const float quad = fma(mul(q0.z, dx), dx, mul(mul(q1.x, dy), dy));
+  const float power = fma(-0.5f, quad, -mul(mul(q0.w, dx), dy));
   G = expf(power);
-  alpha = fminf(0.99f, q1.y * G);
+  alpha = fminf(0.99f, mul(q1.y, G));
   return power <= 0.0f && alpha >= 1.0f / 255.0f;
 }
 
-// Reference formulas (backward.cu:552-663) for one pixel; slots
-// (mx, my, conic a, conic b), (conic c, opacity, depth, r), (g, b, skip, position).
+// The ten (nine without a depth loss) sums of an entry over its lanes' pixels.
+constexpr int kSums = 10;
+template <int kLanes>
+__device__ __forceinline__ void combine_lanes(float (&v)[kSums]) {
+#pragma unroll
+  for (int d = 32 / kLanes; d < 32; d <<= 1)
+#pragma unroll
+    for (int k = 0; k < kSums; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], d);
+}
+
+// Reference formulas (backward.cu:552-663) for one pixel; entries (mx, my,
+// conic a, conic b), (conic c, opacity, depth, r), (g, b, _, _).
 // The reference keeps the colour, depth and alpha composited behind the current
 // entry per channel and multiplies their differences by the upstream planes;
 // the chain is linear in them, so one number serves: B, the upstream-weighted
@@ -249,67 +235,83 @@ struct RefChain {
     T = tf;
     tf_bg = tf * (p.bg[0] * p.dLp0 + p.bg[1] * p.dLp1 + p.bg[2] * p.dLp2);
   }
-  // Gaussian id's record as its slot's three float4s
-  static __device__ __forceinline__ void gather(const BackwardArgs& a, uint32_t id, float4& r0, float4& r1, float4& r2) {
-    const float4* r = reinterpret_cast<const float4*>(a.bwd_record) + 4 * size_t(id);
-    r0 = __ldg(r);
-    r1 = __ldg(r + 1);
-    r2 = __ldg(r + 2);
+  static __device__ __forceinline__ void gather(const BackwardArgs& a, GroupLoad& g) {
+    const float* r = a.bwd_record + 16 * size_t(g.id);
+    ldg32(r, g.q0, g.q1);
+    g.q2 = __ldg(reinterpret_cast<const float4*>(r) + 2);
+  }
+  static __device__ __forceinline__ float4 depth_colour(const GroupLoad& g) {
+    return make_float4(g.q1.z, g.q1.w, g.q2.x, g.q2.y);
+  }
+  template <int kLanes>
+  static __device__ __forceinline__ void evaluate(BwdWarp& s, const GroupLoad& g, float bx, float by) {
+    constexpr int kEntries = 32 / kLanes, kRows = 4 / kLanes;
+    const int lane = int(threadIdx.x & 31u), e = lane % kEntries, r0 = (lane / kEntries) * kRows;
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      const uint4 l0 = *reinterpret_cast<const uint4*>(s.last + 8 * (r0 + r));
+      const uint4 l1 = *reinterpret_cast<const uint4*>(s.last + 8 * (r0 + r) + 4);
+      const uint32_t last[8] = {l0.x, l0.y, l0.z, l0.w, l1.x, l1.y, l1.z, l1.w};
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        float G, alpha;
+        const bool ok = ref_eval(g.q0, g.q1, bx + float(c), by + float(r0 + r), G, alpha) && g.pos < last[c];
+        const int at = (8 * (r0 + r) + c) * kTableStride + e;
+        s.alpha[at] = ok ? alpha : 0.f;
+        s.value[at] = ok ? G : 0.f;
+      }
+    }
   }
 
-  // kIlp entries, in order, at e (past the group's end: records that contribute
-  // nothing); o: u, w of each.  The evaluations are independent and overlap;
-  // only T and B run through the entries.  kFull false: state only (the entries
-  // behind a split tile's segment).
-  template <bool kFull>
-  __device__ __forceinline__ void step(const float4* e, const BwdPixel& p, float pxf, float pyf, float2 (&o)[kIlp]) {
-    float G[kIlp], al[kIlp], y[kIlp], q[kIlp];
-    bool ok[kIlp];
+  // kSteps entries of the pixel's chain: alphas and values become w and u.  T
+  // in [~1e-4, 1] (the forward stops before T < 1e-4) and 1 - alpha in [0.01,
+  // 1]: T / (1 - alpha) from the correctly rounded reciprocal and one remainder
+  // correction; exactly T where alpha is 0.
+  __device__ __forceinline__ void steps(const BwdPixel& p, const float4* dc, float (&alpha)[kSteps],
+                                        float (&value)[kSteps]) {
+    float q[kSteps], y[kSteps];
 #pragma unroll
-    for (int k = 0; k < kIlp; ++k) {
-      const float4 q0 = e[kRecVec * k], q1 = e[kRecVec * k + 1], q2 = e[kRecVec * k + 2];
-      ok[k] = ref_eval(q0, q1, pxf, pyf, G[k], al[k]) && __float_as_uint(q2.w) < p.last;
-      y[k] = rcp_markstein(1.f - al[k]);
-      q[k] = q1.w * p.dLp0 + q2.x * p.dLp1 + q2.y * p.dLp2;
-      if constexpr (kDA) q[k] += q1.z * p.dLd + p.dLa;
+    for (int k = 0; k < kSteps; ++k) {
+      const float4 c = dc[k];
+      q[k] = c.y * p.dLp0 + c.z * p.dLp1 + c.w * p.dLp2;
+      if constexpr (kDA) q[k] += c.x * p.dLd + p.dLa;
+      y[k] = rcp_markstein(1.f - alpha[k]);
     }
 #pragma unroll
-    for (int k = 0; k < kIlp; ++k) {
-      // T / (1 - alpha), T in [~1e-4, 1] (the forward stops before T < 1e-4)
-      // and 1 - alpha in [0.01, 1]: the quotient from the correctly rounded
-      // reciprocal and one remainder correction
-      const float t = T * y[k], Tn = fma(fma(-(1.f - al[k]), t, T), y[k], t);
+    for (int k = 0; k < kSteps; ++k) {
+      const float t = T * y[k];
+      T = fma(fma(-(1.f - alpha[k]), t, T), y[k], t);
       const float d = q[k] - B;
-      // alpha <= 0.99 and T finite keep both factors finite; G itself may be
-      // infinite where the entry is skipped
-      if constexpr (kFull)
-        o[k] = make_float2(ok[k] ? G[k] * (d * Tn - tf_bg * y[k]) : 0.f, ok[k] ? al[k] * Tn : 0.f);
-      T = ok[k] ? Tn : T;
-      B = ok[k] ? B + al[k] * d : B;
+      B += alpha[k] * d;
+      value[k] *= d * T - tf_bg * y[k];
+      alpha[k] *= T;
     }
   }
 
-  // Lane j's entry over the block's 32 pixels, and its atomics.
-  static __device__ __forceinline__ void reduce(const BackwardArgs& a, const BwdWarp& s, int j, uint32_t id, float bx,
+  // The lane's entry over its pixels, and its atomics.
+  template <int kLanes>
+  static __device__ __forceinline__ void reduce(const BackwardArgs& a, const BwdWarp& s, const GroupLoad& g, float bx,
                                                 float by, float hW, float hH) {
-    const float4 q0 = s.rec[kRecVec * j], q1 = s.rec[kRecVec * j + 1];
+    constexpr int kEntries = 32 / kLanes, kRows = 4 / kLanes;
+    const int lane = int(threadIdx.x & 31u), e = lane % kEntries, r0 = (lane / kEntries) * kRows;
     float S = 0.f, Sx = 0.f, Sy = 0.f, Sxx = 0.f, Sxy = 0.f, Syy = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f, cd = 0.f;
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const float dy = q0.y - (by + float(r));
+    for (int r = 0; r < kRows; ++r) {
+      const float dy = g.q0.y - (by + float(r0 + r));
       float rs = 0.f, rx = 0.f;
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
-        const float2 uw = s.uw[j][8 * r + c];
-        const float4 up = s.up[8 * r + c];
-        const float dx = q0.x - (bx + float(c)), t = uw.x * dx;
-        rs += uw.x;
+        const int px = 8 * (r0 + r) + c;
+        const float u = s.value[px * kTableStride + e], w = s.alpha[px * kTableStride + e];
+        const float4 up = s.up[px];
+        const float dx = g.q0.x - (bx + float(c)), t = u * dx;
+        rs += u;
         rx += t;
         Sxx += t * dx;
-        c0 += uw.y * up.x;
-        c1 += uw.y * up.y;
-        c2 += uw.y * up.z;
-        if constexpr (kDA) cd += uw.y * up.w;
+        c0 += w * up.x;
+        c1 += w * up.y;
+        c2 += w * up.z;
+        if constexpr (kDA) cd += w * up.w;
       }
       S += rs;
       Sx += rx;
@@ -318,138 +320,124 @@ struct RefChain {
       Sy += t;
       Syy += t * dy;
     }
-    // no pixel of the block took the entry
-    if (S == 0.f && Sxx == 0.f && Syy == 0.f && c0 == 0.f && c1 == 0.f && c2 == 0.f && cd == 0.f) return;
-    const float h = -0.5f * q1.y;
-    atomicAdd(a.dL_dcolors + 3 * size_t(id), c0);
-    atomicAdd(a.dL_dcolors + 3 * size_t(id) + 1, c1);
-    atomicAdd(a.dL_dcolors + 3 * size_t(id) + 2, c2);
-    if constexpr (kDA) atomicAdd(a.acc_depth + id, cd);
-    atomicAdd(a.dL_dmean2D + 3 * size_t(id), -q1.y * hW * (q0.z * Sx + q0.w * Sy));
-    atomicAdd(a.dL_dmean2D + 3 * size_t(id) + 1, -q1.y * hH * (q1.x * Sy + q0.w * Sx));
-    atomicAdd(a.acc_cov + 4 * size_t(id), h * Sxx);
-    atomicAdd(a.acc_cov + 4 * size_t(id) + 1, h * Sxy);
-    atomicAdd(a.acc_cov + 4 * size_t(id) + 3, h * Syy);
-    atomicAdd(a.dL_dopacity + id, S);
+    float v[kSums] = {S, Sx, Sy, Sxx, Sxy, Syy, c0, c1, c2, cd};
+    combine_lanes<kLanes>(v);
+    // no pixel of the block took the entry (or the lane has none)
+    if (lane >= g.count || g.id >= uint32_t(a.P)) return;
+    if (v[0] == 0.f && v[3] == 0.f && v[5] == 0.f && v[6] == 0.f && v[7] == 0.f && v[8] == 0.f && v[9] == 0.f) return;
+    const float A = g.q0.z, B = g.q0.w, C = g.q1.x, o = g.q1.y, h = -0.5f * o;
+    const size_t id = g.id;
+    atomicAdd(a.dL_dcolors + 3 * id, v[6]);
+    atomicAdd(a.dL_dcolors + 3 * id + 1, v[7]);
+    atomicAdd(a.dL_dcolors + 3 * id + 2, v[8]);
+    if constexpr (kDA) atomicAdd(a.acc_depth + id, v[9]);
+    atomicAdd(a.dL_dmean2D + 3 * id, -o * hW * (A * v[1] + B * v[2]));
+    atomicAdd(a.dL_dmean2D + 3 * id + 1, -o * hH * (C * v[2] + B * v[1]));
+    atomicAdd(a.acc_cov + 4 * id, h * v[3]);
+    atomicAdd(a.acc_cov + 4 * id + 1, h * v[4]);
+    atomicAdd(a.acc_cov + 4 * id + 3, h * v[5]);
+    atomicAdd(a.dL_dopacity + id, v[0]);
   }
 };
 
-// The forward's Gaussian value (blend.cu), split at its division so that a
-// warp's divisions can run branch-free together.
-__device__ __forceinline__ float gauss_num_fwd(float px, float py, float mx, float my, float cxx, float cxy,
-                                               float cyy) {
-  using namespace fp;
-  const float dx = sub(px, mx), dy = sub(py, my);
-  const float tX = d2<BL_TX>(dx, cyy, dy, cxy);
-  const float tY = s2<BL_TY>(-dx, cxy, dy, cxx);
-  return s2<BL_NUM>(tX, dx, tY, dy);
-}
-
-// Exact derivative of the forward blend for one pixel; slots
-// (mx, my, cxx, cxy), (cyy, det, opacity, depth), (r, g, b, position).  The
-// suffix sums behind the current entry (colour including the background,
-// depth, weight) enter only through their upstream-weighted sum D.
+// Exact derivative of the forward blend for one pixel; entries (mx, my, opacity,
+// _), (cxx, cxy, cyy, det), (depth, r, g, b).  The suffix sums behind the
+// current entry (colour including the background, depth, weight) enter only
+// through their upstream-weighted sum D.
 struct ExactChain {
   float T, D;
   __device__ __forceinline__ ExactChain(const BackwardArgs& a, const BwdPixel& p) {
     T = p.inside ? a.T_final[p.pix] : 0.0f;
     D = T * (p.bg[0] * p.dLp0 + p.bg[1] * p.dLp1 + p.bg[2] * p.dLp2);
   }
-  static __device__ __forceinline__ void gather(const BackwardArgs& a, uint32_t id, float4& r0, float4& r1, float4& r2) {
-    const float4* r = reinterpret_cast<const float4*>(a.record) + 4 * size_t(id);
-    const float4 m = __ldg(r), o = __ldg(r + 1), c = __ldg(r + 2), dc = __ldg(r + 3);
-    r0 = make_float4(m.x, m.y, c.x, c.y);
-    r1 = make_float4(c.z, c.w, o.w, dc.x);
-    r2 = make_float4(dc.y, dc.z, dc.w, 0.f);
+  static __device__ __forceinline__ void gather(const BackwardArgs& a, GroupLoad& g) {
+    const float* r = a.record + 16 * size_t(g.id);
+    float4 o;
+    ldg32(r, g.q0, o);
+    g.q0.z = o.w;
+    ldg32(r + 8, g.q1, g.q2);
   }
-
-  // As RefChain::step.  u = dL/dalpha g: nothing passes the 0.99 clamp (a
-  // negative mahalanobis distance, mapped to 1000 by the forward, has g = 0).
-  template <bool kFull>
-  __device__ __forceinline__ void step(const float4* e, const BwdPixel& p, float pxf, float pyf, float2 (&o)[kIlp]) {
-    float num[kIlp], det[kIlp], opac[kIlp], q[kIlp];
-    bool ok[kIlp], in_range = true;
+  static __device__ __forceinline__ float4 depth_colour(const GroupLoad& g) { return g.q2; }
+  // The forward's own Gaussian values and decisions; the value is 0 where
+  // alpha is clamped to 0.99, past which no gradient goes.
+  template <int kLanes>
+  static __device__ __forceinline__ void evaluate(BwdWarp& s, const GroupLoad& g, float bx, float by) {
+    const int e = int(threadIdx.x & 31u) % (32 / kLanes);
+    gauss_values<kLanes>(g.q0.x, g.q0.y, g.q1, bx, by, [&](int p, float v) {
+      const float og = mul(g.q0.z, v);
+      const bool ok = og >= 1.0f / 255.0f && g.pos < s.last[p];
+      s.alpha[p * kTableStride + e] = ok ? fminf(0.99f, og) : 0.f;
+      s.value[p * kTableStride + e] = ok && og < 0.99f ? v : 0.f;
+    });
+  }
+  __device__ __forceinline__ void steps(const BwdPixel& p, const float4* dc, float (&alpha)[kSteps],
+                                        float (&value)[kSteps]) {
+    float q[kSteps], ia[kSteps];
 #pragma unroll
-    for (int k = 0; k < kIlp; ++k) {
-      const float4 q0 = e[kRecVec * k], q1 = e[kRecVec * k + 1], q2 = e[kRecVec * k + 2];
-      num[k] = gauss_num_fwd(pxf, pyf, q0.x, q0.y, q0.z, q0.w, q1.x);
-      det[k] = q1.y;
-      opac[k] = q1.z;
-      in_range = in_range && div_in_range(num[k], q1.y);
-      q[k] = q2.x * p.dLp0 + q2.y * p.dLp1 + q2.z * p.dLp2 + q1.w * p.dLd + p.dLa;
-      ok[k] = __float_as_uint(q2.w) < p.last;
-    }
-    // the forward's Gaussian values (same division as the blend)
-    float m[kIlp], g[kIlp], og[kIlp], ia[kIlp];
-    if (__all_sync(0xffffffffu, in_range)) {
-#pragma unroll
-      for (int k = 0; k < kIlp; ++k) m[k] = div_markstein(num[k], det[k]);
-    } else {
-#pragma unroll
-      for (int k = 0; k < kIlp; ++k) m[k] = div(num[k], det[k]);
+    for (int k = 0; k < kSteps; ++k) {
+      const float4 c = dc[k];
+      q[k] = c.y * p.dLp0 + c.z * p.dLp1 + c.w * p.dLp2 + c.x * p.dLd + p.dLa;
+      ia[k] = rcp_markstein(1.0f - alpha[k]);  // 1 - alpha in [0.01, 1]
     }
 #pragma unroll
-    for (int k = 0; k < kIlp; ++k) {
-      g[k] = expf(mul(-0.5f, m[k] < 0.0f ? 1000.0f : m[k]));
-      og[k] = mul(opac[k], g[k]);
-      ok[k] = ok[k] && og[k] >= 1.0f / 255.0f;
-      ia[k] = rcp_markstein(1.0f - fminf(0.99f, og[k]));  // 1 - alpha in [0.01, 1]
-    }
-#pragma unroll
-    for (int k = 0; k < kIlp; ++k) {
-      const float al = fminf(0.99f, og[k]);
-      const float Tn = T * ia[k];  // transmittance in front of this entry
-      const float aT = al * Tn;
-      if constexpr (kFull)
-        o[k] = make_float2(ok[k] && og[k] < 0.99f ? (q[k] * Tn - D * ia[k]) * g[k] : 0.f, ok[k] ? aT : 0.f);
-      T = ok[k] ? Tn : T;
-      D = ok[k] ? D + q[k] * aT : D;
+    for (int k = 0; k < kSteps; ++k) {
+      T *= ia[k];  // transmittance in front of this entry
+      value[k] *= q[k] * T - D * ia[k];
+      alpha[k] *= T;
+      D += q[k] * alpha[k];
     }
   }
 
   // With e = cyy dx - cxy dy and f = cxx dy - cxy dx (offsets from the mean),
   // d(num / det) = 2 (e, f) / det over the offsets and -(e e, 2 e f, f f) / det^2
   // over the covariance.
-  static __device__ __forceinline__ void reduce(const BackwardArgs& a, const BwdWarp& s, int j, uint32_t id, float bx,
+  template <int kLanes>
+  static __device__ __forceinline__ void reduce(const BackwardArgs& a, const BwdWarp& s, const GroupLoad& g, float bx,
                                                 float by, float hW, float hH) {
-    const float4 q0 = s.rec[kRecVec * j], q1 = s.rec[kRecVec * j + 1];
+    constexpr int kEntries = 32 / kLanes, kRows = 4 / kLanes;
+    const int lane = int(threadIdx.x & 31u), en = lane % kEntries, r0 = (lane / kEntries) * kRows;
     float S = 0.f, Se = 0.f, Sf = 0.f, See = 0.f, Sef = 0.f, Sff = 0.f, c0 = 0.f, c1 = 0.f, c2 = 0.f, cd = 0.f;
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const float dy = (by + float(r)) - q0.y, ey = -q0.w * dy, fy = q0.z * dy;
+    for (int r = 0; r < kRows; ++r) {
+      const float dy = (by + float(r0 + r)) - g.q0.y, ey = -g.q1.y * dy, fy = g.q1.x * dy;
 #pragma unroll
       for (int c = 0; c < 8; ++c) {
-        const float2 uw = s.uw[j][8 * r + c];
-        const float4 up = s.up[8 * r + c];
-        const float dx = (bx + float(c)) - q0.x;
-        const float e = q1.x * dx + ey, f = fy - q0.w * dx;
-        const float te = uw.x * e, tf = uw.x * f;
-        S += uw.x;
+        const int px = 8 * (r0 + r) + c;
+        const float u = s.value[px * kTableStride + en], w = s.alpha[px * kTableStride + en];
+        const float4 up = s.up[px];
+        const float dx = (bx + float(c)) - g.q0.x;
+        const float e = g.q1.z * dx + ey, f = fy - g.q1.y * dx;
+        const float te = u * e, tf = u * f;
+        S += u;
         Se += te;
         Sf += tf;
         See += te * e;
         Sef += te * f;
         Sff += tf * f;
-        c0 += uw.y * up.x;
-        c1 += uw.y * up.y;
-        c2 += uw.y * up.z;
-        cd += uw.y * up.w;
+        c0 += w * up.x;
+        c1 += w * up.y;
+        c2 += w * up.z;
+        cd += w * up.w;
       }
     }
-    if (S == 0.f && See == 0.f && Sff == 0.f && c0 == 0.f && c1 == 0.f && c2 == 0.f && cd == 0.f) return;
+    float v[kSums] = {S, Se, Sf, See, Sef, Sff, c0, c1, c2, cd};
+    combine_lanes<kLanes>(v);
+    if (lane >= g.count || g.id >= uint32_t(a.P)) return;
+    if (v[0] == 0.f && v[3] == 0.f && v[5] == 0.f && v[6] == 0.f && v[7] == 0.f && v[8] == 0.f && v[9] == 0.f) return;
     // det >= 0.09 (the forward's +0.3 low-pass on a positive semi-definite
     // covariance), where rcp_markstein is the correctly rounded 1/det
-    const float idet = rcp_markstein(q1.y), k1 = q1.z * idet, k2 = k1 * idet;
-    atomicAdd(a.dL_dcolors + 3 * size_t(id), c0);
-    atomicAdd(a.dL_dcolors + 3 * size_t(id) + 1, c1);
-    atomicAdd(a.dL_dcolors + 3 * size_t(id) + 2, c2);
-    atomicAdd(a.acc_depth + id, cd);
-    atomicAdd(a.dL_dmean2D + 3 * size_t(id), k1 * hW * Se);
-    atomicAdd(a.dL_dmean2D + 3 * size_t(id) + 1, k1 * hH * Sf);
-    atomicAdd(a.acc_cov + 4 * size_t(id), 0.5f * k2 * See);
-    atomicAdd(a.acc_cov + 4 * size_t(id) + 1, k2 * Sef);
-    atomicAdd(a.acc_cov + 4 * size_t(id) + 2, 0.5f * k2 * Sff);
-    atomicAdd(a.dL_dopacity + id, S);
+    const float idet = rcp_markstein(g.q1.w), k1 = g.q0.z * idet, k2 = k1 * idet;
+    const size_t id = g.id;
+    atomicAdd(a.dL_dcolors + 3 * id, v[6]);
+    atomicAdd(a.dL_dcolors + 3 * id + 1, v[7]);
+    atomicAdd(a.dL_dcolors + 3 * id + 2, v[8]);
+    atomicAdd(a.acc_depth + id, v[9]);
+    atomicAdd(a.dL_dmean2D + 3 * id, k1 * hW * v[1]);
+    atomicAdd(a.dL_dmean2D + 3 * id + 1, k1 * hH * v[2]);
+    atomicAdd(a.acc_cov + 4 * id, 0.5f * k2 * v[3]);
+    atomicAdd(a.acc_cov + 4 * id + 1, k2 * v[4]);
+    atomicAdd(a.acc_cov + 4 * id + 2, 0.5f * k2 * v[5]);
+    atomicAdd(a.dL_dopacity + id, v[0]);
   }
 };
 
@@ -461,32 +449,17 @@ __device__ __forceinline__ BwdPixel make_bwd_pixel(const BackwardArgs& a, int ti
   return BwdPixel(a, tile, tile - int(it.tile_base), block, it.W, it.H, size_t(it.pix_base), it.bg);
 }
 
-// Work item b's tile and segment: the first kSplitWays * split items are the
-// segments of the `split` heaviest tiles (segment 0..kSplitWays-1), the rest
-// one whole tile each (segment -1), heaviest first.
-template <int kSplitWays>
-__device__ __forceinline__ int item_tile(const BackwardArgs& a, int b, int& seg) {
-  if (b < kSplitWays * a.split) {
-    seg = b % kSplitWays;
-    return int(a.order_bwd[b / kSplitWays]);
-  }
-  seg = -1;
-  return int(a.order_bwd[b - (kSplitWays - 1) * a.split]);
-}
-
-template <typename Chain, int kSplitWays>
-__global__ void __launch_bounds__(32 * kBwdWarps, 16 / kBwdWarps) render_bwd_kernel(BackwardArgs a) {
-  __shared__ BwdWarp s_warp[kBwdWarps];
-  int seg;
-  const int tile = item_tile<kSplitWays>(a, int(blockIdx.x) / kBwdParts, seg);
-  const int warp = int(threadIdx.x >> 5), lane = int(threadIdx.x & 31);
-  const int block = (int(blockIdx.x) % kBwdParts) * kBwdWarps + warp;
+template <typename Chain>
+__global__ void __launch_bounds__(32, 16) render_bwd_kernel(BackwardArgs a) {
+  __shared__ BwdWarp s;
+  const int tile = int(a.order_bwd[blockIdx.x / 8]);  // heaviest first
+  const int lane = int(threadIdx.x), block = int(blockIdx.x) % 8;
   const BwdPixel p = make_bwd_pixel(a, tile, block);
-  if (p.walk <= 0) return;  // warp-uniform
-  BwdWarp& s = s_warp[warp];
+  if (p.walk <= 0) return;
   s.up[lane] = make_float4(p.dLp0, p.dLp1, p.dLp2, p.dLd);
+  s.last[lane] = p.last;
   Chain ch(a, p);
-  const float pxf = float(p.tp.px), pyf = float(p.tp.py);
+  const float bx = float(p.tp.bx), by = float(p.tp.by);
   const float hW = 0.5f * float(p.W), hH = 0.5f * float(p.H);
   const uint32_t* list = a.point_list + p.range.x;
   BlockWalk walk;
@@ -499,64 +472,62 @@ __global__ void __launch_bounds__(32 * kBwdWarps, 16 / kBwdWarps) render_bwd_ker
   walk.bx = p.tp.bx;
   walk.by = p.tp.by;
 
-  // Positions of the next group, and lane j's id in it (an id of num_records
-  // or more -- a list left inconsistent by a sort whose bounded wait ran out,
-  // which its error word reports -- is skipped, never read).
-  auto pack = [&](uint32_t& pos, uint32_t& id) {
+  // The next group's positions and ids (the lanes' entries as the chain's
+  // evaluate spreads them).  An id of num_records or more -- a list left
+  // inconsistent by a sort whose bounded wait ran out, which its error word
+  // reports -- is skipped, never read.
+  auto pack = [&](GroupLoad& g) {
     __syncwarp();
-    const int n = walk.next(s.slot);
-    pos = lane < n ? s.slot[lane] : 0u;
-    id = lane < n ? __ldg(list + pos) : ~0u;
-    return n;
+    g.count = walk.fill(s.queue);
+    const int e = g.count > 16 ? lane : g.count > 8 ? lane & 15 : lane & 7;
+    g.pos = e < g.count ? s.queue[walk.head + e] : ~0u;  // past every pixel's last contributor
+    walk.head += g.count;
+    g.id = e < g.count ? __ldg(list + g.pos) : ~0u;
   };
-  auto gather = [&](GroupLoad& g, uint32_t pos, uint32_t id, int n) {
-    g.id = id;
-    g.count = n;
-    g.r0 = g.r1 = g.r2 = make_float4(0.f, 0.f, 0.f, 0.f);  // opacity 0: contributes nothing
-    if (id < uint32_t(a.P)) Chain::gather(a, id, g.r0, g.r1, g.r2);
-    g.r2.w = __uint_as_float(id < uint32_t(a.P) ? pos : ~0u);  // past every pixel's last contributor
+  auto gather = [&](GroupLoad& g) {
+    // opacity 0, in gauss_values' range: contributes nothing
+    g.q0 = make_float4(-1024.f, -1024.f, 0.f, 0.f);
+    g.q1 = make_float4(1.f, 0.f, 1.f, 1.f);
+    g.q2 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (g.id < uint32_t(a.P)) Chain::gather(a, g);
+    else g.pos = ~0u;
   };
-  auto run = [&](int lo, int top, auto full) {
-    constexpr bool kFull = decltype(full)::value;
-    walk.start(lo, top);
-    GroupLoad g;
-    uint32_t pos, id;
-    int n = pack(pos, id);
-    gather(g, pos, id, n);
-    n = n > 0 ? pack(pos, id) : 0;
-    while (g.count > 0) {
-      const int count = g.count;
-      const uint32_t cur = g.id;
-      s.rec[kRecVec * lane] = g.r0;
-      s.rec[kRecVec * lane + 1] = g.r1;
-      s.rec[kRecVec * lane + 2] = g.r2;
-      gather(g, pos, id, n);             // the next group's records and
-      n = n > 0 ? pack(pos, id) : 0;     // the ids of the one after it are in flight below
-      __syncwarp();
-      for (int j = 0; j < count; j += kIlp) {
-        float2 o[kIlp];
-        ch.template step<kFull>(s.rec + kRecVec * j, p, pxf, pyf, o);
-        if constexpr (kFull) {
-#pragma unroll
-          for (int k = 0; k < kIlp; ++k) s.uw[j + k][lane] = o[k];
-        }
-      }
-      __syncwarp();
-      if constexpr (kFull) {
-        if (lane < count && cur < uint32_t(a.P))
-          Chain::reduce(a, s, lane, cur, float(p.tp.bx), float(p.tp.by), hW, hH);
-        __syncwarp();
-      }
+  walk.start(0, p.walk);
+  GroupLoad g, next;
+  pack(g);
+  gather(g);
+  if (g.count > 0) pack(next);
+  while (g.count > 0) {
+    const int count = g.count;
+    if (count > 16) Chain::template evaluate<1>(s, g, bx, by);
+    else if (count > 8) Chain::template evaluate<2>(s, g, bx, by);
+    else Chain::template evaluate<4>(s, g, bx, by);
+    s.dc[lane] = Chain::depth_colour(g);
+    GroupLoad after;
+    gather(next);                     // the next group's records and
+    if (next.count > 0) pack(after);  // the ids of the one after it are in flight below
+    __syncwarp();
+    float* al = s.alpha + lane * kTableStride;
+    float* va = s.value + lane * kTableStride;
+    for (int e = 0; e < count; e += kSteps) {
+      float4* xa = reinterpret_cast<float4*>(al + e);
+      float4* xv = reinterpret_cast<float4*>(va + e);
+      const float4 a0 = xa[0], a1 = xa[1], v0 = xv[0], v1 = xv[1];
+      float x[kSteps] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+      float v[kSteps] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+      ch.steps(p, s.dc + e, x, v);
+      xa[0] = make_float4(x[0], x[1], x[2], x[3]);
+      xa[1] = make_float4(x[4], x[5], x[6], x[7]);
+      xv[0] = make_float4(v[0], v[1], v[2], v[3]);
+      xv[1] = make_float4(v[4], v[5], v[6], v[7]);
     }
-  };
-  if (seg < 0) {
-    run(0, p.walk, std::true_type{});
-  } else {
-    int lo, hi;
-    segment_of<kSplitWays>(p.walk, seg, lo, hi);
-    run(hi, p.walk, std::false_type{});
     __syncwarp();
-    run(lo, hi, std::true_type{});
+    if (count > 16) Chain::template reduce<1>(a, s, g, bx, by, hW, hH);
+    else if (count > 8) Chain::template reduce<2>(a, s, g, bx, by, hW, hH);
+    else Chain::template reduce<4>(a, s, g, bx, by, hW, hH);
+    __syncwarp();
+    g = next;
+    next = after;
   }
 }
 
@@ -1417,26 +1388,12 @@ void launch_backward_groups(const BackwardArgs& a, cudaStream_t stream) {
 void launch_backward_render(const BackwardArgs& a, cudaStream_t stream) {
   const int tiles = a.items ? a.total_tiles : ((a.W + kTile - 1) / kTile) * ((a.H + kTile - 1) / kTile);
   if (tiles <= 0) return;
-  BackwardArgs b = a;
-  int sms = 148, dev = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // the heaviest tiles by largest contributor count: knob quarters of the SM count
-  b.split = min(tiles / 4, sms * tune_value(kTuneBwdSplit) / 4);
-  const int ways = tune_value(kTuneBwdWays);
   stage_begin(kStBwdRender, stream);
-  const int grid = (tiles + (ways - 1) * b.split) * kBwdParts;
   const bool da = a.dL_ddepth != nullptr || a.dL_dalpha != nullptr;  // a loss reaches depth or alpha
-  auto launch = [&](auto kernel) { kernel<<<grid, 32 * kBwdWarps, 0, stream>>>(b); };
-  if (ways == 3) {
-    if (a.grad_mode == 1) launch(render_bwd_kernel<ExactChain, 3>);
-    else if (da) launch(render_bwd_kernel<RefChain<true>, 3>);
-    else launch(render_bwd_kernel<RefChain<false>, 3>);
-  } else {
-    if (a.grad_mode == 1) launch(render_bwd_kernel<ExactChain, 2>);
-    else if (da) launch(render_bwd_kernel<RefChain<true>, 2>);
-    else launch(render_bwd_kernel<RefChain<false>, 2>);
-  }
+  auto launch = [&](auto kernel) { kernel<<<tiles * 8, 32, 0, stream>>>(a); };
+  if (a.grad_mode == 1) launch(render_bwd_kernel<ExactChain>);
+  else if (da) launch(render_bwd_kernel<RefChain<true>>);
+  else launch(render_bwd_kernel<RefChain<false>>);
   stage_end(kStBwdRender, stream, 1);
 }
 

@@ -27,21 +27,6 @@ namespace {
 
 constexpr int kBlendIlp = 4;  // list entries the queue-fed blend evaluates together per warp
 
-// The reference's Gaussian value (gaussEval.h:7-29) in two halves: the
-// mahalanobis numerator, then exp(-0.5 * num / det) with negative distances
-// mapped to 1000.
-__device__ __forceinline__ float gauss_num(float px, float py, float mx, float my, float cxx, float cxy, float cyy) {
-  using namespace fp;
-  const float dx = sub(px, mx), dy = sub(py, my);
-  const float tX = d2<BL_TX>(dx, cyy, dy, cxy);
-  const float tY = s2<BL_TY>(-dx, cxy, dy, cxx);
-  return s2<BL_NUM>(tX, dx, tY, dy);
-}
-__device__ __forceinline__ float gauss_from_m(float m) {
-  if (m < 0.0f) m = 1000.0f;
-  return expf(mul(-0.5f, m));
-}
-
 struct BlendPixel {
   float C0 = 0.f, C1 = 0.f, C2 = 0.f, Wt = 0.f, D = 0.f, T = 1.0f;
   uint32_t last = 0;
@@ -136,54 +121,14 @@ struct BlendEntry {
 };
 
 // Alphas of a group's entries at the block's 32 pixels, into the alpha table (0
-// where an entry is skipped): up to 32 / kLanes entries, a lane per entry and
-// 4 / kLanes pixel rows.  The entry stays in the lane's registers, so its
-// reciprocal determinant and the per-row and per-column products are computed
-// once; a row's pixels go through each stage together, so their divisions and
-// exponentials overlap.
-//
-// Per value the arithmetic is gauss_num's and gauss_from_m's, with the quotient
-// by the determinant from div_markstein and its sign from the numerator.  Both
-// hold while the determinant and the variances are in [2^-20, 2^20] and the
-// mean is not within 2^-12 of a pixel in both coordinates without being on it:
-// then a numerator is 0 or above 2^-126 in magnitude (each of its two nested
-// sums of products cancels to no less than 2^-47 of its terms), its quotient
-// does not underflow, and one too small for div_markstein's range still gives
-// exp(-quotient / 2) = 1.  Any other entry is evaluated with the IEEE division.
+// where an entry is skipped): gauss_values' lanes and pixels.
 template <int kLanes>
 __device__ __forceinline__ void group_alphas(BlendWarp& s, const BlendEntry& en, float bx, float by) {
-  constexpr int kEntries = 32 / kLanes, kRows = 4 / kLanes;
-  const int lane = int(threadIdx.x & 31u), e = lane % kEntries, r0 = (lane / kEntries) * kRows;
-  float* out = s.alpha + 8 * r0 * kAlphaStride + e;
-  const float4 m = en.m, c = en.c;
-  const float y = rcp_markstein(c.w);
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) {
-    float num[8], g[8];
-#pragma unroll
-    for (int col = 0; col < 8; ++col)
-      num[col] = gauss_num(bx + float(col), by + float(r0 + r), m.x, m.y, c.x, c.y, c.z);
-#pragma unroll
-    for (int col = 0; col < 8; ++col) g[col] = div_markstein_y(num[col], c.w, y);
-#pragma unroll
-    for (int col = 0; col < 8; ++col) g[col] = expf(mul(-0.5f, g[col]));
-#pragma unroll
-    for (int col = 0; col < 8; ++col) {
-      const float al = fminf(0.99f, mul(m.z, g[col]));
-      out[(8 * r + col) * kAlphaStride] = al >= 1.0f / 255.0f && !(num[col] < 0.0f) ? al : 0.0f;
-    }
-  }
-  const float fx = fabsf(m.x - rintf(m.x)), fy = fabsf(m.y - rintf(m.y));
-  auto in = [](float v) { return v >= 0x1p-20f && v <= 0x1p20f; };
-  if (!(in(c.w) && in(c.x) && in(c.z) && fabsf(m.x) <= 0x1p24f && fabsf(m.y) <= 0x1p24f &&
-        (fmaxf(fx, fy) >= 0x1p-12f || fmaxf(fx, fy) == 0.0f))) {
-#pragma unroll 1
-    for (int p = 0; p < 8 * kRows; ++p) {
-      const float num = gauss_num(bx + float(p & 7), by + float(r0 + (p >> 3)), m.x, m.y, c.x, c.y, c.z);
-      const float al = fminf(0.99f, mul(m.z, gauss_from_m(div(num, c.w))));
-      out[p * kAlphaStride] = al >= 1.0f / 255.0f ? al : 0.0f;
-    }
-  }
+  const int e = int(threadIdx.x & 31u) % (32 / kLanes);
+  gauss_values<kLanes>(en.m.x, en.m.y, en.c, bx, by, [&](int p, float g) {
+    const float al = fminf(0.99f, mul(en.m.z, g));
+    s.alpha[p * kAlphaStride + e] = al >= 1.0f / 255.0f ? al : 0.0f;
+  });
 }
 
 // One CTA per kBlendWarps blocks of a tile; its warps never wait for one
@@ -286,7 +231,7 @@ __global__ void __launch_bounds__(32 * kBlendWarps, kBlendResident / kBlendWarps
   BlendEntry en;
   auto load_group = [&](int count) {
     const int e = count > 16 ? lane : count > 8 ? lane & 15 : lane & 7;
-    // past the count: opacity 0, so alpha 0, and operands in group_alphas' range
+    // past the count: opacity 0, so alpha 0, and operands in gauss_values' range
     en.m = make_float4(-1024.f, -1024.f, 0.f, 0.f);
     en.c = make_float4(1.f, 0.f, 1.f, 1.f);
     en.dc = make_float4(0.f, 0.f, 0.f, 0.f);

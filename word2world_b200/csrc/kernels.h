@@ -201,7 +201,6 @@ struct BackwardArgs {
   const uint32_t* order_bwd;  // tile order by largest contributor count (written by the blend)
   const uint32_t* masks;      // the blend's block masks (tile_walk.cuh mask_row); null: test each entry
   const uint32_t* masks_valid;
-  int split;               // heaviest tiles whose walks are split over several CTAs (set at launch)
   const float* T_final;
   const float* out_alpha;
   const float* dL_dcolor;
@@ -336,11 +335,12 @@ enum WaitStage { kWaitScan = 0, kWaitSort = 1, kWaitPreprocess = 2, kNumWaitStag
 uint32_t spin_limit();
 long long unpublished_tile(int stage);
 
-// Run-time launch shapes chosen by the autotuner (w2w_tune_set): warps per
-// blend CTA (4: two CTAs per tile, 8: one), how many of the heaviest tiles the
-// per-pixel backward splits (in quarters of the SM count) and into how many
-// segments.  None of them changes a result beyond the order of float atomic
-// additions.
+// Run-time launch shapes chosen by the autotuner (w2w_tune_set).  None of them
+// changes a result beyond the order of float atomic additions.  Three no longer
+// select anything and are accepted for their callers' sake: the per-pixel
+// backward runs one warp per block of a tile whatever backward_split and
+// backward_ways say, the per-tile blend one kernel whatever blend_stage says;
+// blend_warps picks the queue-fed blend's consumer warps.
 // The fourth knob picks how a single-view call builds its sorted list: 0 key
 // emission + radix sort (duplicate.cu, sort.cu), 1 binning from the
 // depth-ordered Gaussians (binning.cu); both give the same list.

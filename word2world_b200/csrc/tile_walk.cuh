@@ -10,7 +10,6 @@
 
 namespace w2w {
 
-constexpr int kRecVec = 3;  // float4s of an entry staged in shared memory
 
 // Pixel of this thread in tile `tile` of a grid `gw` tiles wide.
 struct TilePixel {
@@ -52,20 +51,66 @@ __host__ __device__ __forceinline__ size_t mask_row(uint32_t first, int tile, in
   return 8 * (size_t(first >> 5) + size_t(tile)) + size_t(block) * size_t((n + 31) >> 5);
 }
 
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
-  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gmem_src) : "memory");
+// The reference's Gaussian value (gaussEval.h:7-29) in two halves: the
+// mahalanobis numerator, then exp(-0.5 * num / det) with negative distances
+// mapped to 1000.
+__device__ __forceinline__ float gauss_num(float px, float py, float mx, float my, float cxx, float cxy, float cyy) {
+  using namespace fp;
+  const float dx = sub(px, mx), dy = sub(py, my);
+  const float tX = d2<BL_TX>(dx, cyy, dy, cxy);
+  const float tY = s2<BL_TY>(-dx, cxy, dy, cxx);
+  return s2<BL_NUM>(tX, dx, tY, dy);
 }
-__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) {
-  const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(gmem_src) : "memory");
+__device__ __forceinline__ float gauss_from_m(float m) {
+  if (m < 0.0f) m = 1000.0f;
+  return expf(mul(-0.5f, m));
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-// All but this thread's newest kPending groups of copies have landed (and are
-// visible to it).
-template <int kPending>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(kPending) : "memory");
+
+// The forward's Gaussian values of a lane's entry -- mean (mx, my), covariance
+// and determinant c = (cxx, cxy, cyy, det) -- at pixels of the block at
+// (bx, by): emit(p, value) for the lane's 32 / kLanes pixels p (a lane per entry
+// and 4 / kLanes pixel rows: lane l takes entry l % (32 / kLanes)).  The entry
+// stays in registers, so its reciprocal determinant and the per-row and
+// per-column products are computed once; a row's pixels go through each stage
+// together, so their divisions and exponentials overlap.
+//
+// Per value the arithmetic is gauss_num's and gauss_from_m's, with the quotient
+// by the determinant from div_markstein and its sign from the numerator.  Both
+// hold while the determinant and the variances are in [2^-20, 2^20] and the
+// mean is not within 2^-12 of a pixel in both coordinates without being on it:
+// then a numerator is 0 or above 2^-126 in magnitude (each of its two nested
+// sums of products cancels to no less than 2^-47 of its terms), its quotient
+// does not underflow, and one too small for div_markstein's range still gives
+// exp(-quotient / 2) = 1.  Any other entry is evaluated with the IEEE division.
+template <int kLanes, typename Emit>
+__device__ __forceinline__ void gauss_values(float mx, float my, float4 c, float bx, float by, Emit&& emit) {
+  constexpr int kRows = 4 / kLanes;
+  const int r0 = (int(threadIdx.x & 31u) / (32 / kLanes)) * kRows;
+  const float fx = fabsf(mx - rintf(mx)), fy = fabsf(my - rintf(my));
+  auto in = [](float v) { return v >= 0x1p-20f && v <= 0x1p20f; };
+  if (in(c.w) && in(c.x) && in(c.z) && fabsf(mx) <= 0x1p24f && fabsf(my) <= 0x1p24f &&
+      (fmaxf(fx, fy) >= 0x1p-12f || fmaxf(fx, fy) == 0.0f)) {
+    const float y = rcp_markstein(c.w);
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      float num[8], g[8];
+#pragma unroll
+      for (int col = 0; col < 8; ++col)
+        num[col] = gauss_num(bx + float(col), by + float(r0 + r), mx, my, c.x, c.y, c.z);
+#pragma unroll
+      for (int col = 0; col < 8; ++col) g[col] = div_markstein_y(num[col], c.w, y);
+#pragma unroll
+      for (int col = 0; col < 8; ++col) g[col] = expf(mul(-0.5f, g[col]));
+#pragma unroll
+      for (int col = 0; col < 8; ++col) emit(8 * (r0 + r) + col, num[col] < 0.0f ? 0.0f : g[col]);
+    }
+  } else {
+#pragma unroll 1
+    for (int p = 8 * r0; p < 8 * (r0 + kRows); ++p) {
+      const float num = gauss_num(bx + float(p & 7), by + float(p >> 3), mx, my, c.x, c.y, c.z);
+      emit(p, gauss_from_m(div(num, c.w)));
+    }
+  }
 }
 
 }  // namespace w2w

@@ -73,13 +73,9 @@ namespace {
 const char* kTuneNames[kNumTuneKnobs] = {"blend_warps", "backward_split", "backward_ways",
                                          "binning",     "blend_queue",    "preprocess_blocks",
                                          "planned_forward", "blend_stage"};
-// defaults: 4-warp blend CTAs, the heaviest half-SM-count tiles' backward
-// walks split in two (backward_split 2 measured 3.09 against 3.21 ms per 4-view
-// step for 4, same B200), radix sort, per-tile blend, 4 projection CTAs per SM,
-// planned forward on, blend batches copied with cp.async (five 4-warp CTAs per
-// SM: 1416-1423 against 1388-1396 views/s for the 4-view step with the views
-// on their own streams; alone the kernel takes 0.218 against 0.199 ms, so a
-// single-stream caller's autotuning may pick 0)
+// defaults: four consumer warps in the queue-fed blend, radix sort, per-tile
+// blend, 4 projection CTAs per SM, planned forward on; backward_split,
+// backward_ways and blend_stage select nothing (kernels.h)
 std::atomic<int> g_tune[kNumTuneKnobs] = {{4}, {2}, {2}, {0}, {0}, {4}, {1}, {1}};
 bool tune_valid(int knob, int v) {
   switch (knob) {
