@@ -452,7 +452,7 @@ __device__ __forceinline__ BwdPixel make_bwd_pixel(const BackwardArgs& a, int ti
 template <typename Chain>
 __global__ void __launch_bounds__(32, 16) render_bwd_kernel(BackwardArgs a) {
   __shared__ BwdWarp s;
-  const int tile = int(a.order_bwd[blockIdx.x / 8]);  // heaviest first
+  const int tile = int(a.order[blockIdx.x / 8]);  // heaviest first
   const int lane = int(threadIdx.x), block = int(blockIdx.x) % 8;
   const BwdPixel p = make_bwd_pixel(a, tile, block);
   if (p.walk <= 0) return;

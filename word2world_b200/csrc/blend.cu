@@ -605,40 +605,9 @@ __global__ void __launch_bounds__(32 * (kW + 1)) blend_queue_kernel(BlendArgs a,
 
 }  // namespace
 
-// Bucket sort of the tiles by decreasing list length (quarter-octave buckets;
-// order within a bucket is arbitrary).  One CTA.
-__global__ void __launch_bounds__(1024) tile_order_kernel(const uint2* ranges, const uint32_t* counts, int num_tiles,
-                                                          uint32_t* order, uint32_t* zero, uint32_t* counter) {
-  if (counter != nullptr && threadIdx.x == 0) *counter = 0u;
-  constexpr int kBuckets = 130;
-  __shared__ uint32_t s_cnt[kBuckets];
-  __shared__ uint32_t s_pos[kBuckets];
-  auto bucket = [](uint32_t n) -> int {
-    if (n == 0) return 0;
-    const int e = 31 - __clz(n);
-    const uint32_t q = e >= 2 ? (n >> (e - 2)) & 3u : (n << (2 - e)) & 3u;
-    return 1 + 4 * e + int(q);
-  };
-  for (int i = threadIdx.x; i < kBuckets; i += blockDim.x) s_cnt[i] = 0;
-  if (zero != nullptr)
-    for (int t = threadIdx.x; t < num_tiles; t += blockDim.x) zero[t] = 0u;
-  __syncthreads();
-  auto weight = [&](int t) -> uint32_t {
-    if (counts) return counts[t];
-    const uint2 r = ranges[t];
-    return r.y - r.x;
-  };
-  for (int t = threadIdx.x; t < num_tiles; t += blockDim.x) atomicAdd(&s_cnt[bucket(weight(t))], 1u);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    uint32_t acc = 0;
-    for (int b = kBuckets - 1; b >= 0; --b) {
-      s_pos[b] = acc;
-      acc += s_cnt[b];
-    }
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < num_tiles; t += blockDim.x) order[atomicAdd(&s_pos[bucket(weight(t))], 1u)] = uint32_t(t);
+__global__ void __launch_bounds__(1024) tile_order_kernel(const uint2* ranges, int num_tiles, uint32_t* order,
+                                                          uint32_t* zero, uint32_t* counter) {
+  tile_order_block(ranges, num_tiles, order, zero, counter);
 }
 
 namespace {
@@ -710,19 +679,17 @@ void launch_blend(const BlendArgs& a, cudaStream_t stream) {
   if (tiles <= 0) return;
   const int warps = tune_value(kTuneBlendWarps);
   const bool queue = tune_value(kTuneBlendQueue) == 1 && a.queue != nullptr;
-  stage_begin(kStOther, stream);
-  // a tile's warps combine their contributor counts in its maximum: clear
+  // a tile's warps combine their contributor counts in its maximum, cleared
   // first; the queue counter starts at zero
-  tile_order_kernel<<<1, 1024, 0, stream>>>(a.ranges, nullptr, tiles, a.order, a.tile_max, queue ? a.queue : nullptr);
-  stage_end(kStOther, stream, 1);
+  if (!a.ordered) {
+    stage_begin(kStOther, stream);
+    tile_order_kernel<<<1, 1024, 0, stream>>>(a.ranges, tiles, a.order, a.tile_max, a.queue);
+    stage_end(kStOther, stream, 1);
+  }
   stage_begin(kStBlend, stream);
   const bool queued = queue && (warps == 4 ? launch_queue<4>(a, tiles, stream) : launch_queue<8>(a, tiles, stream));
   if (!queued) blend_kernel<<<tiles * (8 / kBlendWarps), 32 * kBlendWarps, 0, stream>>>(a);
   stage_end(kStBlend, stream, 1);
-  // the backward's order: by the largest contributor count the blend just found
-  stage_begin(kStOther, stream);
-  tile_order_kernel<<<1, 1024, 0, stream>>>(nullptr, a.tile_max, tiles, a.order_bwd, nullptr, nullptr);
-  stage_end(kStOther, stream, 1);
 }
 
 }  // namespace w2w

@@ -99,7 +99,7 @@ __global__ void write_bin_header(BinHeader* h, KeyPlan k, uint32_t R, uint32_t p
   h->tile_bits = k.tile_bits;
   h->passes = passes;
   h->num_rendered = R;
-  for (int i = 0; i < 8; ++i) h->tile_counter[i] = 0;
+  for (int i = 0; i <= kMaxPasses; ++i) h->tile_counter[i] = 0;
 }
 
 template <typename K>
@@ -134,8 +134,26 @@ size_t sort_scratch_layout(long long n, size_t* keys_tmp, size_t* vals_tmp, size
   *vals_tmp = take(nn * 4);
   *hist = take(size_t(kMaxPasses) * kMaxBins * 4);
   *status = take(sort_status_words(n) * 4);
-  *counters = take(kMaxPasses * 4);
+  *counters = take((kMaxPasses + 1) * 4);
   return align256(o);
+}
+
+// The emission's share of a render's bookkeeping (DuplicateArgs): the binning
+// header, and the span the sort needs cleared -- its histograms, tile counts and
+// the used passes' status words, contiguous in the layout -- with the sort told so.
+void set_emission(DuplicateArgs& d, SortArgs& so, void* binning_state, const BinLayout& BL, BinHeader* header,
+                  const KeyPlan& kp, int passes, long long n, const GeomHeader* plan) {
+  d.header = header;
+  d.plan = plan;
+  d.tile_bits = uint32_t(kp.tile_bits);
+  d.passes = uint32_t(passes);
+  d.depth_prefix = kp.prefix;
+  const long long tile = sort_tile_keys(kp.key64, n);
+  const size_t bytes = BL.status - BL.hist +
+                       size_t(passes > 0 ? passes : 1) * kMaxBins * 4 * size_t((n + tile - 1) / tile);
+  d.clear = at<uint4>(binning_state, BL.hist);
+  d.clear_vecs = uint32_t((bytes + 15) / 16);
+  so.cleared = true;
 }
 
 // Whether entry points with bounded device waits read their error word back
@@ -234,7 +252,7 @@ size_t w2w_image_offset(int W, int H, const char* name) {
   if (!strcmp(name, "T_final")) return L.T_final;
   if (!strcmp(name, "tile_max")) return L.tile_max;
   if (!strcmp(name, "order")) return L.order;
-  if (!strcmp(name, "order_bwd")) return L.order_bwd;
+  if (!strcmp(name, "order_bwd")) return L.order;  // the backward takes the blend's order
   return size_t(-1);
 }
 
@@ -285,7 +303,7 @@ static void launch_depth_order(const w2w_settings* s, void* geom_state, const w2
     const int passes = sort_passes(kp.depth_bits);
     so.clear_span = at<void>(geom_state, L.dsort_hist);
     so.clear_bytes = L.dsort_status - L.dsort_hist +
-                     size_t(passes) * kMaxBins * 4 * size_t((P + sort_tile_keys(0) - 1) / sort_tile_keys(0));
+                     size_t(passes) * kMaxBins * 4 * size_t((P + sort_tile_keys(0, P) - 1) / sort_tile_keys(0, P));
     so.spin_limit = spin_limit();
     so.unpublished_tile = unpublished_tile(kWaitSort);
     so.stage_hist = so.stage_pass = kStDepthSort;
@@ -409,6 +427,7 @@ int w2w_forward_render(const w2w_settings* s, const void* geom_state, const w2w_
   uint2* ranges = at<uint2>(image_state, IL.ranges);
   const uint32_t* point_list = nullptr;
   const void* err_word = nullptr;  // the binning header's error word
+  bool ordered = false;            // the sort writes the tiles' order
   if (R == 0) {
     cudaMemsetAsync(ranges, 0, sizeof(uint2) * size_t(T), st);
   } else if ((info->reserved & kInfoDepthOrder) != 0u) {
@@ -447,9 +466,6 @@ int w2w_forward_render(const w2w_settings* s, const void* geom_state, const w2w_
     const int passes = sort_passes(kp.bits);
     BinHeader* bh = at<BinHeader>(binning_state, BL.header);
     err_word = &bh->error;
-    stage_begin(kStOther, st);
-    write_bin_header<<<1, 1, 0, st>>>(bh, kp, uint32_t(R), uint32_t(passes), nullptr, nullptr);
-    stage_end(kStOther, st, 1);
     // the sort result lands in (keysA, valsA); key emission targets the
     // buffer that makes the ping-pong end there
     const bool odd = (passes % 2) == 1;
@@ -466,8 +482,9 @@ int w2w_forward_render(const w2w_settings* s, const void* geom_state, const w2w_
     d.depth = at<float>(geom_state, GL.depth);
     d.keys = odd ? keysB : keysA;
     d.vals = odd ? valsB : valsA;
-    launch_duplicate(d, st);
     SortArgs so{};
+    set_emission(d, so, binning_state, BL, bh, kp, passes, R, nullptr);
+    launch_duplicate(d, st);
     so.n = R; so.key64 = kp.key64; so.begin_bit = 0; so.bits = kp.bits;
     so.keys_in = d.keys; so.vals_in = d.vals;
     so.match_rank = 1;  // emitted Gaussian by Gaussian: few distinct digits per warp
@@ -481,11 +498,10 @@ int w2w_forward_render(const w2w_settings* s, const void* geom_state, const w2w_
     so.num_tiles = T;
     so.tile_hist = at<uint32_t>(binning_state, BL.tile_hist);
     so.ranges = ranges;
-    // hist, tile_hist and the used status words are contiguous; the tile
-    // counters were cleared by write_bin_header
-    so.clear_span = at<void>(binning_state, BL.hist);
-    so.clear_bytes = BL.status - BL.hist + size_t(passes > 0 ? passes : 1) * kMaxBins * 4 *
-                     size_t((R + sort_tile_keys(kp.key64) - 1) / sort_tile_keys(kp.key64));
+    so.order = at<uint32_t>(image_state, IL.order);
+    so.order_zero = at<uint32_t>(image_state, IL.tile_max);
+    so.order_counter = at<uint32_t>(image_state, IL.queue);
+    ordered = true;
     so.spin_limit = spin_limit();
     so.unpublished_tile = unpublished_tile(kWaitSort);
     launch_sort(so, st);
@@ -508,7 +524,7 @@ int w2w_forward_render(const w2w_settings* s, const void* geom_state, const w2w_
   b.T_final = at<float>(image_state, IL.T_final);
   b.tile_max = at<uint32_t>(image_state, IL.tile_max);
   b.order = at<uint32_t>(image_state, IL.order);
-  b.order_bwd = at<uint32_t>(image_state, IL.order_bwd);
+  b.ordered = ordered;
   b.queue = at<uint32_t>(image_state, IL.queue);
   b.error = const_cast<uint32_t*>(static_cast<const uint32_t*>(err_word));
   b.spin_limit = spin_limit();
@@ -618,28 +634,6 @@ long long w2w_binning_layout_count(long long num_rendered, size_t state_bytes, i
 
 }  // extern "C"
 
-// The planned render's header: the caller's key plan, checked against the
-// view's own count and depth range (the projection pass's header).
-__global__ void plan_bin_header(BinHeader* h, const GeomHeader* g, uint32_t capacity, KeyPlan k, uint32_t passes) {
-  const uint32_t R = g->num_rendered;
-  const uint32_t dmin = ~g->depth_min, dmax = g->depth_max;
-  const uint32_t x = dmin ^ dmax;
-  int need = 0;
-  while (need < 32 && (x >> need) != 0u) ++need;
-  const bool ok = R <= capacity && need <= k.depth_bits && (g->error & (kErrTimeout | kErrCapacity)) == 0u;
-  h->error = 0u;
-  h->masks_valid = 1u;
-  h->key64 = k.key64;
-  h->depth_bits = k.depth_bits;
-  h->depth_prefix = k.depth_bits >= 32 ? 0u : (dmin & ~((1u << k.depth_bits) - 1u));
-  h->tile_bits = k.tile_bits;
-  h->passes = passes;
-  h->num_rendered = R;
-  h->n_sort = ok ? R : 0u;
-  h->replan = ok ? 0u : 1u;
-  for (int i = 0; i < 8; ++i) h->tile_counter[i] = 0;
-}
-
 extern "C" {
 
 int w2w_forward_render_planned(const w2w_settings* s, const void* geom_state, long long capacity, int depth_bits,
@@ -660,10 +654,6 @@ int w2w_forward_render_planned(const w2w_settings* s, const void* geom_state, lo
   kp.key64 = kp.bits > 32 ? 1 : 0;
   const int passes = sort_passes(kp.bits);
   BinHeader* bh = at<BinHeader>(binning_state, BL.header);
-  stage_begin(kStOther, st);
-  plan_bin_header<<<1, 1, 0, st>>>(bh, at<GeomHeader>(geom_state, GL.header), uint32_t(capacity), kp,
-                                   uint32_t(passes));
-  stage_end(kStOther, st, 1);
   // the sort result lands in (keysA, valsA); key emission targets the buffer
   // that makes the ping-pong end there
   const bool odd = (passes % 2) == 1;
@@ -681,9 +671,9 @@ int w2w_forward_render_planned(const w2w_settings* s, const void* geom_state, lo
   d.depth = at<float>(geom_state, GL.depth);
   d.keys = odd ? keysB : keysA;
   d.vals = odd ? valsB : valsA;
-  d.n_dev = &bh->n_sort;
-  launch_duplicate(d, st);
   SortArgs so{};
+  set_emission(d, so, binning_state, BL, bh, kp, passes, capacity, at<GeomHeader>(geom_state, GL.header));
+  launch_duplicate(d, st);
   so.n = capacity; so.key64 = kp.key64; so.begin_bit = 0; so.bits = kp.bits;
   so.keys_in = d.keys; so.vals_in = d.vals;
   so.match_rank = 1;  // emitted Gaussian by Gaussian: few distinct digits per warp
@@ -698,9 +688,9 @@ int w2w_forward_render_planned(const w2w_settings* s, const void* geom_state, lo
   so.num_tiles = T;
   so.tile_hist = at<uint32_t>(binning_state, BL.tile_hist);
   so.ranges = at<uint2>(image_state, IL.ranges);
-  so.clear_span = at<void>(binning_state, BL.hist);
-  so.clear_bytes = BL.status - BL.hist + size_t(passes > 0 ? passes : 1) * kMaxBins * 4 *
-                   size_t((capacity + sort_tile_keys(kp.key64) - 1) / sort_tile_keys(kp.key64));
+  so.order = at<uint32_t>(image_state, IL.order);
+  so.order_zero = at<uint32_t>(image_state, IL.tile_max);
+  so.order_counter = at<uint32_t>(image_state, IL.queue);
   so.spin_limit = spin_limit();
   so.unpublished_tile = unpublished_tile(kWaitSort);
   launch_sort(so, st);
@@ -718,7 +708,7 @@ int w2w_forward_render_planned(const w2w_settings* s, const void* geom_state, lo
   b.T_final = at<float>(image_state, IL.T_final);
   b.tile_max = at<uint32_t>(image_state, IL.tile_max);
   b.order = at<uint32_t>(image_state, IL.order);
-  b.order_bwd = at<uint32_t>(image_state, IL.order_bwd);
+  b.ordered = true;
   b.queue = at<uint32_t>(image_state, IL.queue);
   b.error = &bh->error;
   b.spin_limit = spin_limit();
@@ -747,6 +737,35 @@ int w2w_state_error(const void* state, int which, w2w_stream_t stream) {
   return int(e);
 }
 
+// Zeroes up to four spans of floats (a backward's accumulators) in one launch.
+struct ZeroSpans {
+  float* p[4];
+  unsigned long long n[4];  // floats
+};
+static __global__ void __launch_bounds__(256) zero_spans_kernel(ZeroSpans z) {
+  const unsigned long long i0 = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned long long step = (unsigned long long)gridDim.x * blockDim.x;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if ((reinterpret_cast<uintptr_t>(z.p[k]) & 15u) == 0u) {
+      for (unsigned long long i = i0; i < z.n[k] / 4; i += step)
+        reinterpret_cast<float4*>(z.p[k])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (i0 < z.n[k] % 4) z.p[k][z.n[k] - 1 - i0] = 0.f;
+    } else {
+      for (unsigned long long i = i0; i < z.n[k]; i += step) z.p[k][i] = 0.f;
+    }
+  }
+}
+static void zero_accumulators(void* scratch, size_t scratch_bytes, float* mean2D, float* colors, float* opacity,
+                              long long P, cudaStream_t st) {
+  const unsigned long long n = (unsigned long long)P;
+  const ZeroSpans z{{static_cast<float*>(scratch), mean2D, colors, opacity}, {scratch_bytes / 4, 3 * n, 3 * n, n}};
+  const long long blocks = (P * 12 + 1023) / 1024;  // a float4 per thread
+  stage_begin(kStOther, st);
+  zero_spans_kernel<<<unsigned(blocks < 1184 ? blocks : 1184), 256, 0, st>>>(z);
+  stage_end(kStOther, st, 1);
+}
+
 struct RawGrads {
   const float *svec, *quat, *logit, *sh_dc, *sh_ac;
   float *d_sh_dc, *d_sh_ac;
@@ -768,10 +787,7 @@ static int backward_impl(const w2w_settings* s, const float* means3D, const floa
   const ImageLayout IL(W, H);
   float* acc_cov = static_cast<float*>(scratch);
   float* acc_depth = at<float>(scratch, align256(size_t(P) * 16));
-  cudaMemsetAsync(scratch, 0, w2w_backward_scratch_bytes(P), st);
-  cudaMemsetAsync(dL_dmeans2D, 0, sizeof(float) * 3 * size_t(P), st);
-  cudaMemsetAsync(dL_dcolors, 0, sizeof(float) * 3 * size_t(P), st);
-  cudaMemsetAsync(dL_dopacity, 0, sizeof(float) * size_t(P), st);
+  zero_accumulators(scratch, w2w_backward_scratch_bytes(P), dL_dmeans2D, dL_dcolors, dL_dopacity, P, st);
   BackwardArgs a{};
   a.P = P; a.W = W; a.H = H; a.degree = s->degree; a.M = s->M; a.grad_mode = grad_mode;
   a.h_x = float(W) / (2.0f * s->tan_fovx);
@@ -794,8 +810,7 @@ static int backward_impl(const w2w_settings* s, const float* means3D, const floa
     a.masks_valid = &at<BinHeader>(binning_state, BL.header)->masks_valid;
   }
   a.n_contrib = at<uint32_t>(image_state, IL.n_contrib);
-  a.tile_max = at<uint32_t>(image_state, IL.tile_max);
-  a.order_bwd = at<uint32_t>(image_state, IL.order_bwd);
+  a.order = at<uint32_t>(image_state, IL.order);
   a.T_final = at<float>(image_state, IL.T_final);
   a.out_alpha = out_alpha;
   a.dL_dcolor = dL_dcolor; a.dL_ddepth = dL_ddepth; a.dL_dalpha = dL_dalpha;
@@ -1129,7 +1144,6 @@ int w2w_blend(const w2w_settings* s, const void* geom_state, const uint32_t* ran
   b.T_final = at<float>(image_state, IL.T_final);
   b.tile_max = at<uint32_t>(image_state, IL.tile_max);
   b.order = at<uint32_t>(image_state, IL.order);
-  b.order_bwd = at<uint32_t>(image_state, IL.order_bwd);
   b.queue = at<uint32_t>(image_state, IL.queue);
   b.spin_limit = spin_limit();
   launch_blend(b, S(stream));
@@ -1337,6 +1351,7 @@ int w2w_batch_forward_render(const w2w_batch_item* items, int n, const void* geo
   uint2* ranges = at<uint2>(image_state, IL.ranges);
   const uint32_t* point_list = nullptr;
   const void* err_word = nullptr;  // the binning header's error word
+  bool ordered = false;            // the sort writes the tiles' order
   if (R == 0) {
     cudaMemsetAsync(ranges, 0, sizeof(uint2) * size_t(T), st);
   } else {
@@ -1346,9 +1361,6 @@ int w2w_batch_forward_render(const w2w_batch_item* items, int n, const void* geo
     const int passes = sort_passes(kp.bits);
     BinHeader* bh = at<BinHeader>(binning_state, BL.header);
     err_word = &bh->error;
-    stage_begin(kStOther, st);
-    write_bin_header<<<1, 1, 0, st>>>(bh, kp, uint32_t(R), uint32_t(passes), nullptr, nullptr);
-    stage_end(kStOther, st, 1);
     const bool odd = (passes % 2) == 1;
     void* keysA = at<void>(binning_state, BL.keysA);
     void* keysB = at<void>(binning_state, BL.keysB);
@@ -1364,8 +1376,9 @@ int w2w_batch_forward_render(const w2w_batch_item* items, int n, const void* geo
     d.depth = at<float>(geom_state, GL.depth);
     d.keys = odd ? keysB : keysA;
     d.vals = odd ? valsB : valsA;
-    launch_duplicate(d, st);
     SortArgs so{};
+    set_emission(d, so, binning_state, BL, bh, kp, passes, R, nullptr);
+    launch_duplicate(d, st);
     so.n = R; so.key64 = kp.key64; so.begin_bit = 0; so.bits = kp.bits;
     so.keys_in = d.keys; so.vals_in = d.vals;
     so.match_rank = 1;  // emitted Gaussian by Gaussian: few distinct digits per warp
@@ -1379,11 +1392,10 @@ int w2w_batch_forward_render(const w2w_batch_item* items, int n, const void* geo
     so.num_tiles = T;
     so.tile_hist = at<uint32_t>(binning_state, BL.tile_hist);
     so.ranges = ranges;
-    // hist, tile_hist and the used status words are contiguous; the tile
-    // counters were cleared by write_bin_header
-    so.clear_span = at<void>(binning_state, BL.hist);
-    so.clear_bytes = BL.status - BL.hist + size_t(passes > 0 ? passes : 1) * kMaxBins * 4 *
-                     size_t((R + sort_tile_keys(kp.key64) - 1) / sort_tile_keys(kp.key64));
+    so.order = at<uint32_t>(image_state, IL.order);
+    so.order_zero = at<uint32_t>(image_state, IL.tile_max);
+    so.order_counter = at<uint32_t>(image_state, IL.queue);
+    ordered = true;
     so.spin_limit = spin_limit();
     so.unpublished_tile = unpublished_tile(kWaitSort);
     launch_sort(so, st);
@@ -1407,7 +1419,7 @@ int w2w_batch_forward_render(const w2w_batch_item* items, int n, const void* geo
   b.T_final = at<float>(image_state, IL.T_final);
   b.tile_max = at<uint32_t>(image_state, IL.tile_max);
   b.order = at<uint32_t>(image_state, IL.order);
-  b.order_bwd = at<uint32_t>(image_state, IL.order_bwd);
+  b.ordered = ordered;
   b.queue = at<uint32_t>(image_state, IL.queue);
   b.error = const_cast<uint32_t*>(static_cast<const uint32_t*>(err_word));
   b.spin_limit = spin_limit();
@@ -1457,10 +1469,7 @@ static int batch_backward_begin(const w2w_batch_item* items, int n, const void* 
   if (!scratch || scratch_bytes < w2w_batch_backward_scratch_bytes(items, n)) return W2W_ERR_SCRATCH;
   const int T = t.tiles;
   const ImageLayout IL(size_t(t.pixels), size_t(T));
-  cudaMemsetAsync(scratch, 0, w2w_batch_backward_scratch_bytes(items, n), st);
-  cudaMemsetAsync(dL_dmeans2D, 0, sizeof(float) * 3 * size_t(E), st);
-  cudaMemsetAsync(dL_dcolors, 0, sizeof(float) * 3 * size_t(E), st);
-  cudaMemsetAsync(dL_dopacity, 0, sizeof(float) * size_t(E), st);
+  zero_accumulators(scratch, w2w_batch_backward_scratch_bytes(items, n), dL_dmeans2D, dL_dcolors, dL_dopacity, E, st);
   batch_gaussian_args(n, E, t.M, geom_state, radii, grad_mode, scratch, dL_dmeans2D, dL_dcolors, dL_dopacity, a);
   a.total_tiles = T;
   a.ranges = at<uint2>(image_state, IL.ranges);
@@ -1471,8 +1480,7 @@ static int batch_backward_begin(const w2w_batch_item* items, int n, const void* 
     a.masks_valid = &at<BinHeader>(binning_state, BL.header)->masks_valid;
   }
   a.n_contrib = at<uint32_t>(image_state, IL.n_contrib);
-  a.tile_max = at<uint32_t>(image_state, IL.tile_max);
-  a.order_bwd = at<uint32_t>(image_state, IL.order_bwd);
+  a.order = at<uint32_t>(image_state, IL.order);
   a.T_final = at<float>(image_state, IL.T_final);
   a.out_alpha = out_alpha;
   a.dL_dcolor = dL_dcolor; a.dL_ddepth = dL_ddepth; a.dL_dalpha = dL_dalpha;

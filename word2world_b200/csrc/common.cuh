@@ -329,7 +329,15 @@ __device__ __forceinline__ void stage_span(const float* src, int len, float* s, 
 }
 
 
-constexpr int kSortTileMin = 4096;  // smallest onesweep tile of any key type: status words are sized for it
+constexpr int kSortTileMin = 4096;    // smallest onesweep tile of any key type: status words are sized for it,
+constexpr int kSortTileSmall = 2048;  // but for counts up to kSortSmall, whose tiles are this small
+constexpr long long kSortSmall = 700000;
+// Onesweep tiles to size status words for (never fewer for more keys).
+__host__ __device__ constexpr long long sort_status_tiles(long long n) {
+  const long long m = n < kSortSmall ? n : kSortSmall;
+  const long long small = (m + kSortTileSmall - 1) / kSortTileSmall, large = (n + kSortTileMin - 1) / kSortTileMin;
+  return small > large ? small : large;
+}
 constexpr int kMaxPasses = 8;
 constexpr int kMaxDigitBits = 9;             // digit width: ceil(bits / ceil(bits / 9))
 constexpr int kMaxBins = 1 << kMaxDigitBits;
@@ -372,15 +380,15 @@ struct GeomLayout {
     dtmp_vals = take(p * 4);
     dprefix = take((p + 1) * 4);
     dsort_hist = take(size_t(kMaxPasses) * kMaxBins * 4);
-    dsort_counters = take(size_t(kMaxPasses) * 4);
-    dsort_status = take(size_t(kMaxPasses) * kMaxBins * ((p + kSortTileMin - 1) / kSortTileMin + 1) * 4);
+    dsort_counters = take(size_t(kMaxPasses + 1) * 4);
+    dsort_status = take(size_t(kMaxPasses) * kMaxBins * size_t(sort_status_tiles(P) + 1) * 4);
     dscan = take(256 + ((p + kScanTileElems - 1) / kScanTileElems + 1) * 8);
     total = align256(o);
   }
 };
 
 struct ImageLayout {
-  size_t n_contrib, ranges, T_final, tile_max, order, order_bwd, queue, total;
+  size_t n_contrib, ranges, T_final, tile_max, order, queue, total;
   __host__ __device__ ImageLayout(int W, int H)
       : ImageLayout(size_t(W) * size_t(H), size_t((W + kTile - 1) / kTile) * size_t((H + kTile - 1) / kTile)) {}
   // a batch: all items' pixels and tiles back to back
@@ -392,7 +400,6 @@ struct ImageLayout {
     T_final = take(hw * 4);
     tile_max = take(tiles * 4);
     order = take(tiles * 4);
-    order_bwd = take(tiles * 4);
     queue = take(4);  // the persistent blend's tile queue counter
     total = align256(o);
   }
@@ -411,7 +418,8 @@ struct BinHeader {
   uint32_t n_sort;         // planned render: instances the emission and sort process (R, or 0 to replan)
   uint32_t replan;         // planned render: 1 when R or the depth range did not fit the plan
   uint32_t pad[6];
-  uint32_t tile_counter[8];  // per-pass tile acquisition counters (onesweep)
+  // per-pass tile acquisition counters (onesweep), then the histogram's finished blocks
+  uint32_t tile_counter[kMaxPasses + 1];
 };
 
 constexpr int kSortThreads = 256;
@@ -422,7 +430,7 @@ struct BinLayout {
     size_t o = 0;
     auto take = [&](size_t bytes) { size_t a = align256(o); o = a + bytes; return a; };
     const size_t r = size_t(R > 0 ? R : 1);
-    const size_t sort_tiles = (r + kSortTileMin - 1) / kSortTileMin;
+    const size_t sort_tiles = size_t(sort_status_tiles((long long)r));
     header = take(sizeof(BinHeader));
     keysA = take(r * 8);
     keysB = take(r * 8);

@@ -13,6 +13,12 @@
 // Batched calls: every view's Gaussians emit into its own slot range, with its
 // own tile grid, and tile ids offset by the view's first global tile.
 //
+// The kernel also writes the binning state's header (a planned render's: the
+// caller's key plan, checked against the view's own count and depth range; one
+// that does not fit emits nothing and makes the sort process nothing) and clears
+// the sort's histograms and status words: a one-thread kernel and a memset of
+// their own cost about 5 us a view in launches and gaps.
+//
 // Load balance: each warp expands 32 consecutive Gaussians; every lane emits
 // one entry per round, so large and small Gaussians cost the same per entry
 // and stores to consecutive slots are coalesced.
@@ -30,8 +36,32 @@ __global__ void __launch_bounds__(kDupThreads) duplicate_kernel(DuplicateArgs a)
   const int warp_global = (blockIdx.x * kDupThreads + threadIdx.x) >> 5;
   const int g = warp_global * 32 + lane;
   uint32_t p0 = 0, cnt = 0, start = 0, x0 = 0, y0 = 0, w = 1, dlow = 0, gwv = uint32_t(a.gw), tbase = 0;
-  // a planned render's instance count is read from device memory (a.R is then the capacity)
-  const uint32_t Rlim = a.n_dev != nullptr ? min(*a.n_dev, a.R) : a.R;
+  uint32_t R = a.R, prefix = a.depth_prefix;
+  bool fits = true;
+  if (a.plan != nullptr) {  // a.R is the capacity
+    R = a.plan->num_rendered;
+    const uint32_t dmin = ~a.plan->depth_min, x = dmin ^ a.plan->depth_max;
+    const uint32_t need = x == 0u ? 0u : 32u - uint32_t(__clz(x));
+    fits = R <= a.R && need <= a.depth_bits && (a.plan->error & (kErrTimeout | kErrCapacity)) == 0u;
+    prefix = a.depth_bits >= 32 ? 0u : (dmin & ~((1u << a.depth_bits) - 1u));
+  }
+  const uint32_t Rlim = fits ? R : 0u;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    BinHeader* h = a.header;
+    h->error = 0u;
+    h->masks_valid = 1u;  // the blend that follows writes the block masks
+    h->key64 = kKey64 ? 1u : 0u;
+    h->depth_bits = a.depth_bits;
+    h->depth_prefix = prefix;
+    h->tile_bits = a.tile_bits;
+    h->passes = a.passes;
+    h->num_rendered = R;
+    h->n_sort = Rlim;
+    h->replan = fits ? 0u : 1u;
+    for (int i = 0; i <= kMaxPasses; ++i) h->tile_counter[i] = 0u;
+  }
+  for (uint32_t i = blockIdx.x * kDupThreads + threadIdx.x; i < a.clear_vecs; i += gridDim.x * kDupThreads)
+    a.clear[i] = make_uint4(0u, 0u, 0u, 0u);
   if (g < a.P) {  // Gaussians that emit nothing have an empty rectangle
     uint32_t end = Rlim;
     if (a.items != nullptr) {  // batched: this view's tile grid, first tile id and end slot
@@ -103,7 +133,8 @@ __global__ void __launch_bounds__(kDupThreads) duplicate_kernel(DuplicateArgs a)
 
 void launch_duplicate(const DuplicateArgs& a, cudaStream_t stream) {
   if (a.P <= 0 || a.R == 0) return;
-  const int blocks = (a.P + kDupThreads - 1) / kDupThreads;
+  // enough blocks to clear 16 KB each when the Gaussians need fewer
+  const int blocks = max((a.P + kDupThreads - 1) / kDupThreads, min(296, int(a.clear_vecs / 1024u)));
   stage_begin(kStDuplicate, stream);
   if (a.key64) duplicate_kernel<true><<<blocks, kDupThreads, 0, stream>>>(a);
   else duplicate_kernel<false><<<blocks, kDupThreads, 0, stream>>>(a);

@@ -100,7 +100,15 @@ struct DuplicateArgs {
   const float* depth;
   void* keys;
   uint32_t* vals;
-  const uint32_t* n_dev = nullptr;  // planned render: the instance count in device memory (R is then the capacity)
+  // The emission also writes the binning state's header -- it is the first
+  // kernel of a render -- and clears what the sort needs zeroed.  plan: a planned
+  // render's projection header (the plan is checked against its count and depth
+  // range, R is then the capacity); null: the header is written as given.
+  BinHeader* header;
+  const GeomHeader* plan;
+  uint32_t tile_bits, passes, depth_prefix;
+  uint4* clear;         // 16-byte aligned span
+  uint32_t clear_vecs;  // uint4s in it
 };
 void launch_duplicate(const DuplicateArgs& a, cudaStream_t stream);
 
@@ -124,7 +132,7 @@ struct SortArgs {
   uint32_t* vals_tmp;
   uint32_t* hist;        // [kMaxPasses * kMaxBins]
   uint32_t* status;      // [kMaxPasses * sort_tiles * kMaxBins]
-  uint32_t* counters;    // [kMaxPasses]
+  uint32_t* counters;    // [kMaxPasses + 1]: per pass, then the histogram's finished blocks
   uint32_t* error;
   uint32_t spin_limit = kSpinLimit;  // bounded waits (spin_limit())
   long long unpublished_tile = -1;   // first pass: tile that skips publishing (tests; -1 = none)
@@ -135,6 +143,12 @@ struct SortArgs {
   int num_tiles;
   uint32_t* tile_hist;
   uint2* ranges;
+  // with ranges (else ignored): the tiles by decreasing list length, and the
+  // words to clear on the way (tile_order_block)
+  uint32_t* order = nullptr;
+  uint32_t* order_zero = nullptr;
+  uint32_t* order_counter = nullptr;
+  bool cleared = false;  // the caller has zeroed hist, the used status words, counters and tile_hist
   // optional: one span to zero instead of the four buffers above (hist, the
   // used status words, counters, tile_hist), when the caller's layout makes
   // them contiguous
@@ -142,7 +156,7 @@ struct SortArgs {
   size_t clear_bytes;
 };
 int sort_passes(int bits);
-long long sort_tile_keys(int key64);  // keys per onesweep tile for the key width
+long long sort_tile_keys(int key64, long long n);  // keys per onesweep tile for the key width and count
 int sort_digit_bits(int bits);
 void launch_sort(const SortArgs& a, cudaStream_t stream);
 size_t sort_status_words(long long n);
@@ -163,8 +177,8 @@ struct BlendArgs {
   uint32_t* n_contrib;
   float* T_final;
   uint32_t* tile_max;
-  uint32_t* order;      // tiles by decreasing list length (the blend's processing order)
-  uint32_t* order_bwd;  // tiles by decreasing largest contributor count (the backward's)
+  uint32_t* order;      // tiles by decreasing list length (the processing order, the backward's too)
+  bool ordered = false;  // the sort has written order and cleared tile_max and queue
   uint32_t* queue;      // the persistent blend's queue counter (cleared before its launch), or null
   uint32_t* error;      // error word for the persistent blend's bounded waits, or null
   uint32_t* masks_valid;  // the binning header's block-mask flag (the persistent blend clears it), or null
@@ -197,8 +211,7 @@ struct BackwardArgs {
   const uint2* ranges;
   const uint32_t* point_list;
   const uint32_t* n_contrib;
-  const uint32_t* tile_max;
-  const uint32_t* order_bwd;  // tile order by largest contributor count (written by the blend)
+  const uint32_t* order;      // the blend's tile order
   const uint32_t* masks;      // the blend's block masks (tile_walk.cuh mask_row); null: test each entry
   const uint32_t* masks_valid;
   const float* T_final;

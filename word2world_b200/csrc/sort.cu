@@ -8,11 +8,12 @@
 //
 //   1. histogram kernel: one read of the keys gives the digit histogram of
 //      every pass, plus the histogram of key >> tile_shift (the per-tile
-//      instance counts);
-//   2. offsets kernel: exclusive scans of those histograms; the tile scan is
-//      the per-tile [start, end) range table (empty tiles get (0, 0), as the
-//      reference's memset leaves them);
-//   3. one onesweep kernel per digit: each CTA takes the next tile (6144 32-bit or 5120 64-bit keys)
+//      instance counts).  Its last block to finish scans those histograms; the
+//      tile scan is the per-tile [start, end) range table (empty tiles get (0,
+//      0), as the reference's memset leaves them), and the tiles' processing
+//      order follows from it (two one-block kernels before: 7 us a view with
+//      their launches);
+//   2. one onesweep kernel per digit: each CTA takes the next tile (6144 32-bit or 5120 64-bit keys)
 //      (acquired through an atomic counter, so every earlier tile is already
 //      running), ranks its keys stably (warp match.any or per-bit ballots), publishes its
 //      per-digit counts and looks back over earlier tiles for their prefix
@@ -31,6 +32,7 @@
 // stable 2-bit passes produce, so equal keys keep their input order.
 #include "common.cuh"
 #include "kernels.h"
+#include "tile_walk.cuh"
 
 namespace w2w {
 namespace {
@@ -38,9 +40,14 @@ namespace {
 constexpr uint32_t kStatAgg = 1u << 30;
 constexpr uint32_t kStatInc = 2u << 30;
 constexpr uint32_t kStatMask = (1u << 30) - 1u;
-constexpr int kHistThreads = 256;
-constexpr int kSmemTileBins = 8192;
-
+// Threads of a histogram block: 256, four blocks to an SM, while the tile counts
+// fit beside the digit histograms in a quarter of the shared memory; 1024 and
+// one block beyond that, up to kSmemTileBins tiles; past it the tile counts go
+// straight to memory.  (12 views, 9216 tiles: 205 us with global counts, %HB%
+// with 1024 threads.)
+constexpr int kHistThreads = 256, kHistThreadsBig = 1024;
+constexpr int kSmemTileBinsSmall = 8192;
+constexpr int kSmemTileBins = 48 * 1024;
 // Width of pass p's digit.
 __host__ __device__ __forceinline__ int pass_width(int p, int dbits, int bits) {
   const int left = bits - p * dbits;
@@ -90,42 +97,6 @@ __device__ __forceinline__ void count_run(const K (&k)[kHistRun], int cnt, int s
   if (cur < limit) atomicAdd(&counters[cur], run);
 }
 
-template <typename K>
-__global__ void __launch_bounds__(kHistThreads)
-hist_kernel(const K* __restrict__ keys, long long n, int begin_bit, int passes, int dbits, int bits,
-            uint32_t* __restrict__ hist, int tile_shift, int num_tiles, uint32_t* __restrict__ tile_hist,
-            const uint32_t* __restrict__ n_dev) {
-  extern __shared__ uint32_t smem[];
-  uint32_t* sh = smem;                      // passes * kMaxBins
-  uint32_t* st = smem + passes * kMaxBins;  // num_tiles when they fit
-  const bool tiles_in_smem = tile_hist != nullptr && num_tiles <= kSmemTileBins;
-  for (int i = threadIdx.x; i < passes * kMaxBins; i += blockDim.x) sh[i] = 0;
-  if (tiles_in_smem)
-    for (int i = threadIdx.x; i < num_tiles; i += blockDim.x) st[i] = 0;
-  __syncthreads();
-  // n < 2^30 (checked by every caller); a planned render's count is in device memory
-  const uint32_t nn = n_dev != nullptr ? min(*n_dev, uint32_t(n)) : uint32_t(n);
-  const bool vec = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0u;
-  const uint32_t runs = (nn + kHistRun - 1) / kHistRun;
-  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < runs; c += gridDim.x * blockDim.x) {
-    K k[kHistRun];
-    const uint32_t i0 = c * kHistRun;
-    load_run(keys, i0, nn, vec, k);
-    const int cnt = int(min(uint32_t(kHistRun), nn - i0));
-    for (int p = 0; p < passes; ++p)
-      count_run(k, cnt, begin_bit + dbits * p, (1u << pass_width(p, dbits, bits)) - 1u, 0xffffffffu,
-                sh + p * kMaxBins);
-    if (tile_hist != nullptr)
-      count_run(k, cnt, tile_shift, 0xffffffffu, uint32_t(num_tiles), tiles_in_smem ? st : tile_hist);
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < passes * kMaxBins; i += blockDim.x)
-    if (sh[i]) atomicAdd(&hist[i], sh[i]);
-  if (tiles_in_smem)
-    for (int i = threadIdx.x; i < num_tiles; i += blockDim.x)
-      if (st[i]) atomicAdd(&tile_hist[i], st[i]);
-}
-
 // Block-wide exclusive scan of one value per thread (blockDim.x <= 1024).
 __device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s_warp, uint32_t* total) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
@@ -155,30 +126,96 @@ __device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s_warp, uint32_t*
 }
 
 // Digit histograms -> exclusive digit offsets (in place); tile histogram ->
-// [start, end) ranges.  One block of 1024 threads.
-__global__ void __launch_bounds__(1024)
-offsets_kernel(uint32_t* hist, int passes, const uint32_t* tile_hist, int num_tiles, uint2* ranges) {
+// [start, end) ranges.  The whole block; the counts are other blocks' atomics,
+// read past the L1.
+__device__ __forceinline__ void offsets_block(uint32_t* hist, int passes, const uint32_t* tile_hist, int num_tiles,
+                                              uint2* ranges) {
   __shared__ uint32_t s_warp[32];
-  __shared__ uint32_t s_carry;
   for (int p = 0; p < passes; ++p) {
-    const uint32_t v = threadIdx.x < kMaxBins ? hist[p * kMaxBins + threadIdx.x] : 0u;
-    const uint32_t ex = block_exclusive_scan(v, s_warp, nullptr);
-    if (threadIdx.x < kMaxBins) hist[p * kMaxBins + threadIdx.x] = ex;
-    __syncthreads();
+    // kMaxBins bins over the block's threads, consecutive ones to a thread
+    const int per = kMaxBins > int(blockDim.x) ? kMaxBins / int(blockDim.x) : 1;
+    const int b0 = int(threadIdx.x) * per;
+    uint32_t v[kMaxBins / kHistThreads], sum = 0;
+#pragma unroll
+    for (int k = 0; k < kMaxBins / kHistThreads; ++k) {
+      v[k] = k < per && b0 + k < kMaxBins ? __ldcg(hist + p * kMaxBins + b0 + k) : 0u;
+      sum += v[k];
+    }
+    uint32_t ex = block_exclusive_scan(sum, s_warp, nullptr);
+#pragma unroll
+    for (int k = 0; k < kMaxBins / kHistThreads; ++k) {
+      if (k < per && b0 + k < kMaxBins) hist[p * kMaxBins + b0 + k] = ex;
+      ex += v[k];
+    }
   }
   if (tile_hist == nullptr || ranges == nullptr) return;
-  if (threadIdx.x == 0) s_carry = 0;
+  constexpr int kPer = 4;  // tiles per thread and round
+  uint32_t carry = 0;
+  for (int base = 0; base < num_tiles; base += int(blockDim.x) * kPer) {
+    const int t0 = base + int(threadIdx.x) * kPer;
+    uint32_t c[kPer], sum = 0, tot;
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      c[k] = t0 + k < num_tiles ? __ldcg(tile_hist + t0 + k) : 0u;
+      sum += c[k];
+    }
+    uint32_t start = carry + block_exclusive_scan(sum, s_warp, &tot);
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      if (t0 + k < num_tiles) ranges[t0 + k] = c[k] ? make_uint2(start, start + c[k]) : make_uint2(0u, 0u);
+      start += c[k];
+    }
+    carry += tot;
+  }
+}
+
+template <typename K>
+__global__ void __launch_bounds__(kHistThreadsBig)
+hist_kernel(const K* __restrict__ keys, long long n, int begin_bit, int passes, int dbits, int bits,
+            uint32_t* __restrict__ hist, int tile_shift, int num_tiles, uint32_t* __restrict__ tile_hist,
+            const uint32_t* __restrict__ n_dev, uint2* __restrict__ ranges, uint32_t* done, uint32_t* order,
+            uint32_t* order_zero, uint32_t* order_counter) {
+  extern __shared__ uint32_t smem[];
+  uint32_t* sh = smem;                      // passes * kMaxBins
+  uint32_t* st = smem + passes * kMaxBins;  // num_tiles when they fit
+  const bool tiles_in_smem = tile_hist != nullptr && num_tiles <= kSmemTileBins;
+  for (int i = threadIdx.x; i < passes * kMaxBins; i += blockDim.x) sh[i] = 0;
+  if (tiles_in_smem)
+    for (int i = threadIdx.x; i < num_tiles; i += blockDim.x) st[i] = 0;
   __syncthreads();
-  for (int base = 0; base < num_tiles; base += blockDim.x) {
-    const int t = base + threadIdx.x;
-    const uint32_t c = t < num_tiles ? tile_hist[t] : 0u;
-    uint32_t tot;
-    const uint32_t ex = block_exclusive_scan(c, s_warp, &tot);
-    const uint32_t start = s_carry + ex;
-    if (t < num_tiles) ranges[t] = c ? make_uint2(start, start + c) : make_uint2(0u, 0u);
-    __syncthreads();
-    if (threadIdx.x == 0) s_carry += tot;
-    __syncthreads();
+  // n < 2^30 (checked by every caller); a planned render's count is in device memory
+  const uint32_t nn = n_dev != nullptr ? min(*n_dev, uint32_t(n)) : uint32_t(n);
+  const bool vec = (reinterpret_cast<uintptr_t>(keys) & 15u) == 0u;
+  const uint32_t runs = (nn + kHistRun - 1) / kHistRun;
+  for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < runs; c += gridDim.x * blockDim.x) {
+    K k[kHistRun];
+    const uint32_t i0 = c * kHistRun;
+    load_run(keys, i0, nn, vec, k);
+    const int cnt = int(min(uint32_t(kHistRun), nn - i0));
+    for (int p = 0; p < passes; ++p)
+      count_run(k, cnt, begin_bit + dbits * p, (1u << pass_width(p, dbits, bits)) - 1u, 0xffffffffu,
+                sh + p * kMaxBins);
+    if (tile_hist != nullptr)
+      count_run(k, cnt, tile_shift, 0xffffffffu, uint32_t(num_tiles), tiles_in_smem ? st : tile_hist);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < passes * kMaxBins; i += blockDim.x)
+    if (sh[i]) atomicAdd(&hist[i], sh[i]);
+  if (tiles_in_smem)
+    for (int i = threadIdx.x; i < num_tiles; i += blockDim.x)
+      if (st[i]) atomicAdd(&tile_hist[i], st[i]);
+  // the last block to get here has every block's counts
+  __shared__ bool s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) + 1u == gridDim.x;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  offsets_block(hist, passes, tile_hist, num_tiles, ranges);
+  if (ranges != nullptr && order != nullptr) {
+    __syncthreads();  // the ranges are this block's own
+    tile_order_block(ranges, num_tiles, order, order_zero, order_counter);
   }
 }
 
@@ -246,20 +283,28 @@ struct LookbackWindow {
 // 59.7, 68.0 us) and 16 at 3 (59.8 us); 64-bit keys (20M pairs) 20 items at 2
 // CTAs/SM 174.5 us, against 16 / 24 at 2 (186.8, 203.0 us) and 12 / 16 at 3
 // (218.7, 211.2 us).
-template <typename K>
+// Up to kSortSmall keys (114 tiles of 6144: fewer than the SMs) the pass is one
+// tile's own chain of load, count, rank, look back and reorder, which a tile of
+// 2048 keys runs in half the time (kSmall): %SMALL%
+template <typename K, bool kSmall>
 struct OnesweepShape;
+template <typename K>
+struct OnesweepShape<K, true> {
+  static constexpr int kItems = 8, kMinBlocks = 3;
+};
 template <>
-struct OnesweepShape<uint32_t> {
+struct OnesweepShape<uint32_t, false> {
   static constexpr int kItems = 24, kMinBlocks = 2;
 };
 template <>
-struct OnesweepShape<uint64_t> {
+struct OnesweepShape<uint64_t, false> {
   static constexpr int kItems = 20, kMinBlocks = 2;
 };
-template <typename K>
-__host__ __device__ constexpr int onesweep_tile() { return kSortThreads * OnesweepShape<K>::kItems; }
-static_assert(onesweep_tile<uint32_t>() >= kSortTileMin && onesweep_tile<uint64_t>() >= kSortTileMin,
-              "scratch is sized for tiles of at least kSortTileMin keys");
+template <typename K, bool kSmall>
+__host__ __device__ constexpr int onesweep_tile() { return kSortThreads * OnesweepShape<K, kSmall>::kItems; }
+static_assert(onesweep_tile<uint32_t, false>() >= kSortTileMin && onesweep_tile<uint64_t, false>() >= kSortTileMin &&
+                  onesweep_tile<uint32_t, true>() >= kSortTileSmall && onesweep_tile<uint64_t, true>() >= kSortTileSmall,
+              "status words are sized for tiles of at least this many keys");
 
 template <typename K>
 struct OnesweepShared {
@@ -272,7 +317,7 @@ struct OnesweepShared {
 
 // One tile of a pass.  kFull: every key of the tile exists (all tiles but the
 // last), so the per-key bounds checks drop out.  Indices are 32-bit (n < 2^30).
-template <typename K, int kWidth, bool kFull, bool kMatch>
+template <typename K, int kWidth, bool kFull, bool kMatch, bool kSmall>
 __device__ __forceinline__ void onesweep_tile_pass(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
                                                    K* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t n,
                                                    int shift, const uint32_t* __restrict__ digit_base,
@@ -280,8 +325,8 @@ __device__ __forceinline__ void onesweep_tile_pass(const K* __restrict__ kin, co
                                                    uint32_t spin_limit, bool publish, OnesweepShared<K>& sm,
                                                    K* s_keys, uint32_t* s_vals) {
   constexpr int kWarps = kSortThreads / 32;
-  constexpr int kItems = OnesweepShape<K>::kItems;
-  constexpr int kTile = onesweep_tile<K>();
+  constexpr int kItems = OnesweepShape<K, kSmall>::kItems;
+  constexpr int kTile = onesweep_tile<K, kSmall>();
   constexpr int bins = 1 << kWidth;
   const uint32_t dmask = uint32_t(bins) - 1u;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -399,13 +444,13 @@ __device__ __forceinline__ void onesweep_tile_pass(const K* __restrict__ kin, co
 // match.any (keys whose warps hold few distinct digits, such as the
 // rasterizer's, emitted Gaussian by Gaussian) or with one ballot per digit
 // bit (constant cost whatever the keys: random keys).
-template <typename K, int kWidth, bool kMatch>
-__global__ void __launch_bounds__(kSortThreads, OnesweepShape<K>::kMinBlocks)
+template <typename K, int kWidth, bool kMatch, bool kSmall>
+__global__ void __launch_bounds__(kSortThreads, (OnesweepShape<K, kSmall>::kMinBlocks))
 onesweep_kernel(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restrict__ kout,
                 uint32_t* __restrict__ vout, long long n, int shift,
                 const uint32_t* __restrict__ digit_base, uint32_t* status, uint32_t* counter, uint32_t* err,
                 uint32_t spin_limit, long long unpublished_tile, const uint32_t* __restrict__ n_dev) {
-  constexpr int kTile = onesweep_tile<K>();
+  constexpr int kTile = onesweep_tile<K, kSmall>();
   static_assert(kSortThreads * 2 >= kMaxBins, "at most two digits per thread");
   __shared__ __align__(16) OnesweepShared<K> sm;
   extern __shared__ __align__(16) unsigned char s_dyn[];
@@ -430,32 +475,32 @@ onesweep_kernel(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* 
   if ((unsigned long long)tile * kTile >= nn) return;
   const bool publish = (long long)tile != unpublished_tile;
   if ((unsigned long long)(tile + 1) * kTile <= nn)
-    onesweep_tile_pass<K, kWidth, true, kMatch>(kin, vin, kout, vout, nn, shift, digit_base, status, err, tile, spin_limit,
+    onesweep_tile_pass<K, kWidth, true, kMatch, kSmall>(kin, vin, kout, vout, nn, shift, digit_base, status, err, tile, spin_limit,
                                         publish, sm, s_keys, s_vals);
   else
-    onesweep_tile_pass<K, kWidth, false, kMatch>(kin, vin, kout, vout, nn, shift, digit_base, status, err, tile, spin_limit,
+    onesweep_tile_pass<K, kWidth, false, kMatch, kSmall>(kin, vin, kout, vout, nn, shift, digit_base, status, err, tile, spin_limit,
                                          publish, sm, s_keys, s_vals);
 }
 
-template <typename K, int kWidth, bool kMatch>
+template <typename K, int kWidth, bool kMatch, bool kSmall>
 void launch_onesweep_w(int tiles, cudaStream_t stream, const K* kin, const uint32_t* vin, K* kout, uint32_t* vout,
                        long long n, int shift, const uint32_t* digit_base, uint32_t* status, uint32_t* counter,
                        uint32_t* err, uint32_t spin_limit, long long unpublished, const uint32_t* n_dev) {
-  const size_t dyn = (sizeof(K) + sizeof(uint32_t)) * size_t(onesweep_tile<K>());
+  const size_t dyn = (sizeof(K) + sizeof(uint32_t)) * size_t(onesweep_tile<K, kSmall>());
   // the shared-memory opt-in is set once per device (a driver call per launch
   // would widen the gap the device waits between launches)
   static bool opted[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !opted[dev]) {
-    cudaFuncSetAttribute(onesweep_kernel<K, kWidth, kMatch>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn));
+    cudaFuncSetAttribute(onesweep_kernel<K, kWidth, kMatch, kSmall>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn));
     if (dev >= 0 && dev < 64) opted[dev] = true;
   }
-  onesweep_kernel<K, kWidth, kMatch><<<tiles, kSortThreads, dyn, stream>>>(kin, vin, kout, vout, n, shift, digit_base,
+  onesweep_kernel<K, kWidth, kMatch, kSmall><<<tiles, kSortThreads, dyn, stream>>>(kin, vin, kout, vout, n, shift, digit_base,
                                                                     status, counter, err, spin_limit, unpublished, n_dev);
 }
 
-template <typename K>
+template <typename K, bool kSmall>
 void launch_onesweep(int width, int tiles, cudaStream_t stream, const K* kin, const uint32_t* vin, K* kout,
                      uint32_t* vout, long long n, int shift, const uint32_t* digit_base, uint32_t* status,
                      uint32_t* counter, uint32_t* err, uint32_t spin_limit, long long unpublished, bool match,
@@ -464,10 +509,10 @@ void launch_onesweep(int width, int tiles, cudaStream_t stream, const K* kin, co
 #define W2W_ONESWEEP_CASE(W)                                                                                      \
   case W:                                                                                                         \
     if (match)                                                                                                    \
-      launch_onesweep_w<K, W, true>(tiles, stream, kin, vin, kout, vout, n, shift, digit_base, status, counter,   \
+      launch_onesweep_w<K, W, true, kSmall>(tiles, stream, kin, vin, kout, vout, n, shift, digit_base, status, counter,   \
                                     err, spin_limit, unpublished, n_dev);                                         \
     else                                                                                                          \
-      launch_onesweep_w<K, W, false>(tiles, stream, kin, vin, kout, vout, n, shift, digit_base, status, counter,  \
+      launch_onesweep_w<K, W, false, kSmall>(tiles, stream, kin, vin, kout, vout, n, shift, digit_base, status, counter,  \
                                      err, spin_limit, unpublished, n_dev);                                        \
     break;
     W2W_ONESWEEP_CASE(1) W2W_ONESWEEP_CASE(2) W2W_ONESWEEP_CASE(3) W2W_ONESWEEP_CASE(4) W2W_ONESWEEP_CASE(5)
@@ -484,12 +529,16 @@ void run_sort(const SortArgs& a, cudaStream_t stream) {
   const int dbits = sort_digit_bits(a.bits);
   const long long n = a.n;
   if (n <= 0) return;
-  const long long tiles = (n + onesweep_tile<K>() - 1) / onesweep_tile<K>();
-  if (a.clear_span != nullptr) {  // the caller's layout puts everything to clear in one span
+  const bool small = n <= kSortSmall;
+  const long long tile_keys = sort_tile_keys(sizeof(K) == 8 ? 1 : 0, n);
+  const long long tiles = (n + tile_keys - 1) / tile_keys;
+  if (a.cleared) {
+    // nothing to clear
+  } else if (a.clear_span != nullptr) {  // the caller's layout puts everything to clear in one span
     cudaMemsetAsync(a.clear_span, 0, a.clear_bytes, stream);
   } else {
     cudaMemsetAsync(a.hist, 0, sizeof(uint32_t) * kMaxBins * kMaxPasses, stream);
-    cudaMemsetAsync(a.counters, 0, sizeof(uint32_t) * kMaxPasses, stream);
+    cudaMemsetAsync(a.counters, 0, sizeof(uint32_t) * (kMaxPasses + 1), stream);
     cudaMemsetAsync(a.status, 0, sizeof(uint32_t) * kMaxBins * size_t(tiles) * size_t(passes > 0 ? passes : 1),
                     stream);
     if (a.tile_hist) cudaMemsetAsync(a.tile_hist, 0, sizeof(uint32_t) * size_t(a.num_tiles), stream);
@@ -500,20 +549,22 @@ void run_sort(const SortArgs& a, cudaStream_t stream) {
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // a few blocks per SM: each block's flush is passes * kMaxBins global atomics (4 per SM measured
     // 0.119 ms of histogram per 4-view step against 0.129 with 2 and 0.135 with 8)
-    const long long want = (n + kHistThreads * kHistRun * 4 - 1) / (kHistThreads * kHistRun * 4);
-    const int grid = int(max(1LL, min(want, (long long)sms * 4)));
     const bool tiles_in_smem = a.tile_hist != nullptr && a.num_tiles <= kSmemTileBins;
+    const bool big = tiles_in_smem && a.num_tiles > kSmemTileBinsSmall;
+    const int threads = big ? kHistThreadsBig : kHistThreads;
+    const long long per_block = (long long)threads * kHistRun * 4;
+    const int grid = int(max(1LL, min((n + per_block - 1) / per_block, (long long)sms * (big ? 1 : 4))));
     const size_t smem =
         sizeof(uint32_t) * (size_t(passes) * kMaxBins + (tiles_in_smem ? size_t(a.num_tiles) : 0));
-    if (smem > 48 * 1024)
+    if (smem > 40 * 1024)  // beside the scans' own
       cudaFuncSetAttribute(hist_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     const int st_hist = a.stage_hist >= 0 ? a.stage_hist : kStSortHist;
     stage_begin(st_hist, stream);
-    hist_kernel<K><<<grid, kHistThreads, smem, stream>>>(reinterpret_cast<const K*>(a.keys_in), n, a.begin_bit,
-                                                         passes, dbits, a.bits, a.hist, a.tile_shift,
-                                                         a.num_tiles, a.tile_hist, a.n_dev);
-    offsets_kernel<<<1, 1024, 0, stream>>>(a.hist, passes, a.tile_hist, a.num_tiles, a.ranges);
-    stage_end(st_hist, stream, 2);
+    hist_kernel<K><<<grid, threads, smem, stream>>>(reinterpret_cast<const K*>(a.keys_in), n, a.begin_bit,
+                                                    passes, dbits, a.bits, a.hist, a.tile_shift,
+                                                    a.num_tiles, a.tile_hist, a.n_dev, a.ranges,
+                                                    a.counters + kMaxPasses, a.order, a.order_zero, a.order_counter);
+    stage_end(st_hist, stream, 1);
   }
   const K* kin = reinterpret_cast<const K*>(a.keys_in);
   const uint32_t* vin = a.vals_in;
@@ -523,10 +574,13 @@ void run_sort(const SortArgs& a, cudaStream_t stream) {
     uint32_t* vout = to_out ? a.vals_out : a.vals_tmp;
     const int st_pass = a.stage_pass >= 0 ? a.stage_pass : kStSortPass;
     stage_begin(st_pass, stream);
-    launch_onesweep<K>(pass_width(p, dbits, a.bits), int(tiles), stream, kin, vin, kout, vout, n,
-                       a.begin_bit + dbits * p, a.hist + kMaxBins * p,
-                       a.status + size_t(p) * kMaxBins * size_t(tiles), a.counters + p, a.error,
-                       a.spin_limit, p == 0 ? a.unpublished_tile : -1LL, a.match_rank != 0, a.n_dev);
+    auto pass = [&](auto launch) {
+      launch(pass_width(p, dbits, a.bits), int(tiles), stream, kin, vin, kout, vout, n, a.begin_bit + dbits * p,
+             a.hist + kMaxBins * p, a.status + size_t(p) * kMaxBins * size_t(tiles), a.counters + p, a.error,
+             a.spin_limit, p == 0 ? a.unpublished_tile : -1LL, a.match_rank != 0, a.n_dev);
+    };
+    if (small) pass(launch_onesweep<K, true>);
+    else pass(launch_onesweep<K, false>);
     stage_end(st_pass, stream, 1);
     kin = kout;
     vin = vout;
@@ -539,7 +593,10 @@ void run_sort(const SortArgs& a, cudaStream_t stream) {
 
 }  // namespace
 
-long long sort_tile_keys(int key64) { return key64 ? onesweep_tile<uint64_t>() : onesweep_tile<uint32_t>(); }
+long long sort_tile_keys(int key64, long long n) {
+  if (n <= kSortSmall) return key64 ? onesweep_tile<uint64_t, true>() : onesweep_tile<uint32_t, true>();
+  return key64 ? onesweep_tile<uint64_t, false>() : onesweep_tile<uint32_t, false>();
+}
 
 int sort_passes(int bits) { return bits <= 0 ? 0 : (bits + kMaxDigitBits - 1) / kMaxDigitBits; }
 
@@ -549,7 +606,7 @@ int sort_digit_bits(int bits) {
 }
 
 size_t sort_status_words(long long n) {
-  const long long tiles = (n + kSortTileMin - 1) / kSortTileMin;
+  const long long tiles = sort_status_tiles(n);
   return size_t(kMaxPasses) * kMaxBins * size_t(tiles > 0 ? tiles : 1);
 }
 
