@@ -487,7 +487,6 @@ int w2w_forward_render(const w2w_settings* s, const void* geom_state, const w2w_
     launch_duplicate(d, st);
     so.n = R; so.key64 = kp.key64; so.begin_bit = 0; so.bits = kp.bits;
     so.keys_in = d.keys; so.vals_in = d.vals;
-    so.match_rank = 1;  // emitted Gaussian by Gaussian: few distinct digits per warp
     so.keys_out = keysA; so.vals_out = valsA;
     so.keys_tmp = keysB; so.vals_tmp = valsB;
     so.hist = at<uint32_t>(binning_state, BL.hist);
@@ -676,7 +675,6 @@ int w2w_forward_render_planned(const w2w_settings* s, const void* geom_state, lo
   launch_duplicate(d, st);
   so.n = capacity; so.key64 = kp.key64; so.begin_bit = 0; so.bits = kp.bits;
   so.keys_in = d.keys; so.vals_in = d.vals;
-  so.match_rank = 1;  // emitted Gaussian by Gaussian: few distinct digits per warp
   so.n_dev = &bh->n_sort;
   so.keys_out = keysA; so.vals_out = valsA;
   so.keys_tmp = keysB; so.vals_tmp = valsB;
@@ -1381,7 +1379,6 @@ int w2w_batch_forward_render(const w2w_batch_item* items, int n, const void* geo
     launch_duplicate(d, st);
     so.n = R; so.key64 = kp.key64; so.begin_bit = 0; so.bits = kp.bits;
     so.keys_in = d.keys; so.vals_in = d.vals;
-    so.match_rank = 1;  // emitted Gaussian by Gaussian: few distinct digits per warp
     so.keys_out = keysA; so.vals_out = valsA;
     so.keys_tmp = keysB; so.vals_tmp = valsB;
     so.hist = at<uint32_t>(binning_state, BL.hist);

@@ -15,17 +15,18 @@
 //      their launches);
 //   2. one onesweep kernel per digit: each CTA takes the next tile (6144 32-bit or 5120 64-bit keys)
 //      (acquired through an atomic counter, so every earlier tile is already
-//      running), ranks its keys stably (warp match.any or per-bit ballots), publishes its
+//      running), ranks its keys stably (per-bit warp ballots), publishes its
 //      per-digit counts and looks back over earlier tiles for their prefix
 //      (decoupled lookback), then scatters through shared memory so the
 //      global stores are coalesced.  Every wait is bounded: a wait that runs
 //      out sets kErrTimeout and the kernel finishes without hanging.
 //
-// Ranking: match.any costs little when a warp's 32 keys hold few distinct
-// digits, as the rasterizer's keys do (emitted Gaussian by Gaussian): 1.5 %
-// faster per pass than ballots there; on random keys (the standalone sort) it
-// measured 12 % slower than one ballot per digit bit, so SortArgs::match_rank
-// chooses.
+// Ranking: one ballot per digit bit, four operations each (match_bit).  A
+// match.any per key costs more the more distinct digits a warp's 32 keys hold:
+// it was 1.5 % faster than six-operation ballots on the rasterizer's keys
+// (emitted Gaussian by Gaussian), and is 18 % slower than these (a 9-bit pass
+// over 5.9M pairs 54 against 46 us; 20M random 64-bit pairs, 44 bits: 914 us of
+// passes with six operations, 857 with four).
 //
 // Stability: keys are ranked in input order within a warp, warps in order
 // within a tile, tiles in order globally -- the same order the reference's
@@ -315,9 +316,29 @@ struct OnesweepShared {
   uint32_t tile;
 };
 
+// The lanes of `pm` whose `bit` of d agrees with this lane's: one test, one
+// ballot, one select and one three-input logic operation.  (As a ternary over
+// the ballot and its complement it compiled to six operations; the ranking's
+// are most of a 64-bit pass's, and the ALU its busiest pipe.)
+__device__ __forceinline__ uint32_t match_bit(uint32_t pm, uint32_t d, uint32_t bit) {
+  uint32_t r;
+  asm volatile("{\n\t"
+               ".reg .pred p;\n\t"
+               ".reg .b32 t, b, m;\n\t"
+               "and.b32 t, %2, %3;\n\t"
+               "setp.ne.u32 p, t, 0;\n\t"
+               "vote.sync.ballot.b32 b, p, 0xffffffff;\n\t"
+               "selp.b32 m, 0xffffffff, 0, p;\n\t"
+               "lop3.b32 %0, %1, b, m, 0x90;\n\t"  // pm & ~(ballot ^ m)
+               "}"
+               : "=r"(r)
+               : "r"(pm), "r"(d), "r"(bit));
+  return r;
+}
+
 // One tile of a pass.  kFull: every key of the tile exists (all tiles but the
 // last), so the per-key bounds checks drop out.  Indices are 32-bit (n < 2^30).
-template <typename K, int kWidth, bool kFull, bool kMatch, bool kSmall>
+template <typename K, int kWidth, bool kFull, bool kSmall>
 __device__ __forceinline__ void onesweep_tile_pass(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
                                                    K* __restrict__ kout, uint32_t* __restrict__ vout, uint32_t n,
                                                    int shift, const uint32_t* __restrict__ digit_base,
@@ -378,21 +399,14 @@ __device__ __forceinline__ void onesweep_tile_pass(const K* __restrict__ kin, co
 
   // stable rank within the tile's digit: warp base + earlier items of the warp
   // + earlier lanes of this item holding the same digit (the lanes holding
-  // it: one match.any, or one ballot per digit bit; see "Ranking" above)
+  // it: match_bit)
 #pragma unroll
   for (int i = 0; i < kItems; ++i) {
     const uint32_t d = uint32_t(k[i] >> shift) & dmask;
     const bool valid = kFull || wbase + uint32_t(i * 32) < n;
     uint32_t pm = kFull ? 0xffffffffu : __ballot_sync(0xffffffffu, valid);
-    if constexpr (kMatch) {
-      pm &= __match_any_sync(0xffffffffu, d);
-    } else {
 #pragma unroll
-      for (int bt = 0; bt < kWidth; ++bt) {
-        const uint32_t bal = __ballot_sync(0xffffffffu, (d >> bt) & 1u);
-        pm &= ((d >> bt) & 1u) ? bal : ~bal;
-      }
-    }
+    for (int bt = 0; bt < kWidth; ++bt) pm = match_bit(pm, d, 1u << bt);
     const uint32_t before = valid ? sm.wcnt[warp][d] : 0u;
     rank[i] = before + __popc(pm & lt);
     __syncwarp();
@@ -440,11 +454,8 @@ __device__ __forceinline__ void onesweep_tile_pass(const K* __restrict__ kin, co
   }
 }
 
-// kWidth: this pass's digit width (compile-time).  kMatch: rank with
-// match.any (keys whose warps hold few distinct digits, such as the
-// rasterizer's, emitted Gaussian by Gaussian) or with one ballot per digit
-// bit (constant cost whatever the keys: random keys).
-template <typename K, int kWidth, bool kMatch, bool kSmall>
+// kWidth: this pass's digit width (compile-time).
+template <typename K, int kWidth, bool kSmall>
 __global__ void __launch_bounds__(kSortThreads, (OnesweepShape<K, kSmall>::kMinBlocks))
 onesweep_kernel(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restrict__ kout,
                 uint32_t* __restrict__ vout, long long n, int shift,
@@ -475,14 +486,14 @@ onesweep_kernel(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* 
   if ((unsigned long long)tile * kTile >= nn) return;
   const bool publish = (long long)tile != unpublished_tile;
   if ((unsigned long long)(tile + 1) * kTile <= nn)
-    onesweep_tile_pass<K, kWidth, true, kMatch, kSmall>(kin, vin, kout, vout, nn, shift, digit_base, status, err, tile, spin_limit,
+    onesweep_tile_pass<K, kWidth, true, kSmall>(kin, vin, kout, vout, nn, shift, digit_base, status, err, tile, spin_limit,
                                         publish, sm, s_keys, s_vals);
   else
-    onesweep_tile_pass<K, kWidth, false, kMatch, kSmall>(kin, vin, kout, vout, nn, shift, digit_base, status, err, tile, spin_limit,
+    onesweep_tile_pass<K, kWidth, false, kSmall>(kin, vin, kout, vout, nn, shift, digit_base, status, err, tile, spin_limit,
                                          publish, sm, s_keys, s_vals);
 }
 
-template <typename K, int kWidth, bool kMatch, bool kSmall>
+template <typename K, int kWidth, bool kSmall>
 void launch_onesweep_w(int tiles, cudaStream_t stream, const K* kin, const uint32_t* vin, K* kout, uint32_t* vout,
                        long long n, int shift, const uint32_t* digit_base, uint32_t* status, uint32_t* counter,
                        uint32_t* err, uint32_t spin_limit, long long unpublished, const uint32_t* n_dev) {
@@ -493,27 +504,22 @@ void launch_onesweep_w(int tiles, cudaStream_t stream, const K* kin, const uint3
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64 || !opted[dev]) {
-    cudaFuncSetAttribute(onesweep_kernel<K, kWidth, kMatch, kSmall>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn));
+    cudaFuncSetAttribute(onesweep_kernel<K, kWidth, kSmall>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn));
     if (dev >= 0 && dev < 64) opted[dev] = true;
   }
-  onesweep_kernel<K, kWidth, kMatch, kSmall><<<tiles, kSortThreads, dyn, stream>>>(kin, vin, kout, vout, n, shift, digit_base,
+  onesweep_kernel<K, kWidth, kSmall><<<tiles, kSortThreads, dyn, stream>>>(kin, vin, kout, vout, n, shift, digit_base,
                                                                     status, counter, err, spin_limit, unpublished, n_dev);
 }
 
 template <typename K, bool kSmall>
 void launch_onesweep(int width, int tiles, cudaStream_t stream, const K* kin, const uint32_t* vin, K* kout,
                      uint32_t* vout, long long n, int shift, const uint32_t* digit_base, uint32_t* status,
-                     uint32_t* counter, uint32_t* err, uint32_t spin_limit, long long unpublished, bool match,
-                     const uint32_t* n_dev) {
+                     uint32_t* counter, uint32_t* err, uint32_t spin_limit, long long unpublished, const uint32_t* n_dev) {
   switch (width) {
-#define W2W_ONESWEEP_CASE(W)                                                                                      \
-  case W:                                                                                                         \
-    if (match)                                                                                                    \
-      launch_onesweep_w<K, W, true, kSmall>(tiles, stream, kin, vin, kout, vout, n, shift, digit_base, status, counter,   \
-                                    err, spin_limit, unpublished, n_dev);                                         \
-    else                                                                                                          \
-      launch_onesweep_w<K, W, false, kSmall>(tiles, stream, kin, vin, kout, vout, n, shift, digit_base, status, counter,  \
-                                     err, spin_limit, unpublished, n_dev);                                        \
+#define W2W_ONESWEEP_CASE(W)                                                                                    \
+  case W:                                                                                                       \
+    launch_onesweep_w<K, W, kSmall>(tiles, stream, kin, vin, kout, vout, n, shift, digit_base, status, counter, \
+                                    err, spin_limit, unpublished, n_dev);                                       \
     break;
     W2W_ONESWEEP_CASE(1) W2W_ONESWEEP_CASE(2) W2W_ONESWEEP_CASE(3) W2W_ONESWEEP_CASE(4) W2W_ONESWEEP_CASE(5)
     W2W_ONESWEEP_CASE(6) W2W_ONESWEEP_CASE(7) W2W_ONESWEEP_CASE(8) W2W_ONESWEEP_CASE(9)
@@ -577,7 +583,7 @@ void run_sort(const SortArgs& a, cudaStream_t stream) {
     auto pass = [&](auto launch) {
       launch(pass_width(p, dbits, a.bits), int(tiles), stream, kin, vin, kout, vout, n, a.begin_bit + dbits * p,
              a.hist + kMaxBins * p, a.status + size_t(p) * kMaxBins * size_t(tiles), a.counters + p, a.error,
-             a.spin_limit, p == 0 ? a.unpublished_tile : -1LL, a.match_rank != 0, a.n_dev);
+             a.spin_limit, p == 0 ? a.unpublished_tile : -1LL, a.n_dev);
     };
     if (small) pass(launch_onesweep<K, true>);
     else pass(launch_onesweep<K, false>);
