@@ -28,13 +28,52 @@
 namespace w2w {
 namespace {
 
-constexpr int kDupThreads = 256;
+constexpr uint32_t kScanAgg = 1u << 30, kScanInc = 2u << 30, kScanMask = (1u << 30) - 1u;
 
-template <bool kKey64>
-__global__ void __launch_bounds__(kDupThreads) duplicate_kernel(DuplicateArgs a) {
+// The sum of the blocks before `tile`, by warp 0 (decoupled lookback, 32 status
+// words a step; a status word carries its flag and count together).  Bounded.
+__device__ __forceinline__ uint32_t lookback_sum(const uint32_t* status, int tile, uint32_t spin_limit,
+                                                 uint32_t* error) {
   const int lane = threadIdx.x & 31;
-  const int warp_global = (blockIdx.x * kDupThreads + threadIdx.x) >> 5;
-  const int g = warp_global * 32 + lane;
+  uint32_t sum = 0, spins = 0;
+  int t = tile - 1;
+  while (t >= 0) {
+    const int q = t - lane;
+    const uint32_t w = q >= 0 ? ld_relaxed(status + q) : kScanInc;
+    const uint32_t inc = __ballot_sync(0xffffffffu, (w & ~kScanMask) == kScanInc);
+    const uint32_t ready = __ballot_sync(0xffffffffu, (w & ~kScanMask) != 0u);
+    const uint32_t need = inc ? ((inc & (0u - inc)) << 1) - 1u : 0xffffffffu;
+    if ((ready & need) != need) {
+      if (++spins > spin_limit) {
+        if (lane == 0) atomicOr(error, kErrTimeout);
+        break;
+      }
+      continue;
+    }
+    sum += __reduce_add_sync(0xffffffffu, (need >> lane) & 1u ? w & kScanMask : 0u);
+    if (inc) break;
+    t -= 32;
+  }
+  return sum;
+}
+
+// kOrdered: thread j takes the j-th Gaussian by depth, and the entries follow
+// one another in that order (their count scanned here), instead of Gaussian j
+// and the slots it owns: the list is then sorted by depth already, and the sort
+// has only the tile digits left.
+template <bool kKey64, bool kOrdered>
+__global__ void __launch_bounds__(kDupThreads) duplicate_kernel(DuplicateArgs a) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int block = blockIdx.x;
+  if constexpr (kOrdered) {  // blocks in the order they start, so that lookback waits on running ones
+    __shared__ int s_block;
+    if (threadIdx.x == 0) s_block = int(atomicAdd(a.scan_counter, 1u));
+    __syncthreads();
+    block = s_block;
+  }
+  const int j = block * kDupThreads + int(threadIdx.x);
+  uint32_t g = uint32_t(j);
+  if constexpr (kOrdered) g = j < a.P ? a.order[j] : ~0u;
   uint32_t p0 = 0, cnt = 0, start = 0, x0 = 0, y0 = 0, w = 1, dlow = 0, gwv = uint32_t(a.gw), tbase = 0;
   uint32_t R = a.R, prefix = a.depth_prefix;
   bool fits = true;
@@ -46,9 +85,9 @@ __global__ void __launch_bounds__(kDupThreads) duplicate_kernel(DuplicateArgs a)
     prefix = a.depth_bits >= 32 ? 0u : (dmin & ~((1u << a.depth_bits) - 1u));
   }
   const uint32_t Rlim = fits ? R : 0u;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  if (block == 0 && threadIdx.x == 0) {
     BinHeader* h = a.header;
-    h->error = 0u;
+    if constexpr (!kOrdered) h->error = 0u;  // else cleared before the depth sort, which reports there too
     h->masks_valid = 1u;  // the blend that follows writes the block masks
     h->key64 = kKey64 ? 1u : 0u;
     h->depth_bits = a.depth_bits;
@@ -62,10 +101,11 @@ __global__ void __launch_bounds__(kDupThreads) duplicate_kernel(DuplicateArgs a)
   }
   for (uint32_t i = blockIdx.x * kDupThreads + threadIdx.x; i < a.clear_vecs; i += gridDim.x * kDupThreads)
     a.clear[i] = make_uint4(0u, 0u, 0u, 0u);
-  if (g < a.P) {  // Gaussians that emit nothing have an empty rectangle
+  if (block * kDupThreads >= a.P) return;  // a block that only clears
+  if (g < uint32_t(a.P)) {  // Gaussians that emit nothing have an empty rectangle
     uint32_t end = Rlim;
     if (a.items != nullptr) {  // batched: this view's tile grid, first tile id and end slot
-      const int item = find_item_elem(a.items, a.num_items, uint32_t(g));
+      const int item = find_item_elem(a.items, a.num_items, g);
       gwv = uint32_t(a.items[item].gw);
       tbase = a.items[item].tile_base;
       end = a.item_end[item];
@@ -93,6 +133,28 @@ __global__ void __launch_bounds__(kDupThreads) duplicate_kernel(DuplicateArgs a)
   }
   const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
   const uint32_t excl = incl - cnt;
+  uint32_t before = 0;  // kOrdered: entries before this warp's
+  if constexpr (kOrdered) {
+    __shared__ uint32_t s_warp[kDupThreads / 32], s_before;
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t mine = 0, all = 0;
+#pragma unroll
+    for (int w2 = 0; w2 < kDupThreads / 32; ++w2) {
+      if (w2 < warp) mine += s_warp[w2];
+      all += s_warp[w2];
+    }
+    if (warp == 0) {
+      if (lane == 0 && block > 0) st_relaxed(a.scan_status + block, kScanAgg | all);
+      const uint32_t b = lookback_sum(a.scan_status, block, a.spin_limit, &a.header->error);
+      if (lane == 0) {
+        st_relaxed(a.scan_status + block, kScanInc | ((b + all) & kScanMask));
+        s_before = b;
+      }
+    }
+    __syncthreads();
+    before = s_before + mine;
+  }
   for (uint32_t base = 0; base < total; base += 32) {
     const uint32_t e = base + lane;
     // owner lane: number of lanes whose inclusive count is <= e
@@ -112,18 +174,20 @@ __global__ void __launch_bounds__(kDupThreads) duplicate_kernel(DuplicateArgs a)
     const uint32_t odl = __shfl_sync(0xffffffffu, dlow, o);
     const uint32_t ogw = __shfl_sync(0xffffffffu, gwv, o);
     const uint32_t otb = __shfl_sync(0xffffffffu, tbase, o);
+    const uint32_t og = __shfl_sync(0xffffffffu, g, o);
     if (e < total) {
       const uint32_t p = op0 + (e - oex);
       const uint32_t k = p - ost;
       const uint32_t ty = oy0 + k / ow, tx = ox0 + k % ow;
       const uint32_t tile = otb + ty * ogw + tx;
-      if (p < Rlim) {
+      const uint32_t at = kOrdered ? before + e : p;
+      if (at < Rlim) {
         if constexpr (kKey64) {
-          reinterpret_cast<uint64_t*>(a.keys)[p] = (uint64_t(tile) << a.depth_bits) | odl;
+          reinterpret_cast<uint64_t*>(a.keys)[at] = (uint64_t(tile) << a.depth_bits) | odl;
         } else {
-          reinterpret_cast<uint32_t*>(a.keys)[p] = (a.depth_bits >= 32 ? 0u : (tile << a.depth_bits)) | odl;
+          reinterpret_cast<uint32_t*>(a.keys)[at] = (a.depth_bits >= 32 ? 0u : (tile << a.depth_bits)) | odl;
         }
-        a.vals[p] = uint32_t(warp_global * 32 + o);
+        a.vals[at] = og;
       }
     }
   }
@@ -136,8 +200,13 @@ void launch_duplicate(const DuplicateArgs& a, cudaStream_t stream) {
   // enough blocks to clear 16 KB each when the Gaussians need fewer
   const int blocks = max((a.P + kDupThreads - 1) / kDupThreads, min(296, int(a.clear_vecs / 1024u)));
   stage_begin(kStDuplicate, stream);
-  if (a.key64) duplicate_kernel<true><<<blocks, kDupThreads, 0, stream>>>(a);
-  else duplicate_kernel<false><<<blocks, kDupThreads, 0, stream>>>(a);
+  if (a.order != nullptr) {
+    if (a.key64) duplicate_kernel<true, true><<<blocks, kDupThreads, 0, stream>>>(a);
+    else duplicate_kernel<false, true><<<blocks, kDupThreads, 0, stream>>>(a);
+  } else {
+    if (a.key64) duplicate_kernel<true, false><<<blocks, kDupThreads, 0, stream>>>(a);
+    else duplicate_kernel<false, false><<<blocks, kDupThreads, 0, stream>>>(a);
+  }
   stage_end(kStDuplicate, stream, 1);
 }
 

@@ -109,7 +109,14 @@ struct DuplicateArgs {
   uint32_t tile_bits, passes, depth_prefix;
   uint4* clear;         // 16-byte aligned span
   uint32_t clear_vecs;  // uint4s in it
+  // Emission in depth order: the Gaussians by depth bits (stable), the scan's
+  // status words (one per kDupThreads Gaussians) and block counter, zeroed
+  const uint32_t* order = nullptr;
+  uint32_t* scan_status;
+  uint32_t* scan_counter;
+  uint32_t spin_limit = kSpinLimit;
 };
+constexpr int kDupThreads = 256;
 void launch_duplicate(const DuplicateArgs& a, cudaStream_t stream);
 
 // LSD radix sort of packed keys (uint32 or uint64) with uint32 values over
