@@ -78,6 +78,7 @@ struct __align__(16) BwdWarp {
 // window at the offset a scan over the lanes gives it: about 80 instructions
 // per 512 positions, where taking the words one by one cost 40 per 32 and was
 // the longest walks' largest part (91k of 222k cycles).
+template <bool kWide>
 struct BlockWalk {
   const uint32_t* words;
   const float* record;
@@ -99,7 +100,7 @@ struct BlockWalk {
         const uint32_t id = __ldg(list + pos);
         if (id < num_records) {
           float4 r0, r1;  // the blend's record
-          ldg32(record + 16 * size_t(id), r0, r1);
+          ldg32<kWide>(record + 16 * size_t(id), r0, r1);
           reach = block_test(r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, bx, by);
         }
       }
@@ -235,9 +236,10 @@ struct RefChain {
     T = tf;
     tf_bg = tf * (p.bg[0] * p.dLp0 + p.bg[1] * p.dLp1 + p.bg[2] * p.dLp2);
   }
+  template <bool kWide>
   static __device__ __forceinline__ void gather(const BackwardArgs& a, GroupLoad& g) {
     const float* r = a.bwd_record + 16 * size_t(g.id);
-    ldg32(r, g.q0, g.q1);
+    ldg32<kWide>(r, g.q0, g.q1);
     g.q2 = __ldg(reinterpret_cast<const float4*>(r) + 2);
   }
   static __device__ __forceinline__ float4 depth_colour(const GroupLoad& g) {
@@ -350,12 +352,13 @@ struct ExactChain {
     T = p.inside ? a.T_final[p.pix] : 0.0f;
     D = T * (p.bg[0] * p.dLp0 + p.bg[1] * p.dLp1 + p.bg[2] * p.dLp2);
   }
+  template <bool kWide>
   static __device__ __forceinline__ void gather(const BackwardArgs& a, GroupLoad& g) {
     const float* r = a.record + 16 * size_t(g.id);
     float4 o;
-    ldg32(r, g.q0, o);
+    ldg32<kWide>(r, g.q0, o);
     g.q0.z = o.w;
-    ldg32(r + 8, g.q1, g.q2);
+    ldg32<kWide>(r + 8, g.q1, g.q2);
   }
   static __device__ __forceinline__ float4 depth_colour(const GroupLoad& g) { return g.q2; }
   // The forward's own Gaussian values and decisions; the value is 0 where
@@ -449,7 +452,7 @@ __device__ __forceinline__ BwdPixel make_bwd_pixel(const BackwardArgs& a, int ti
   return BwdPixel(a, tile, tile - int(it.tile_base), block, it.W, it.H, size_t(it.pix_base), it.bg);
 }
 
-template <typename Chain>
+template <typename Chain, bool kWide>
 __global__ void __launch_bounds__(32, 16) render_bwd_kernel(BackwardArgs a) {
   __shared__ BwdWarp s;
   const int tile = int(a.order[blockIdx.x / 8]);  // heaviest first
@@ -462,7 +465,7 @@ __global__ void __launch_bounds__(32, 16) render_bwd_kernel(BackwardArgs a) {
   const float bx = float(p.tp.bx), by = float(p.tp.by);
   const float hW = 0.5f * float(p.W), hH = 0.5f * float(p.H);
   const uint32_t* list = a.point_list + p.range.x;
-  BlockWalk walk;
+  BlockWalk<kWide> walk;
   // the blend's block masks, when this binning state has them
   const bool use_masks = a.masks_valid != nullptr && *a.masks_valid != 0u;
   walk.words = use_masks ? a.masks + mask_row(p.range.x, tile, int(p.range.y - p.range.x), block) : nullptr;
@@ -489,7 +492,7 @@ __global__ void __launch_bounds__(32, 16) render_bwd_kernel(BackwardArgs a) {
     g.q0 = make_float4(-1024.f, -1024.f, 0.f, 0.f);
     g.q1 = make_float4(1.f, 0.f, 1.f, 1.f);
     g.q2 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (g.id < uint32_t(a.P)) Chain::gather(a, g);
+    if (g.id < uint32_t(a.P)) Chain::template gather<kWide>(a, g);
     else g.pos = ~0u;
   };
   walk.start(0, p.walk);
@@ -1390,10 +1393,14 @@ void launch_backward_render(const BackwardArgs& a, cudaStream_t stream) {
   if (tiles <= 0) return;
   stage_begin(kStBwdRender, stream);
   const bool da = a.dL_ddepth != nullptr || a.dL_dalpha != nullptr;  // a loss reaches depth or alpha
-  auto launch = [&](auto kernel) { kernel<<<tiles * 8, 32, 0, stream>>>(a); };
-  if (a.grad_mode == 1) launch(render_bwd_kernel<ExactChain>);
-  else if (da) launch(render_bwd_kernel<RefChain<true>>);
-  else launch(render_bwd_kernel<RefChain<false>>);
+  const bool wide = ((reinterpret_cast<uintptr_t>(a.record) | reinterpret_cast<uintptr_t>(a.bwd_record)) & 31u) == 0u;
+  auto launch = [&](auto kernel, auto narrow) {
+    if (wide) kernel<<<tiles * 8, 32, 0, stream>>>(a);
+    else narrow<<<tiles * 8, 32, 0, stream>>>(a);
+  };
+  if (a.grad_mode == 1) launch(render_bwd_kernel<ExactChain, true>, render_bwd_kernel<ExactChain, false>);
+  else if (da) launch(render_bwd_kernel<RefChain<true>, true>, render_bwd_kernel<RefChain<true>, false>);
+  else launch(render_bwd_kernel<RefChain<false>, true>, render_bwd_kernel<RefChain<false>, false>);
   stage_end(kStBwdRender, stream, 1);
 }
 

@@ -144,6 +144,7 @@ __device__ __forceinline__ void group_alphas(BlendWarp& s, const BlendEntry& en,
 // per entry and 32 pixels for the alphas, 16 for the pixels' chains, 1.3 per
 // tested entry); at small scenes, and at the end of large ones, the busiest
 // warp's chain.
+template <bool kWide>
 __global__ void __launch_bounds__(32 * kBlendWarps, kBlendResident / kBlendWarps) blend_kernel(BlendArgs a) {
   constexpr int kParts = 8 / kBlendWarps;  // CTAs per tile
   __shared__ BlendWarp s_warp[kBlendWarps];
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(32 * kBlendWarps, kBlendResident / kBlendWarps
       t0[q] = make_float4(0.f, 0.f, -1.f, 0.f);  // hy < 0: reaches nothing
       t1[q] = make_float4(0.f, 0.f, 0.f, 0.f);
       if (id[q] < a.num_records) {
-        ldg32(records + 4 * size_t(id[q]), t0[q], t1[q]);
+        ldg32<kWide>(records + 4 * size_t(id[q]), t0[q], t1[q]);
       }
     }
   };
@@ -238,9 +239,9 @@ __global__ void __launch_bounds__(32 * kBlendWarps, kBlendResident / kBlendWarps
     if (e < count) {
       const float4* r = records + 4 * size_t(s.ring[(head + uint32_t(e)) & (kRing - 1)].x);
       float4 o;
-      ldg32(r, en.m, o);
+      ldg32<kWide>(r, en.m, o);
       en.m.z = o.w;
-      ldg32(r + 2, en.c, en.dc);
+      ldg32<kWide>(r + 2, en.c, en.dc);
     }
   };
   int count = 0;
@@ -605,9 +606,24 @@ __global__ void __launch_bounds__(32 * (kW + 1)) blend_queue_kernel(BlendArgs a,
 
 }  // namespace
 
+// The tiles' processing order from their ranges (tile_walk.cuh), with `zero` (the
+// blend's per-tile maximum) and `counter` (the persistent blend's queue)
+// cleared.  One block.
 __global__ void __launch_bounds__(1024) tile_order_kernel(const uint2* ranges, int num_tiles, uint32_t* order,
                                                           uint32_t* zero, uint32_t* counter) {
-  tile_order_block(ranges, num_tiles, order, zero, counter);
+  __shared__ uint32_t s_cnt[kTileBuckets], s_pos[kTileBuckets];
+  if (counter != nullptr && threadIdx.x == 0) *counter = 0u;
+  for (int i = threadIdx.x; i < kTileBuckets; i += blockDim.x) s_cnt[i] = 0u;
+  __syncthreads();
+  for (int t = threadIdx.x; t < num_tiles; t += blockDim.x) {
+    zero[t] = 0u;
+    atomicAdd(&s_cnt[tile_bucket(ranges[t].y - ranges[t].x)], 1u);
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) bucket_positions(s_cnt, s_pos);
+  __syncthreads();
+  for (int t = threadIdx.x; t < num_tiles; t += blockDim.x)
+    order[atomicAdd(&s_pos[tile_bucket(ranges[t].y - ranges[t].x)], 1u)] = uint32_t(t);
 }
 
 namespace {
@@ -688,7 +704,11 @@ void launch_blend(const BlendArgs& a, cudaStream_t stream) {
   }
   stage_begin(kStBlend, stream);
   const bool queued = queue && (warps == 4 ? launch_queue<4>(a, tiles, stream) : launch_queue<8>(a, tiles, stream));
-  if (!queued) blend_kernel<<<tiles * (8 / kBlendWarps), 32 * kBlendWarps, 0, stream>>>(a);
+  if (!queued) {
+    auto launch = [&](auto kernel) { kernel<<<tiles * (8 / kBlendWarps), 32 * kBlendWarps, 0, stream>>>(a); };
+    if ((reinterpret_cast<uintptr_t>(a.record) & 31u) == 0u) launch(blend_kernel<true>);
+    else launch(blend_kernel<false>);
+  }
   stage_end(kStBlend, stream, 1);
 }
 

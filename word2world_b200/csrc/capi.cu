@@ -214,8 +214,12 @@ void launch_list(DuplicateArgs d, const KeyPlan& kp, long long n, int T, void* b
   const long long tile = sort_tile_keys(kp.key64, n);
   const size_t bytes = BL.status - BL.hist +
                        size_t(passes > 0 ? passes : 1) * kMaxBins * 4 * size_t((n + tile - 1) / tile);
-  d.clear = at<uint4>(binning_state, BL.hist);
-  d.clear_vecs = uint32_t((bytes + 15) / 16);
+  if ((reinterpret_cast<uintptr_t>(binning_state) & 15u) == 0u) {
+    d.clear = at<uint4>(binning_state, BL.hist);
+    d.clear_vecs = uint32_t((bytes + 15) / 16);
+  } else {
+    cudaMemsetAsync(at<void>(binning_state, BL.hist), 0, bytes, st);
+  }
   launch_duplicate(d, st);
   SortArgs so{};
   so.n = n; so.key64 = kp.key64; so.begin_bit = by_depth ? kp.depth_bits : 0; so.bits = sort_bits;

@@ -168,12 +168,20 @@ __device__ __forceinline__ CullParams make_cull_params(float A, float B, float C
   return p;
 }
 
-// 32 bytes (32-byte aligned) in one load: half the load instructions, and half
-// the L1 wavefronts of a gather, of two 16-byte ones.
+// 32 bytes in one load where the address allows it (kWide: 32-byte aligned):
+// half the load instructions, and half the L1 wavefronts of a gather, of two
+// 16-byte ones.  The state buffers are the caller's, aligned to 16 at least;
+// kernels that gather records are compiled for both.
+template <bool kWide>
 __device__ __forceinline__ void ldg32(const void* p, float4& a, float4& b) {
-  asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-               : "l"(p));
+  if constexpr (kWide) {
+    asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(p));
+  } else {
+    a = __ldg(reinterpret_cast<const float4*>(p));
+    b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+  }
 }
 
 __device__ __forceinline__ float sqrt_approx(float x) {

@@ -107,8 +107,8 @@ struct DuplicateArgs {
   BinHeader* header;
   const GeomHeader* plan;
   uint32_t tile_bits, passes, depth_prefix;
-  uint4* clear;         // 16-byte aligned span
-  uint32_t clear_vecs;  // uint4s in it
+  uint4* clear = nullptr;  // 16-byte aligned span
+  uint32_t clear_vecs = 0;  // uint4s in it
   // Emission in depth order: the Gaussians by depth bits (stable), the scan's
   // status words (one per kDupThreads Gaussians) and block counter, zeroed
   const uint32_t* order = nullptr;

@@ -11,8 +11,7 @@
 //      instance counts).  Its last block to finish scans those histograms; the
 //      tile scan is the per-tile [start, end) range table (empty tiles get (0,
 //      0), as the reference's memset leaves them), and the tiles' processing
-//      order follows from it (two one-block kernels before: 7 us a view with
-//      their launches);
+//      order follows from it (two one-block kernels before);
 //   2. one onesweep kernel per digit: each CTA takes the next tile (6144 32-bit or 5120 64-bit keys)
 //      (acquired through an atomic counter, so every earlier tile is already
 //      running), ranks its keys stably (per-bit warp ballots), publishes its
@@ -126,47 +125,83 @@ __device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s_warp, uint32_t*
   return r;
 }
 
-// Digit histograms -> exclusive digit offsets (in place); tile histogram ->
-// [start, end) ranges.  The whole block; the counts are other blocks' atomics,
-// read past the L1.
-__device__ __forceinline__ void offsets_block(uint32_t* hist, int passes, const uint32_t* tile_hist, int num_tiles,
-                                              uint2* ranges) {
-  __shared__ uint32_t s_warp[32];
-  for (int p = 0; p < passes; ++p) {
-    // kMaxBins bins over the block's threads, consecutive ones to a thread
-    const int per = kMaxBins > int(blockDim.x) ? kMaxBins / int(blockDim.x) : 1;
-    const int b0 = int(threadIdx.x) * per;
-    uint32_t v[kMaxBins / kHistThreads], sum = 0;
+// What the histogram's last block makes of the counts (other blocks' atomics,
+// read past the L1): digit histograms -> exclusive digit offsets, in place, a
+// warp per pass; tile histogram -> [start, end) ranges, and the tiles by
+// decreasing length (tile_bucket's buckets, heaviest first; order within a
+// bucket is arbitrary), with the blend's per-tile maximum and queue cleared.
+// Sixteen tiles to a thread: up to 4096 tiles are one round, whose counts stay in
+// registers from the scan to the ordering.
+constexpr int kTilesPer = 16;
+__device__ __forceinline__ void finish_counts(uint32_t* hist, int passes, const uint32_t* tile_hist, int num_tiles,
+                                              uint2* ranges, uint32_t* order, uint32_t* order_zero,
+                                              uint32_t* order_counter) {
+  __shared__ uint32_t s_warp[32], s_cnt[kTileBuckets], s_pos[kTileBuckets];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int per = min(kTilesPer, (num_tiles + int(blockDim.x) - 1) / int(blockDim.x));
+  const int round = int(blockDim.x) * per;
+  uint32_t c[kTilesPer], carry = 0;
+  auto load = [&](int t0) {
 #pragma unroll
-    for (int k = 0; k < kMaxBins / kHistThreads; ++k) {
-      v[k] = k < per && b0 + k < kMaxBins ? __ldcg(hist + p * kMaxBins + b0 + k) : 0u;
-      sum += v[k];
+    for (int k = 0; k < kTilesPer; ++k) c[k] = k < per && t0 + k < num_tiles ? __ldcg(tile_hist + t0 + k) : 0u;
+  };
+  const bool tiles = tile_hist != nullptr && ranges != nullptr;
+  if (tiles) load(int(threadIdx.x) * per);  // the first round's, in flight with the digits'
+  for (int p = warp; p < passes; p += int(blockDim.x >> 5)) {
+    static_assert(kMaxBins == 512, "sixteen bins to a lane");
+    uint2* h = reinterpret_cast<uint2*>(hist + p * kMaxBins) + 8 * lane;
+    uint2 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = __ldcg(h + k);
+    uint32_t sum = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sum += v[k].x + v[k].y;
+    uint32_t ex = sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t o = __shfl_up_sync(0xffffffffu, ex, d);
+      if (lane >= d) ex += o;
     }
-    uint32_t ex = block_exclusive_scan(sum, s_warp, nullptr);
+    ex -= sum;
 #pragma unroll
-    for (int k = 0; k < kMaxBins / kHistThreads; ++k) {
-      if (k < per && b0 + k < kMaxBins) hist[p * kMaxBins + b0 + k] = ex;
-      ex += v[k];
+    for (int k = 0; k < 8; ++k) {
+      h[k] = make_uint2(ex, ex + v[k].x);
+      ex += v[k].x + v[k].y;
     }
   }
-  if (tile_hist == nullptr || ranges == nullptr) return;
-  constexpr int kPer = 4;  // tiles per thread and round
-  uint32_t carry = 0;
-  for (int base = 0; base < num_tiles; base += int(blockDim.x) * kPer) {
-    const int t0 = base + int(threadIdx.x) * kPer;
-    uint32_t c[kPer], sum = 0, tot;
+  if (!tiles) return;
+  if (order != nullptr) {
+    if (order_counter != nullptr && threadIdx.x == 0) *order_counter = 0u;
+    for (int i = threadIdx.x; i < kTileBuckets; i += blockDim.x) s_cnt[i] = 0u;
+  }
+  for (int base = 0; base < num_tiles; base += round) {
+    const int t0 = base + int(threadIdx.x) * per;
+    if (base > 0) load(t0);
+    uint32_t sum = 0, tot;
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-      c[k] = t0 + k < num_tiles ? __ldcg(tile_hist + t0 + k) : 0u;
-      sum += c[k];
-    }
-    uint32_t start = carry + block_exclusive_scan(sum, s_warp, &tot);
+    for (int k = 0; k < kTilesPer; ++k) sum += c[k];
+    uint32_t start = carry + block_exclusive_scan(sum, s_warp, &tot);  // synchronises the block
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) {
-      if (t0 + k < num_tiles) ranges[t0 + k] = c[k] ? make_uint2(start, start + c[k]) : make_uint2(0u, 0u);
+    for (int k = 0; k < kTilesPer; ++k) {
+      if (k < per && t0 + k < num_tiles) {
+        ranges[t0 + k] = c[k] ? make_uint2(start, start + c[k]) : make_uint2(0u, 0u);
+        if (order != nullptr) atomicAdd(&s_cnt[tile_bucket(c[k])], 1u);
+        if (order != nullptr && order_zero != nullptr) order_zero[t0 + k] = 0u;
+      }
       start += c[k];
     }
     carry += tot;
+  }
+  if (order == nullptr) return;
+  __syncthreads();
+  if (warp == 0) bucket_positions(s_cnt, s_pos);
+  __syncthreads();
+  for (int base = 0; base < num_tiles; base += round) {
+    const int t0 = base + int(threadIdx.x) * per;
+    if (num_tiles > round) load(t0);
+#pragma unroll
+    for (int k = 0; k < kTilesPer; ++k)
+      if (k < per && t0 + k < num_tiles) order[atomicAdd(&s_pos[tile_bucket(c[k])], 1u)] = uint32_t(t0 + k);
   }
 }
 
@@ -213,11 +248,7 @@ hist_kernel(const K* __restrict__ keys, long long n, int begin_bit, int passes, 
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  offsets_block(hist, passes, tile_hist, num_tiles, ranges);
-  if (ranges != nullptr && order != nullptr) {
-    __syncthreads();  // the ranges are this block's own
-    tile_order_block(ranges, num_tiles, order, order_zero, order_counter);
-  }
+  finish_counts(hist, passes, tile_hist, num_tiles, ranges, order, order_zero, order_counter);
 }
 
 // Decoupled lookback for the adjacent digits d, d + 1 (d even).  A tile
@@ -558,7 +589,7 @@ void run_sort(const SortArgs& a, cudaStream_t stream) {
     const bool tiles_in_smem = a.tile_hist != nullptr && a.num_tiles <= kSmemTileBins;
     const bool big = tiles_in_smem && a.num_tiles > kSmemTileBinsSmall;
     const int threads = big ? kHistThreadsBig : kHistThreads;
-    const long long per_block = (long long)threads * kHistRun * 4;
+    const long long per_block = (long long)threads * kHistRun;
     const int grid = int(max(1LL, min((n + per_block - 1) / per_block, (long long)sms * (big ? 1 : 4))));
     const size_t smem =
         sizeof(uint32_t) * (size_t(passes) * kMaxBins + (tiles_in_smem ? size_t(a.num_tiles) : 0));

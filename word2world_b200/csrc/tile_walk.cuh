@@ -31,51 +31,34 @@ struct TilePixel {
 // Tiles are processed heaviest first: CTA b takes tile order[b], where order
 // lists the tiles by decreasing list length (quarter-octave buckets; order
 // within a bucket is arbitrary), so the heaviest start in the first wave
-// instead of wherever the raster order puts them.  `zero`, when given, is
-// cleared over num_tiles entries on the way (the blend's per-tile maximum), and
-// `counter`, when given, set to zero (the persistent blend's queue).  The whole
-// block calls it; what it reads of `ranges` is this block's own or an earlier
-// kernel's.  The backward takes the same order: sorting the tiles again by the
+// instead of wherever the raster order puts them.  The sort's histogram writes
+// it (sort.cu), or a kernel of its own where there is no sort (blend.cu).  The
+// backward takes the same order: sorting the tiles again by the
 // contributor counts the blend found cost 3 us a view and won nothing (378
 // against 383 us of backward per 4 views at 500k, 93 against 90 at 16k).
-__device__ __forceinline__ void tile_order_block(const uint2* ranges, int num_tiles, uint32_t* order, uint32_t* zero,
-                                                 uint32_t* counter) {
-  if (counter != nullptr && threadIdx.x == 0) *counter = 0u;
-  constexpr int kBuckets = 130;
-  __shared__ uint32_t s_cnt[kBuckets];
-  __shared__ uint32_t s_pos[kBuckets];
-  auto bucket = [&](int t) -> int {
-    const uint2 r = ranges[t];
-    const uint32_t n = r.y - r.x;
-    if (n == 0) return 0;
-    const int e = 31 - __clz(n);
-    const uint32_t q = e >= 2 ? (n >> (e - 2)) & 3u : (n << (2 - e)) & 3u;
-    return 1 + 4 * e + int(q);
-  };
-  for (int i = threadIdx.x; i < kBuckets; i += blockDim.x) s_cnt[i] = 0;
-  __syncthreads();
-  for (int t = threadIdx.x; t < num_tiles; t += blockDim.x) {
-    if (zero != nullptr) zero[t] = 0u;
-    atomicAdd(&s_cnt[bucket(t)], 1u);
-  }
-  __syncthreads();
-  if (threadIdx.x < 32) {  // first position of each bucket, the heaviest first: a warp takes 32 buckets at a time
-    uint32_t before = 0;
-    for (int b0 = kBuckets - 1; b0 >= 0; b0 -= 32) {
-      const int b = b0 - int(threadIdx.x);
-      const uint32_t c = b >= 0 ? s_cnt[b] : 0u;
-      uint32_t x = c;
+constexpr int kTileBuckets = 130;
+__device__ __forceinline__ int tile_bucket(uint32_t n) {
+  if (n == 0) return 0;
+  const int e = 31 - __clz(n);
+  const uint32_t q = e >= 2 ? (n >> (e - 2)) & 3u : (n << (2 - e)) & 3u;
+  return 1 + 4 * e + int(q);
+}
+// First position of each bucket, the heaviest first, by one warp (32 buckets a step).
+__device__ __forceinline__ void bucket_positions(const uint32_t* cnt, uint32_t* pos) {
+  const int lane = threadIdx.x & 31;
+  uint32_t before = 0;
+  for (int b0 = kTileBuckets - 1; b0 >= 0; b0 -= 32) {
+    const int b = b0 - lane;
+    const uint32_t c = b >= 0 ? cnt[b] : 0u;
+    uint32_t x = c;
 #pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t o = __shfl_up_sync(0xffffffffu, x, d);
-        if (int(threadIdx.x) >= d) x += o;
-      }
-      if (b >= 0) s_pos[b] = before + x - c;
-      before += __shfl_sync(0xffffffffu, x, 31);
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t o = __shfl_up_sync(0xffffffffu, x, d);
+      if (lane >= d) x += o;
     }
+    if (b >= 0) pos[b] = before + x - c;
+    before += __shfl_sync(0xffffffffu, x, 31);
   }
-  __syncthreads();
-  for (int t = threadIdx.x; t < num_tiles; t += blockDim.x) order[atomicAdd(&s_pos[bucket(t)], 1u)] = uint32_t(t);
 }
 
 // Block masks the forward blend leaves for the backward passes: for every
