@@ -541,6 +541,7 @@ __global__ void __launch_bounds__(32, 16) render_bwd_kernel(BackwardArgs a) {
 // 192-byte-strided row per thread.
 // ---------------------------------------------------------------------------
 constexpr int kGaussThreads = 128;
+constexpr int kGaussRow = 52;  // floats of shared memory per Gaussian (store_rows; the staged rows need 49)
 
 __device__ __forceinline__ int sh_stride(int M) {
   const int r = 3 * (M < 16 ? M : 16);
@@ -580,26 +581,47 @@ __device__ __forceinline__ void sh_stage_in(const float* shs, int M, int i0, int
   __syncwarp();
 }
 
-// Write the span of 32 rows of `len` floats at dst: row g's element c is
-// coefficient (c + off) / 3, channel (c + off) % 3 of Gaussian g, the product of
-// its basis value and colour factor in s (row g at g * 21: 16 basis, 3 factors).
-__device__ __forceinline__ void store_span(float* dst, int len, const float* s, int off) {
-  const int lane = threadIdx.x & 31, nf = 8 * len;
-  float4* q = reinterpret_cast<float4*>(dst);
-  for (int f = lane; f < nf; f += 32) {
-    int g = (4 * f) / len, c = 4 * f - g * len;
+// 32 rows of dL/dSH (48 floats each) of 16-byte aligned arrays: each lane puts
+// its products into s, and the warp writes them out as contiguous 16-byte
+// pieces, without the index arithmetic of a lane per output element.  s holds
+// 32 rows of 52 floats (an odd number of 16-byte pieces), which start at
+// conflict-free banks.
+__device__ __forceinline__ void store_rows(float* dsh, float* s, const float (&basis)[16], const float (&cf)[3],
+                                           bool active) {
+  const int lane = threadIdx.x & 31;
+  float4* s4 = reinterpret_cast<float4*>(s);
+#pragma unroll
+  for (int q = 0; q < 12; ++q) {
     float o[4];
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      const int e = c + off, k = e / 3, ch = e - 3 * k;
-      o[w] = s[g * 21 + k] * s[g * 21 + 16 + ch];
-      if (++c == len) {
-        c = 0;
-        ++g;
-      }
-    }
-    q[f] = make_float4(o[0], o[1], o[2], o[3]);
+    for (int w = 0; w < 4; ++w) o[w] = active ? basis[(4 * q + w) / 3] * cf[(4 * q + w) % 3] : 0.f;
+    s4[13 * lane + q] = make_float4(o[0], o[1], o[2], o[3]);
   }
+  __syncwarp();
+  float4* dst = reinterpret_cast<float4*>(dsh);
+#pragma unroll
+  for (int q = 0; q < 12; ++q) {
+    const int f = 32 * q + lane, g = f / 12;
+    dst[f] = s4[f + g];  // piece f % 12 of row g at 13 g
+  }
+}
+
+// The same for the raw path's arrays: rows of 3 and of 45 floats, both odd, lie
+// in s as they lie in memory.
+__device__ __forceinline__ void store_rows_raw(float* ddc, float* dac, float* s, const float (&basis)[16],
+                                               const float (&cf)[3], bool active) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int ch = 0; ch < 3; ++ch) s[3 * lane + ch] = active ? basis[0] * cf[ch] : 0.f;
+#pragma unroll
+  for (int e = 0; e < 45; ++e) s[kRawAc + 45 * lane + e] = active ? basis[1 + e / 3] * cf[e % 3] : 0.f;
+  __syncwarp();
+  const float4* s4 = reinterpret_cast<const float4*>(s);
+  if (lane < 24) reinterpret_cast<float4*>(ddc)[lane] = s4[lane];
+  float4* dst = reinterpret_cast<float4*>(dac);
+#pragma unroll
+  for (int q = 0; q < 12; ++q)
+    if (32 * q + lane < 360) dst[32 * q + lane] = s4[kRawAc / 4 + 32 * q + lane];
 }
 
 // dsh rows [i0, i0 + n) ([P, M, 3]) = basis[k] * cf[ch] (k < 16; 0 beyond),
@@ -609,15 +631,15 @@ __device__ __forceinline__ void sh_store_outer(float* dsh, int M, int i0, int n,
   constexpr int kRow = 21;  // 16 basis + 3 colour factors, odd stride
   const int lane = threadIdx.x & 31, rg = 3 * M;
   __syncwarp();  // the SH rows in s have been read
+  if (M == 16 && n == 32 && aligned16(dsh)) {
+    store_rows(dsh + size_t(i0) * 48, s, basis, cf, active);
+    return;
+  }
 #pragma unroll
   for (int k = 0; k < 16; ++k) s[lane * kRow + k] = active ? basis[k] : 0.f;
 #pragma unroll
   for (int ch = 0; ch < 3; ++ch) s[lane * kRow + 16 + ch] = active ? cf[ch] : 0.f;
   __syncwarp();
-  if (M == 16 && n == 32 && aligned16(dsh)) {
-    store_span(dsh + size_t(i0) * 48, 48, s, 0);
-    return;
-  }
   if (rg > 0) {
     constexpr int kInFlight = 8;
     const int total = n * rg;
@@ -644,15 +666,16 @@ __device__ __forceinline__ void sh_store_outer(float* dsh, int M, int i0, int n,
 
 // The raw path's SH rows: coefficient 0 from sh_dc ([P, 1, 3]), the rest from
 // sh_ac ([P, M - 1, 3]).  Same staging as sh_stage_in.  Warp-collective.
-__device__ __forceinline__ void sh_stage_in_raw(const float* dc, const float* ac, int M, int i0, int n, float* s,
+// Returns true for full rows that are on their way asynchronously as they lie in
+// memory (sh_ac only, 45 floats a row): copy_wait and a warp barrier complete
+// them.
+__device__ __forceinline__ bool sh_stage_in_raw(const float* dc, const float* ac, int M, int i0, int n, float* s,
                                                 int stride) {
   constexpr int kInFlight = 8;
   const int rs = 3 * (M < 16 ? M : 16), ra = 3 * (M - 1), lane = threadIdx.x & 31;
-  if (M == 16 && n == 32 && aligned16(dc) && aligned16(ac)) {
-    stage_span(dc + size_t(i0) * 3, 3, s, stride, 0);
-    stage_span(ac + size_t(i0) * 45, 45, s, stride, 3);
-    __syncwarp();
-    return;
+  if (M == 16 && n == 32 && aligned16(ac)) {
+    copy_span_async(s, ac + size_t(i0) * 45, 32 * 45);
+    return true;
   }
   if (rs > 0) {
     const int total = n * rs;
@@ -675,6 +698,7 @@ __device__ __forceinline__ void sh_stage_in_raw(const float* dc, const float* ac
     }
   }
   __syncwarp();
+  return false;
 }
 
 // sh_store_outer for the raw path: coefficient 0 to ddc, the rest to dac.
@@ -682,17 +706,16 @@ __device__ __forceinline__ void sh_store_outer_raw(float* ddc, float* dac, int M
                                                    const float (&basis)[16], const float (&cf)[3], bool active) {
   constexpr int kRow = 21;
   const int lane = threadIdx.x & 31, rg = 3 * M, ra = 3 * (M - 1);
-  __syncwarp();
+  __syncwarp();  // the SH rows in s have been read
+  if (M == 16 && n == 32 && aligned16(ddc) && aligned16(dac)) {
+    store_rows_raw(ddc + size_t(i0) * 3, dac + size_t(i0) * 45, s, basis, cf, active);
+    return;
+  }
 #pragma unroll
   for (int k = 0; k < 16; ++k) s[lane * kRow + k] = active ? basis[k] : 0.f;
 #pragma unroll
   for (int ch = 0; ch < 3; ++ch) s[lane * kRow + 16 + ch] = active ? cf[ch] : 0.f;
   __syncwarp();
-  if (M == 16 && n == 32 && aligned16(ddc) && aligned16(dac)) {
-    store_span(ddc + size_t(i0) * 3, 3, s, 0);
-    store_span(dac + size_t(i0) * 45, 45, s, 3);
-    return;
-  }
   if (rg > 0) {
     constexpr int kInFlight = 8;
     const int total = n * rg;
@@ -767,13 +790,12 @@ struct GView {
   }
   __device__ __forceinline__ float4 rotation() const {
     if (quat != nullptr) {
-      const float w = __ldg(&quat[4 * gi]), x = __ldg(&quat[4 * gi + 1]), y = __ldg(&quat[4 * gi + 2]),
-                  z = __ldg(&quat[4 * gi + 3]);
+      const float4 q = load_quat(quat, gi);
+      const float w = q.x, x = q.y, y = q.z, z = q.w;
       const float inv = __frcp_rn(fmaxf(sqrtf((w * w + y * y) + (x * x + z * z)), 1e-12f));
       return make_float4(w * inv, x * inv, y * inv, z * inv);
     }
-    return make_float4(__ldg(&rotations[4 * gi]), __ldg(&rotations[4 * gi + 1]), __ldg(&rotations[4 * gi + 2]),
-                       __ldg(&rotations[4 * gi + 3]));
+    return load_quat(rotations, gi);
   }
 };
 
@@ -809,14 +831,13 @@ __device__ __forceinline__ void store_gout(const BackwardArgs& a, int i, const G
   for (int k = 0; k < 4; ++k) a.dL_drotations[4 * i + k] = o.rot[k];
 }
 
-// One Gaussian (radius > 0) of the reference-formula pass: every output but
-// dL_dsh, plus the SH basis and masked colour gradient dL_dsh is built from.
-// sh_row: this Gaussian's SH coefficients (staged in shared memory).
-__device__ __forceinline__ void ref_gaussian(const BackwardArgs& a, int i, const GView& gv, const float* sh_row, float (&basis)[16],
-                                             float (&cf)[3], GOut& o) {
-  const int M = a.M;
+// One Gaussian (radius > 0) of the reference-formula pass, in two parts: the
+// covariance and mean gradients (sd: dL/dmean so far), which need no SH
+// coefficient, then every other output but dL_dsh, plus the SH basis and masked
+// colour gradient dL_dsh is built from.
+__device__ __forceinline__ void ref_gaussian_geometry(const BackwardArgs& a, int i, const GView& gv, GOut& o,
+                                                      float (&dc)[6], float (&sd)[3]) {
   const float* mats = gv.mats;
-  const float* cam = mats + 32;
   const float* view = mats;
   const float* proj = mats + 16;
   const float cx = __ldg(&gv.means3D[3 * gv.gi]), cy = __ldg(&gv.means3D[3 * gv.gi + 1]), cz = __ldg(&gv.means3D[3 * gv.gi + 2]);
@@ -864,7 +885,6 @@ __device__ __forceinline__ void ref_gaussian(const BackwardArgs& a, int i, const
   const float dinv2 = 1.0f / (den * den + 1e-7f);
   const float gx = __ldg(&a.acc_cov[4 * i]), gy = __ldg(&a.acc_cov[4 * i + 1]), gz = __ldg(&a.acc_cov[4 * i + 3]);
   float ga = 0.f, gb = 0.f, gc = 0.f;
-  float dc[6];
   if (dinv2 > 0) {
     ga = dinv2 * (-cc * cc * gx + 2.0f * cb * cc * gy + (den - ca * cc) * gz);
     gb = dinv2 * 2.0f * (cb * cc * gx - (den + 2.0f * cb * cb) * gy + ca * cb * gz);
@@ -894,8 +914,9 @@ __device__ __forceinline__ void ref_gaussian(const BackwardArgs& a, int i, const
   const float gvy = mask_y * (-h_y * z_inv2 * gJ12);
   const float gvz = -h_x * z_inv2 * gJ00 - h_y * z_inv2 * gJ11 + 2.0f * h_x * px * z_inv3 * gJ02 +
                     2.0f * h_y * py * z_inv3 * gJ12;
-  float sd[3] = {view[0] * gvx + view[1] * gvy + view[2] * gvz, view[4] * gvx + view[5] * gvy + view[6] * gvz,
-                 view[8] * gvx + view[9] * gvy + view[10] * gvz};
+  sd[0] = view[0] * gvx + view[1] * gvy + view[2] * gvz;
+  sd[1] = view[4] * gvx + view[5] * gvy + view[6] * gvz;
+  sd[2] = view[8] * gvx + view[9] * gvy + view[10] * gvz;
 
   // ---- backwardPreprocessingKernel ----
   const float cw = proj[3] * cx + proj[7] * cy + proj[11] * cz + proj[15];
@@ -912,6 +933,16 @@ __device__ __forceinline__ void ref_gaussian(const BackwardArgs& a, int i, const
   sd[0] += (view[2] - view[3] * vzz) * gd;
   sd[1] += (view[6] - view[7] * vzz) * gd;
   sd[2] += (view[10] - view[11] * vzz) * gd;
+}
+
+// sh_row: this Gaussian's SH coefficients (staged in shared memory), of which
+// coefficient 0, whose basis value is constant, is not read.
+__device__ __forceinline__ void ref_gaussian_rest(const BackwardArgs& a, int i, const GView& gv, const float* sh_row,
+                                                  const float (&dc)[6], float (&sd)[3], float (&basis)[16],
+                                                  float (&cf)[3], GOut& o) {
+  const int M = a.M;
+  const float* cam = gv.mats + 32;
+  const float cx = __ldg(&gv.means3D[3 * gv.gi]), cy = __ldg(&gv.means3D[3 * gv.gi + 1]), cz = __ldg(&gv.means3D[3 * gv.gi + 2]);
   // SH (all 16 bands, colour-clamp masks)
   const float ox = cx - cam[0], oy = cy - cam[1], oz = cz - cam[2];
   const float msq = ox * ox + oy * oy + oz * oz;
@@ -1007,8 +1038,8 @@ __device__ __forceinline__ void ref_gaussian(const BackwardArgs& a, int i, const
   dq.z = 4.f * (-sz * (a31 * xx + a32 * xw + a33 * qxz) + sy * (a21 * zw + a22 * yy + a23 * yw) - sx * (a12 * xw + a13 * xx + a11 * qxy));
   dq.w = 4.f * (sz * (a31 * xw - a32 * xx + a33 * qxy) - sy * (a21 * qxz - a22 * zw + a23 * qyz) + sx * (a12 * qyz - a13 * zz + a11 * yy));
   if (gv.quat != nullptr) {  // raw path: rotation = q / max(|q|, 1e-12)
-    const float q0 = __ldg(&gv.quat[4 * gv.gi]), q1 = __ldg(&gv.quat[4 * gv.gi + 1]),
-                q2 = __ldg(&gv.quat[4 * gv.gi + 2]), q3 = __ldg(&gv.quat[4 * gv.gi + 3]);
+    const float4 qv = load_quat(gv.quat, gv.gi);
+    const float q0 = qv.x, q1 = qv.y, q2 = qv.z, q3 = qv.w;
     const float n = sqrtf(q0 * q0 + q1 * q1 + q2 * q2 + q3 * q3);
     if (n > 1e-12f) {  // (g - r (r . g)) / n with r = q / n
       const float inv = __frcp_rn(n);
@@ -1025,11 +1056,14 @@ __device__ __forceinline__ void ref_gaussian(const BackwardArgs& a, int i, const
   o.rot[3] = dq.w;
 }
 
-// 8 CTAs per SM (64 registers, no spills; shared memory allows 9): more
-// Gaussians' loads in flight (0.452 -> 0.415 ms per 4-view step against the
-// default 6 CTAs at 80 registers).
+// Bound by memory: 556 bytes a Gaussian, 4.5 TB/s at 500k and 5 TB/s at 1M.  The
+// raw SH rows arrive asynchronously under the covariance gradients, and dL/dSH
+// leaves as products each lane forms for its own row (store_rows): 78 -> 62 us a
+// view at 500k, 142 -> 112 us at 1M, against rows staged through registers and
+// outputs whose factors every lane looked up by index.  8 CTAs per SM (64
+// registers): more Gaussians' loads in flight.
 __global__ void __launch_bounds__(kGaussThreads, 8) gaussians_ref_kernel(BackwardArgs a) {
-  __shared__ float s_sh[kGaussThreads / 32][32 * kShStride];
+  __shared__ __align__(16) float s_sh[kGaussThreads / 32][32 * kGaussRow];
   // view, projection, camera position: shared memory is never aliased by the
   // outputs, so these stay in place across the output stores
   __shared__ float s_mats[35];
@@ -1046,18 +1080,26 @@ __global__ void __launch_bounds__(kGaussThreads, 8) gaussians_ref_kernel(Backwar
   const int n = min(32, a.P - i0);
   const int i = i0 + lane;
   const int stride = sh_stride(a.M);
-  const GView gv = make_gview(a, lane < n ? i : i0, s_mats);
+  const float* row = sw + lane * stride;
   if (a.items == nullptr) {
-    if (a.sh_dc != nullptr) sh_stage_in_raw(a.sh_dc, a.sh_ac, a.M, i0, n, sw, stride);
-    else sh_stage_in(a.shs, a.M, i0, n, sw, stride);
+    if (a.sh_dc != nullptr) {
+      if (sh_stage_in_raw(a.sh_dc, a.sh_ac, a.M, i0, n, sw, stride)) row = sw + 45 * lane - 3;
+    } else {
+      sh_stage_in(a.shs, a.M, i0, n, sw, stride);
+    }
   } else {
     batch_sh_stage_in(a, i0, n, sw, stride);
   }
+  const GView gv = make_gview(a, lane < n ? i : i0, s_mats);
   float basis[16], cf[3] = {0.f, 0.f, 0.f};
   const bool active = lane < n && a.radii[i] > 0;
+  GOut o;
+  float dcov[6], sd[3];
+  if (active) ref_gaussian_geometry(a, i, gv, o, dcov, sd);
+  copy_wait();
+  __syncwarp();
   if (active) {
-    GOut o;
-    ref_gaussian(a, i, gv, sw + lane * stride, basis, cf, o);
+    ref_gaussian_rest(a, i, gv, row, dcov, sd, basis, cf, o);
     store_gout(a, i, o);
   } else if (lane < n) {
     for (int k = 0; k < 3; ++k) a.dL_dmeans3D[3 * i + k] = 0.f;
@@ -1239,7 +1281,7 @@ __device__ __forceinline__ void exact_gaussian(const BackwardArgs& a, int i, con
 }
 
 __global__ void __launch_bounds__(kGaussThreads) gaussians_exact_kernel(BackwardArgs a) {
-  __shared__ float s_sh[kGaussThreads / 32][32 * kShStride];
+  __shared__ __align__(16) float s_sh[kGaussThreads / 32][32 * kGaussRow];
   // view, projection, camera position: shared memory is never aliased by the
   // outputs, so these stay in place across the output stores
   __shared__ float s_mats[35];
@@ -1291,7 +1333,7 @@ __global__ void __launch_bounds__(kGaussThreads) gaussians_exact_kernel(Backward
 // ---------------------------------------------------------------------------
 template <int kMode>
 __global__ void __launch_bounds__(kGaussThreads) gaussians_group_kernel(BackwardArgs a) {
-  __shared__ float s_sh[kGaussThreads / 32][32 * kShStride];
+  __shared__ __align__(16) float s_sh[kGaussThreads / 32][32 * kGaussRow];
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   float* sw = s_sh[threadIdx.x >> 5];
@@ -1336,7 +1378,11 @@ __global__ void __launch_bounds__(kGaussThreads) gaussians_group_kernel(Backward
       float basis[16], cf[3];
       GOut o;
       if (kMode == 1) exact_gaussian(a, int(i), gv, sh_row, basis, cf, o);
-      else ref_gaussian(a, int(i), gv, sh_row, basis, cf, o);
+      else {
+        float dcov[6], sd[3];
+        ref_gaussian_geometry(a, int(i), gv, o, dcov, sd);
+        ref_gaussian_rest(a, int(i), gv, sh_row, dcov, sd, basis, cf, o);
+      }
 #pragma unroll
       for (int c = 0; c < 3; ++c) am[c] = add(am[c], o.m3[c]);
 #pragma unroll

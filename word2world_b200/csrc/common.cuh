@@ -295,6 +295,33 @@ constexpr int kPreThreads = 256;  // Gaussians per preprocess block (one scan ti
 constexpr int kShStride = 49;  // odd row stride: row reads by 32 threads hit 32 banks
 
 __host__ __device__ __forceinline__ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0u; }
+// Quaternion i of p, in one load where p is 16-byte aligned.
+__device__ __forceinline__ float4 load_quat(const float* p, int i) {
+  if (aligned16(p)) return __ldg(reinterpret_cast<const float4*>(p) + i);
+  return make_float4(__ldg(p + 4 * i), __ldg(p + 4 * i + 1), __ldg(p + 4 * i + 2), __ldg(p + 4 * i + 3));
+}
+
+// Asynchronous copies of 16-byte pieces to shared memory (both sides aligned):
+// no registers and no store instructions in between, and what follows runs
+// under them.  copy_wait() completes this thread's copies (other lanes' need
+// the warp barrier after theirs).
+__device__ __forceinline__ void copy_async16(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;"
+               :: "r"(uint32_t(__cvta_generic_to_shared(dst))), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// Warp-collective: `floats` (a multiple of 4) contiguous floats.
+__device__ __forceinline__ void copy_span_async(float* dst, const float* src, int floats) {
+  for (int f = 4 * int(threadIdx.x & 31); f < floats; f += 128) copy_async16(dst + f, src + f);
+}
+// The raw SH rows of 32 Gaussians as they lie in memory: sh_dc's rows of 3, then
+// sh_ac's rows of 45 (both strides are odd: 32 lanes at their own rows hit 32
+// banks).
+constexpr int kRawAc = 3 * 32;
+__device__ __forceinline__ void copy_raw_rows_async(float* dst, const float* dc, const float* ac, size_t i0) {
+  copy_span_async(dst, dc + i0 * 3, 32 * 3);
+  copy_span_async(dst + kRawAc, ac + i0 * 45, 32 * 45);
+}
 
 // Vector forms for a full warp of degree-3 rows (M == 16): the warp's rows are
 // one contiguous span, moved as float4s (coalesced 16-byte accesses; the span

@@ -178,15 +178,16 @@ __device__ __forceinline__ float xmy(float x, float y, float xx, float yy) {
 }
 
 // SH colour (gaussianForwardPass.cu:195-263); coefficients needed by a degree
-// are used only when stored (degree d needs (d+1)^2 of them).
-__device__ __forceinline__ void sh_colour(const float* __restrict__ sh, int M, int deg, float px, float py, float pz,
+// are used only when stored (degree d needs (d+1)^2 of them).  Coefficient 0 is
+// at dc, coefficient k > 0 at sh + 3 k.
+__device__ __forceinline__ void sh_colour(const float* dc, const float* sh, int M, int deg, float px, float py, float pz,
                                           const float* __restrict__ campos, float rgb[3], uint8_t clamped[3]) {
   using namespace fp;
   const float vx = sub(px, campos[0]), vy = sub(py, campos[1]), vz = sub(pz, campos[2]);
   const float l2 = s3<SH_DOT>(vx, vx, vy, vy, vz, vz);
   const float inv = __frcp_rn(__fsqrt_rn(l2));
   const float x = mul(vx, inv), y = mul(vy, inv), z = mul(vz, inv);
-  float o0 = mul(kC0, sh[0]), o1 = mul(kC0, sh[1]), o2 = mul(kC0, sh[2]);
+  float o0 = mul(kC0, dc[0]), o1 = mul(kC0, dc[1]), o2 = mul(kC0, dc[2]);
   auto acc = [&](float coef, int idx) {
     o0 = s1<SH_ACC>(coef, sh[3 * idx + 0], o0);
     o1 = s1<SH_ACC>(coef, sh[3 * idx + 1], o1);
@@ -229,11 +230,22 @@ __device__ __forceinline__ void sh_colour(const float* __restrict__ sh, int M, i
   for (int k = 0; k < 3; ++k) clamped[k] = rgb[k] < 0.0f ? 1 : 0;
 }
 
-// 4 CTAs per SM (64 registers, a few spilled): measured 2 % faster than 3 at 80.
+// What bounds it: latency, at 32 warps per SM (registers and staged rows both
+// allow four CTAs) and some 2000 instructions a Gaussian; DRAM runs at 2.5 of
+// 6.5 TB/s.  So the order of the work hides what it can: the raw degree-3 rows
+// (M == 16) of a full warp travel to shared memory asynchronously, as they lie
+// in memory, under the projection, the culling and the block's scan; the scan's
+// aggregate is published before the colours are computed, so that the lookback
+// after them finds its predecessors'.  Per view at 500k Gaussians 91 -> 84 us
+// (copies) -> 78 us (order of the scan), at 1M 161 -> 133 us, at 16k 12.2 -> 8.4
+// us.  Coalesced stores of the short rows, 32-byte record stores and a lookback
+// of 128 tiles a step made no difference; blocks of 128 or 64 threads were slower
+// (93, 100 us).  3 CTAs per SM at 80 registers: 88 us, 2 at 128: 96 us (4 spill
+// 80 bytes).
 // kRaw: the raw parameters of Renderer.render, activated here (PreprocessArgs).
-// kStage: degree-3 rows (M == 16) of a full warp are staged through shared
-// memory as coalesced float4 spans (dynamic shared memory, kStageBytes) instead
-// of each thread gathering its own 192-byte row.
+// kStage: degree-3 rows are staged through shared memory (dynamic, kStageBytes)
+// instead of each thread gathering its own 192-byte row; activated parameters'
+// rows of 48 floats are spread over rows of 49 on the way.
 constexpr int kStageBytes = kPreThreads * kShStride * 4;
 
 // kMinBlocks: CTAs per SM the register budget is sized for (the tuning knob
@@ -280,85 +292,50 @@ preprocess_kernel(PreprocessArgs a) {
     staged = f == find_item_elem(a.items, a.num_items, uint32_t(i0 + 31)) && a.items[f].M == 16;
     span = a.items[f].shs + size_t(i0 - int(a.items[f].elem_base)) * 48;
   }
-  const float* srow = s_rows + int(threadIdx.x >> 5) * 32 * kShStride;
+  const int lane32 = int(threadIdx.x & 31);
+  float* const w = s_rows + int(threadIdx.x >> 5) * 32 * kShStride;
   if (staged) {
-    float* w = s_rows + int(threadIdx.x >> 5) * 32 * kShStride;
-    if (kRaw) {
-      stage_span(a.sh_dc + size_t(i0) * 3, 3, w, kShStride, 0);
-      stage_span(a.sh_ac + size_t(i0) * 45, 45, w, kShStride, 3);
-    } else {
-      stage_span(span, 48, w, kShStride, 0);
-    }
-    __syncwarp();
+    if (kRaw) copy_raw_rows_async(w, a.sh_dc, a.sh_ac, size_t(i0));
+    else stage_span(span, 48, w, kShStride, 0);
   }
-  srow += int(threadIdx.x & 31) * kShStride;
+  const float* dc = kRaw ? w + 3 * lane32 : w + lane32 * kShStride;
+  const float* row = kRaw ? w + kRawAc + 45 * lane32 - 3 : dc;  // coefficient k at row + 3 k
 
   uint32_t alloc = 0, emit = 0;
   uint32_t depth_bits = 0;
+  Geometry g;
+  float px = 0.f, py = 0.f, pz = 0.f, opacity = 0.f;
   if (i < P) {
-    const float px = means3D[3 * gi], py = means3D[3 * gi + 1], pz = means3D[3 * gi + 2];
-    float sx, sy, sz, opacity;
-    float4 q;
+    const float* sp = kRaw ? a.svec : scales;
+    px = __ldg(means3D + 3 * gi);
+    py = __ldg(means3D + 3 * gi + 1);
+    pz = __ldg(means3D + 3 * gi + 2);
+    float sx = __ldg(sp + 3 * gi), sy = __ldg(sp + 3 * gi + 1), sz = __ldg(sp + 3 * gi + 2);
+    float4 q = load_quat(kRaw ? a.quat : rotations, gi);
+    opacity = __ldg((kRaw ? a.logit : opacities) + gi);
     if constexpr (kRaw) {
-      sx = expf(a.svec[3 * gi]);
-      sy = expf(a.svec[3 * gi + 1]);
-      sz = expf(a.svec[3 * gi + 2]);
-      q = act_normalize(a.quat[4 * gi], a.quat[4 * gi + 1], a.quat[4 * gi + 2], a.quat[4 * gi + 3]);
-      opacity = act_sigmoid(a.logit[gi]);
-    } else {
-      sx = scales[3 * gi];
-      sy = scales[3 * gi + 1];
-      sz = scales[3 * gi + 2];
-      q = make_float4(rotations[4 * gi], rotations[4 * gi + 1], rotations[4 * gi + 2], rotations[4 * gi + 3]);
-      opacity = opacities[gi];
+      sx = expf(sx);
+      sy = expf(sy);
+      sz = expf(sz);
+      q = act_normalize(q.x, q.y, q.z, q.w);
+      opacity = act_sigmoid(opacity);
     }
-    Geometry g;
     project(view, proj, focal, float(Wd), float(Hd), px, py, pz, sx, sy, sz, q, g);
     float* cov3 = a.cov3D + 6 * size_t(i);
 #pragma unroll
     for (int k = 0; k < 6; ++k) cov3[k] = g.cov3[k];
-
-    // SH colour
-    float rgb[3];
-    uint8_t clampf[3];
-    const float* shp = kRaw ? nullptr : shs + size_t(gi) * M * 3;
-    if (staged) {
-      sh_colour(srow, 16, degree, px, py, pz, campos, rgb, clampf);
-    } else if constexpr (kRaw) {  // the row is sh_dc (3 floats) then sh_ac (3 (M - 1) floats); M <= 16
-      float buf[48];
-      const float* dc = a.sh_dc + 3 * size_t(gi);
-      const float* ac = a.sh_ac + size_t(gi) * 3 * (M - 1);
-      // only the coefficients the degree uses: (degree + 1)^2 of the M stored
-      const int used = 3 * min(M, (degree + 1) * (degree + 1));
-#pragma unroll
-      for (int k = 0; k < 3; ++k) buf[k] = __ldg(dc + k);
-#pragma unroll
-      for (int k = 3; k < 48; ++k) buf[k] = k < used ? __ldg(ac + (k - 3)) : 0.f;
-      sh_colour(buf, M, degree, px, py, pz, campos, rgb, clampf);
-    } else if constexpr (kSh16) {
-      float buf[48];
-      const float4* s4 = reinterpret_cast<const float4*>(shp);
-#pragma unroll
-      for (int k = 0; k < 12; ++k) {
-        const float4 t = __ldg(s4 + k);
-        buf[4 * k] = t.x; buf[4 * k + 1] = t.y; buf[4 * k + 2] = t.z; buf[4 * k + 3] = t.w;
-      }
-      sh_colour(buf, 16, degree, px, py, pz, campos, rgb, clampf);
-    } else {
-      sh_colour(shp, M, degree, px, py, pz, campos, rgb, clampf);
-    }
-    reinterpret_cast<float*>(a.rgb)[3 * i] = rgb[0];
-    reinterpret_cast<float*>(a.rgb)[3 * i + 1] = rgb[1];
-    reinterpret_cast<float*>(a.rgb)[3 * i + 2] = rgb[2];
-    a.clamped[3 * i] = clampf[0];
-    a.clamped[3 * i + 1] = clampf[1];
-    a.clamped[3 * i + 2] = clampf[2];
-
+  }
+  float skip = -__int_as_float(0x7f800000), rec_depth = 0.f;
+  CullParams cp{-1.0f, 0.f, 0.f, 0.f, 0.f};
+  if (i < P) {
     int radius = 0;
     uint32_t rect_lo = 0, rect_hi = 0;
     BlendRecord rec{};
     if (g.visible) {
-      // ADR culling (ADRculling.cu:39-107)
+      // ADR culling (ADRculling.cu:39-107); the divisions by the tile size are by a
+      // power of two, so multiplying by its inverse rounds the same
+      constexpr float kInvTile = 1.0f / kTile;
+      static_assert((kTile & (kTile - 1)) == 0, "");
       using namespace fp;
       const float ht = mul(add(g.cxx, g.cyy), 0.5f);
       const float dsq = s1<ADR_DELTA>(ht, ht, -g.det);
@@ -370,10 +347,10 @@ preprocess_kernel(PreprocessArgs a) {
         const float adapt = __fsqrt_rn(mul(mul(2.0f, ymax), ln));
         const float mr = fminf(adapt, allp);
         radius = int(ceilf(mr));
-        int x0 = int(div(sub(g.mx, mr), 16.0f));
-        int y0 = int(div(sub(g.my, mr), 16.0f));
-        int x1 = int(div(add(add(g.mx, mr), 15.0f), 16.0f));
-        int y1 = int(div(add(add(g.my, mr), 15.0f), 16.0f));
+        int x0 = int(mul(sub(g.mx, mr), kInvTile));
+        int y0 = int(mul(sub(g.my, mr), kInvTile));
+        int x1 = int(mul(add(add(g.mx, mr), 15.0f), kInvTile));
+        int y1 = int(mul(add(add(g.my, mr), 15.0f), kInvTile));
         x0 = max(0, x0); y0 = max(0, y0);
         x1 = min(gw, x1); y1 = min(gh, y1);
         x1 = max(x1, x0); y1 = max(y1, y0);
@@ -381,10 +358,10 @@ preprocess_kernel(PreprocessArgs a) {
         if (a.compat_spill) {
           // emission rectangle of prepareSort.cu:279-282 (integer radius, floor/ceil)
           const float rf = float(radius);
-          const int ex0 = min(gw, max(0, int(floorf(div(sub(g.mx, rf), 16.0f)))));
-          const int ex1 = min(gw, max(0, int(ceilf(div(add(g.mx, rf), 16.0f)))));
-          const int ey0 = min(gh, max(0, int(floorf(div(sub(g.my, rf), 16.0f)))));
-          const int ey1 = min(gh, max(0, int(ceilf(div(add(g.my, rf), 16.0f)))));
+          const int ex0 = min(gw, max(0, int(floorf(mul(sub(g.mx, rf), kInvTile)))));
+          const int ex1 = min(gw, max(0, int(ceilf(mul(add(g.mx, rf), kInvTile)))));
+          const int ey0 = min(gh, max(0, int(floorf(mul(sub(g.my, rf), kInvTile)))));
+          const int ey1 = min(gh, max(0, int(ceilf(mul(add(g.my, rf), kInvTile)))));
           x0 = ex0; x1 = ex1; y0 = ey0; y1 = ey1;
         }
         emit = uint32_t(x1 - x0) * uint32_t(y1 - y0);
@@ -396,7 +373,6 @@ preprocess_kernel(PreprocessArgs a) {
       rec.det = d2<BL_DET>(g.cxx, g.cyy, g.cxy, g.cxy);
       rec.opacity = opacity;
       rec.depth = g.depth;
-      rec.r = rgb[0]; rec.g = rgb[1]; rec.b = rgb[2];
       reinterpret_cast<float4*>(a.conic)[i] = make_float4(g.conic[0], g.conic[1], g.conic[2], opacity);
       reinterpret_cast<float2*>(a.means2D)[i] = make_float2(g.mx, g.my);
       a.depth[i] = g.depth;
@@ -411,8 +387,6 @@ preprocess_kernel(PreprocessArgs a) {
     a.tiles[i] = alloc;
     reinterpret_cast<uint2*>(a.rect)[i] = make_uint2(rect_lo, rect_hi);
     // backward skip threshold (BackwardRecord::skip) and block-culling parameters
-    float skip = -__int_as_float(0x7f800000);
-    CullParams cp{-1.0f, 0.f, 0.f, 0.f, 0.f};
     if (g.visible) {
       skip = opacity > 0.0f ? -logf(255.0f * opacity) - 1e-4f : __int_as_float(0x7f800000);
       cp = make_cull_params(g.conic[0], g.conic[1], g.conic[2], opacity);
@@ -421,18 +395,10 @@ preprocess_kernel(PreprocessArgs a) {
     rp[0] = make_float4(rec.mx, rec.my, cp.hy, cp.beta);
     rp[1] = make_float4(cp.gamma, cp.eps, cp.vr, rec.opacity);
     rp[2] = make_float4(rec.cxx, rec.cxy, rec.cyy, rec.det);
-    rp[3] = make_float4(rec.depth, rec.r, rec.g, rec.b);
     float4* bp = reinterpret_cast<float4*>(a.bwd_record) + 4 * size_t(i);
-    if (g.visible) {
-      bp[0] = make_float4(g.mx, g.my, g.conic[0], g.conic[1]);
-      bp[1] = make_float4(g.conic[2], opacity, g.depth, rgb[0]);
-      bp[2] = make_float4(rgb[1], rgb[2], skip, cp.hy);
-      bp[3] = make_float4(cp.beta, cp.gamma, cp.eps, cp.vr);
-    } else {
-      bp[0] = bp[1] = bp[2] = make_float4(0.f, 0.f, 0.f, 0.f);
-      bp[3] = make_float4(0.f, 0.f, 0.f, 0.f);
-      bp[2].w = -1.0f;
-    }
+    bp[0] = g.visible ? make_float4(g.mx, g.my, g.conic[0], g.conic[1]) : make_float4(0.f, 0.f, 0.f, 0.f);
+    bp[3] = g.visible ? make_float4(cp.beta, cp.gamma, cp.eps, cp.vr) : make_float4(0.f, 0.f, 0.f, 0.f);
+    rec_depth = rec.depth;
   }
 
   // depth-bit range of Gaussians that emit keys (sizes the sort)
@@ -476,6 +442,60 @@ preprocess_kernel(PreprocessArgs a) {
   }
   __syncthreads();
   const Pair block_total = s_warp[kPreThreads / 32 - 1];
+  // published before the colours are computed, so that the tiles after this one
+  // rarely wait for it
+  const bool publish = (long long)tile != a.unpublished_tile;
+  if (threadIdx.x == 0 && publish)
+    st_relaxed64(a.scan_status + tile, pack(tile == 0 ? kFlagInc : kFlagAgg, block_total));
+
+  if (staged) {  // the rows were copied while the geometry was computed
+    if (kRaw) copy_wait();
+    __syncwarp();
+  }
+  if (i < P) {
+    // SH colour
+    float rgb[3];
+    uint8_t clampf[3];
+    const float* shp = kRaw ? nullptr : shs + size_t(gi) * M * 3;
+    if (staged) {
+      sh_colour(dc, row, 16, degree, px, py, pz, campos, rgb, clampf);
+    } else if constexpr (kRaw) {  // the row is sh_dc (3 floats) then sh_ac (3 (M - 1) floats); M <= 16
+      float buf[48];
+      const float* first = a.sh_dc + 3 * size_t(gi);
+      const float* ac = a.sh_ac + size_t(gi) * 3 * (M - 1);
+      // only the coefficients the degree uses: (degree + 1)^2 of the M stored
+      const int used = 3 * min(M, (degree + 1) * (degree + 1));
+#pragma unroll
+      for (int k = 0; k < 3; ++k) buf[k] = __ldg(first + k);
+#pragma unroll
+      for (int k = 3; k < 48; ++k) buf[k] = k < used ? __ldg(ac + (k - 3)) : 0.f;
+      sh_colour(buf, buf, M, degree, px, py, pz, campos, rgb, clampf);
+    } else if constexpr (kSh16) {
+      float buf[48];
+      const float4* s4 = reinterpret_cast<const float4*>(shp);
+#pragma unroll
+      for (int k = 0; k < 12; ++k) {
+        const float4 t = __ldg(s4 + k);
+        buf[4 * k] = t.x; buf[4 * k + 1] = t.y; buf[4 * k + 2] = t.z; buf[4 * k + 3] = t.w;
+      }
+      sh_colour(buf, buf, 16, degree, px, py, pz, campos, rgb, clampf);
+    } else {
+      sh_colour(shp, shp, M, degree, px, py, pz, campos, rgb, clampf);
+    }
+    reinterpret_cast<float*>(a.rgb)[3 * i] = rgb[0];
+    reinterpret_cast<float*>(a.rgb)[3 * i + 1] = rgb[1];
+    reinterpret_cast<float*>(a.rgb)[3 * i + 2] = rgb[2];
+    a.clamped[3 * i] = clampf[0];
+    a.clamped[3 * i + 1] = clampf[1];
+    a.clamped[3 * i + 2] = clampf[2];
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    reinterpret_cast<float4*>(a.record)[4 * size_t(i) + 3] =
+        g.visible ? make_float4(rec_depth, rgb[0], rgb[1], rgb[2]) : none;
+    float4* bp = reinterpret_cast<float4*>(a.bwd_record) + 4 * size_t(i);
+    bp[1] = g.visible ? make_float4(g.conic[2], opacity, g.depth, rgb[0]) : none;
+    bp[2] = g.visible ? make_float4(rgb[1], rgb[2], skip, cp.hy) : make_float4(0.f, 0.f, 0.f, -1.0f);
+  }
+
   // decoupled lookback by warp 0; each status word carries its flag and pair
   // together and nothing else written by its tile is read, so relaxed
   // accesses suffice.  Each step reads the 32 tiles before t at once and,
@@ -484,14 +504,9 @@ preprocess_kernel(PreprocessArgs a) {
   // left); a serial walk would cost one L2 round trip per tile.
   if (warp == 0) {
     unsigned long long* status = a.scan_status;
-    const bool publish = (long long)tile != a.unpublished_tile;
     if (tile == 0) {
-      if (lane == 0) {
-        if (publish) st_relaxed64(status + tile, pack(kFlagInc, block_total));
-        s_prefix = Pair{0, 0, 0};
-      }
+      if (lane == 0) s_prefix = Pair{0, 0, 0};
     } else {
-      if (lane == 0 && publish) st_relaxed64(status + tile, pack(kFlagAgg, block_total));
       // (0, 0, 0) is an identity on both sides for every pair that occurs
       Pair ex{0, 0, 0};
       long long t = int(tile) - 1;
