@@ -312,11 +312,18 @@ int w2w_activate_backward(long long P, int K, const float* g_opacity, const floa
  * sides) of opacity * exp(-1/2 d^T Sigma^-1 d), Sigma given by its upper
  * triangle (xx, xy, xz, yy, yz, zz).  Each Gaussian is binned once into the
  * blocks that hold its mean instead of being tested by every voxel.
- * w2w_voxel_field takes device pointers and enqueues on `stream` (its
- * temporaries come from the stream-ordered allocator; it synchronises the
- * stream once, to size them); w2w_compute_voxel_field is the reference's
+ * w2w_voxel_field takes device pointers and enqueues on `stream`; its
+ * temporaries come from the stream-ordered allocator.  w2w_voxel_field_in takes
+ * them from the caller instead: w2w_voxel_field_scratch bytes (256-byte
+ * aligned; 0 where the pairs of Gaussians and blocks have to be counted first,
+ * and then taken from the allocator).  Both read the status back and so
+ * synchronise the stream.  w2w_compute_voxel_field is the reference's
  * entry point (compute_voxel_field_cuda), with host pointers.  2 <= R <= 2048,
  * 1 <= B <= 1000, 0 <= relax_ratio <= 64; non-finite means are not supported. */
+size_t w2w_voxel_field_scratch(int n, int resolution, int num_blocks, float relax_ratio);
+int w2w_voxel_field_in(const float* means, const float* covs, const float* opacities, int n, int resolution,
+                       int num_blocks, float relax_ratio, float* occ, void* scratch, size_t scratch_bytes,
+                       w2w_stream_t stream);
 int w2w_voxel_field(const float* means, const float* covs, const float* opacities, int n, int resolution,
                     int num_blocks, float relax_ratio, float* occ, w2w_stream_t stream);
 int w2w_compute_voxel_field(float* h_occ, const float* h_means, const float* h_covs, const float* h_opacities,

@@ -643,8 +643,11 @@ Tensor voxel_field(const Tensor& means, const Tensor& covs, const Tensor& opacit
   TORCH_CHECK(m.numel() == 3 * n && c.numel() == 6 * n && o.numel() == n,
               "means [N,3], covs [N,6] (xx, xy, xz, yy, yz, zz), opacities [N] expected");
   Tensor occ = torch::empty({resolution, resolution, resolution}, m.options());
-  check(w2w_voxel_field(m.data_ptr<float>(), c.data_ptr<float>(), o.data_ptr<float>(), int(n), int(resolution),
-                        int(num_blocks), float(relax_ratio), occ.data_ptr<float>(), cur_stream()),
+  const size_t bytes = w2w_voxel_field_scratch(int(n), int(resolution), int(num_blocks), float(relax_ratio));
+  Tensor scratch = torch::empty({int64_t(bytes)}, m.options().dtype(torch::kUInt8));
+  check(w2w_voxel_field_in(m.data_ptr<float>(), c.data_ptr<float>(), o.data_ptr<float>(), int(n), int(resolution),
+                           int(num_blocks), float(relax_ratio), occ.data_ptr<float>(), scratch.data_ptr(), bytes,
+                           cur_stream()),
         "w2w_voxel_field");
   return occ;
 }

@@ -1008,19 +1008,60 @@ int w2w_activate_backward(long long P, int K, const float* g_opacity, const floa
   return check_launch();
 }
 
-int w2w_voxel_field(const float* means, const float* covs, const float* opacities, int n, int resolution,
-                    int num_blocks, float relax_ratio, float* occ, w2w_stream_t stream) {
-  if (n < 0 || resolution < 2 || resolution > 2048 || num_blocks < 1 || num_blocks > 1000 ||
-      !(relax_ratio >= 0.0f && relax_ratio <= 64.0f) || !occ)
-    return W2W_ERR_INVALID;
-  if (n > 0 && (!means || !covs || !opacities)) return W2W_ERR_INVALID;
-  cudaStream_t st = S(stream);
-  const size_t voxels = size_t(resolution) * resolution * resolution;
-  if (n == 0) {
-    cudaMemsetAsync(occ, 0, voxels * 4, st);
-    return check_launch();
+// Pairs of a Gaussian on the voxel field's route without a count, or 0 for the
+// other.  A mean lies within at most floor(1 + 2 relax) + 1 of an axis's grown
+// blocks (the hundredth is far above the bounds' rounding).  Up to 2^20 slots
+// (and blocks) in all: 16 bytes each, and the sort's passes over the unused ones are cheaper
+// than the scan and the host's wait for the total that they replace (20k
+// Gaussians with eight slots, 64^3 voxels: 149 us a call counted, 85 with slots).
+constexpr long long kVoxelSlotMax = 1LL << 20;
+static int voxel_slots(int n, int num_blocks, float relax_ratio) {
+  const long long m = std::min((long long)num_blocks + 1, (long long)std::floor(2.0 * relax_ratio + 1.01) + 1);
+  const long long nb = num_blocks + 1LL;
+  return m * m * m * n <= kVoxelSlotMax && nb * nb * nb <= kVoxelSlotMax ? int(m * m * m) : 0;
+}
+
+// The route without a count: its scratch, of which [err, zero_end) starts zeroed.
+struct VoxelLayout {
+  size_t rec, keys_a, vals_a, keys_b, vals_b, ranges, err, hist, counters, status, tile_hist, zero_end, total;
+  int bits;
+  VoxelLayout(int n, int num_blocks, int slots) {
+    size_t o = 0;
+    auto take = [&](size_t bytes) { size_t a = align256(o); o = a + bytes; return a; };
+    const size_t nb = size_t(num_blocks) + 1, blocks = nb * nb * nb, pairs = size_t(n) * size_t(slots);
+    const size_t tile = size_t(sort_tile_keys(0, (long long)pairs));
+    bits = ceil_log2(uint32_t(blocks) + 1u);  // the key past the last block too
+    rec = take(size_t(n) * 48);
+    keys_a = take(pairs * 4);
+    vals_a = take(pairs * 4);
+    keys_b = take(pairs * 4);
+    vals_b = take(pairs * 4);
+    ranges = take(blocks * 8);
+    err = take(4);
+    hist = take(size_t(kMaxPasses) * kMaxBins * 4);
+    counters = take(size_t(kMaxPasses + 1) * 4);
+    status = take(size_t(sort_passes(bits)) * kMaxBins * 4 * ((pairs + tile - 1) / tile));
+    tile_hist = take(blocks * 4);
+    zero_end = o;
+    total = align256(o);
   }
-  const int nb = num_blocks + 1;  // the last voxel of an axis falls in block num_blocks
+};
+
+static bool voxel_ok(int n, int resolution, int num_blocks, float relax_ratio) {
+  return n >= 0 && resolution >= 2 && resolution <= 2048 && num_blocks >= 1 && num_blocks <= 1000 &&
+         relax_ratio >= 0.0f && relax_ratio <= 64.0f;
+}
+
+static int voxel_result(uint32_t err) {
+  if (err & kErrTimeout) return W2W_ERR_TIMEOUT;
+  if (err) return W2W_ERR_CAPACITY;
+  return check_launch();
+}
+
+// The pairs counted, their total read back, and room for them taken from the
+// stream-ordered allocator.
+static int voxel_field_counted(const VoxelArgs& args, cudaStream_t st) {
+  const int nb = args.B + 1;  // the last voxel of an axis falls in block B
   const int nblocks = nb * nb * nb;
   std::vector<void*> bufs;
   auto alloc = [&](size_t bytes) -> void* {
@@ -1033,11 +1074,8 @@ int w2w_voxel_field(const float* means, const float* covs, const float* opacitie
     for (void* p : bufs) cudaFreeAsync(p, st);
     bufs.clear();
   };
-  VoxelArgs a{};
-  a.P = n; a.R = resolution; a.B = num_blocks;
-  a.bs = 2.0f / float(num_blocks);
-  a.relax = relax_ratio;
-  a.means = means; a.covs = covs; a.opacities = opacities; a.occ = occ;
+  VoxelArgs a = args;
+  const int n = a.P;
   a.rec = static_cast<float4*>(alloc(size_t(n) * 48));
   a.count = static_cast<uint32_t*>(alloc(size_t(n) * 4));
   uint32_t* offsets = static_cast<uint32_t*>(alloc(size_t(n) * 4));
@@ -1053,7 +1091,7 @@ int w2w_voxel_field(const float* means, const float* covs, const float* opacitie
   const long long pairs = (long long)tail[0] + tail[1];
   if (pairs >= (1LL << 30)) { release(); return W2W_ERR_CAPACITY; }
   if (pairs == 0) {
-    cudaMemsetAsync(occ, 0, voxels * 4, st);
+    cudaMemsetAsync(a.occ, 0, size_t(a.R) * a.R * a.R * 4, st);
     release();
     return check_launch();
   }
@@ -1088,10 +1126,79 @@ int w2w_voxel_field(const float* means, const float* covs, const float* opacitie
   const cudaError_t se = cudaStreamSynchronize(st);
   release();
   if (se != cudaSuccess) return check_launch();
-  if (err & kErrTimeout) return W2W_ERR_TIMEOUT;
-  if (err) return W2W_ERR_CAPACITY;
-  return check_launch();
+  return voxel_result(err);
 }
+
+size_t w2w_voxel_field_scratch(int n, int resolution, int num_blocks, float relax_ratio) {
+  if (n == 0 || !voxel_ok(n, resolution, num_blocks, relax_ratio)) return 0;
+  const int slots = voxel_slots(n, num_blocks, relax_ratio);
+  return slots > 0 ? VoxelLayout(n, num_blocks, slots).total : 0;
+}
+
+int w2w_voxel_field_in(const float* means, const float* covs, const float* opacities, int n, int resolution,
+                       int num_blocks, float relax_ratio, float* occ, void* scratch, size_t scratch_bytes,
+                       w2w_stream_t stream) {
+  if (!voxel_ok(n, resolution, num_blocks, relax_ratio) || !occ) return W2W_ERR_INVALID;
+  if (n > 0 && (!means || !covs || !opacities)) return W2W_ERR_INVALID;
+  cudaStream_t st = S(stream);
+  if (n == 0) {
+    cudaMemsetAsync(occ, 0, size_t(resolution) * resolution * resolution * 4, st);
+    return check_launch();
+  }
+  VoxelArgs a{};
+  a.P = n; a.R = resolution; a.B = num_blocks;
+  a.bs = 2.0f / float(num_blocks);
+  a.relax = relax_ratio;
+  a.means = means; a.covs = covs; a.opacities = opacities; a.occ = occ;
+  const int slots = voxel_slots(n, num_blocks, relax_ratio);
+  if (slots == 0) return voxel_field_counted(a, st);
+  const VoxelLayout L(n, num_blocks, slots);
+  if (!scratch || scratch_bytes < L.total || (reinterpret_cast<uintptr_t>(scratch) & 255u) != 0u)
+    return W2W_ERR_SCRATCH;
+  VoxelArgs v = a;
+  const int nb = num_blocks + 1;
+  SortArgs so{};
+  so.n = (long long)n * slots; so.key64 = 0; so.begin_bit = 0; so.bits = L.bits;
+  const bool odd = sort_passes(L.bits) % 2 == 1;  // the result lands in the a buffers
+  so.keys_out = at<uint32_t>(scratch, L.keys_a); so.vals_out = at<uint32_t>(scratch, L.vals_a);
+  so.keys_tmp = at<uint32_t>(scratch, L.keys_b); so.vals_tmp = at<uint32_t>(scratch, L.vals_b);
+  v.rec = at<float4>(scratch, L.rec);
+  v.keys = at<uint32_t>(scratch, odd ? L.keys_b : L.keys_a);
+  v.vals = at<uint32_t>(scratch, odd ? L.vals_b : L.vals_a);
+  v.slots = slots;
+  v.error = at<uint32_t>(scratch, L.err);
+  so.keys_in = v.keys; so.vals_in = v.vals;
+  so.hist = at<uint32_t>(scratch, L.hist); so.status = at<uint32_t>(scratch, L.status);
+  so.counters = at<uint32_t>(scratch, L.counters); so.error = v.error;
+  so.tile_shift = 0; so.num_tiles = nb * nb * nb;
+  so.tile_hist = at<uint32_t>(scratch, L.tile_hist); so.ranges = at<uint2>(scratch, L.ranges);
+  so.cleared = true;
+  so.spin_limit = spin_limit();
+  so.unpublished_tile = unpublished_tile(kWaitSort);
+  cudaMemsetAsync(v.error, 0, L.zero_end - L.err, st);
+  launch_voxel_prepare(v, st);
+  launch_sort(so, st);
+  launch_voxel_field(v, so.vals_out, so.ranges, st);
+  uint32_t err = 0;
+  cudaMemcpyAsync(&err, v.error, 4, cudaMemcpyDeviceToHost, st);
+  if (cudaStreamSynchronize(st) != cudaSuccess) return check_launch();
+  if (err == kErrRange) return voxel_field_counted(a, st);
+  return voxel_result(err);
+}
+
+int w2w_voxel_field(const float* means, const float* covs, const float* opacities, int n, int resolution,
+                    int num_blocks, float relax_ratio, float* occ, w2w_stream_t stream) {
+  const size_t bytes = w2w_voxel_field_scratch(n, resolution, num_blocks, relax_ratio);
+  void* scratch = nullptr;
+  if (bytes > 0 && occ && means && covs && opacities &&
+      cudaMallocAsync(&scratch, bytes, S(stream)) != cudaSuccess)
+    return W2W_ERR_CUDA;
+  const int rc = w2w_voxel_field_in(means, covs, opacities, n, resolution, num_blocks, relax_ratio, occ, scratch,
+                                    bytes, stream);
+  if (scratch) cudaFreeAsync(scratch, S(stream));
+  return rc;
+}
+
 
 int w2w_compute_voxel_field(float* h_occ, const float* h_means, const float* h_covs, const float* h_opacities,
                             int n, int resolution, int num_blocks, float relax_ratio) {

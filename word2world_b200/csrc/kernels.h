@@ -330,6 +330,8 @@ struct VoxelArgs {
   uint32_t* keys;     // [pairs] block ids
   uint32_t* vals;     // [pairs] Gaussian ids
   float* occ;         // [R^3], x fastest
+  int slots = 0;      // > 0: this many pairs per Gaussian, unused ones with key (B + 1)^3
+  uint32_t* error = nullptr;  // slots > 0: set where a Gaussian has more
 };
 void launch_voxel_prepare(const VoxelArgs& a, cudaStream_t stream);
 void launch_voxel_emit(const VoxelArgs& a, cudaStream_t stream);

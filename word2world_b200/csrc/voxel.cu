@@ -15,6 +15,12 @@
 // reference's summation order), and each voxel walks only its block's list;
 // the inverse covariance is computed once per Gaussian instead of once per
 // voxel-Gaussian pair.
+//
+// A Gaussian lies in at most floor(1 + 2 relax) + 1 blocks of an axis.  Where
+// that makes few enough pairs (voxel_slots, capi.cu) every Gaussian gets that
+// many slots and fills the unused ones with a key past the last block, which the
+// stable sort moves to the end: no count, scan, or read of the total on the host
+// before the pairs can be emitted.  Otherwise they are counted and scanned.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -55,7 +61,9 @@ __device__ __forceinline__ void vox_span(float m, const VoxelArgs& a, int& lo, i
 }
 
 // Per Gaussian: the inverse covariance (cofactors over the regularised
-// determinant), its record, and the number of blocks it is binned into.
+// determinant), its record, and the number of blocks it is binned into; with
+// kSlots, its pairs instead of their number.
+template <bool kSlots>
 __global__ void __launch_bounds__(kVoxThreads) voxel_prepare_kernel(VoxelArgs a) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= a.P) return;
@@ -74,8 +82,30 @@ __global__ void __launch_bounds__(kVoxThreads) voxel_prepare_kernel(VoxelArgs a)
   vox_span(mx, a, xl, xh);
   vox_span(my, a, yl, yh);
   vox_span(mz, a, zl, zh);
-  a.count[g] = uint32_t(max(xh - xl + 1, 0) * max(yh - yl + 1, 0) * max(zh - zl + 1, 0));
+  if constexpr (!kSlots) {
+    a.count[g] = uint32_t(max(xh - xl + 1, 0) * max(yh - yl + 1, 0) * max(zh - zl + 1, 0));
+  } else {
+    const int nb = a.B + 1;
+    uint32_t* keys = a.keys + size_t(g) * a.slots;
+    uint32_t* vals = a.vals + size_t(g) * a.slots;
+    int s = 0;
+    for (int z = zl; z <= zh; ++z)
+      for (int y = yl; y <= yh; ++y)
+        for (int x = xl; x <= xh; ++x) {
+          if (s < a.slots) {
+            keys[s] = uint32_t(x + nb * (y + nb * z));
+            vals[s] = uint32_t(g);
+          }
+          ++s;
+        }
+    if (s > a.slots) atomicOr(a.error, kErrRange);  // only a mean that is not a number; counted then
+    for (; s < a.slots; ++s) {
+      keys[s] = uint32_t(nb * nb * nb);
+      vals[s] = uint32_t(g);
+    }
+  }
 }
+
 
 // Per Gaussian: its (block, Gaussian) pairs at its scanned offset, blocks in
 // x-fastest order.
@@ -97,33 +127,60 @@ __global__ void __launch_bounds__(kVoxThreads) voxel_emit_kernel(VoxelArgs a) {
       }
 }
 
-// One thread per voxel, x fastest within a CTA of 8 x 8 x 4 voxels, so a
-// warp's voxels share a block and its list entries are broadcast loads.
+// Opacity times the Gaussian's value at (x, y, z) from its record.
+__device__ __forceinline__ float vox_value(const float4& q0, const float4& q1, const float4& q2, float x, float y,
+                                           float z) {
+  const float dx = x - q0.x, dy = y - q0.y, dz = z - q0.z;
+  float power = -0.5f * (dx * dx * q1.x + dy * dy * q1.w + dz * dz * q2.y) - dx * dy * q1.y - dx * dz * q1.z -
+                dy * dz * q2.x;
+  if (power > 0) power = -1e10f;
+  return q0.w * expf(power);
+}
+
+// Two voxels per thread, neighbours in z, x fastest within a CTA of 8 x 8 x 8
+// voxels, so a warp's voxels share a block and its list entries are broadcast
+// loads, each used for 64 voxels.  Bound by the pairs' arithmetic (about 20
+// operations and an exponential each) once the loads are shared and four
+// entries' are in flight: 64^3 voxels of 20k Gaussians, 67 entries to a block,
+// 31 us with a voxel per thread and 29 with two.
 __global__ void __launch_bounds__(kVoxThreads) voxel_field_kernel(VoxelArgs a, const uint32_t* __restrict__ list,
                                                                     const uint2* __restrict__ ranges) {
   const int i = blockIdx.x * 8 + (threadIdx.x & 7);
   const int j = blockIdx.y * 8 + ((threadIdx.x >> 3) & 7);
-  const int k = blockIdx.z * 4 + (threadIdx.x >> 6);
+  const int k = blockIdx.z * 8 + 2 * (threadIdx.x >> 6);
   const int R = a.R;
   if (i >= R || j >= R || k >= R) return;
-  const float x = vox_coord(i, R), y = vox_coord(j, R), z = vox_coord(k, R);
+  const float x = vox_coord(i, R), y = vox_coord(j, R), z0 = vox_coord(k, R), z1 = vox_coord(k + 1, R);
   const int nb = a.B + 1;
   // voxel coordinates lie in [-1, 1], so their blocks lie in [0, B]; the
   // clamp only guards the ranges array
-  const int blk = vox_block_clamped(x, a.bs, a.B) +
-                  nb * (vox_block_clamped(y, a.bs, a.B) + nb * vox_block_clamped(z, a.bs, a.B));
-  const uint2 r = ranges[blk];
-  float val = 0.0f;
-  for (uint32_t e = r.x; e < r.y; ++e) {
-    const float4* rec = a.rec + 3 * size_t(__ldg(list + e));
-    const float4 q0 = __ldg(rec), q1 = __ldg(rec + 1), q2 = __ldg(rec + 2);
-    const float dx = x - q0.x, dy = y - q0.y, dz = z - q0.z;
-    float power = -0.5f * (dx * dx * q1.x + dy * dy * q1.w + dz * dz * q2.y) - dx * dy * q1.y - dx * dz * q1.z -
-                  dy * dz * q2.x;
-    if (power > 0) power = -1e10f;
-    val += q0.w * expf(power);
+  const int bx = vox_block_clamped(x, a.bs, a.B), by = vox_block_clamped(y, a.bs, a.B);
+  const int b0 = vox_block_clamped(z0, a.bs, a.B), b1 = vox_block_clamped(z1, a.bs, a.B);
+  const bool two = k + 1 < R;
+  float* out = a.occ + size_t(i) + size_t(R) * (size_t(j) + size_t(R) * size_t(k));
+  const uint2 r = ranges[bx + nb * (by + nb * b0)];
+  float v0 = 0.0f, v1 = 0.0f;
+  if (two && b0 == b1) {
+#pragma unroll 4
+    for (uint32_t e = r.x; e < r.y; ++e) {
+      const float4* rec = a.rec + 3 * size_t(__ldg(list + e));
+      const float4 q0 = __ldg(rec), q1 = __ldg(rec + 1), q2 = __ldg(rec + 2);
+      v0 += vox_value(q0, q1, q2, x, y, z0);
+      v1 += vox_value(q0, q1, q2, x, y, z1);
+    }
+  } else {  // the pair straddles two blocks, or the grid's edge
+    for (uint32_t e = r.x; e < r.y; ++e) {
+      const float4* rec = a.rec + 3 * size_t(__ldg(list + e));
+      v0 += vox_value(__ldg(rec), __ldg(rec + 1), __ldg(rec + 2), x, y, z0);
+    }
+    const uint2 r1 = two ? ranges[bx + nb * (by + nb * b1)] : make_uint2(0u, 0u);
+    for (uint32_t e = r1.x; e < r1.y; ++e) {
+      const float4* rec = a.rec + 3 * size_t(__ldg(list + e));
+      v1 += vox_value(__ldg(rec), __ldg(rec + 1), __ldg(rec + 2), x, y, z1);
+    }
   }
-  a.occ[size_t(i) + size_t(R) * (size_t(j) + size_t(R) * size_t(k))] = val;
+  out[0] = v0;
+  if (two) out[size_t(R) * size_t(R)] = v1;
 }
 
 }  // namespace
@@ -131,7 +188,9 @@ __global__ void __launch_bounds__(kVoxThreads) voxel_field_kernel(VoxelArgs a, c
 void launch_voxel_prepare(const VoxelArgs& a, cudaStream_t stream) {
   if (a.P <= 0) return;
   stage_begin(kStOther, stream);
-  voxel_prepare_kernel<<<(a.P + kVoxThreads - 1) / kVoxThreads, kVoxThreads, 0, stream>>>(a);
+  const int blocks = (a.P + kVoxThreads - 1) / kVoxThreads;
+  if (a.slots > 0) voxel_prepare_kernel<true><<<blocks, kVoxThreads, 0, stream>>>(a);
+  else voxel_prepare_kernel<false><<<blocks, kVoxThreads, 0, stream>>>(a);
   stage_end(kStOther, stream, 1);
 }
 
@@ -143,7 +202,7 @@ void launch_voxel_emit(const VoxelArgs& a, cudaStream_t stream) {
 }
 
 void launch_voxel_field(const VoxelArgs& a, const uint32_t* list, const uint2* ranges, cudaStream_t stream) {
-  const dim3 grid((a.R + 7) / 8, (a.R + 7) / 8, (a.R + 3) / 4);
+  const dim3 grid((a.R + 7) / 8, (a.R + 7) / 8, (a.R + 7) / 8);
   stage_begin(kStOther, stream);
   voxel_field_kernel<<<grid, kVoxThreads, 0, stream>>>(a, list, ranges);
   stage_end(kStOther, stream, 1);
