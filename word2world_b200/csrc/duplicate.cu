@@ -22,6 +22,13 @@
 // Load balance: each warp expands 32 consecutive Gaussians; every lane emits
 // one entry per round, so large and small Gaussians cost the same per entry
 // and stores to consecutive slots are coalesced.
+//
+// Bound by the rounds' instructions and by latency (order -> gathers -> lookback
+// -> rounds), not by the bytes written.  A round finds its owners in five
+// shuffles and takes six or seven words from them, and the row of a cell comes
+// from a multiplication where that is exact.  In depth order, per view: 100k
+// Gaussians, 2.4M instances, 25 -> 22.6 us; 500k, 5.9M, 47 -> 44.6; 1M, 36M, 141
+// -> 120-128, against eleven words and a division.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -155,6 +162,13 @@ __global__ void __launch_bounds__(kDupThreads) duplicate_kernel(DuplicateArgs a)
     __syncthreads();
     before = s_before + mine;
   }
+  // what an entry's lane needs of its owner, in as few words as it takes: entry
+  // e is rectangle cell e + cell; the row by a multiplication where that is
+  // exact (cell numbers and widths below 2^16)
+  const uint32_t cell = p0 - excl - start, slot = p0 - excl, corner = x0 | (y0 << 16);
+  const uint32_t inv = w > 1u ? 0xffffffffu / w + 1u : 0u;
+  const bool batched = a.items != nullptr;
+  const bool small = __all_sync(0xffffffffu, w < 65536u && p0 - start + cnt <= 65536u);
   for (uint32_t base = 0; base < total; base += 32) {
     const uint32_t e = base + lane;
     // owner lane: number of lanes whose inclusive count is <= e
@@ -165,30 +179,27 @@ __global__ void __launch_bounds__(kDupThreads) duplicate_kernel(DuplicateArgs a)
       if (t <= e) o += b;
     }
     o = min(o, 31);
-    const uint32_t op0 = __shfl_sync(0xffffffffu, p0, o);
-    const uint32_t oex = __shfl_sync(0xffffffffu, excl, o);
-    const uint32_t ost = __shfl_sync(0xffffffffu, start, o);
-    const uint32_t ox0 = __shfl_sync(0xffffffffu, x0, o);
-    const uint32_t oy0 = __shfl_sync(0xffffffffu, y0, o);
+    const uint32_t k = e + __shfl_sync(0xffffffffu, cell, o);
+    const uint32_t oc = __shfl_sync(0xffffffffu, corner, o);
     const uint32_t ow = __shfl_sync(0xffffffffu, w, o);
+    const uint32_t oi = __shfl_sync(0xffffffffu, inv, o);
     const uint32_t odl = __shfl_sync(0xffffffffu, dlow, o);
-    const uint32_t ogw = __shfl_sync(0xffffffffu, gwv, o);
-    const uint32_t otb = __shfl_sync(0xffffffffu, tbase, o);
     const uint32_t og = __shfl_sync(0xffffffffu, g, o);
-    if (e < total) {
-      const uint32_t p = op0 + (e - oex);
-      const uint32_t k = p - ost;
-      const uint32_t ty = oy0 + k / ow, tx = ox0 + k % ow;
-      const uint32_t tile = otb + ty * ogw + tx;
-      const uint32_t at = kOrdered ? before + e : p;
-      if (at < Rlim) {
-        if constexpr (kKey64) {
-          reinterpret_cast<uint64_t*>(a.keys)[at] = (uint64_t(tile) << a.depth_bits) | odl;
-        } else {
-          reinterpret_cast<uint32_t*>(a.keys)[at] = (a.depth_bits >= 32 ? 0u : (tile << a.depth_bits)) | odl;
-        }
-        a.vals[at] = og;
+    const uint32_t at = kOrdered ? before + e : e + __shfl_sync(0xffffffffu, slot, o);
+    uint32_t ogw = uint32_t(a.gw), otb = 0;
+    if (batched) {
+      ogw = __shfl_sync(0xffffffffu, gwv, o);
+      otb = __shfl_sync(0xffffffffu, tbase, o);
+    }
+    if (e < total && at < Rlim) {
+      const uint32_t row = small ? (ow > 1u ? __umulhi(k, oi) : k) : k / ow;
+      const uint32_t tile = otb + ((oc >> 16) + row) * ogw + (oc & 0xffffu) + (k - row * ow);
+      if constexpr (kKey64) {
+        reinterpret_cast<uint64_t*>(a.keys)[at] = (uint64_t(tile) << a.depth_bits) | odl;
+      } else {
+        reinterpret_cast<uint32_t*>(a.keys)[at] = (a.depth_bits >= 32 ? 0u : (tile << a.depth_bits)) | odl;
       }
+      a.vals[at] = og;
     }
   }
 }
