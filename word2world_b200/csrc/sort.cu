@@ -43,7 +43,7 @@ constexpr uint32_t kStatMask = (1u << 30) - 1u;
 // Threads of a histogram block: 256, four blocks to an SM, while the tile counts
 // fit beside the digit histograms in a quarter of the shared memory; 1024 and
 // one block beyond that, up to kSmemTileBins tiles; past it the tile counts go
-// straight to memory.  (12 views, 9216 tiles: 205 us with global counts, %HB%
+// straight to memory.  (12 views, 9216 tiles: 205 us with global counts, 38
 // with 1024 threads.)
 constexpr int kHistThreads = 256, kHistThreadsBig = 1024;
 constexpr int kSmemTileBinsSmall = 8192;
@@ -317,7 +317,7 @@ struct LookbackWindow {
 // (218.7, 211.2 us).
 // Up to kSortSmall keys (114 tiles of 6144: fewer than the SMs) the pass is one
 // tile's own chain of load, count, rank, look back and reorder, which a tile of
-// 2048 keys runs in half the time (kSmall): %SMALL%
+// 2048 keys runs in half the time (kSmall): 78k 27-bit keys, 9.6 -> 5 us a pass.
 template <typename K, bool kSmall>
 struct OnesweepShape;
 template <typename K>
