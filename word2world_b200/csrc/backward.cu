@@ -454,6 +454,7 @@ __device__ __forceinline__ BwdPixel make_bwd_pixel(const BackwardArgs& a, int ti
 
 template <typename Chain, bool kWide>
 __global__ void __launch_bounds__(32, 16) render_bwd_kernel(BackwardArgs a) {
+  grid_wait();
   __shared__ BwdWarp s;
   const int tile = int(a.order[blockIdx.x / 8]);  // heaviest first
   const int lane = int(threadIdx.x), block = int(blockIdx.x) % 8;
@@ -1063,6 +1064,7 @@ __device__ __forceinline__ void ref_gaussian_rest(const BackwardArgs& a, int i, 
 // outputs whose factors every lane looked up by index.  8 CTAs per SM (64
 // registers): more Gaussians' loads in flight.
 __global__ void __launch_bounds__(kGaussThreads, 8) gaussians_ref_kernel(BackwardArgs a) {
+  grid_wait();
   __shared__ __align__(16) float s_sh[kGaussThreads / 32][32 * kGaussRow];
   // view, projection, camera position: shared memory is never aliased by the
   // outputs, so these stay in place across the output stores
@@ -1281,6 +1283,7 @@ __device__ __forceinline__ void exact_gaussian(const BackwardArgs& a, int i, con
 }
 
 __global__ void __launch_bounds__(kGaussThreads) gaussians_exact_kernel(BackwardArgs a) {
+  grid_wait();
   __shared__ __align__(16) float s_sh[kGaussThreads / 32][32 * kGaussRow];
   // view, projection, camera position: shared memory is never aliased by the
   // outputs, so these stay in place across the output stores
@@ -1333,6 +1336,7 @@ __global__ void __launch_bounds__(kGaussThreads) gaussians_exact_kernel(Backward
 // ---------------------------------------------------------------------------
 template <int kMode>
 __global__ void __launch_bounds__(kGaussThreads) gaussians_group_kernel(BackwardArgs a) {
+  grid_wait();
   __shared__ __align__(16) float s_sh[kGaussThreads / 32][32 * kGaussRow];
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -1429,8 +1433,8 @@ void launch_backward_groups(const BackwardArgs& a, cudaStream_t stream) {
   if (a.group_rows <= 0 || a.num_groups <= 0) return;
   const long long blocks = (a.group_rows + kGaussThreads - 1) / kGaussThreads;
   stage_begin(kStBwdGaussians, stream);
-  if (a.grad_mode == 1) gaussians_group_kernel<1><<<unsigned(blocks), kGaussThreads, 0, stream>>>(a);
-  else gaussians_group_kernel<0><<<unsigned(blocks), kGaussThreads, 0, stream>>>(a);
+  launch_after(a.grad_mode == 1 ? gaussians_group_kernel<1> : gaussians_group_kernel<0>, unsigned(blocks),
+               kGaussThreads, 0, stream, a);
   stage_end(kStBwdGaussians, stream, 1);
 }
 
@@ -1441,8 +1445,8 @@ void launch_backward_render(const BackwardArgs& a, cudaStream_t stream) {
   const bool da = a.dL_ddepth != nullptr || a.dL_dalpha != nullptr;  // a loss reaches depth or alpha
   const bool wide = ((reinterpret_cast<uintptr_t>(a.record) | reinterpret_cast<uintptr_t>(a.bwd_record)) & 31u) == 0u;
   auto launch = [&](auto kernel, auto narrow) {
-    if (wide) kernel<<<tiles * 8, 32, 0, stream>>>(a);
-    else narrow<<<tiles * 8, 32, 0, stream>>>(a);
+    if (wide) launch_after(kernel, unsigned(tiles * 8), 32, 0, stream, a);
+    else launch_after(narrow, unsigned(tiles * 8), 32, 0, stream, a);
   };
   if (a.grad_mode == 1) launch(render_bwd_kernel<ExactChain, true>, render_bwd_kernel<ExactChain, false>);
   else if (da) launch(render_bwd_kernel<RefChain<true>, true>, render_bwd_kernel<RefChain<true>, false>);
@@ -1454,8 +1458,8 @@ void launch_backward_gaussians(const BackwardArgs& a, cudaStream_t stream) {
   if (a.P <= 0) return;
   const int blocks = (a.P + kGaussThreads - 1) / kGaussThreads;
   stage_begin(kStBwdGaussians, stream);
-  if (a.grad_mode == 1) gaussians_exact_kernel<<<blocks, kGaussThreads, 0, stream>>>(a);
-  else gaussians_ref_kernel<<<blocks, kGaussThreads, 0, stream>>>(a);
+  launch_after(a.grad_mode == 1 ? gaussians_exact_kernel : gaussians_ref_kernel, unsigned(blocks), kGaussThreads, 0,
+               stream, a);
   stage_end(kStBwdGaussians, stream, 1);
 }
 

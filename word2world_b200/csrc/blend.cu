@@ -146,6 +146,7 @@ __device__ __forceinline__ void group_alphas(BlendWarp& s, const BlendEntry& en,
 // warp's chain.
 template <bool kWide>
 __global__ void __launch_bounds__(32 * kBlendWarps, kBlendResident / kBlendWarps) blend_kernel(BlendArgs a) {
+  grid_wait();
   constexpr int kParts = 8 / kBlendWarps;  // CTAs per tile
   __shared__ BlendWarp s_warp[kBlendWarps];
   const int tile = int(a.order[blockIdx.x / kParts]);
@@ -705,7 +706,9 @@ void launch_blend(const BlendArgs& a, cudaStream_t stream) {
   stage_begin(kStBlend, stream);
   const bool queued = queue && (warps == 4 ? launch_queue<4>(a, tiles, stream) : launch_queue<8>(a, tiles, stream));
   if (!queued) {
-    auto launch = [&](auto kernel) { kernel<<<tiles * (8 / kBlendWarps), 32 * kBlendWarps, 0, stream>>>(a); };
+    auto launch = [&](auto kernel) {
+      launch_after(kernel, unsigned(tiles * (8 / kBlendWarps)), 32 * kBlendWarps, 0, stream, a);
+    };
     if ((reinterpret_cast<uintptr_t>(a.record) & 31u) == 0u) launch(blend_kernel<true>);
     else launch(blend_kernel<false>);
   }

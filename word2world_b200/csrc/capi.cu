@@ -597,7 +597,7 @@ int w2w_forward_render(const w2w_settings* s, const void* geom_state, const w2w_
 // ---- planned forward --------------------------------------------------------
 // A render whose sort and blend are launched before the host knows the view's
 // instance count R: the binning state is laid out for a capacity C and the
-// keys carry a guessed number of depth bits; a one-thread kernel checks both
+// keys carry a guessed number of depth bits; the emission checks both
 // against the projection pass's header on the device and either lets the
 // emission, histogram, sort passes and blend process R instances (read from
 // device memory), or sets `replan` and makes them process none, after which

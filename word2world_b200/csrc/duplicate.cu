@@ -70,6 +70,7 @@ __device__ __forceinline__ uint32_t lookback_sum(const uint32_t* status, int til
 // has only the tile digits left.
 template <bool kKey64, bool kOrdered>
 __global__ void __launch_bounds__(kDupThreads) duplicate_kernel(DuplicateArgs a) {
+  grid_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int block = blockIdx.x;
   if constexpr (kOrdered) {  // blocks in the order they start, so that lookback waits on running ones
@@ -212,11 +213,11 @@ void launch_duplicate(const DuplicateArgs& a, cudaStream_t stream) {
   const int blocks = max((a.P + kDupThreads - 1) / kDupThreads, min(296, int(a.clear_vecs / 1024u)));
   stage_begin(kStDuplicate, stream);
   if (a.order != nullptr) {
-    if (a.key64) duplicate_kernel<true, true><<<blocks, kDupThreads, 0, stream>>>(a);
-    else duplicate_kernel<false, true><<<blocks, kDupThreads, 0, stream>>>(a);
+    if (a.key64) launch_after(duplicate_kernel<true, true>, unsigned(blocks), kDupThreads, 0, stream, a);
+    else launch_after(duplicate_kernel<false, true>, unsigned(blocks), kDupThreads, 0, stream, a);
   } else {
-    if (a.key64) duplicate_kernel<true, false><<<blocks, kDupThreads, 0, stream>>>(a);
-    else duplicate_kernel<false, false><<<blocks, kDupThreads, 0, stream>>>(a);
+    if (a.key64) launch_after(duplicate_kernel<true, false>, unsigned(blocks), kDupThreads, 0, stream, a);
+    else launch_after(duplicate_kernel<false, false>, unsigned(blocks), kDupThreads, 0, stream, a);
   }
   stage_end(kStDuplicate, stream, 1);
 }

@@ -12,8 +12,8 @@
 //      tile scan is the per-tile [start, end) range table (empty tiles get (0,
 //      0), as the reference's memset leaves them), and the tiles' processing
 //      order follows from it (two one-block kernels before);
-//   2. one onesweep kernel per digit: each CTA takes the next tile (6144 32-bit or 5120 64-bit keys)
-//      (acquired through an atomic counter, so every earlier tile is already
+//   2. one onesweep kernel per digit: each CTA takes the next tile (6144 32-bit
+//      or 5120 64-bit keys, 2048 up to kSortSmall keys; acquired through an atomic counter, so every earlier tile is already
 //      running), ranks its keys stably (per-bit warp ballots), publishes its
 //      per-digit counts and looks back over earlier tiles for their prefix
 //      (decoupled lookback), then scatters through shared memory so the
@@ -212,6 +212,7 @@ hist_kernel(const K* __restrict__ keys, long long n, int begin_bit, int passes, 
             const uint32_t* __restrict__ n_dev, uint2* __restrict__ ranges, uint32_t* done, uint32_t* order,
             uint32_t* order_zero, uint32_t* order_counter) {
   extern __shared__ uint32_t smem[];
+  grid_wait();
   uint32_t* sh = smem;                      // passes * kMaxBins
   uint32_t* st = smem + passes * kMaxBins;  // num_tiles when they fit
   const bool tiles_in_smem = tile_hist != nullptr && num_tiles <= kSmemTileBins;
@@ -498,6 +499,7 @@ onesweep_kernel(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* 
   extern __shared__ __align__(16) unsigned char s_dyn[];
   K* s_keys = reinterpret_cast<K*>(s_dyn);
   uint32_t* s_vals = reinterpret_cast<uint32_t*>(s_dyn + sizeof(K) * kTile);
+  grid_wait();
   if (threadIdx.x == 0) sm.tile = atomicAdd(counter, 1u);
   // n < 2^30 (checked by every caller).  A planned render launches tiles for
   // its capacity and reads the count from device memory: a tile past the
@@ -538,8 +540,8 @@ void launch_onesweep_w(int tiles, cudaStream_t stream, const K* kin, const uint3
     cudaFuncSetAttribute(onesweep_kernel<K, kWidth, kSmall>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(dyn));
     if (dev >= 0 && dev < 64) opted[dev] = true;
   }
-  onesweep_kernel<K, kWidth, kSmall><<<tiles, kSortThreads, dyn, stream>>>(kin, vin, kout, vout, n, shift, digit_base,
-                                                                    status, counter, err, spin_limit, unpublished, n_dev);
+  launch_after(onesweep_kernel<K, kWidth, kSmall>, unsigned(tiles), kSortThreads, dyn, stream, kin, vin, kout, vout, n,
+               shift, digit_base, status, counter, err, spin_limit, unpublished, n_dev);
 }
 
 template <typename K, bool kSmall>
@@ -597,10 +599,10 @@ void run_sort(const SortArgs& a, cudaStream_t stream) {
       cudaFuncSetAttribute(hist_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     const int st_hist = a.stage_hist >= 0 ? a.stage_hist : kStSortHist;
     stage_begin(st_hist, stream);
-    hist_kernel<K><<<grid, threads, smem, stream>>>(reinterpret_cast<const K*>(a.keys_in), n, a.begin_bit,
-                                                    passes, dbits, a.bits, a.hist, a.tile_shift,
-                                                    a.num_tiles, a.tile_hist, a.n_dev, a.ranges,
-                                                    a.counters + kMaxPasses, a.order, a.order_zero, a.order_counter);
+    launch_after(hist_kernel<K>, unsigned(grid), unsigned(threads), smem, stream,
+                 reinterpret_cast<const K*>(a.keys_in), n, a.begin_bit, passes, dbits, a.bits, a.hist, a.tile_shift,
+                 a.num_tiles, a.tile_hist, a.n_dev, a.ranges, a.counters + kMaxPasses, a.order, a.order_zero,
+                 a.order_counter);
     stage_end(st_hist, stream, 1);
   }
   const K* kin = reinterpret_cast<const K*>(a.keys_in);
