@@ -315,7 +315,10 @@ struct LookbackWindow {
 // at 2 CTAs/SM 51.7 us, against 20 / 22 / 26 / 28 / 32 at 2 (57.9, 55.6, 55.8,
 // 59.7, 68.0 us) and 16 at 3 (59.8 us); 64-bit keys (20M pairs) 20 items at 2
 // CTAs/SM 174.5 us, against 16 / 24 at 2 (186.8, 203.0 us) and 12 / 16 at 3
-// (218.7, 211.2 us).
+// (218.7, 211.2 us).  With the four-operation ballots the shapes stand in the
+// same order: 64-bit, 9 bits, 20M pairs, 181 us, against 198 / 193 / 216 with 16 /
+// 22 / 24 at 2 and 217 with 16 at 3; 32-bit, 6 bits, 36M pairs, 191 us, against
+// 222 / 215 with 22 / 28 at 2 and 226 with 16 at 3.
 // Up to kSortSmall keys (114 tiles of 6144: fewer than the SMs) the pass is one
 // tile's own chain of load, count, rank, look back and reorder, which a tile of
 // 2048 keys runs in half the time (kSmall): 78k 27-bit keys, 9.6 -> 5 us a pass.
