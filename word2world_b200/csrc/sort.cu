@@ -11,7 +11,7 @@
 //      instance counts).  Its last block to finish scans those histograms; the
 //      tile scan is the per-tile [start, end) range table (empty tiles get (0,
 //      0), as the reference's memset leaves them), and the tiles' processing
-//      order follows from it (two one-block kernels before);
+//      order follows from it;
 //   2. one onesweep kernel per digit: each CTA takes the next tile (6144 32-bit
 //      or 5120 64-bit keys, 2048 up to kSortSmall keys; acquired through an atomic counter, so every earlier tile is already
 //      running), ranks its keys stably (per-bit warp ballots), publishes its
@@ -131,7 +131,11 @@ __device__ uint32_t block_exclusive_scan(uint32_t v, uint32_t* s_warp, uint32_t*
 // decreasing length (tile_bucket's buckets, heaviest first; order within a
 // bucket is arbitrary), with the blend's per-tile maximum and queue cleared.
 // Sixteen tiles to a thread: up to 4096 tiles are one round, whose counts stay in
-// registers from the scan to the ordering.
+// registers from the scan to the ordering; fewer tiles spread over the threads.
+// One block's chain of loads and scans, which is what a small histogram takes:
+// per view (whole kernel, with a run of keys a thread) 16k Gaussians 13.8 -> 10.2
+// us, 50k 14.1 -> 10.6, 1M 102 -> 94, against a block-wide scan per pass and four
+// tiles a thread read twice.
 constexpr int kTilesPer = 16;
 __device__ __forceinline__ void finish_counts(uint32_t* hist, int passes, const uint32_t* tile_hist, int num_tiles,
                                               uint2* ranges, uint32_t* order, uint32_t* order_zero,
