@@ -222,6 +222,16 @@ __device__ __forceinline__ void combine_lanes(float (&v)[kSums]) {
     for (int k = 0; k < kSums; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], d);
 }
 
+// Nothing to add: mostly an entry that no pixel of the block took.  Each sum
+// counts: the others may cancel (a Gaussian centred between two pixels under an
+// upstream gradient of opposite signs has a mean gradient and nothing else).
+__device__ __forceinline__ bool all_zero(const float (&v)[kSums]) {
+  bool zero = true;
+#pragma unroll
+  for (int k = 0; k < kSums; ++k) zero = zero && v[k] == 0.f;
+  return zero;
+}
+
 // Reference formulas (backward.cu:552-663) for one pixel; entries (mx, my,
 // conic a, conic b), (conic c, opacity, depth, r), (g, b, _, _).
 // The reference keeps the colour, depth and alpha composited behind the current
@@ -324,9 +334,8 @@ struct RefChain {
     }
     float v[kSums] = {S, Sx, Sy, Sxx, Sxy, Syy, c0, c1, c2, cd};
     combine_lanes<kLanes>(v);
-    // no pixel of the block took the entry (or the lane has none)
     if (lane >= g.count || g.id >= uint32_t(a.P)) return;
-    if (v[0] == 0.f && v[3] == 0.f && v[5] == 0.f && v[6] == 0.f && v[7] == 0.f && v[8] == 0.f && v[9] == 0.f) return;
+    if (all_zero(v)) return;
     const float A = g.q0.z, B = g.q0.w, C = g.q1.x, o = g.q1.y, h = -0.5f * o;
     const size_t id = g.id;
     atomicAdd(a.dL_dcolors + 3 * id, v[6]);
@@ -426,7 +435,7 @@ struct ExactChain {
     float v[kSums] = {S, Se, Sf, See, Sef, Sff, c0, c1, c2, cd};
     combine_lanes<kLanes>(v);
     if (lane >= g.count || g.id >= uint32_t(a.P)) return;
-    if (v[0] == 0.f && v[3] == 0.f && v[5] == 0.f && v[6] == 0.f && v[7] == 0.f && v[8] == 0.f && v[9] == 0.f) return;
+    if (all_zero(v)) return;
     // det >= 0.09 (the forward's +0.3 low-pass on a positive semi-definite
     // covariance), where rcp_markstein is the correctly rounded 1/det
     const float idet = rcp_markstein(g.q1.w), k1 = g.q0.z * idet, k2 = k1 * idet;
