@@ -30,6 +30,8 @@
 // Stability: keys are ranked in input order within a warp, warps in order
 // within a tile, tiles in order globally -- the same order the reference's
 // stable 2-bit passes produce, so equal keys keep their input order.
+#include <atomic>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "tile_walk.cuh"
@@ -569,6 +571,18 @@ void launch_onesweep(int width, int tiles, cudaStream_t stream, const K* kin, co
   }
 }
 
+// The histogram's shared-memory opt-in, once per device and for the most that
+// any launch asks for: the limit is the kernel's, not the launch's, so one set
+// to a launch's own size could be lowered by another thread before that launch.
+template <typename K>
+void hist_opt_in(int dev) {
+  constexpr int kMost = int(sizeof(uint32_t)) * (kMaxPasses * kMaxBins + kSmemTileBins);
+  static std::atomic<bool> opted[64];
+  if (dev >= 0 && dev < 64 && opted[dev].load(std::memory_order_acquire)) return;
+  const cudaError_t e = cudaFuncSetAttribute(hist_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
+  if (e == cudaSuccess && dev >= 0 && dev < 64) opted[dev].store(true, std::memory_order_release);
+}
+
 template <typename K>
 void run_sort(const SortArgs& a, cudaStream_t stream) {
   const int passes = sort_passes(a.bits);
@@ -602,8 +616,7 @@ void run_sort(const SortArgs& a, cudaStream_t stream) {
     const int grid = int(max(1LL, min((n + per_block - 1) / per_block, (long long)sms * (big ? 1 : 4))));
     const size_t smem =
         sizeof(uint32_t) * (size_t(passes) * kMaxBins + (tiles_in_smem ? size_t(a.num_tiles) : 0));
-    if (smem > 40 * 1024)  // beside the scans' own
-      cudaFuncSetAttribute(hist_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (smem > 40 * 1024) hist_opt_in<K>(dev);  // beside the scans' own
     const int st_hist = a.stage_hist >= 0 ? a.stage_hist : kStSortHist;
     stage_begin(st_hist, stream);
     launch_after(hist_kernel<K>, unsigned(grid), unsigned(threads), smem, stream,
