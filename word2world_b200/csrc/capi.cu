@@ -831,6 +831,7 @@ static int backward_impl(const w2w_settings* s, const float* means3D, const floa
   a.clamped = at<uint8_t>(geom_state, GL.clamped);
   a.record = at<float>(geom_state, GL.record);
   a.bwd_record = at<float>(geom_state, GL.bwd_record);
+  a.wild = &at<GeomHeader>(geom_state, GL.header)->wild;
   a.ranges = at<uint2>(image_state, IL.ranges);
   a.point_list = R > 0 ? at<uint32_t>(binning_state, BinLayout(R, num_tiles(W, H)).valsA) : nullptr;
   if (R > 0) {
@@ -1551,6 +1552,7 @@ static void batch_gaussian_args(int n, long long E, int M, const void* geom_stat
   a.clamped = at<uint8_t>(geom_state, GL.clamped);
   a.record = at<float>(geom_state, GL.record);
   a.bwd_record = at<float>(geom_state, GL.bwd_record);
+  a.wild = &at<GeomHeader>(geom_state, GL.header)->wild;
   a.dL_dmean2D = dL_dmeans2D; a.dL_dopacity = dL_dopacity; a.dL_dcolors = dL_dcolors;
   a.acc_cov = static_cast<float*>(scratch);
   a.acc_depth = at<float>(scratch, align256(size_t(E) * 16));

@@ -303,6 +303,10 @@ static_assert(sizeof(BackwardRecord) == 64, "BackwardRecord layout");
 // ---------------------------------------------------------------------------
 __host__ __device__ constexpr size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
+// Small enough that no product or sum of the per-pixel passes overflows with it;
+// false for infinities and NaN.
+__device__ __forceinline__ bool tame(float x) { return fabsf(x) <= 0x1p58f; }
+
 // Device-written header at the start of the geometry state.
 struct GeomHeader {
   uint32_t error;          // kErr* bits
@@ -311,7 +315,8 @@ struct GeomHeader {
   uint32_t num_rendered;   // sum of tiles touched (the reference's R)
   uint32_t scan_tiles_done;
   uint32_t scan_tile_counter;
-  uint32_t pad[10];
+  uint32_t wild;           // nonzero: a Gaussian that emits keys has a position, covariance, depth or colour that is not tame
+  uint32_t pad[9];
 };
 
 constexpr int kPreThreads = 256;  // Gaussians per preprocess block (one scan tile)

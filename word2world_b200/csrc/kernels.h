@@ -214,6 +214,7 @@ struct BackwardArgs {
   const uint8_t* clamped;
   const float* record;
   const float* bwd_record;
+  const uint32_t* wild;  // GeomHeader::wild
   const uint2* ranges;
   const uint32_t* point_list;
   const uint32_t* n_contrib;

@@ -326,6 +326,7 @@ preprocess_kernel(PreprocessArgs a) {
     for (int k = 0; k < 6; ++k) cov3[k] = g.cov3[k];
   }
   float skip = -__int_as_float(0x7f800000), rec_depth = 0.f;
+  bool tame_geometry = true;
   CullParams cp{-1.0f, 0.f, 0.f, 0.f, 0.f};
   if (i < P) {
     int radius = 0;
@@ -399,6 +400,7 @@ preprocess_kernel(PreprocessArgs a) {
     bp[0] = g.visible ? make_float4(g.mx, g.my, g.conic[0], g.conic[1]) : make_float4(0.f, 0.f, 0.f, 0.f);
     bp[3] = g.visible ? make_float4(cp.beta, cp.gamma, cp.eps, cp.vr) : make_float4(0.f, 0.f, 0.f, 0.f);
     rec_depth = rec.depth;
+    tame_geometry = tame(rec.mx) && tame(rec.my) && tame(rec.cxx) && tame(rec.cxy) && tame(rec.cyy) && tame(rec.depth);
   }
 
   // depth-bit range of Gaussians that emit keys (sizes the sort)
@@ -488,6 +490,7 @@ preprocess_kernel(PreprocessArgs a) {
     a.clamped[3 * i] = clampf[0];
     a.clamped[3 * i + 1] = clampf[1];
     a.clamped[3 * i + 2] = clampf[2];
+    if (emit > 0 && !(tame_geometry && tame(rgb[0]) && tame(rgb[1]) && tame(rgb[2]))) atomicOr(&hdr->wild, 1u);
     const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
     reinterpret_cast<float4*>(a.record)[4 * size_t(i) + 3] =
         g.visible ? make_float4(rec_depth, rgb[0], rgb[1], rgb[2]) : none;
