@@ -21,6 +21,7 @@
 #include "kernels.h"
 #include "tile_walk.cuh"
 
+#include <cfloat>
 #include <type_traits>
 
 namespace w2w {
@@ -390,9 +391,9 @@ struct ExactChain {
   static __device__ __forceinline__ void evaluate(BwdWarp& s, const GroupLoad& g, float bx, float by) {
     const int e = int(threadIdx.x & 31u) % (32 / kLanes);
     gauss_values<kLanes>(g.q0.x, g.q0.y, g.q1, bx, by, [&](int p, float v) {
-      const float og = mul(g.q0.z, v);
-      const bool ok = og >= 1.0f / 255.0f && g.pos < s.last[p];
-      s.alpha[p * kTableStride + e] = ok ? fminf(0.99f, og) : 0.f;
+      const float og = mul(g.q0.z, v), al = fminf(0.99f, og);  // 0.99 for NaN (an infinite opacity times 0)
+      const bool ok = al >= 1.0f / 255.0f && g.pos < s.last[p];
+      s.alpha[p * kTableStride + e] = ok ? al : 0.f;
       s.value[p * kTableStride + e] = ok && og < 0.99f ? v : 0.f;
     });
   }
@@ -455,7 +456,8 @@ struct ExactChain {
     if (all_zero(v)) return;
     // det >= 0.09 (the forward's +0.3 low-pass on a positive semi-definite
     // covariance), where rcp_markstein is the correctly rounded 1/det
-    const float idet = rcp_markstein(g.q1.w), k1 = g.q0.z * idet, k2 = k1 * idet;
+    // An infinite opacity is clamped at every pixel: the geometric sums are 0.
+    const float idet = rcp_markstein(g.q1.w), k1 = (fabsf(g.q0.z) <= FLT_MAX ? g.q0.z : 0.f) * idet, k2 = k1 * idet;
     const size_t id = g.id;
     atomicAdd(a.dL_dcolors + 3 * id, v[6]);
     atomicAdd(a.dL_dcolors + 3 * id + 1, v[7]);
