@@ -21,6 +21,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 namespace w2w {
 namespace {
@@ -36,7 +37,10 @@ struct BlendPixel {
   // or the pixel has terminated), depths and colours dc[k]; `at` becomes e + k of
   // the last one blended.  Only the transmittance runs through them: it never
   // grows, so the entry that would take it below 1e-4 and all after it are the
-  // ones whose product lies below, and their weight is 0.
+  // ones whose product lies below, and their weight is 0.  Weight 0 keeps an entry
+  // out by multiplication while its depth and colour are finite; kSelect: by
+  // selection.
+  template <bool kSelect>
   __device__ __forceinline__ void step(const float (&v)[8], const float4* dc, int e, int& at) {
     float t = T;
 #pragma unroll
@@ -44,7 +48,7 @@ struct BlendPixel {
       const float nT = mul(t, sub(1.0f, v[k]));
       const bool alive = nT >= 0.0001f;
       const float aT = alive ? mul(v[k], t) : 0.0f;
-      const float4 q = dc[k];
+      const float4 q = kSelect && aT == 0.0f ? make_float4(0.f, 0.f, 0.f, 0.f) : dc[k];
       C0 = fma(q.y, aT, C0);
       C1 = fma(q.z, aT, C1);
       C2 = fma(q.w, aT, C2);
@@ -60,14 +64,17 @@ struct BlendPixel {
   // Entry with alpha `al` and depth and colour `dc`, 1-based list position `pos`.
   // Branch-free: the updates are selected, so a warp's lanes never diverge.
   // An entry that does not accumulate adds exactly zero: its weight aT is
-  // selected to 0, colours and depth are finite, and C, Wt and D are never
-  // -0 (non-negative colours and weights, positive depths), so x + c * 0 = x.
+  // selected to 0, colours and depth are finite (or, kSelect, selected to 0 too),
+  // and C, Wt and D are never -0 (non-negative colours and weights, positive
+  // depths), so x + c * 0 = x.
+  template <bool kSelect>
   __device__ __forceinline__ void step(float al, float4 dc, uint32_t pos) {
     const bool blend = !done && al >= 1.0f / 255.0f;
     const float nT = mul(T, sub(1.0f, al));
     const bool term = blend && nT < 0.0001f;
     const bool acc = blend && !term;
     const float aT = acc ? mul(al, T) : 0.0f;
+    if (kSelect && !acc) dc = make_float4(0.f, 0.f, 0.f, 0.f);
     C0 = fma(dc.y, aT, C0);
     C1 = fma(dc.z, aT, C1);
     C2 = fma(dc.w, aT, C2);
@@ -254,29 +261,33 @@ __global__ void __launch_bounds__(32 * kBlendWarps, kBlendResident / kBlendWarps
     count = int(min(tail - head, 32u));
     load_group(count);
   }
-  while (count > 0 && !done) {
-    if (count > 16) group_alphas<1>(s, en, float(tp.bx), float(tp.by));
-    else if (count > 8) group_alphas<2>(s, en, float(tp.bx), float(tp.by));
-    else group_alphas<4>(s, en, float(tp.bx), float(tp.by));
-    s.dc[lane] = en.dc;
-    const uint32_t first = head;
-    head += uint32_t(count);
-    refill();  // synchronises the warp
-    const int next = int(min(tail - head, 32u));
-    load_group(next);
-    const float* mine = s.alpha + (pix.done ? 32 : lane) * kAlphaStride;  // a terminated pixel: zeros
-    int at = -1;  // this pixel's last blended entry of the group
-    for (int e = 0; e < count; e += 8) {
-      const float4 a0 = *reinterpret_cast<const float4*>(mine + e), a1 = *reinterpret_cast<const float4*>(mine + e + 4);
-      const float v[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-      pix.step(v, s.dc + e, e, at);
-      if (pix.done) mine = s.alpha + 32 * kAlphaStride;
+  auto run = [&](auto select) {
+    while (count > 0 && !done) {
+      if (count > 16) group_alphas<1>(s, en, float(tp.bx), float(tp.by));
+      else if (count > 8) group_alphas<2>(s, en, float(tp.bx), float(tp.by));
+      else group_alphas<4>(s, en, float(tp.bx), float(tp.by));
+      s.dc[lane] = en.dc;
+      const uint32_t first = head;
+      head += uint32_t(count);
+      refill();  // synchronises the warp
+      const int next = int(min(tail - head, 32u));
+      load_group(next);
+      const float* mine = s.alpha + (pix.done ? 32 : lane) * kAlphaStride;  // a terminated pixel: zeros
+      int at = -1;  // this pixel's last blended entry of the group
+      for (int e = 0; e < count; e += 8) {
+        const float4 a0 = *reinterpret_cast<const float4*>(mine + e), a1 = *reinterpret_cast<const float4*>(mine + e + 4);
+        const float v[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+        pix.template step<decltype(select)::value>(v, s.dc + e, e, at);
+        if (pix.done) mine = s.alpha + 32 * kAlphaStride;
+      }
+      if (at >= 0) pix.last = s.ring[(first + uint32_t(at)) & (kRing - 1)].y;
+      done = __all_sync(0xffffffffu, pix.done) != 0;
+      __syncwarp();
+      count = next;
     }
-    if (at >= 0) pix.last = s.ring[(first + uint32_t(at)) & (kRing - 1)].y;
-    done = __all_sync(0xffffffffu, pix.done) != 0;
-    __syncwarp();
-    count = next;
-  }
+  };
+  if (a.wild == nullptr || *a.wild == 0u) run(std::false_type{});
+  else run(std::true_type{});
   // the mask words not yet written (the backward reads none past the last contributor)
   if (row != nullptr && (c & 31) != 0 && c < chunks && lane < (c & 31)) row[(c & ~31) + lane] = word;
   if (inside) {
@@ -422,6 +433,7 @@ __global__ void __launch_bounds__(32 * (kW + 1)) blend_queue_kernel(BlendArgs a,
   QueueShared<kW>& s = *reinterpret_cast<QueueShared<kW>*>((reinterpret_cast<uintptr_t>(q_raw) + 127) & ~uintptr_t(127));
   const int warp = int(threadIdx.x >> 5), lane = int(threadIdx.x & 31);
   const uint32_t limit = a.spin_limit;
+  const uint32_t wild = a.wild != nullptr ? *a.wild : 0u;
   volatile uint32_t* abort = &s.abort;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kQStages; ++i) {
@@ -591,7 +603,9 @@ __global__ void __launch_bounds__(32 * (kW + 1)) blend_queue_kernel(BlendArgs a,
 #pragma unroll
         for (int kk = 0; kk < kBlendIlp; ++kk) {
           const int jj = j[kk] < 0 ? j[0] : j[kk];
-          pix.step(j[kk] < 0 ? 0.0f : al[kk], sr[kQRec * jj + 3], base + uint32_t(j[kk]));
+          const float v = j[kk] < 0 ? 0.0f : al[kk];
+          if (wild == 0u) pix.step<false>(v, sr[kQRec * jj + 3], base + uint32_t(j[kk]));
+          else pix.step<true>(v, sr[kQRec * jj + 3], base + uint32_t(j[kk]));
         }
         if (__all_sync(0xffffffffu, pix.done)) break;
       }

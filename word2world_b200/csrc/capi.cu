@@ -574,6 +574,7 @@ int w2w_forward_render(const w2w_settings* s, const void* geom_state, const w2w_
   b.ranges = ranges;
   b.point_list = point_list;
   b.record = R > 0 ? at<float>(geom_state, GeomLayout(s->P).record) : nullptr;
+  b.wild = R > 0 ? &at<GeomHeader>(geom_state, GeomLayout(s->P).header)->wild : nullptr;
   b.num_records = uint32_t(s->P);
   if (R > 0) {
     const BinLayout BL(R, T);
@@ -728,6 +729,7 @@ int w2w_forward_render_planned(const w2w_settings* s, const void* geom_state, lo
   b.ranges = at<uint2>(image_state, IL.ranges);
   b.point_list = at<uint32_t>(binning_state, BL.valsA);
   b.record = at<float>(geom_state, GL.record);
+  b.wild = &at<GeomHeader>(geom_state, GL.header)->wild;
   b.num_records = uint32_t(s->P);
   b.masks = at<uint32_t>(binning_state, BL.masks);
   b.masks_valid = &bh->masks_valid;
@@ -1274,6 +1276,7 @@ int w2w_blend(const w2w_settings* s, const void* geom_state, const uint32_t* ran
   b.ranges = own;
   b.point_list = point_list;
   b.record = at<float>(geom_state, GeomLayout(s->P).record);
+  b.wild = &at<GeomHeader>(geom_state, GeomLayout(s->P).header)->wild;
   b.num_records = uint32_t(s->P);
   b.bg = s->background;
   b.out_color = out_color; b.out_depth = out_depth; b.out_alpha = out_alpha;
@@ -1515,6 +1518,7 @@ int w2w_batch_forward_render(const w2w_batch_item* items, int n, const void* geo
   b.ranges = ranges;
   b.point_list = point_list;
   b.record = R > 0 ? at<float>(geom_state, GeomLayout(E).record) : nullptr;
+  b.wild = R > 0 ? &at<GeomHeader>(geom_state, GeomLayout(E).header)->wild : nullptr;
   b.num_records = uint32_t(E);
   if (R > 0) {
     const BinLayout BL(R, T);

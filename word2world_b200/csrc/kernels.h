@@ -175,6 +175,7 @@ struct BlendArgs {
   const uint32_t* point_list;
   const float* record;
   uint32_t num_records;  // records (Gaussians, or batch elements); larger ids in the list are skipped
+  const uint32_t* wild;  // GeomHeader::wild; null: no entries
   uint32_t* masks;       // block masks for the backward passes (tile_walk.cuh mask_row), or null
   const float* bg;
   float* out_color;
