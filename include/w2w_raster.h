@@ -501,8 +501,9 @@ int w2w_tune_set(int knob, int value);
  * w2w_test_set_spin_limit: the iteration limit of every bounded device wait
  * (0 restores the default, 2^22 polls: a second or two); returns the previous
  * limit.  w2w_test_unpublished_tile: the CTA of tile `tile` of a stage (0: the
- * stand-alone scans, 1: the first pass of every sort, 2: the scan fused into
- * w2w_forward_geometry) skips publishing its status, so that the waits behind
+ * stand-alone scans, 1: the first pass of every sort but 3's, 2: the scan fused into
+ * w2w_forward_geometry, 3: the first pass of a depth-ordered emission's own sort of
+ * the Gaussians, 4: that emission's scan) skips publishing its status, so that the waits behind
  * it run out and the call reports W2W_ERR_TIMEOUT; -1 turns it off.  Returns
  * the previous tile (-2 for an unknown stage).  Nothing faults or hangs: every
  * wait ends at its limit.  Process-wide settings read at launch. */

@@ -195,11 +195,13 @@ void launch_list(DuplicateArgs d, const KeyPlan& kp, long long n, int T, void* b
     so.error = &bh->error;
     so.tile_shift = 0; so.num_tiles = 0; so.tile_hist = nullptr; so.ranges = nullptr;
     so.spin_limit = spin_limit();
+    so.unpublished_tile = unpublished_tile(kWaitEmitSort);
     so.stage_hist = so.stage_pass = kStDepthSort;
     cudaMemsetAsync(&bh->error, 0, 4, st);
     launch_sort(so, st);
     d.order = so.vals_out;
     d.spin_limit = spin_limit();
+    d.unpublished_tile = unpublished_tile(kWaitEmit);
   }
   d.R = uint32_t(n); d.key64 = kp.key64; d.depth_bits = uint32_t(kp.depth_bits);
   d.keys = odd ? keysB : keysA;

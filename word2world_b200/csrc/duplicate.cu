@@ -153,10 +153,11 @@ __global__ void __launch_bounds__(kDupThreads) duplicate_kernel(DuplicateArgs a)
       all += s_warp[w2];
     }
     if (warp == 0) {
-      if (lane == 0 && block > 0) st_relaxed(a.scan_status + block, kScanAgg | all);
+      const bool publish = block != a.unpublished_tile;
+      if (lane == 0 && block > 0 && publish) st_relaxed(a.scan_status + block, kScanAgg | all);
       const uint32_t b = lookback_sum(a.scan_status, block, a.spin_limit, &a.header->error);
       if (lane == 0) {
-        st_relaxed(a.scan_status + block, kScanInc | ((b + all) & kScanMask));
+        if (publish) st_relaxed(a.scan_status + block, kScanInc | ((b + all) & kScanMask));
         s_before = b;
       }
     }

@@ -115,6 +115,7 @@ struct DuplicateArgs {
   uint32_t* scan_status;
   uint32_t* scan_counter;
   uint32_t spin_limit = kSpinLimit;
+  long long unpublished_tile = -1;  // block that skips publishing (tests; -1 = none)
 };
 constexpr int kDupThreads = 256;
 void launch_duplicate(const DuplicateArgs& a, cudaStream_t stream);
@@ -354,7 +355,11 @@ size_t scan_status_words(long long n);
 // tile of that stage whose CTA skips publishing its status, so that the waits
 // behind it run out and report kErrTimeout (tests only; -1 = none).  Both are
 // host-side settings read when a kernel is launched.
-enum WaitStage { kWaitScan = 0, kWaitSort = 1, kWaitPreprocess = 2, kNumWaitStages = 3 };
+enum WaitStage {
+  kWaitScan = 0, kWaitSort = 1, kWaitPreprocess = 2,
+  kWaitEmitSort = 3, kWaitEmit = 4,  // the emission in depth order: the sort of its Gaussians, its scan
+  kNumWaitStages = 5
+};
 uint32_t spin_limit();
 long long unpublished_tile(int stage);
 

@@ -65,7 +65,7 @@ void stage_end(int stage, cudaStream_t s, int kernels) {
 }
 
 std::atomic<uint32_t> g_spin_limit{kSpinLimit};
-std::atomic<long long> g_unpublished[kNumWaitStages] = {{-1}, {-1}, {-1}};
+std::atomic<long long> g_unpublished[kNumWaitStages] = {{-1}, {-1}, {-1}, {-1}, {-1}};
 
 uint32_t spin_limit() { return g_spin_limit.load(std::memory_order_relaxed); }
 
