@@ -1097,8 +1097,9 @@ static int voxel_field_counted(const VoxelArgs& args, cudaStream_t st) {
   if (pairs >= (1LL << 30)) { release(); return W2W_ERR_CAPACITY; }
   if (pairs == 0) {
     cudaMemsetAsync(a.occ, 0, size_t(a.R) * a.R * a.R * 4, st);
+    const int rc = read_error_word(at<uint32_t>(scan_scratch, 4), st);
     release();
-    return check_launch();
+    return rc != W2W_OK ? rc : check_launch();
   }
   a.keys = static_cast<uint32_t*>(alloc(size_t(pairs) * 4));
   a.vals = static_cast<uint32_t*>(alloc(size_t(pairs) * 4));
@@ -1113,14 +1114,17 @@ static int voxel_field_counted(const VoxelArgs& args, cudaStream_t st) {
     release();
     return W2W_ERR_CUDA;
   }
-  launch_voxel_emit(a, st);
   cudaMemsetAsync(at<uint32_t>(sort_scratch, er), 0, 4, st);
+  a.error = at<uint32_t>(sort_scratch, er);
+  a.scan_error = at<uint32_t>(scan_scratch, 4);
+  a.pairs = uint32_t(pairs);
+  launch_voxel_emit(a, st);
   SortArgs so{};
   so.n = pairs; so.key64 = 0; so.begin_bit = 0; so.bits = ceil_log2(uint32_t(nblocks));
   so.keys_in = a.keys; so.vals_in = a.vals; so.keys_out = keys_out; so.vals_out = vals_out;
   so.keys_tmp = at<void>(sort_scratch, kt); so.vals_tmp = at<uint32_t>(sort_scratch, vt);
   so.hist = at<uint32_t>(sort_scratch, hi); so.status = at<uint32_t>(sort_scratch, stt);
-  so.counters = at<uint32_t>(sort_scratch, ct); so.error = at<uint32_t>(sort_scratch, er);
+  so.counters = at<uint32_t>(sort_scratch, ct); so.error = a.error;
   so.tile_shift = 0; so.num_tiles = nblocks; so.tile_hist = tile_hist; so.ranges = ranges;
   so.spin_limit = spin_limit();
   so.unpublished_tile = unpublished_tile(kWaitSort);

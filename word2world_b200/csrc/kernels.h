@@ -334,7 +334,9 @@ struct VoxelArgs {
   uint32_t* vals;     // [pairs] Gaussian ids
   float* occ;         // [R^3], x fastest
   int slots = 0;      // > 0: this many pairs per Gaussian, unused ones with key (B + 1)^3
-  uint32_t* error = nullptr;  // slots > 0: set where a Gaussian has more
+  uint32_t* error = nullptr;  // the sort's error word; slots > 0: set where a Gaussian has more
+  uint32_t pairs = 0;         // counted: room in keys and vals
+  const uint32_t* scan_error = nullptr;  // counted: the scan's error word, passed on to `error`
 };
 void launch_voxel_prepare(const VoxelArgs& a, cudaStream_t stream);
 void launch_voxel_emit(const VoxelArgs& a, cudaStream_t stream);

@@ -108,9 +108,11 @@ __global__ void __launch_bounds__(kVoxThreads) voxel_prepare_kernel(VoxelArgs a)
 
 
 // Per Gaussian: its (block, Gaussian) pairs at its scanned offset, blocks in
-// x-fastest order.
+// x-fastest order.  Offsets that a scan left inconsistent when its bounded wait
+// ran out may lie past the pairs' room: nothing is written there.
 __global__ void __launch_bounds__(kVoxThreads) voxel_emit_kernel(VoxelArgs a) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  if (g == 0 && *a.scan_error != 0u) atomicOr(a.error, *a.scan_error);
   if (g >= a.P || a.count[g] == 0) return;
   int xl, xh, yl, yh, zl, zh;
   vox_span(a.means[3 * g], a, xl, xh);
@@ -121,8 +123,10 @@ __global__ void __launch_bounds__(kVoxThreads) voxel_emit_kernel(VoxelArgs a) {
   for (int z = zl; z <= zh; ++z)
     for (int y = yl; y <= yh; ++y)
       for (int x = xl; x <= xh; ++x) {
-        a.keys[o] = uint32_t(x + nb * (y + nb * z));
-        a.vals[o] = uint32_t(g);
+        if (o < a.pairs) {
+          a.keys[o] = uint32_t(x + nb * (y + nb * z));
+          a.vals[o] = uint32_t(g);
+        }
         ++o;
       }
 }
@@ -135,6 +139,13 @@ __device__ __forceinline__ float vox_value(const float4& q0, const float4& q1, c
                 dy * dz * q2.x;
   if (power > 0) power = -1e10f;
   return q0.w * expf(power);
+}
+
+// A list entry's record.  An id past the last Gaussian (a list left inconsistent
+// by a sort whose bounded wait ran out, which its error word reports) reads the
+// last one's.
+__device__ __forceinline__ const float4* vox_record(const VoxelArgs& a, const uint32_t* list, uint32_t e) {
+  return a.rec + 3 * size_t(min(__ldg(list + e), uint32_t(a.P - 1)));
 }
 
 // Two voxels per thread, neighbours in z, x fastest within a CTA of 8 x 8 x 8
@@ -163,19 +174,19 @@ __global__ void __launch_bounds__(kVoxThreads) voxel_field_kernel(VoxelArgs a, c
   if (two && b0 == b1) {
 #pragma unroll 4
     for (uint32_t e = r.x; e < r.y; ++e) {
-      const float4* rec = a.rec + 3 * size_t(__ldg(list + e));
+      const float4* rec = vox_record(a, list, e);
       const float4 q0 = __ldg(rec), q1 = __ldg(rec + 1), q2 = __ldg(rec + 2);
       v0 += vox_value(q0, q1, q2, x, y, z0);
       v1 += vox_value(q0, q1, q2, x, y, z1);
     }
   } else {  // the pair straddles two blocks, or the grid's edge
     for (uint32_t e = r.x; e < r.y; ++e) {
-      const float4* rec = a.rec + 3 * size_t(__ldg(list + e));
+      const float4* rec = vox_record(a, list, e);
       v0 += vox_value(__ldg(rec), __ldg(rec + 1), __ldg(rec + 2), x, y, z0);
     }
     const uint2 r1 = two ? ranges[bx + nb * (by + nb * b1)] : make_uint2(0u, 0u);
     for (uint32_t e = r1.x; e < r1.y; ++e) {
-      const float4* rec = a.rec + 3 * size_t(__ldg(list + e));
+      const float4* rec = vox_record(a, list, e);
       v1 += vox_value(__ldg(rec), __ldg(rec + 1), __ldg(rec + 2), x, y, z1);
     }
   }
