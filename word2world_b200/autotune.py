@@ -37,6 +37,10 @@ CANDIDATES = {
     "preprocess_blocks": [4, 3, 2],
     "blend_stage": [1, 0],
 }
+# Knobs that are accepted but select nothing: their trials would time one build
+# against itself, and a lucky one would lower the mark that real gains have to
+# beat.  Timed only by a caller's own candidates or timer.
+INERT = frozenset({"backward_split", "backward_ways", "blend_stage"})
 
 
 def bucket_key(width: int, height: int, P: int, grad_mode: str = "reference", device=None) -> str:
@@ -64,6 +68,7 @@ class Autotuner:
         self.reps, self.warmup, self.min_gain = int(reps), int(warmup), float(min_gain)
         self.cache: dict = {}
         self.log: list = []
+        self._own_timer = timer is None
         self._timer = timer or self._cuda_time
         if path and os.path.exists(path):
             with open(path) as f:
@@ -96,6 +101,8 @@ class Autotuner:
         knobs (with the timings in ``self.log``)."""
         cands = candidates or CANDIDATES
         best = {k: v for k, v in current().items() if k in cands}
+        if candidates is None and self._own_timer:
+            cands = {k: v for k, v in cands.items() if k not in INERT}
         apply(best)
         best_ms = self._timer(step)
         self.log.append((dict(best), best_ms))
