@@ -382,7 +382,7 @@ preprocess_kernel(PreprocessArgs a) {
       reinterpret_cast<float2*>(a.means2D)[i] = make_float2(0.f, 0.f);
       a.depth[i] = 0.f;
     }
-    if (radius <= 0) { alloc = 0; emit = 0; }
+    if (radius <= 0) { alloc = 0; emit = 0; rect_lo = 0; rect_hi = 0; }  // the emission reads the rectangle alone
     if (emit > 0) depth_bits = __float_as_uint(g.depth);
     a.radii[i] = radius;
     a.tiles[i] = alloc;
