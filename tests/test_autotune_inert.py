@@ -11,13 +11,14 @@ except ImportError:
     pytest.skip("extension not built", allow_module_level=True)
 
 
-def test_inert_knobs_are_not_timed(monkeypatch, tmp_path):
+@pytest.mark.parametrize("queue", [0, 1])  # the faster blend: per tile, or the queue-fed one that blend_warps shapes
+def test_inert_knobs_are_not_timed(monkeypatch, tmp_path, queue):
     before, seen = autotune.current(), []
-    times = iter([1.0] + [0.5, 1.0] * 50)  # every other trial looks like a gain
 
-    def timed(self, step):
-        seen.append(autotune.current())
-        return next(times)
+    def timed(self, step):  # every trial with the faster blend looks like a gain
+        k = autotune.current()
+        seen.append(k)
+        return 1.0 - 0.02 * len(seen) + (0.0 if k["blend_queue"] == queue else 10.0)
 
     monkeypatch.setattr(autotune.Autotuner, "_cuda_time", timed)
     path = str(tmp_path / "tune.json")
@@ -28,4 +29,5 @@ def test_inert_knobs_are_not_timed(monkeypatch, tmp_path):
     assert all(k[i] == before[i] for k in seen for i in autotune.INERT)
     assert set(best) == set(before) and all(best[i] == before[i] for i in autotune.INERT)
     assert all(json.load(open(path))["bucket"][i] == before[i] for i in autotune.INERT)
-    assert any(best[k] != before[k] for k in best)
+    assert best["blend_queue"] == queue
+    assert any(k["blend_warps"] != before["blend_warps"] for k in seen) == (queue == 1)

@@ -39,7 +39,8 @@ CANDIDATES = {
 }
 # Knobs that are accepted but select nothing: their trials would time one build
 # against itself, and a lucky one would lower the mark that real gains have to
-# beat.  Timed only by a caller's own candidates or timer.
+# beat.  Timed only by a caller's own candidates or timer; so is blend_warps while
+# the blend is not the queue-fed one, which alone it shapes.
 INERT = frozenset({"backward_split", "backward_ways", "blend_stage"})
 
 
@@ -101,14 +102,15 @@ class Autotuner:
         knobs (with the timings in ``self.log``)."""
         cands = candidates or CANDIDATES
         best = {k: v for k, v in current().items() if k in cands}
-        if candidates is None and self._own_timer:
-            cands = {k: v for k, v in cands.items() if k not in INERT}
+        skip_inert = candidates is None and self._own_timer
         apply(best)
         best_ms = self._timer(step)
         self.log.append((dict(best), best_ms))
         for _ in range(rounds):
             changed = False
             for knob, values in cands.items():
+                if skip_inert and (knob in INERT or (knob == "blend_warps" and best["blend_queue"] == 0)):
+                    continue
                 for v in values:
                     if v == best[knob]:
                         continue
