@@ -1,11 +1,11 @@
 // Backward pass.
 //
-// Per-pixel pass (reference backward.cu:521-665): one CTA per tile, pixels
-// walk the tile's list back to front, recomputing each pair's alpha from the
-// stored state (final transmittance and last-contributor index) instead of
-// storing per-pair values.  Each entry's per-pixel contributions are summed
-// across the warp with shuffles and added with one atomic per warp (the
-// reference issues ten atomics per pixel-Gaussian pair).  A tile starts at its
+// Per-pixel pass (reference backward.cu:521-665): one warp, and one CTA, per 8x4
+// pixel block, its pixels walking the tile's list back to front, recomputing each
+// pair's alpha from the stored state (final transmittance and last-contributor
+// index) instead of storing per-pair values.  Each entry's sums over the block's
+// pixels are formed by its own lane and added with one atomic each (the reference
+// issues ten atomics per pixel-Gaussian pair).  A block starts at its pixels'
 // largest contributor count: entries past it are skipped by every pixel.
 //
 // Per-Gaussian pass: the reference's computeCov2DCUDA (backward.cu:27-227) and
@@ -59,12 +59,6 @@ namespace {
 // heaviest tiles' walks into segments, each replaying the chain behind it, no
 // longer pays: a replay costs steps 1 and 2, three quarters of the work (470
 // us per 4 views at 500k without, 678 with half an SM count of tiles cut).
-// ---------------------------------------------------------------------------
-constexpr int kGroup = 32;        // entries per group
-constexpr int kSteps = 8;         // of them in flight through a pixel's chain
-constexpr int kWindow = 512;      // list positions whose mask bits are expanded together, 16 per lane
-constexpr int kTableStride = 36;  // floats per pixel row: rows start on 16 bytes, 8 rows cover the banks
-
 //
 // A skipped pair's zeros keep it out of the chain and the sums by
 // multiplication, as long as all that they meet is finite.  kSelect: they are
@@ -73,6 +67,11 @@ constexpr int kTableStride = 36;  // floats per pixel row: rows start on 16 byte
 // have such an upstream gradient.  A whole walk is compiled either way: a test
 // per group of entries instead, its loops the same, cost 1 to 3 % of a step (1M
 // Gaussians 1364 -> 1385 us, a batch of six scenes 1012 -> 1040).
+// ---------------------------------------------------------------------------
+constexpr int kGroup = 32;        // entries per group
+constexpr int kSteps = 8;         // of them in flight through a pixel's chain
+constexpr int kWindow = 512;      // list positions whose mask bits are expanded together, 16 per lane
+constexpr int kTableStride = 36;  // floats per pixel row: rows start on 16 bytes, 8 rows cover the banks
 
 // A warp's shared memory.
 struct __align__(16) BwdWarp {
@@ -454,8 +453,9 @@ struct ExactChain {
     combine_lanes<kLanes>(v);
     if (lane >= g.count || g.id >= uint32_t(a.P)) return;
     if (all_zero(v)) return;
-    // det >= 0.09 (the forward's +0.3 low-pass on a positive semi-definite
-    // covariance), where rcp_markstein is the correctly rounded 1/det
+    // |det| >= 1e-8 (the projection drops a smaller one): rcp_markstein's rounding
+    // depends on the significand alone while det, its approximate reciprocal and
+    // the remainder are normal numbers, so this is the correctly rounded 1/det.
     // An infinite opacity is clamped at every pixel: the geometric sums are 0.
     const float idet = rcp_markstein(g.q1.w), k1 = (fabsf(g.q0.z) <= FLT_MAX ? g.q0.z : 0.f) * idet, k2 = k1 * idet;
     const size_t id = g.id;

@@ -302,8 +302,9 @@ __global__ void __launch_bounds__(32 * kBlendWarps, kBlendResident / kBlendWarps
     a.out_color[hw + cp] = fma(pix.T, bg[1], pix.C1);
     a.out_color[2 * hw + cp] = fma(pix.T, bg[2], pix.C2);
   }
-  // largest contributor count in the tile (the backward starts there); the
-  // tile's warps combine theirs (tile_max is cleared before the launch)
+  // largest contributor count in the tile, for inspection of the image state (the
+  // backward's blocks start at their own pixels' counts); the tile's warps combine
+  // theirs (tile_max is cleared before the launch)
   const uint32_t wm = __reduce_max_sync(0xffffffffu, pix.last);
   if (lane == 0 && wm != 0u) atomicMax(&a.tile_max[tile], wm);
 }

@@ -51,7 +51,8 @@ __device__ __forceinline__ float rcp_approx(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-// RN(1/b) for |b| in [2^-20, 2^60].
+// RN(1/b) for |b| in [2^-60, 2^60]: the approximation, the remainder (2^-48 at
+// least) and the result are normal numbers, so b's exponent changes no rounding.
 __device__ __forceinline__ float rcp_markstein(float b) {
   const float y0 = rcp_approx(b);
   return fma(fma(-b, y0, 1.0f), y0, y0);
@@ -284,9 +285,10 @@ struct __align__(16) BlendRecord {
 };
 static_assert(sizeof(BlendRecord) == 64, "BlendRecord layout");
 
-// Per-Gaussian record read by the reference-formula backward pass, 64 bytes.
-// skip: -ln(255 o) - 1e-4; a pair whose exponent is below it has
-// alpha < 1/255 for certain, so its exp is not evaluated.
+// Per-Gaussian record of the reference-formula backward pass, 64 bytes, of which
+// it reads the first ten floats.  Nothing reads the rest any more: skip is
+// -ln(255 o) - 1e-4 (an exponent below it has alpha < 1/255 for certain), and a
+// list without block masks is tested with the blend's record.
 struct __align__(16) BackwardRecord {
   float mx, my;
   float conic_a, conic_b, conic_c;  // inverse 2-D covariance

@@ -151,7 +151,7 @@ struct SortArgs {
   uint32_t* tile_hist;
   uint2* ranges;
   // with ranges (else ignored): the tiles by decreasing list length, and the
-  // words to clear on the way (tile_order_block)
+  // words to clear on the way (finish_counts)
   uint32_t* order = nullptr;
   uint32_t* order_zero = nullptr;
   uint32_t* order_counter = nullptr;
@@ -184,7 +184,7 @@ struct BlendArgs {
   float* out_alpha;
   uint32_t* n_contrib;
   float* T_final;
-  uint32_t* tile_max;
+  uint32_t* tile_max;   // per tile the largest contributor count (inspection only)
   uint32_t* order;      // tiles by decreasing list length (the processing order, the backward's too)
   bool ordered = false;  // the sort has written order and cleared tile_max and queue
   uint32_t* queue;      // the persistent blend's queue counter (cleared before its launch), or null

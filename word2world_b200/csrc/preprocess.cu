@@ -240,8 +240,11 @@ __device__ __forceinline__ void sh_colour(const float* dc, const float* sh, int 
 // (copies) -> 78 us (order of the scan), at 1M 161 -> 133 us, at 16k 12.2 -> 8.4
 // us.  Coalesced stores of the short rows, 32-byte record stores and a lookback
 // of 128 tiles a step made no difference; blocks of 128 or 64 threads were slower
-// (93, 100 us).  3 CTAs per SM at 80 registers: 88 us, 2 at 128: 96 us (4 spill
-// 80 bytes).
+// (93, 100 us).  4 CTAs per SM (64 registers, 100 bytes spilled) suit
+// one stream, where 3 (80 registers) take the same time and 2 (128) more: a 500k
+// render 386, 389 and 396 us, a 16k step 777, 773 and 770.  With every view on its
+// own stream 3 let other views' blocks in: 1.97 ms a 4-view step of 500k against
+// 2.00 to 2.02; that caller's tuning run picks them.
 // kRaw: the raw parameters of Renderer.render, activated here (PreprocessArgs).
 // kStage: degree-3 rows are staged through shared memory (dynamic, kStageBytes)
 // instead of each thread gathering its own 192-byte row; activated parameters'
@@ -387,7 +390,7 @@ preprocess_kernel(PreprocessArgs a) {
     a.radii[i] = radius;
     a.tiles[i] = alloc;
     reinterpret_cast<uint2*>(a.rect)[i] = make_uint2(rect_lo, rect_hi);
-    // backward skip threshold (BackwardRecord::skip) and block-culling parameters
+    // BackwardRecord::skip, and the block-culling parameters
     if (g.visible) {
       skip = opacity > 0.0f ? -logf(255.0f * opacity) - 1e-4f : __int_as_float(0x7f800000);
       cp = make_cull_params(g.conic[0], g.conic[1], g.conic[2], opacity);
